@@ -3,6 +3,7 @@
 // device allocation of the handle-owned arrays, and dispatch to the kernels.
 #include "../../include/dndsb.h"
 #include "solver.cuh"
+#include "wall_flux.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -544,7 +545,7 @@ extern "C"
         rc |= dev_alloc((void **)&e->e.redBuf, sizeof(real) * kRedBufLen);
         rc |= dev_alloc((void **)&e->e.errWord, sizeof(int));
         rc |= dev_alloc((void **)&e->e.errDeferred, sizeof(int));
-        rc |= dev_alloc((void **)&e->e.fluxWall, sizeof(real) * 8);
+        rc |= dev_alloc((void **)&e->e.fluxWall, sizeof(real) * kWallFluxLen);
         rc |= dev_alloc((void **)&e->e.objDir, sizeof(real) * 8);
         if (s->nVars == 6)
             rc |= dev_alloc((void **)&e->e.jSource, sizeof(real) * m.nCell * 6);
@@ -564,7 +565,7 @@ extern "C"
         cudaMemset(e->e.lambdaFace, 0, sizeof(real) * m.nFace);
         cudaMemset(e->e.lambdaConv, 0, sizeof(real) * m.nFace);
         cudaMemset(e->e.errDeferred, 0, sizeof(int));
-        cudaMemset(e->e.fluxWall, 0, sizeof(real) * 8);
+        cudaMemset(e->e.fluxWall, 0, sizeof(real) * kWallFluxLen);
         *out = e;
         return DNDSB_OK;
     }

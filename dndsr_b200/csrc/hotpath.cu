@@ -4,6 +4,7 @@
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "sa.cuh"
+#include "wall_flux.cuh"
 
 namespace dndsb
 {
@@ -623,16 +624,20 @@ int vr_swap(int64_t n, real *a, real *b, cudaStream_t st)
 }
 
 // wall-flux integral of EvaluateRHS.hxx:599-607: minus the face fluxes of the BCWall / BCWallIsothermal faces
-// (and of BCWallInvis faces when muGas < 1e-99), summed over the boundary-face list in a fixed order (one
-// block: thread partial sums over a fixed stride, then a fixed tree)
+// (and of BCWallInvis faces when muGas < 1e-99), summed in a fixed order: the boundary-face list in a fixed
+// grid stride, fixed trees per block and over the blocks' sums.
+// Bound by the latency of the chain face -> zone -> type -> flux row, so the list is spread over up to
+// kWallFluxBlocks blocks (about one face per thread up to 38k faces); one block walking the whole list took
+// 58 us for the 19,040 boundary faces of the 249,600-tet bump and 82 us for the 15,120 of a 304k-hex plate, 7 and 6
+// now (the whole residuals 467 -> 415 us and 1,733 -> 1,657 us).
 template <int NV>
-DNDSB_GLOBAL void k_wall_flux_sum(MeshD m, BoundaryD bnd, real muGas, const real *__restrict__ ff, real *out)
+DNDSB_GLOBAL void __launch_bounds__(256) k_wall_flux_part(MeshD m, BoundaryD bnd, real muGas, const real *__restrict__ ff, real *out)
 {
-    __shared__ real sp[256][NV];
+    __shared__ real sp[8][NV];
     real acc[NV];
     for (int v = 0; v < NV; v++)
         acc[v] = 0;
-    for (int64_t ii = threadIdx.x; ii < m.nBndFace; ii += blockDim.x)
+    DNDSB_KERNEL_LOOP(ii, m.nBndFace)
     {
         int64_t f = m.bndFace[ii];
         int zone = m.faceZone[f];
@@ -641,19 +646,47 @@ DNDSB_GLOBAL void k_wall_flux_sum(MeshD m, BoundaryD bnd, real muGas, const real
             for (int v = 0; v < NV; v++)
                 acc[v] -= ff[f * NV + v];
     }
+#pragma unroll
     for (int v = 0; v < NV; v++)
-        sp[threadIdx.x][v] = acc[v];
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1)
     {
-        if ((int)threadIdx.x < w)
-            for (int v = 0; v < NV; v++)
-                sp[threadIdx.x][v] += sp[threadIdx.x + w][v];
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1)
+            acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
+        if ((threadIdx.x & 31) == 0)
+            sp[threadIdx.x >> 5][v] = acc[v];
     }
-    if (threadIdx.x == 0)
-        for (int v = 0; v < NV; v++)
-            out[v] = sp[0][v];
+    __syncthreads();
+    if (threadIdx.x < NV)
+    {
+        real s = 0;
+        for (int w = 0; w < 8; w++)
+            s += sp[w][threadIdx.x];
+        out[blockIdx.x * NV + threadIdx.x] = s;
+    }
+}
+
+// out[v] = the sum of the blocks' partials, one warp per variable
+template <int NV>
+DNDSB_GLOBAL void k_wall_flux_final(int nb, const real *__restrict__ part, real *out)
+{
+    const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    real s = 0;
+    for (int b = lane; b < nb; b += 32)
+        s += part[b * NV + v];
+    for (int o = 16; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0)
+        out[v] = s;
+}
+
+// fluxWall: [8] result, then the blocks' partials
+template <int NV>
+void wall_flux_sum(const MeshD &m, const BoundaryD &bnd, real muGas, const real *ff, real *fluxWall, cudaStream_t st)
+{
+    const int64_t want = (m.nBndFace + 255) / 256;
+    const int nb = (int)(want < kWallFluxBlocks ? want : kWallFluxBlocks);
+    k_wall_flux_part<NV><<<nb, 256, 0, st>>>(m, bnd, muGas, ff, nb == 1 ? fluxWall : fluxWall + 8);
+    if (nb > 1)
+        k_wall_flux_final<NV><<<1, 32 * NV, 0, st>>>(nb, fluxWall + 8, fluxWall);
 }
 
 int eval_rhs(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real *u, const real *uRec, real *rhs, real *faceFlux,
@@ -756,9 +789,9 @@ int eval_rhs_ex(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const 
     if (!(flags & RHSF_DONT_UPDATE_INTEGRATION) && m.nBndFace > 0 && ev.fluxWall)
     {
         if (nv == 5)
-            k_wall_flux_sum<5><<<1, 256, 0, st>>>(m, vr.bnd, s.muGas, ff, ev.fluxWall);
+            wall_flux_sum<5>(m, vr.bnd, s.muGas, ff, ev.fluxWall, st);
         else
-            k_wall_flux_sum<6><<<1, 256, 0, st>>>(m, vr.bnd, s.muGas, ff, ev.fluxWall);
+            wall_flux_sum<6>(m, vr.bnd, s.muGas, ff, ev.fluxWall, st);
     }
     return check(st, evc.errWord, !ev.deferErr);
 }

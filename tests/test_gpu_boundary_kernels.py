@@ -1,0 +1,33 @@
+"""Boundary-face kernels at the sizes where their blocks change shape: lists that fit one block of the wall-flux
+reduction and lists that need several."""
+import numpy as np
+import pytest
+import torch
+
+from dndsr_b200 import mesh as M
+from tests.bump_case import bump_bc, perturbed_state
+from tests.util import VR_HQM_PY
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims", [(3, 2, 2), (4, 4, 6), (12, 6, 5)])  # 64, 256 and 648 boundary faces: one, one and three blocks
+def test_wall_flux_is_the_sum_over_the_wall_faces(dims):
+    from dndsr_b200.solver import EulerEvaluator, VariationalReconstruction
+    m = M.bump_channel_tet(*dims)
+    far = M.freestream(0.8)
+    types, vals, w = bump_bc(far)
+    vr = VariationalReconstruction(m, dict(VR_HQM_PY, maxOrder=1, intOrder=2)).construct(w)
+    ev = EulerEvaluator(vr, dict(nVars=5, riemannSolverType="Roe", muGas=0.0, ignoreVis=True))
+    ev.SetBC(types, vals)
+    u0, rec0 = perturbed_state(m, far, R=3)
+    u, rec = torch.tensor(u0, device="cuda"), torch.tensor(rec0, device="cuda")
+    dt = torch.zeros(m.n_cell, dtype=torch.float64, device="cuda")
+    ev.EvaluateDt(dt, u, 1.0)
+    ev.EvaluateRHS(torch.zeros_like(u), u, rec)
+    ff = ev.get("faceFlux").reshape(-1, 5)[:m.n_face]
+    walls = (m.face2cell[:, 1] < 0) & (types[m.face_zone] == 3)  # slip walls count without viscosity
+    assert walls.sum() > 0
+    # each of the n additions of the two orders rounds a partial sum of at most sum |f|
+    bound = 2 * walls.sum() * np.finfo(float).eps * np.abs(ff[walls]).sum(0)
+    assert np.all(np.abs(ev.get("fluxWallSum")[:5] + ff[walls].sum(0)) <= bound)
