@@ -2,83 +2,107 @@
 //
 // Boundary faces are few (the walls and far-field of a channel are a few
 // percent of the faces), so they run in their own kernels after the interior
-// kernels: one thread per boundary cell adds the boundary term of the VR sweep,
-// one thread per boundary face writes the boundary face flux.  Both are
+// kernels: the boundary term of the VR sweep per boundary cell, the boundary
+// face flux per boundary face, each with one thread per Gauss point.  Both are
 // deterministic (fixed loop orders, no atomics on data).
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "bc.cuh"
 #include "sa.cuh"
+#include "basis_rows.cuh"
 
 namespace dndsb
 {
 namespace
 {
+// Boundary kernels run one thread per (boundary cell or face, Gauss point) in blocks of about 64 threads: there are
+// few boundary faces and their points are long serial chains (ghost state, Riemann solve), so a thread that walks all
+// the points of its face leaves the GPU idle for its whole length.  Thread per cell / face against thread per point:
+// 74 -> 24 us (VR term) and 102 -> 12 us (RHS) for the 5,180 faces of a 36k-tet bump at degree 2 (7 points), 31 -> 21
+// and 33 -> 22 us for the 19,040 faces of a 250k-tet one at degree 1 (3 points).
+inline int bc_rows(int nGf) { return nGf < 64 ? 64 / nGf : 1; }
+
 // VariationalReconstruction_Reconstruction.hxx:19-176 GetBoundaryRHS with the Euler FBoundary of
 // EulerSolver.hxx:163-175, applied as in :568-586:
 //   BCC = sum_{bc faces} sum_q w0^2 phi(x_q) (uBV(compress(u + phi . uRec)) - u) |J| w_q
 //   uRecNew += relax A^-1 BCC     (recordInc: -= A^-1 BCC, nothing when uRecIsZero)
+// Thread (cl, q) of a block: point q of the boundary faces of the block's cell cl, one face slot at a time; the
+// cell's threads then share out the R NV sums over the points (in point order) and the product with A^-1.
 template <int DIM, int P, int NV, typename TC>
 DNDSB_GLOBAL void k_vr_bc(MeshD m, GeomD g, VRD vr, const TC *__restrict__ AAInvB, const real *__restrict__ uRec, real *uRecNew,
                           const real *__restrict__ u, real relax, int recordInc)
 {
-    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
-    DNDSB_KERNEL_LOOP(ii, m.nBndCell)
+    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, RV = R * NV;
+    extern __shared__ real smBc[];
+    const int nG = g.nGf, cl = threadIdx.x / nG, q = threadIdx.x - cl * nG, rows = blockDim.x / nG;
+    const int64_t ii = (int64_t)blockIdx.x * rows + cl;
+    const int64_t c = ii < m.nBndCell ? m.bndCell[ii] : -1;
+    real *sP = smBc + cl * (nG * (R + NV) + RV); // [nG][R + NV]: phi, (uBV - u) |J| w w0^2
+    real *sB = sP + nG * (R + NV);               // [R][NV]: BCC
+    for (int e = q; e < RV; e += nG)
+        sB[e] = 0;
+    for (int k = 0; k < m.nf; k++)
     {
-        int64_t c = m.bndCell[ii];
-        const real *uc = u + c * NV, *rc = uRec + c * R * NV;
-        real BCC[R * NV];
-        for (int i = 0; i < R * NV; i++)
-            BCC[i] = 0;
-        for (int k = 0; k < m.nf; k++)
+        int64_t f = 0;
+        real w0 = 0;
+        if (c >= 0 && m.cellNbr[c * m.nf + k] < 0)
         {
-            if (m.cellNbr[c * m.nf + k] >= 0)
-                continue;
-            int64_t f = m.cell2face[c * m.nf + k] >> 1;
-            real w0 = vr.faceWeight[f * (P + 1)];
-            if (w0 == 0)
-                continue;
-            int zone = m.faceZone[f];
-            for (int q = 0; q < g.nGf; q++)
-            {
-                const real *p = &g.facePP[(f * g.nGf + q) * 3];
-                const real *n = &g.faceNorm[(f * g.nGf + q) * 3];
-                real T[NDOF];
-                cell_basis<DIM, NDOF>(&g.cellCent[c * 3], &g.cellScale[c * 3], &vr.baseMoment[c * NDOF], vr.s.anisotropicLengths, p, 1, T);
-                real UL[NV], ULf[NV], UB[NV];
-                for (int v = 0; v < NV; v++)
-                {
-                    real a = uc[v];
-                    for (int j = 0; j < R; j++)
-                        a += T[1 + j] * rc[j * NV + v];
-                    UL[v] = a;
-                }
-                compress_rec<NV>(uc, UL, ULf);
-                if (!bc_value_fix<NV>(vr.bnd, zone, ULf, n, UB))
-                    for (int v = 0; v < NV; v++)
-                        UB[v] = ULf[v];
-                real JW = g.faceJDet[f * g.nGf + q] * g.faceQw[q] * w0 * w0;
-                for (int i = 0; i < R; i++)
-                    for (int v = 0; v < NV; v++)
-                        BCC[i * NV + v] += T[1 + i] * (UB[v] - uc[v]) * JW;
-            }
+            f = m.cell2face[c * m.nf + k] >> 1;
+            w0 = vr.faceWeight[f * (P + 1)];
         }
-        const TC *Ai = AAInvB + c * (m.nf + 1) * R * R;
-        real sgn = recordInc ? -1.0 : relax;
-        for (int i = 0; i < R; i++)
+        if (!__syncthreads_or(w0 != 0)) // also keeps the last slot's sums apart from this slot's points
+            continue;
+        if (w0 != 0)
         {
-            real acc[NV];
+            const real *uc = u + c * NV, *rc = uRec + c * RV;
+            const real *n = &g.faceNorm[(f * nG + q) * 3];
+            real phi[R];
+            basis_rows<DIM, P, false>(g, vr, c, &g.facePP[(f * nG + q) * 3], phi, nullptr);
+            real UL[NV], ULf[NV], UB[NV];
+#pragma unroll
             for (int v = 0; v < NV; v++)
-                acc[v] = 0;
-            for (int j = 0; j < R; j++)
             {
-                real a = (real)Ai[i * R + j];
-                for (int v = 0; v < NV; v++)
-                    acc[v] += a * BCC[j * NV + v];
+                real a = uc[v];
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    a += phi[j] * rc[j * NV + v];
+                UL[v] = a;
             }
+            compress_rec<NV>(uc, UL, ULf);
+            if (!bc_value_fix<NV>(vr.bnd, m.faceZone[f], ULf, n, UB))
+                for (int v = 0; v < NV; v++)
+                    UB[v] = ULf[v];
+            const real JW = g.faceJDet[f * nG + q] * g.faceQw[q] * w0 * w0;
+            real *row = sP + q * (R + NV);
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                row[i] = phi[i];
             for (int v = 0; v < NV; v++)
-                uRecNew[(c * R + i) * NV + v] += sgn * acc[v];
+                row[R + v] = (UB[v] - uc[v]) * JW;
         }
+        __syncthreads();
+        if (w0 != 0)
+            for (int e = q; e < RV; e += nG)
+            {
+                const int i = e / NV, v = e - i * NV;
+                real a = sB[e];
+                for (int p = 0; p < nG; p++)
+                    a += sP[p * (R + NV) + i] * sP[p * (R + NV) + R + v];
+                sB[e] = a;
+            }
+    }
+    __syncthreads();
+    if (c < 0)
+        return;
+    const TC *Ai = AAInvB + c * (m.nf + 1) * R * R;
+    const real sgn = recordInc ? -1.0 : relax;
+    for (int e = q; e < RV; e += nG)
+    {
+        const int i = e / NV, v = e - i * NV;
+        real acc = 0;
+        for (int j = 0; j < R; j++)
+            acc += (real)Ai[i * R + j] * sB[j * NV + v];
+        uRecNew[c * RV + e] += sgn * acc;
     }
 }
 
@@ -201,95 +225,104 @@ DNDSB_GLOBAL void k_rhs_bc(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const rea
                            real *__restrict__ lam)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
+    extern __shared__ real smBc[];
     const real gamma = s.gamma;
-    DNDSB_KERNEL_LOOP(ii, m.nBndFace)
+    const int nG = g.nGf, fl = threadIdx.x / nG, q = threadIdx.x - fl * nG, rows = blockDim.x / nG;
+    const int64_t ii = (int64_t)blockIdx.x * rows + fl;
+    real *row = smBc + threadIdx.x * (NV + 3); // this point's flux and eigenvalues times |J| w
+    const int64_t f = ii < m.nBndFace ? m.bndFace[ii] : -1;
+    if (f >= 0)
     {
-        int64_t f = m.bndFace[ii];
         int64_t c0 = m.face2cell[f * 2];
         int zone = m.faceZone[f];
         int type = zone >= 0 && zone < vr.bnd.nZone ? vr.bnd.type[zone] : 0;
         const real *ULm = u + c0 * NV, *r0 = uRec + c0 * R * NV, *q0 = uRecG + c0 * R * NV; // values, gradients
         real URm[NV];
-        bool bad = false;
         if (!bc_value<NV>(vr.bnd, zone, ULm, &g.faceMeanNorm[f * 3], URm))
             for (int v = 0; v < NV; v++)
                 URm[v] = ULm[v];
-        real dLambda = dLamCell[c0];
         bool zeroGrad = type == BC_WALL_INVIS || type == BC_OUT || type == BC_FAR || type == BC_SYM;
         bool slip = type == BC_WALL_INVIS || type == BC_SYM;
-        real dc[3];
-        for (int d = 0; d < 3; d++)
-            dc[d] = g.faceCent[f * 3 + d] - g.cellBary[c0 * 3 + d];
-        real fluxEs[NV], lamEs[3] = {0, 0, 0};
+        const real *n = &g.faceNorm[(f * nG + q) * 3];
+        const real *p0 = &g.facePP[(f * nG + q) * 3];
+        real phi[R], dphi[R][DIM];
+        basis_rows<DIM, P, true>(g, vr, c0, p0, phi, dphi);
+        real UL[NV], UR[NV], Fv[NV];
+#pragma unroll
         for (int v = 0; v < NV; v++)
-            fluxEs[v] = 0;
-        for (int q = 0; q < g.nGf; q++)
         {
-            const real *n = &g.faceNorm[(f * g.nGf + q) * 3];
-            const real *p0 = &g.facePP[(f * g.nGf + q) * 3];
-            real T0[(DIM + 1) * NDOF];
-            cell_basis<DIM, NDOF>(&g.cellCent[c0 * 3], &g.cellScale[c0 * 3], &vr.baseMoment[c0 * NDOF], vr.s.anisotropicLengths, p0, DIM + 1,
-                                  T0);
-            real UL[NV], UR[NV], GL[3 * NV];
-            for (int v = 0; v < NV; v++)
-            {
-                real a = ULm[v];
-                real ga[3] = {0, 0, 0};
-                for (int j = 0; j < R; j++)
-                {
-                    real x0 = r0[j * NV + v], y0 = q0[j * NV + v];
-                    a += T0[1 + j] * x0;
-                    for (int d = 0; d < DIM; d++)
-                        ga[d] += T0[(1 + d) * NDOF + 1 + j] * y0;
-                }
-                UL[v] = a;
-                for (int d = 0; d < 3; d++)
-                    GL[d * NV + v] = ga[d];
-            }
-            if (!bc_value_fix<NV>(vr.bnd, zone, UL, n, UR))
-                for (int v = 0; v < NV; v++)
-                    UR[v] = UL[v];
-            real Fv[NV];
-            for (int v = 0; v < NV; v++)
-                Fv[v] = 0;
-            if (!s.ignoreVis && !zeroGrad)
-            {
-                real distBaryPerp = fabs(dot3(dc, n)) * 2.;
-                real distGRP = g.vol[c0] / g.faceArea[f] * 2;
-                distGRP = dmax(dmin(distBaryPerp, distGRP * 2), distGRP * 0.25);
-                real iD = 1.0 / distGRP;
-                real UM[NV], GM[3 * NV], GP[3 * NV];
-                for (int v = 0; v < NV; v++)
-                    UM[v] = 0.5 * (UL[v] + UR[v]);
-                for (int d = 0; d < 3; d++)
-                    for (int v = 0; v < NV; v++)
-                        GM[d * NV + v] = GL[d * NV + v] + iD * (n[d] * (UR[v] - UL[v]));
-                grad_cons2prim<NV>(UM, GM, GP, gamma);
-                if (!slip)
-                    point_viscous_flux<NV>(s, UM, GP, n, type == BC_WALL, Fv);
-            }
-            real F[NV], l0, l1, l4;
-            for (int v = 0; v < NV; v++)
-                F[v] = 0;
-            bad |= !riemann_flux(s.rsType, UL, UR, ULm, URm, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4,
-                                 s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr);
-            if (NV == 6)
-                F[NV - 1] = sa_convective_flux(UL, UR, n, l1);
-            real JW = g.faceJDet[f * g.nGf + q] * g.faceQw[q];
-            for (int v = 0; v < NV; v++)
-                fluxEs[v] -= (F[v] - Fv[v]) * JW;
-            lamEs[0] += l0 * JW, lamEs[1] += l1 * JW, lamEs[2] += l4 * JW;
+            real a = ULm[v];
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                a += phi[j] * r0[j * NV + v];
+            UL[v] = a;
+            Fv[v] = 0;
         }
-        if (lam)
-            for (int i = 0; i < 3; i++)
-                lam[i * m.nFace + f] = lamEs[i] / g.faceArea[f];
-        bool fin = true;
+        if (!bc_value_fix<NV>(vr.bnd, zone, UL, n, UR))
+            for (int v = 0; v < NV; v++)
+                UR[v] = UL[v];
+        if (!s.ignoreVis && !zeroGrad && !slip)
+        {
+            real dc[3];
+            for (int d = 0; d < 3; d++)
+                dc[d] = g.faceCent[f * 3 + d] - g.cellBary[c0 * 3 + d];
+            real distBaryPerp = fabs(dot3(dc, n)) * 2.;
+            real distGRP = g.vol[c0] / g.faceArea[f] * 2;
+            distGRP = dmax(dmin(distBaryPerp, distGRP * 2), distGRP * 0.25);
+            real iD = 1.0 / distGRP;
+            real UM[NV], GM[3 * NV], GP[3 * NV];
+            for (int v = 0; v < NV; v++)
+                UM[v] = 0.5 * (UL[v] + UR[v]);
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                {
+                    real ga = 0;
+                    if (d < DIM)
+#pragma unroll
+                        for (int j = 0; j < R; j++)
+                            ga += dphi[j][d < DIM ? d : 0] * q0[j * NV + v];
+                    GM[d * NV + v] = ga + iD * (n[d] * (UR[v] - UL[v]));
+                }
+            grad_cons2prim<NV>(UM, GM, GP, gamma);
+            point_viscous_flux<NV>(s, UM, GP, n, type == BC_WALL, Fv);
+        }
+        real F[NV], l0, l1, l4;
         for (int v = 0; v < NV; v++)
-            fin = fin && isfinite(fluxEs[v]);
-        if (bad || !fin)
-            atomicOr(err, bad ? (int)DE_NONPHYSICAL : (int)DE_NONFINITE);
+            F[v] = 0;
+        if (!riemann_flux(s.rsType, UL, UR, ULm, URm, n, gamma, dLamCell[c0], s.rsFixScale, s.rsIncFScale, F, l0, l1, l4,
+                          s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr))
+            atomicOr(err, (int)DE_NONPHYSICAL);
+        if (NV == 6)
+            F[NV - 1] = sa_convective_flux(UL, UR, n, l1);
+        real JW = g.faceJDet[f * nG + q] * g.faceQw[q];
         for (int v = 0; v < NV; v++)
-            faceFlux[f * NV + v] = fluxEs[v];
+            row[v] = (F[v] - Fv[v]) * JW;
+        row[NV] = l0 * JW, row[NV + 1] = l1 * JW, row[NV + 2] = l4 * JW;
+    }
+    __syncthreads();
+    // the sums over the points of a face, in point order
+    for (int e = threadIdx.x; e < rows * (NV + 3); e += blockDim.x)
+    {
+        const int fi = e / (NV + 3), v = e - fi * (NV + 3);
+        const int64_t ff = (int64_t)blockIdx.x * rows + fi < m.nBndFace ? m.bndFace[(int64_t)blockIdx.x * rows + fi] : -1;
+        if (ff < 0 || (v >= NV && !lam))
+            continue;
+        real acc = 0;
+        for (int p = 0; p < nG; p++)
+        {
+            const real x = smBc[(fi * nG + p) * (NV + 3) + v];
+            acc = v < NV ? acc - x : acc + x;
+        }
+        if (v >= NV)
+        {
+            lam[(v - NV) * m.nFace + ff] = acc / g.faceArea[ff];
+            continue;
+        }
+        if (!isfinite(acc))
+            atomicOr(err, (int)DE_NONFINITE);
+        faceFlux[ff * NV + v] = acc;
     }
 }
 
@@ -297,16 +330,14 @@ template <int DIM, int P, int NV>
 void launch_vr_bc(const MeshD &m, const GeomD &g, const VRD &vr, const real *uRec, real *uRecNew, const real *u, int recordInc, int useFP32,
                   cudaStream_t st)
 {
+    constexpr int R = ndof_of<DIM>(P) - 1;
+    const int rows = bc_rows(g.nGf);
+    const unsigned nb = (unsigned)((m.nBndCell + rows - 1) / rows);
+    const size_t sh = sizeof(real) * rows * (g.nGf * (R + NV) + R * NV);
     if (useFP32)
-    {
-        auto k = k_vr_bc<DIM, P, NV, float>;
-        DNDSB_LAUNCH(k, m.nBndCell, 64, st, m, g, vr, vr.AAInvB32, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
-    }
+        k_vr_bc<DIM, P, NV, float><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, vr.AAInvB32, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
     else
-    {
-        auto k = k_vr_bc<DIM, P, NV, real>;
-        DNDSB_LAUNCH(k, m.nBndCell, 64, st, m, g, vr, vr.AAInvB, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
-    }
+        k_vr_bc<DIM, P, NV, real><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, vr.AAInvB, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
 }
 
 template <int DIM, int NV>
@@ -328,6 +359,17 @@ int vr_bc_p(const MeshD &m, const GeomD &g, const VRD &vr, const real *uRec, rea
     return ST_UNSUPPORTED;
 }
 
+template <int DIM, int P, int NV>
+void launch_rhs_bc(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, const real *u, const real *uRec, const real *uRecG, real *ff,
+                   cudaStream_t st)
+{
+    const int rows = bc_rows(g.nGf);
+    const unsigned nb = (unsigned)((m.nBndFace + rows - 1) / rows);
+    const size_t sh = sizeof(real) * rows * g.nGf * (NV + 3);
+    k_rhs_bc<DIM, P, NV><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, ev.s, u, uRec, uRecG, ev.deltaLambdaCell, ff, ev.errWord,
+                                                       ev.jacMode == 2 ? ev.lambdaFace0 : nullptr);
+}
+
 template <int DIM, int NV>
 int rhs_bc_p(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, const real *u, const real *uRec, const real *uRecG, real *ff,
              cudaStream_t st)
@@ -335,26 +377,14 @@ int rhs_bc_p(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, con
     switch (vr.P)
     {
     case 1:
-    {
-        auto k = k_rhs_bc<DIM, 1, NV>;
-        DNDSB_LAUNCH(k, m.nBndFace, 64, st, m, g, vr, ev.s, u, uRec, uRecG, ev.deltaLambdaCell, ff, ev.errWord,
-                     ev.jacMode == 2 ? ev.lambdaFace0 : nullptr);
+        launch_rhs_bc<DIM, 1, NV>(m, g, vr, ev, u, uRec, uRecG, ff, st);
         return ST_OK;
-    }
     case 2:
-    {
-        auto k = k_rhs_bc<DIM, 2, NV>;
-        DNDSB_LAUNCH(k, m.nBndFace, 64, st, m, g, vr, ev.s, u, uRec, uRecG, ev.deltaLambdaCell, ff, ev.errWord,
-                     ev.jacMode == 2 ? ev.lambdaFace0 : nullptr);
+        launch_rhs_bc<DIM, 2, NV>(m, g, vr, ev, u, uRec, uRecG, ff, st);
         return ST_OK;
-    }
     case 3:
-    {
-        auto k = k_rhs_bc<DIM, 3, NV>;
-        DNDSB_LAUNCH(k, m.nBndFace, 64, st, m, g, vr, ev.s, u, uRec, uRecG, ev.deltaLambdaCell, ff, ev.errWord,
-                     ev.jacMode == 2 ? ev.lambdaFace0 : nullptr);
+        launch_rhs_bc<DIM, 3, NV>(m, g, vr, ev, u, uRec, uRecG, ff, st);
         return ST_OK;
-    }
     }
     return ST_UNSUPPORTED;
 }

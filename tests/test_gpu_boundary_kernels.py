@@ -1,12 +1,12 @@
 """Boundary-face kernels at the sizes where their blocks change shape: lists that fit one block of the wall-flux
-reduction and lists that need several."""
+reduction and lists that need several, every number of points per face (rows per block)."""
 import numpy as np
 import pytest
 import torch
 
 from dndsr_b200 import mesh as M
-from tests.bump_case import bump_bc, perturbed_state
-from tests.util import VR_HQM_PY
+from tests.bump_case import bump_bc, bump_oracle, perturbed_state
+from tests.util import VR_HQM_PY, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +31,24 @@ def test_wall_flux_is_the_sum_over_the_wall_faces(dims):
     # each of the n additions of the two orders rounds a partial sum of at most sum |f|
     bound = 2 * walls.sum() * np.finfo(float).eps * np.abs(ff[walls]).sum(0)
     assert np.all(np.abs(ev.get("fluxWallSum")[:5] + ff[walls].sum(0)) <= bound)
+
+
+@pytest.mark.parametrize("p,intOrder", [(1, 2), (1, 4), (2, 5), (2, 6), (3, 6)])  # 3, 6, 7, 12, 12 points per face
+def test_points_per_face_against_the_oracle(p, intOrder):
+    """VR boundary term and boundary fluxes, the 1e-12 of the other parity tests; 64 boundary faces, so that the last
+    block of 64 // points rows is ragged."""
+    from dndsr_b200.solver import EulerEvaluator, VariationalReconstruction
+    m = M.renumber_by_color(M.bump_channel_tet(3, 2, 2))
+    o, far, types, vals, w = bump_oracle(m, p, "Roe", 1e-3, 0, intOrder=intOrder, outflow_type=6, inflow_type=7, wall_type=2)
+    vr = VariationalReconstruction(m, dict(VR_HQM_PY, maxOrder=p, intOrder=intOrder)).construct(w)
+    ev = EulerEvaluator(vr, dict(nVars=5, riemannSolverType="Roe", muGas=1e-3, muModel=0, ignoreVis=False))
+    ev.SetBC(types, vals)
+    u0, rec0 = perturbed_state(m, far, R=o.R)
+    u, rec = torch.tensor(u0, device="cuda"), torch.tensor(rec0, device="cuda")
+    new, rhs, dt = torch.zeros_like(rec), torch.zeros_like(u), torch.zeros(m.n_cell, dtype=torch.float64, device="cuda")
+    vr.DoReconstructionIter(rec, new, u, putIntoNew=True)
+    assert relerr(new.cpu().numpy(), o.vr_iter(rec0, u0)) < 1e-12
+    ev.EvaluateDt(dt, u, 5.0)
+    o.eval_dt(u0, 5.0)
+    ev.EvaluateRHS(rhs, u, rec)
+    assert relerr(rhs.cpu().numpy(), o.eval_rhs(u0, rec0)) < 1e-12
