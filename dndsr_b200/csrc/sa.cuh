@@ -52,88 +52,137 @@ DNDSB_HD T sa_convective_flux(const T *UL, const T *UR, const real *n, const T &
     return ((vnL * UL[5] + vnR * UR[5]) - (UR[5] - UL[5]) * lam123) * 0.5;
 }
 
-// RANS_ke.hpp:985-1195 GetSource_SA: mode 0 the source of the SA equation, mode 1 its diagonal
-// Jacobian; G is the conservative gradient [3][6]
+constexpr real kSAFarDistance = 2.5873402367724347e33; // kVeryLarge^(1/6), the largest wall distance taken
+
 template <typename T>
-DNDSB_HD T sa_source(const T *U, const T *G, real muRef, const T &mufPhy, real d, real lLES, real hMax, int mode)
+DNDSB_HD T sa_cube(const T &x) { return x * x * x; }
+// x^(1/6) of x >= 0 (zero derivative at 0, as the power has in dual numbers)
+DNDSB_HD real sa_root6(real x) { return sqrt(cbrt(x)); }
+template <int N>
+DNDSB_HD Dual<N> sa_root6(const Dual<N> &x)
+{
+    Dual<N> r;
+    r.v = sa_root6(x.v);
+    const real s = x.v != 0 ? r.v / (6 * x.v) : 0.0;
+    for (int i = 0; i < N; i++)
+        r.d[i] = s * x.d[i];
+    return r;
+}
+
+// The state enters the source through rho, U5, mu and five invariants of the conservative gradient G [3][6]
+template <typename T>
+struct SAInvariants
+{
+    T ir, velo[3], nuh;                 // 1 / rho, velocity, nuTilde
+    T dRho[3], dNu[3], dV[3][3];        // gradients of rho, nuTilde and the velocity (dV[i][j] = d v_j / d x_i)
+    T om2, ss2, du2, dd, nn;            // vorticity, strain and gradient norms squared; dRho.dNu, dNu.dNu
+};
+
+template <typename T>
+DNDSB_HD void sa_invariants(const T *U, const T *G, real muRef, SAInvariants<T> &q)
+{
+    q.ir = 1.0 / U[0];
+    q.nuh = U[5] * muRef * q.ir;
+    for (int j = 0; j < 3; j++)
+        q.velo[j] = U[1 + j] * q.ir;
+    for (int i = 0; i < 3; i++)
+    {
+        q.dRho[i] = G[i * 6 + 0];
+        q.dNu[i] = (G[i * 6 + 5] * muRef - q.nuh * q.dRho[i]) * q.ir;
+        for (int j = 0; j < 3; j++)
+            q.dV[i][j] = (G[i * 6 + 1 + j] - q.dRho[i] * q.velo[j]) * q.ir;
+    }
+    q.om2 = q.ss2 = q.du2 = 0;
+    for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++)
+        {
+            T o = 0.5 * (q.dV[j][i] - q.dV[i][j]);
+            T sij = q.dV[i][j] + q.dV[j][i];
+            q.om2 += o * o, q.ss2 += sij * sij, q.du2 += q.dV[i][j] * q.dV[i][j];
+        }
+    q.dd = q.dRho[0] * q.dNu[0] + q.dRho[1] * q.dNu[1] + q.dRho[2] * q.dNu[2];
+    q.nn = q.dNu[0] * q.dNu[0] + q.dNu[1] * q.dNu[1] + q.dNu[2] * q.dNu[2];
+}
+
+// RANS_ke.hpp:985-1195 GetSource_SA: production P, destruction D and the diffusion factor fn, from
+// (rho, U5, mu; S, SS, |grad v|).  Bound by the FP64 elementary functions, so whole powers are products, the sixth
+// root is a square root of a cube root, and where a blending factor is exactly 0 or 1 (fe1 <= 1, fB = 1: next to the
+// wall) the functions that it multiplies away are not evaluated.
+template <typename T>
+DNDSB_HD void sa_core(const T &rho, const T &n5, const T &mufPhy, const T &S, const T &SS, const T &diffUNorm, real muRef, real d, real lLES,
+                      real hMax, T &P, T &D, T &fn)
 {
     using C = SAConst;
     const real cw1 = C::cb1 / (C::kappa * C::kappa) + (1 + C::cb2) / C::sigma;
     const real k2 = C::kappa * C::kappa;
-    T nuh = U[5] * muRef / U[0];
-    T Chi = U[5] * muRef / mufPhy;
-    T Chi3 = Chi * Chi * Chi;
+    const T ir = 1.0 / rho;
+    T nuh = n5 * muRef * ir;
+    T Chi = n5 * muRef / mufPhy;
+    T Chi3 = sa_cube(Chi);
     T fnu1 = Chi3 / (Chi3 + C::cnu1 * C::cnu1 * C::cnu1);
     T fnu2 = 1 - Chi / (1 + Chi * fnu1);
-    T velo[3] = {U[1] / U[0], U[2] / U[0], U[3] / U[0]};
-    T diffRho[3], diffNu[3], diffU[3][3];
-    for (int i = 0; i < 3; i++)
-    {
-        diffRho[i] = G[i * 6 + 0];
-        diffNu[i] = (G[i * 6 + 5] * muRef - nuh * diffRho[i]) / U[0];
-        for (int j = 0; j < 3; j++)
-            diffU[i][j] = (G[i * 6 + 1 + j] - diffRho[i] * velo[j]) / U[0];
-    }
-    T om2 = 0, ss2 = 0, du2 = 0;
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++)
-        {
-            T o = 0.5 * (diffU[j][i] - diffU[i][j]);
-            T sij = diffU[i][j] + diffU[j][i];
-            om2 += o * o, ss2 += sij * sij, du2 += diffU[i][j] * diffU[i][j];
-        }
-    T S = sqrt(om2) * sqrt(2.0);
-    T SS = sqrt(ss2) * (1. / sqrt(2.0));
     T SRotCor = 2.0 * dmin(0.0, S - SS);
-    T diffUNorm = sqrt(du2);
     T ft2 = C::ct3 * exp(-C::ct4 * Chi * Chi);
-    // DDES shielding, then the IDDES blend (SADESMode 1)
-    T lRANS = d;
-    T nuTur = mufPhy / U[0] * dmax(Chi * fnu1, 0.0);
-    T nufPhy = mufPhy / U[0];
-    T den = k2 * d * d * dmax(kSmall, diffUNorm);
-    T rd = (nuTur + nufPhy) / den;
-    T fd = 1. - tanh(pow(8 * rd, 3.0));
+    // the IDDES blend of the RANS and LES lengths (SADESMode 1)
+    const real lRANS = d;
+    T nufPhy = mufPhy * ir;
+    T nuTur = nufPhy * dmax(Chi * fnu1, 0.0);
+    T iden = 1.0 / (k2 * d * d * dmax(kSmall, diffUNorm));
     T psiSqr = Chi <= 0 ? T(100.0) : dmin(100.0, (1 - C::cb1 / (cw1 * k2 * 0.424) * (ft2 + (1 - ft2) * fnu2)) / (fnu1 * dmax(kSmall, 1 - ft2)));
     T psi = sqrt(dmax(psiSqr, 1.0));
-    T lDES = lRANS - fd * dmax(0., lRANS - lLES * psi);
+    const real alphaIDDES = 0.25 - d / hMax;
+    const real fB = dmin(2 * exp(-9. * alphaIDDES * alphaIDDES), 1.0);
+    const real cl = 3.55, ct = 1.63;
+    T rdt = nuTur * iden, rdl = nufPhy * iden;
+    const real fe1 = 2. * exp(-(alphaIDDES >= 0 ? 11.09 : 9.0) * alphaIDDES * alphaIDDES);
+    T fe = 0.0;
+    if (fe1 > 1)
     {
-        real alphaIDDES = 0.25 - d / hMax;
-        real fB = dmin(2 * exp(-9. * alphaIDDES * alphaIDDES), 1.0);
-        const real cl = 3.55, ct = 1.63;
-        T rdt = nuTur / den, rdl = nufPhy / den;
-        T ft = tanh(pow(ct * ct * rdt, 3.0));
+        T ft = tanh(sa_cube(T(ct * ct * rdt)));
         T flt = (cl * cl * rdl) * (cl * cl * rdl);
         T fl = tanh((flt * flt) * (flt * flt) * flt);
-        real fe1 = 2. * exp(-(alphaIDDES >= 0 ? 11.09 : 9.0) * alphaIDDES * alphaIDDES);
-        T fe2 = 1. - dmax(ft, fl);
-        T fe = dmax(fe1 - 1., 0.) * psi * fe2;
-        T fdTilde = dmax(fB, tanh(pow(8 * rdt, 3.0)));
-        T lIDDES = fdTilde * (1 + fe) * lRANS + (1 - fdTilde) * lLES * psi;
-        lDES = dmax(lLES * kSmall, lIDDES);
+        fe = (fe1 - 1.) * psi * (1. - dmax(ft, fl));
     }
-    const T dL = lDES; // d = lDES in the reference
+    T dL = (1 + fe) * lRANS;
+    if (fB < 1)
+    {
+        T fdTilde = dmax(fB, tanh(sa_cube(T(8 * rdt))));
+        dL = fdTilde * dL + (1 - fdTilde) * lLES * psi;
+    }
+    dL = dmax(lLES * kSmall, dL);
+    T idL = 1.0 / dL;
+    T nd = nuh * idL; // nuTilde / d
     T Sbar = nuh / (k2 * dL * dL) * fnu2;
     T Sh = Sbar < -C::cnu2 * S ? T(S + S * (C::cnu2 * C::cnu2 * S + C::cnu3 * Sbar) / ((C::cnu3 - 2 * C::cnu2) * S - Sbar)) : T(S + Sbar);
-    T r = dmin(nuh / (Sh * (C::kappa * dL) * (C::kappa * dL) + kVerySmall), C::rlim);
-    T g = r + C::cw2 * (pow(r, 6.0) - r);
-    real cw36 = pow(C::cw3, 6.0);
-    T fw = g * pow((1 + cw36) / (pow(g, 6.0) + cw36), 1. / 6.);
-    T D = (cw1 * fw - C::cb1 / k2 * ft2) * (nuh / lDES) * (nuh / lDES);
-    T P = C::cb1 * (1 - ft2) * (Sh + SRotCor) * nuh;
-    T fn = 1;
-    if (U[5] < 0)
+    if (n5 < 0)
     {
-        T Chi_ = U[5] * muRef / mufPhy;
-        fn = (C::cn1 + pow(Chi_, 3.0)) / (C::cn1 - pow(Chi_, 3.0));
-        D = -cw1 * (nuh / lDES) * (nuh / lDES);
+        T Chi_3 = Chi3;
+        fn = (C::cn1 + Chi_3) / (C::cn1 - Chi_3);
+        D = -cw1 * nd * nd;
         P = C::cb1 * (1 - C::ct3) * fabs(S + SRotCor) * nuh;
+        return;
     }
-    T dd = diffRho[0] * diffNu[0] + diffRho[1] * diffNu[1] + diffRho[2] * diffNu[2];
-    T nn = diffNu[0] * diffNu[0] + diffNu[1] * diffNu[1] + diffNu[2] * diffNu[2];
-    if (mode == 0)
-        return U[0] * (P - D + nn * C::cb2 / C::sigma) / muRef - (U[5] * fn * muRef + mufPhy) / (U[0] * C::sigma) * dd / muRef;
-    return -dmin(U[0] * (dmin(P, 0.0) * 1 - D * 2) / muRef / (fabs(U[5]) + kVerySmall), -kVerySmall);
+    T r = dmin(nuh / (Sh * (C::kappa * dL) * (C::kappa * dL) + kVerySmall), C::rlim);
+    T g = r + C::cw2 * (sa_cube(T(r * r)) - r);
+    const real cw36 = C::cw3 * C::cw3 * C::cw3 * C::cw3 * C::cw3 * C::cw3;
+    T fw = g * sa_root6(T((1 + cw36) / (sa_cube(T(g * g)) + cw36)));
+    fn = 1.0;
+    D = (cw1 * fw - C::cb1 / k2 * ft2) * nd * nd;
+    P = C::cb1 * (1 - ft2) * (Sh + SRotCor) * nuh;
+}
+
+// the source of the SA equation (mode 0 of GetSource_SA); with J (real only) its diagonal Jacobian (mode 1)
+template <typename T>
+DNDSB_HD T sa_source(const T *U, const T *G, real muRef, const T &mufPhy, real d, real lLES, real hMax, real *J = nullptr)
+{
+    using C = SAConst;
+    SAInvariants<T> q;
+    sa_invariants(U, G, muRef, q);
+    T P, D, fn;
+    sa_core(U[0], U[5], mufPhy, T(sqrt(q.om2) * sqrt(2.0)), T(sqrt(q.ss2) * (1. / sqrt(2.0))), T(sqrt(q.du2)), muRef, d, lLES, hMax, P, D, fn);
+    if (J)
+        *J = -dmin(value_of(U[0]) * (dmin(value_of(P), 0.0) * 1 - value_of(D) * 2) / muRef / (::fabs(value_of(U[5])) + kVerySmall), -kVerySmall);
+    return U[0] * (P - D + q.nn * C::cb2 / C::sigma) / muRef - (U[5] * fn * muRef + mufPhy) * q.ir / C::sigma * q.dd / muRef;
 }
 // fluxFace viscous part at one point (EvaluateDt.hxx:1167-1209): laminar plus, for the SA model,
 // mu_t (with Pr_t = 0.9 heat conduction) and the nuTilde diffusion flux
