@@ -23,6 +23,7 @@
 #include "basis_eval.cuh"
 #include "bc.cuh"
 #include "sa.cuh"
+#include "basis_rows.cuh"
 
 namespace dndsb
 {
@@ -70,7 +71,7 @@ DNDSB_D bool interior_point_flux(const EulerSettingsD &s, const T *UL, const T *
 // cell mean (at the face centre), the inner gradient, no viscous flux on slip, far-field and outflow faces
 template <int NV, typename T>
 DNDSB_D bool boundary_point_flux(const EulerSettingsD &s, const BoundaryD &bnd, int zone, int type, const T *ULin, const T *ULm,
-                                 const real *nMean, const T *GL, const real *n, const real *nMV, real distGRP, real dLambda, T *out)
+                                 const real *nMean, const T *GL, const real *n, const real *nMV, real distGRP, real dLambda, T *out, int parts = 3)
 {
     const real gamma = s.gamma;
     T UL[NV], UR[NV], URm[NV];
@@ -87,7 +88,7 @@ DNDSB_D bool boundary_point_flux(const EulerSettingsD &s, const BoundaryD &bnd, 
     T Fv[NV];
     for (int v = 0; v < NV; v++)
         Fv[v] = 0.0;
-    if (!s.ignoreVis && !zeroGrad)
+    if (!s.ignoreVis && !zeroGrad && (parts & 2))
     {
         real iD = 1.0 / distGRP;
         T UM[NV], GM[3 * NV], GP[3 * NV];
@@ -155,23 +156,18 @@ DNDSB_D int zone_type(const BoundaryD &bnd, int zone) { return zone >= 0 && zone
 // wall faces of the wall-flux integral (EvaluateRHS.hxx:599-607)
 DNDSB_D bool is_wall(int type, real muGas) { return type == BC_WALL || type == BC_WALL_ISOTHERMAL || (type == BC_WALL_INVIS && muGas < 1e-99); }
 
-// Face cotangents faceAdj[f][side][R+1][NV] (entry 0: d/du, 1+j: d/duRec_j) of
-//   sum_c w_c . rhs_c   (objDir == nullptr), or of
-//   sum over the wall faces of objDir . (minus their face flux), the wall-flux integral along objDir.
+// Face cotangents faceAdj[f][side][R+1][NV] (entry 0: d/du, 1+j: d/duRec_j) of sum_c w_c . rhs_c, interior faces
 template <int DIM, int P, int NV>
-DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w, const real *__restrict__ objDir,
-                                   const real *__restrict__ u, const real *__restrict__ uRec, const real *__restrict__ dLamCell,
-                                   real *__restrict__ faceAdj, int *err, int bndOnly)
+DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w, const real *__restrict__ u,
+                                   const real *__restrict__ uRec, const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV;
     using DV = Dual<2 * NV>;
     DNDSB_KERNEL_LOOP(f, m.nFace)
     {
         const int64_t c0 = m.face2cell[f * 2], c1 = m.face2cell[f * 2 + 1];
-        const bool bnd = c1 < 0;
-        if (bndOnly && !bnd)
-            continue; // the interior faces' records come from the Gauss-point-parallel kernel
-        const int zone = m.faceZone[f], type = bnd ? zone_type(vr.bnd, zone) : 0;
+        if (c1 < 0)
+            continue; // k_rhs_vjp_bnd_g
         real *o0 = faceAdj + (f * 2) * W, *o1 = faceAdj + (f * 2 + 1) * W;
         for (int i = 0; i < W; i++)
             o0[i] = 0, o1[i] = 0;
@@ -179,18 +175,14 @@ DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, c
         bool any = false;
         for (int v = 0; v < NV; v++)
         {
-            if (objDir)
-                gbar[v] = bnd && is_wall(type, s.muGas) ? -objDir[v] : 0.0;
-            else
-                gbar[v] = w[c0 * NV + v] / g.vol[c0] - (bnd ? 0.0 : w[c1 * NV + v] / g.vol[c1]);
+            gbar[v] = w[c0 * NV + v] / g.vol[c0] - w[c1 * NV + v] / g.vol[c1];
             any = any || gbar[v] != 0.0;
         }
         if (!any)
             continue;
         const real *nMV = s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr;
-        const real *ULm = u + c0 * NV, *URm = bnd ? nullptr : u + c1 * NV;
-        const real dLambda = bnd ? dLamCell[c0] : dmax(dLamCell[c0], dLamCell[c1]);
-        const bool vis = !s.ignoreVis && !(bnd && (type == BC_WALL_INVIS || type == BC_OUT || type == BC_FAR || type == BC_SYM));
+        const real *ULm = u + c0 * NV, *URm = u + c1 * NV;
+        const real dLambda = dmax(dLamCell[c0], dLamCell[c1]);
         real ULbar[NV], URbar[NV], ULmbar[NV], URmbar[NV], GLbar[3 * NV], GRbar[3 * NV];
         for (int i = 0; i < NV; i++)
             ULbar[i] = URbar[i] = ULmbar[i] = URmbar[i] = 0;
@@ -215,60 +207,36 @@ DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, c
             real UL[NV], UR[NV], GL[3 * NV], GR[3 * NV];
             cell_basis<DIM, NDOF>(&g.cellCent[c0 * 3], &g.cellScale[c0 * 3], &vr.baseMoment[c0 * NDOF], vr.s.anisotropicLengths, p0, DIM + 1, T0);
             recon_point_grad<DIM, NDOF, NV>(T0, u + c0 * NV, uRec + c0 * R * NV, UL, GL);
-            if (!bnd)
-            {
-                cell_basis<DIM, NDOF>(&g.cellCent[c1 * 3], &g.cellScale[c1 * 3], &vr.baseMoment[c1 * NDOF], vr.s.anisotropicLengths, p1, DIM + 1,
-                                      T1);
-                recon_point_grad<DIM, NDOF, NV>(T1, u + c1 * NV, uRec + c1 * R * NV, UR, GR);
-            }
-            const int npass = 2 + (vis ? DIM : 0);
+            cell_basis<DIM, NDOF>(&g.cellCent[c1 * 3], &g.cellScale[c1 * 3], &vr.baseMoment[c1 * NDOF], vr.s.anisotropicLengths, p1, DIM + 1, T1);
+            recon_point_grad<DIM, NDOF, NV>(T1, u + c1 * NV, uRec + c1 * R * NV, UR, GR);
+            const int npass = 2 + (s.ignoreVis ? 0 : DIM);
             for (int pass = 0; pass < npass; pass++)
             {
-                // pass 0: (UL, UR) [boundary: (UL, ULm)]; pass 1: (ULm, URm) [boundary: nothing]; 2 + d: (GL_d, GR_d)
-                if (bnd && pass == 1)
-                    continue;
+                // pass 0: (UL, UR); pass 1: (ULm, URm); 2 + d: (GL_d, GR_d)
                 DV a[NV], b[NV], am[NV], bm[NV], ga[3 * NV], gb[3 * NV], out[NV];
                 for (int v = 0; v < NV; v++)
-                {
-                    a[v] = DV(UL[v]), am[v] = DV(ULm[v]);
-                    if (!bnd)
-                        b[v] = DV(UR[v]), bm[v] = DV(URm[v]);
-                }
+                    a[v] = DV(UL[v]), am[v] = DV(ULm[v]), b[v] = DV(UR[v]), bm[v] = DV(URm[v]);
                 for (int i = 0; i < 3 * NV; i++)
-                    ga[i] = DV(GL[i]), gb[i] = DV(bnd ? 0.0 : GR[i]);
+                    ga[i] = DV(GL[i]), gb[i] = DV(GR[i]);
                 const int d = pass - 2;
                 for (int v = 0; v < NV; v++)
                 {
                     if (pass == 0)
-                    {
-                        a[v].d[v] = 1;
-                        if (bnd)
-                            am[v].d[NV + v] = 1;
-                        else
-                            b[v].d[NV + v] = 1;
-                    }
+                        a[v].d[v] = 1, b[v].d[NV + v] = 1;
                     else if (pass == 1)
                         am[v].d[v] = 1, bm[v].d[NV + v] = 1;
                     else
                         ga[d * NV + v].d[v] = 1, gb[d * NV + v].d[NV + v] = 1;
                 }
-                // on interior faces the means enter only the inviscid flux, the gradients only the viscous one
-                bool ok = bnd ? boundary_point_flux<NV>(s, vr.bnd, zone, type, a, am, &g.faceMeanNorm[f * 3], ga, n, nMV, distGRP, dLambda, out)
-                              : interior_point_flux<NV>(s, a, b, am, bm, ga, gb, n, nMV, distGRP, dLambda, out, pass == 0 ? 3 : pass == 1 ? 1 : 2);
-                bad |= !ok;
+                // the means enter only the inviscid flux, the gradients only the viscous one
+                bad |= !interior_point_flux<NV>(s, a, b, am, bm, ga, gb, n, nMV, distGRP, dLambda, out, pass == 0 ? 3 : pass == 1 ? 1 : 2);
                 for (int i = 0; i < NV; i++)
                 {
                     real x0 = 0, x1 = 0;
                     for (int v = 0; v < NV; v++)
                         x0 += out[v].d[i] * Fbar[v], x1 += out[v].d[NV + i] * Fbar[v];
                     if (pass == 0)
-                    {
-                        ULbar[i] += x0;
-                        if (bnd)
-                            ULmbar[i] += x1;
-                        else
-                            URbar[i] += x1;
-                    }
+                        ULbar[i] += x0, URbar[i] += x1;
                     else if (pass == 1)
                         ULmbar[i] += x0, URmbar[i] += x1;
                     else
@@ -278,24 +246,16 @@ DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, c
             // through the basis into (u, uRec) of both sides: U = u + sum_j T_j uRec_j, G_d = sum_j T_{d,j} uRec_j
             for (int v = 0; v < NV; v++)
             {
-                o0[v] += ULbar[v];
+                o0[v] += ULbar[v], o1[v] += URbar[v];
                 for (int j = 0; j < R; j++)
                 {
-                    real a = T0[1 + j] * ULbar[v];
+                    real a = T0[1 + j] * ULbar[v], b = T1[1 + j] * URbar[v];
                     for (int dd = 0; dd < DIM; dd++)
-                        a += T0[(1 + dd) * NDOF + 1 + j] * GLbar[dd * NV + v];
-                    o0[NV + j * NV + v] += a;
-                }
-                if (!bnd)
-                {
-                    o1[v] += URbar[v];
-                    for (int j = 0; j < R; j++)
                     {
-                        real a = T1[1 + j] * URbar[v];
-                        for (int dd = 0; dd < DIM; dd++)
-                            a += T1[(1 + dd) * NDOF + 1 + j] * GRbar[dd * NV + v];
-                        o1[NV + j * NV + v] += a;
+                        a += T0[(1 + dd) * NDOF + 1 + j] * GLbar[dd * NV + v];
+                        b += T1[(1 + dd) * NDOF + 1 + j] * GRbar[dd * NV + v];
                     }
+                    o0[NV + j * NV + v] += a, o1[NV + j * NV + v] += b;
                 }
                 ULbar[v] = URbar[v] = 0;
             }
@@ -306,6 +266,149 @@ DNDSB_GLOBAL void k_rhs_vjp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, c
             o0[v] += ULmbar[v], o1[v] += URmbar[v];
         if (bad)
             atomicOr(err, (int)DE_NONPHYSICAL);
+    }
+}
+
+// The same for the boundary faces (side 0 only; side 1 is in no cell's row), with objDir of the sum over the wall
+// faces of objDir . (minus their face flux), the wall-flux integral along objDir.
+// There are few boundary faces and a pass in dual numbers is a long serial chain, so the passes and the points run
+// side by side: thread (pass, face, point), one warp (the faces that fit it) per pass of NV seeds: the point state,
+// the cell mean (the inviscid flux alone), the gradient along each axis (the viscous flux alone, skipped where the
+// zone has none); the block then shares out the face's W sums over the points, in point order.  A thread that
+// walked all passes and points of a face took 1,227 us for the 3,200 boundary faces of a 76,800-hex SA plate, this
+// kernel 108.
+template <int DIM, int P, int NV>
+DNDSB_GLOBAL void __launch_bounds__(32 * (DIM + 2))
+    k_rhs_vjp_bnd_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w, const real *__restrict__ objDir,
+                    const real *__restrict__ u, const real *__restrict__ uRec, const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
+{
+    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV;
+    constexpr int OM = NV, OG = 2 * NV, OP = OG + DIM * NV, OD = OP + R, ROW = (OD + R * DIM) | 1;
+    __shared__ real sm[32][ROW]; // per point: d/dU, d/du (the mean), d/dG [DIM][NV]; phi [R], its gradient [R][DIM]
+    const int nG = g.nGf, rows = 32 / nG, lane = threadIdx.x & 31, pass = threadIdx.x >> 5;
+    const int fl = lane / nG, q = lane - fl * nG;
+    const int64_t ii = (int64_t)blockIdx.x * rows + fl;
+    const int64_t f = fl < rows && ii < m.nBndFace ? m.bndFace[ii] : -1;
+    if (f >= 0)
+    {
+        const int64_t c0 = m.face2cell[f * 2];
+        const int zone = m.faceZone[f], type = zone_type(vr.bnd, zone);
+        const bool vis = !s.ignoreVis && !(type == BC_WALL_INVIS || type == BC_OUT || type == BC_FAR || type == BC_SYM);
+        real *row = sm[lane];
+        const real JW = g.faceJDet[f * nG + q] * g.faceQw[q];
+        real Fbar[NV];
+        bool any = false;
+        for (int v = 0; v < NV; v++)
+        {
+            const real gb = objDir ? (is_wall(type, s.muGas) ? -objDir[v] : 0.0) : w[c0 * NV + v] / g.vol[c0];
+            any = any || gb != 0.0;
+            Fbar[v] = -JW * gb;
+        }
+        const real *n = &g.faceNorm[(f * nG + q) * 3];
+        real phi[R], dphi[R][DIM], U[NV], G[3 * NV];
+        basis_rows<DIM, P, true>(g, vr, c0, &g.facePP[(f * nG + q) * 3], phi, dphi);
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+        {
+            real a = u[c0 * NV + v], ga[3] = {0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < R; j++)
+            {
+                const real x = uRec[(c0 * R + j) * NV + v];
+                a += phi[j] * x;
+#pragma unroll
+                for (int d = 0; d < DIM; d++)
+                    ga[d] += dphi[j][d] * x;
+            }
+            U[v] = a;
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                G[d * NV + v] = ga[d];
+        }
+        const real distGRP = grp_distance(m, g, f, c0, -1, n);
+        using DV = Dual<NV>;
+        if (pass < 2)
+        {
+            // pass 0 seeds the point state, pass 1 the cell mean, which enters the inviscid flux only
+            if (pass == 0)
+            {
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                {
+                    row[OP + j] = phi[j];
+#pragma unroll
+                    for (int d = 0; d < DIM; d++)
+                        row[OD + j * DIM + d] = dphi[j][d];
+                }
+            }
+            DV a[NV], am[NV], ga[3 * NV], out[NV];
+            for (int v = 0; v < NV; v++)
+                a[v] = DV::var(U[v], pass == 0 ? v : -1), am[v] = DV::var(u[c0 * NV + v], pass == 1 ? v : -1);
+            for (int i = 0; i < 3 * NV; i++)
+                ga[i] = DV(G[i]);
+            if (any && !boundary_point_flux<NV>(s, vr.bnd, zone, type, a, am, &g.faceMeanNorm[f * 3], ga, n,
+                                                s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr, distGRP, dLamCell[c0], out,
+                                                pass == 0 ? 3 : 1))
+                atomicOr(err, (int)DE_NONPHYSICAL);
+            for (int i = 0; i < NV; i++)
+            {
+                real x = 0;
+                for (int v = 0; v < NV; v++)
+                    x += out[v].d[i] * Fbar[v];
+                row[pass * OM + i] = any ? x : 0.0;
+            }
+        }
+        else
+        {
+            const int d = pass - 2;
+            DV Fv[NV];
+            if (any && vis)
+            {
+                real UR[NV];
+                if (!bc_value_fix<NV>(vr.bnd, zone, U, n, UR))
+                    for (int v = 0; v < NV; v++)
+                        UR[v] = U[v];
+                const real iD = 1.0 / distGRP;
+                DV UM[NV], GM[3 * NV], GP[3 * NV];
+                for (int v = 0; v < NV; v++)
+                    UM[v] = DV(0.5 * (U[v] + UR[v]));
+                for (int e = 0; e < 3; e++)
+                    for (int v = 0; v < NV; v++)
+                        GM[e * NV + v] = DV::var(G[e * NV + v] + iD * (n[e] * (UR[v] - U[v])), e == d ? v : -1);
+                grad_cons2prim<NV>(UM, GM, GP, s.gamma);
+                point_viscous_flux<NV>(s, UM, GP, n, type == BC_WALL, Fv);
+            }
+            for (int i = 0; i < NV; i++)
+            {
+                real x = 0;
+                for (int v = 0; v < NV; v++)
+                    x -= Fv[v].d[i] * Fbar[v];
+                row[OG + d * NV + i] = x;
+            }
+        }
+    }
+    __syncthreads();
+    // through the basis into (u, uRec): U = u + sum_j phi_j uRec_j, G_d = sum_j dphi_j,d uRec_j
+    for (int e = threadIdx.x; e < rows * W; e += blockDim.x)
+    {
+        const int fi = e / W, i = e - fi * W, j = i / NV - 1, v = i - (j + 1) * NV;
+        if ((int64_t)blockIdx.x * rows + fi >= m.nBndFace)
+            break;
+        real acc = 0;
+        for (int p = 0; p < nG; p++)
+        {
+            const real *r = sm[fi * nG + p];
+            if (j < 0)
+                acc += r[v] + r[OM + v];
+            else
+            {
+                real x = r[OP + j] * r[v];
+                for (int d = 0; d < DIM; d++)
+                    x += r[OD + j * DIM + d] * r[OG + d * NV + v];
+                acc += x;
+            }
+        }
+        faceAdj[(int64_t)m.bndFace[(int64_t)blockIdx.x * rows + fi] * 2 * W + i] = acc;
     }
 }
 
@@ -427,27 +530,155 @@ DNDSB_GLOBAL void k_flux_gather_g(int64_t nCell, int nf, const int32_t *__restri
     }
 }
 
-// the SA source at the cell Gauss points (hotpath.cu k_sa_source): VJP (mode 0, cotangent w) adds into
-// (du, duRec); JVP (mode 1, tangents du, duRec) adds into dRhs
+// Reverse of sa_source at one point: cot times its derivatives with respect to the state U [6] and the conservative
+// gradient G [3][6].  The source depends on them through rho, U5, mu, S, SS and |grad v| (nonlinearly: one evaluation
+// of sa_core in dual numbers with these six seeds) and through dRho.dNu and dNu.dNu (linearly); the invariants are
+// reversed by hand.
+DNDSB_D void sa_source_rev(const EulerSettingsD &s, const real *U, const real *G, real d, real lLES, real hMax, real cot, real *Ub, real *Gb)
+{
+    using C = SAConst;
+    using D6 = Dual<6>;
+    const real gamma = s.gamma, cp = s.Rgas * gamma / (gamma - 1), muRef = s.muGas;
+    SAInvariants<real> q;
+    sa_invariants(U, G, muRef, q);
+    const real ir = q.ir;
+    // the laminar viscosity and its derivatives to (rho, T)
+    const real m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
+    const real p = (gamma - 1) * (U[4] - 0.5 * m2 * ir), kT = 1.0 / ((gamma - 1) / gamma * cp), Temp = p * kT * ir;
+    const Dual<2> muD = mu_eff(s.muModel, s.muGas, s.TRef, s.CSutherland, Dual<2>::var(U[0], 0), Dual<2>::var(Temp, 1));
+    const real S = sqrt(q.om2), SS = sqrt(q.ss2), dUN = sqrt(q.du2), r2 = sqrt(2.0), i2 = 1. / sqrt(2.0);
+    D6 P, D, fn;
+    sa_core(D6::var(U[0], 0), D6::var(U[5], 1), D6::var(muD.v, 2), D6::var(S * r2, 3), D6::var(SS * i2, 4), D6::var(dUN, 5), muRef, d, lLES, hMax, P,
+            D, fn);
+    // F = rho (P - D + nn cb2 / sigma) / muRef - (U5 fn muRef + mu) / (rho sigma) dd / muRef
+    const real iM = 1.0 / muRef, e = q.dd * ir / C::sigma * iM, src = P.v - D.v + q.nn * C::cb2 / C::sigma;
+    real db[6];
+    for (int i = 0; i < 6; i++)
+        db[i] = cot * (U[0] * (P.d[i] - D.d[i]) * iM - U[5] * muRef * fn.d[i] * e);
+    real rhob = db[0] + cot * (src * iM + (U[5] * fn.v * muRef + muD.v) * ir * e);
+    real n5b = db[1] - cot * fn.v * muRef * e;
+    const real mub = db[2] - cot * e;
+    const real omb = S > 0 ? db[3] * r2 * 0.5 / S : 0.0, ssb = SS > 0 ? db[4] * i2 * 0.5 / SS : 0.0, dub = dUN > 0 ? db[5] * 0.5 / dUN : 0.0;
+    const real ddb = -cot * (U[5] * fn.v * muRef + muD.v) * ir / C::sigma * iM, nnb = cot * U[0] * C::cb2 / C::sigma * iM;
+    rhob += mub * muD.d[0];
+    const real Tb = mub * muD.d[1], pb = Tb * kT * ir;
+    rhob += -Tb * Temp * ir + pb * (gamma - 1) * 0.5 * m2 * ir * ir;
+    real vb[3] = {0, 0, 0}, nuhb = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+    {
+        const real nb = ddb * q.dRho[i] + 2 * nnb * q.dNu[i];
+        real rb = ddb * q.dNu[i] - nb * q.nuh * ir;
+        Gb[i * 6 + 5] = nb * muRef * ir;
+        nuhb -= nb * q.dRho[i] * ir;
+        rhob -= nb * q.dNu[i] * ir;
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+        {
+            const real A = q.dV[i][j], B = q.dV[j][i];
+            const real Ab = (omb * (A - B) + 4 * ssb * (A + B) + 2 * dub * A) * ir;
+            Gb[i * 6 + 1 + j] = Ab;
+            rb -= Ab * q.velo[j];
+            vb[j] -= Ab * q.dRho[i];
+            rhob -= Ab * A;
+        }
+        Gb[i * 6 + 0] = rb;
+        Gb[i * 6 + 4] = 0;
+    }
+    n5b += nuhb * muRef * ir;
+    rhob -= nuhb * q.nuh * ir;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+    {
+        Ub[1 + j] = vb[j] * ir - pb * (gamma - 1) * U[1 + j] * ir;
+        rhob -= vb[j] * q.velo[j] * ir;
+    }
+    Ub[0] = rhob, Ub[4] = pb * (gamma - 1), Ub[5] = n5b;
+}
+
+// VJP of the SA source at the cell Gauss points (hotpath.cu k_sa_source), cotangent w, added into (du, duRec).
+// One thread per (cell, point), at most 64 a block (the points of a cell are neighbouring lanes), their shares of the
+// W sums of the cell added in point order through shared memory.  Four passes of the whole source in six-seed dual
+// numbers, one thread per cell, took 1,932 us on a 76,800-hex plate, this kernel 154.
 template <int DIM, int P>
-DNDSB_GLOBAL void k_sa_source_d(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ u, const real *__restrict__ uRec,
-                                const real *__restrict__ dWall, int mode, const real *__restrict__ w, const real *__restrict__ tu,
-                                const real *__restrict__ tRec, real *outU, real *outRec)
+DNDSB_GLOBAL void __launch_bounds__(64) k_sa_source_vjp(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ u,
+                                                        const real *__restrict__ uRec, const real *__restrict__ dWall,
+                                                        const real *__restrict__ w, real *du, real *duRec)
+{
+    constexpr int NV = 6, NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV;
+    __shared__ real sm[64][W | 1];
+    const int nG = g.nGc, rows = blockDim.x / nG, cl = threadIdx.x / nG, q = threadIdx.x - cl * nG;
+    const int64_t c = (int64_t)blockIdx.x * rows + cl;
+    if (c < m.nCell)
+    {
+        real phi[R], dphi[R][DIM], U[NV], G[3 * NV];
+        basis_rows<DIM, P, true>(g, vr, c, &g.cellPP[(c * nG + q) * 3], phi, dphi);
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+        {
+            real a = u[c * NV + v], ga[3] = {0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < R; j++)
+            {
+                const real x = uRec[(c * R + j) * NV + v];
+                a += phi[j] * x;
+#pragma unroll
+                for (int d = 0; d < DIM; d++)
+                    ga[d] += dphi[j][d] * x;
+            }
+            U[v] = a;
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                G[d * NV + v] = ga[d];
+        }
+        const real hMax = g.hMax[c], d = dmin(dWall[c * nG + q], kSAFarDistance), lLES = dmin(hMax * kVeryLarge, dmax(d, hMax));
+        real Ub[NV], Gb[3 * NV];
+        sa_source_rev(s, U, G, d, lLES, hMax, g.cellJDet[c * nG + q] * g.cellQw[q] * w[c * NV + 5] / g.vol[c], Ub, Gb);
+        real *row = sm[threadIdx.x];
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+        {
+            row[v] = Ub[v];
+#pragma unroll
+            for (int j = 0; j < R; j++)
+            {
+                real a = phi[j] * Ub[v];
+#pragma unroll
+                for (int dd = 0; dd < DIM; dd++)
+                    a += dphi[j][dd] * Gb[dd * NV + v];
+                row[NV + j * NV + v] = a;
+            }
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < rows * W; e += blockDim.x)
+    {
+        const int ci = e / W, i = e - ci * W;
+        const int64_t cc = (int64_t)blockIdx.x * rows + ci;
+        if (cc >= m.nCell)
+            break;
+        real acc = 0;
+        for (int p = 0; p < nG; p++)
+            acc += sm[ci * nG + p][i];
+        if (i < NV)
+            du[cc * NV + i] += acc;
+        else
+            duRec[cc * R * NV + i - NV] += acc;
+    }
+}
+
+// JVP of the SA source along (tu, tRec), added into dRhs
+template <int DIM, int P>
+DNDSB_GLOBAL void k_sa_source_jvp(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ u, const real *__restrict__ uRec,
+                                  const real *__restrict__ dWall, const real *__restrict__ tu, const real *__restrict__ tRec, real *dRhs)
 {
     constexpr int NV = 6, NDOF = ndof_of<DIM>(P), R = NDOF - 1;
     const real gamma = s.gamma, cp = s.Rgas * gamma / (gamma - 1);
-    using D6 = Dual<6>;
     using D1 = Dual<1>;
     DNDSB_KERNEL_LOOP(c, m.nCell)
     {
         const real hMax = g.hMax[c];
-        const real iv = 1.0 / g.vol[c];
-        const real wb = mode == 0 ? w[c * NV + 5] * iv : 0.0;
-        real aU[NV], aRec[R * NV], dS = 0;
-        for (int i = 0; i < NV; i++)
-            aU[i] = 0;
-        for (int i = 0; i < R * NV; i++)
-            aRec[i] = 0;
+        real dS = 0;
         for (int q = 0; q < g.nGc; q++)
         {
             real T[(DIM + 1) * NDOF];
@@ -455,78 +686,22 @@ DNDSB_GLOBAL void k_sa_source_d(MeshD m, GeomD g, VRD vr, EulerSettingsD s, cons
                                   &g.cellPP[(c * g.nGc + q) * 3], DIM + 1, T);
             real U[NV], G[3 * NV];
             recon_point_grad<DIM, NDOF, NV>(T, u + c * NV, uRec + c * R * NV, U, G);
-            const real d = dmin(dWall[c * g.nGc + q], pow(kVeryLarge, 1. / 6.));
+            const real d = dmin(dWall[c * g.nGc + q], kSAFarDistance);
             const real lLES = dmin(hMax * kVeryLarge, dmax(d, hMax));
-            const real JW = g.cellJDet[c * g.nGc + q] * g.cellQw[q];
-            if (mode == 0)
-            {
-                real Ubar[NV] = {0, 0, 0, 0, 0, 0}, Gbar[3 * NV];
-                for (int i = 0; i < 3 * NV; i++)
-                    Gbar[i] = 0;
-                for (int pass = 0; pass <= DIM; pass++) // pass 0: U; pass 1 + d: G along axis d
-                {
-                    D6 Ud[NV], Gd[3 * NV];
-                    for (int v = 0; v < NV; v++)
-                        Ud[v] = D6(U[v]);
-                    for (int i = 0; i < 3 * NV; i++)
-                        Gd[i] = D6(G[i]);
-                    for (int v = 0; v < NV; v++)
-                    {
-                        if (pass == 0)
-                            Ud[v].d[v] = 1;
-                        else
-                            Gd[(pass - 1) * NV + v].d[v] = 1;
-                    }
-                    D6 pM, a2M, HM;
-                    gas_thermal(Ud[4], Ud[0], D6((Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3]) / (Ud[0] * Ud[0])), gamma, pM, a2M, HM);
-                    D6 Tm = pM / ((gamma - 1) / gamma * cp * Ud[0]);
-                    D6 mu = mu_eff(s.muModel, s.muGas, s.TRef, s.CSutherland, Ud[0], Tm);
-                    D6 S = sa_source(Ud, Gd, s.muGas, mu, d, lLES, hMax, 0);
-                    for (int v = 0; v < NV; v++)
-                    {
-                        if (pass == 0)
-                            Ubar[v] += S.d[v] * JW * wb;
-                        else
-                            Gbar[(pass - 1) * NV + v] += S.d[v] * JW * wb;
-                    }
-                }
-                for (int v = 0; v < NV; v++)
-                {
-                    aU[v] += Ubar[v];
-                    for (int j = 0; j < R; j++)
-                    {
-                        real a = T[1 + j] * Ubar[v];
-                        for (int dd = 0; dd < DIM; dd++)
-                            a += T[(1 + dd) * NDOF + 1 + j] * Gbar[dd * NV + v];
-                        aRec[j * NV + v] += a;
-                    }
-                }
-            }
-            else
-            {
-                real dU[NV], dG[3 * NV];
-                recon_point_grad<DIM, NDOF, NV>(T, tu + c * NV, tRec + c * R * NV, dU, dG);
-                D1 Ud[NV], Gd[3 * NV];
-                for (int v = 0; v < NV; v++)
-                    Ud[v] = D1(U[v]), Ud[v].d[0] = dU[v];
-                for (int i = 0; i < 3 * NV; i++)
-                    Gd[i] = D1(G[i]), Gd[i].d[0] = dG[i];
-                D1 pM, a2M, HM;
-                gas_thermal(Ud[4], Ud[0], D1((Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3]) / (Ud[0] * Ud[0])), gamma, pM, a2M, HM);
-                D1 Tm = pM / ((gamma - 1) / gamma * cp * Ud[0]);
-                D1 mu = mu_eff(s.muModel, s.muGas, s.TRef, s.CSutherland, Ud[0], Tm);
-                dS += sa_source(Ud, Gd, s.muGas, mu, d, lLES, hMax, 0).d[0] * JW;
-            }
-        }
-        if (mode == 0)
-        {
+            real dU[NV], dG[3 * NV];
+            recon_point_grad<DIM, NDOF, NV>(T, tu + c * NV, tRec + c * R * NV, dU, dG);
+            D1 Ud[NV], Gd[3 * NV];
             for (int v = 0; v < NV; v++)
-                outU[c * NV + v] += aU[v];
-            for (int i = 0; i < R * NV; i++)
-                outRec[c * R * NV + i] += aRec[i];
+                Ud[v] = D1(U[v]), Ud[v].d[0] = dU[v];
+            for (int i = 0; i < 3 * NV; i++)
+                Gd[i] = D1(G[i]), Gd[i].d[0] = dG[i];
+            D1 pM, a2M, HM;
+            gas_thermal(Ud[4], Ud[0], D1((Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3]) / (Ud[0] * Ud[0])), gamma, pM, a2M, HM);
+            D1 Tm = pM / ((gamma - 1) / gamma * cp * Ud[0]);
+            D1 mu = mu_eff(s.muModel, s.muGas, s.TRef, s.CSutherland, Ud[0], Tm);
+            dS += sa_source(Ud, Gd, s.muGas, mu, d, lLES, hMax).d[0] * g.cellJDet[c * g.nGc + q] * g.cellQw[q];
         }
-        else
-            outU[c * NV + 5] += dS * iv;
+        dRhs[c * NV + 5] += dS / g.vol[c];
     }
 }
 
@@ -760,15 +935,28 @@ int vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real 
         else if (rc != ST_UNSUPPORTED)
             return rc;
     }
-    auto kf = k_rhs_vjp_face_g<DIM, P, NV>;
-    DNDSB_LAUNCH(kf, m.nFace, 64, st, m, g, vr, ev.s, w, objDir, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord, interiorDone);
+    if (objDir) // the objective lives on the boundary
+        dev_zero(ev.adjBuf, sizeof(real) * m.nFace * 2 * W, st);
+    else if (!interiorDone)
+    {
+        auto kf = k_rhs_vjp_face_g<DIM, P, NV>;
+        DNDSB_LAUNCH(kf, m.nFace, 64, st, m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
+    }
+    if (m.nBndFace > 0)
+    {
+        const int rows = 32 / g.nGf; // at most 16 points per face
+        k_rhs_vjp_bnd_g<DIM, P, NV><<<(unsigned)((m.nBndFace + rows - 1) / rows), 32 * (DIM + 2), 0, st>>>(
+            m, g, vr, ev.s, w, objDir, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
+    }
     auto kg = k_adj_gather_g<W, NV>;
     DNDSB_LAUNCH(kg, m.nCell, 128, st, m.nCell, m.nf, m.cell2face, ev.adjBuf, du, duRec);
-    if (NV == 6 && !objDir)
-    {
-        auto ks = k_sa_source_d<DIM, P>;
-        DNDSB_LAUNCH(ks, m.nCell, 64, st, m, g, vr, ev.s, u, uRec, ev.dWall, 0, w, nullptr, nullptr, du, duRec);
-    }
+    if constexpr (NV == 6)
+        if (!objDir)
+        {
+            const int rows = 64 / g.nGc; // at most 64 points per cell
+            k_sa_source_vjp<DIM, P><<<(unsigned)((m.nCell + rows - 1) / rows), rows * g.nGc, 0, st>>>(m, g, vr, ev.s, u, uRec, ev.dWall, w, du,
+                                                                                                     duRec);
+        }
     return ST_OK;
 }
 
@@ -780,10 +968,10 @@ int jvp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real 
     DNDSB_LAUNCH(kf, m.nFace, 64, st, m, g, vr, ev.s, du, duRec, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
     auto kg = k_flux_gather_g<NV>;
     DNDSB_LAUNCH(kg, m.nCell, 256, st, m.nCell, m.nf, m.cell2face, g.vol, ev.adjBuf, dRhs);
-    if (NV == 6)
+    if constexpr (NV == 6)
     {
-        auto ks = k_sa_source_d<DIM, P>;
-        DNDSB_LAUNCH(ks, m.nCell, 64, st, m, g, vr, ev.s, u, uRec, ev.dWall, 1, nullptr, du, duRec, dRhs, nullptr);
+        auto ks = k_sa_source_jvp<DIM, P>;
+        DNDSB_LAUNCH(ks, m.nCell, 64, st, m, g, vr, ev.s, u, uRec, ev.dWall, du, duRec, dRhs);
     }
     return ST_OK;
 }
