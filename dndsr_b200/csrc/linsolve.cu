@@ -10,10 +10,8 @@
 // Layout.  Inside the solve every cell vector is stored in colour-position
 // order (position p holds cell colorCells[p]), so one colour class is one
 // contiguous range and "neighbour already updated in this sweep" is a range
-// test on the neighbour's position.  Per (position, face slot) the operator
-// keeps {w*n, w*lambda} with w = alpha * A_f / (2 V_c) as one 4-vector and the
-// neighbour's position; per position the scalar diagonal.  The state u is
-// converted once per solve into the solve precision T.
+// test on the neighbour's position.  The scalar-Jacobian operator and its sweeps
+// are in posop.cuh; they are built once per solve in the solve precision T.
 //
 // Precision.  T = double reproduces the FP64 operators; T = float is the
 // FP32 preconditioner of the mixed-precision defect correction (the caller's
@@ -38,66 +36,12 @@
 #include "solver.cuh"
 #include "roejac.cuh"
 #include "ilu.cuh"
+#include "posop.cuh"
 
 namespace dndsb
 {
 namespace
 {
-template <typename T>
-struct Vec4;
-template <>
-struct Vec4<float>
-{
-    using type = float4;
-};
-template <>
-struct Vec4<double>
-{
-    using type = double4;
-};
-
-// ---------------------------------------------------------------------------
-// operator build: LUSGSMatrixInit (EulerEvaluator.hxx:37-159) + packing
-// ---------------------------------------------------------------------------
-// JD: diagonals per cell (1, or NV with the SA source Jacobian)
-template <typename T, int NV>
-constexpr int jd_of() { return NV == 6 ? NV : 1; }
-
-template <typename T, int NV>
-DNDSB_GLOBAL void k_sgsop_build(MeshD m, GeomD g, const real *__restrict__ lamFace, const real *__restrict__ dTau, real dt, real alphaDiag,
-                                const real *__restrict__ u, const real *__restrict__ jSource, const int32_t *__restrict__ cellPos,
-                                int32_t *nbrPos, typename Vec4<T>::type *op, T *jd, T *uT)
-{
-    DNDSB_KERNEL_LOOP(p, m.nCell)
-    {
-        int64_t c = m.colorCells[p];
-        real iv = 1.0 / g.vol[c];
-        real cf = 0.5 * alphaDiag / g.vol[c];
-        real fp = 1.0 / dTau[c] + 1.0 / dt;
-        for (int k = 0; k < m.nf; k++)
-        {
-            int pk = m.cell2face[c * m.nf + k];
-            int64_t f = pk >> 1;
-            real sg = (pk & 1) ? -1.0 : 1.0;
-            fp += (0.5 * alphaDiag) * g.faceArea[f] * lamFace[f] * iv;
-            real w = cf * g.faceArea[f];
-            typename Vec4<T>::type o4;
-            o4.x = (T)(w * g.faceMeanNorm[f * 3] * sg);
-            o4.y = (T)(w * g.faceMeanNorm[f * 3 + 1] * sg);
-            o4.z = (T)(w * g.faceMeanNorm[f * 3 + 2] * sg);
-            o4.w = (T)(w * lamFace[f]);
-            op[p * m.nf + k] = o4;
-            int o = m.cellNbr[c * m.nf + k];
-            nbrPos[p * m.nf + k] = o < 0 ? -1 : cellPos[o];
-        }
-        constexpr int JD = jd_of<T, NV>();
-        for (int v = 0; v < JD; v++)
-            jd[p * JD + v] = (T)(fp + (JD > 1 ? alphaDiag * jSource[c * NV + v] : 0.0));
-        for (int v = 0; v < NV; v++)
-            uT[p * NV + v] = (T)u[c * NV + v];
-    }
-}
-
 // natural order FP64 -> position order T, and back
 template <typename T, int NV>
 DNDSB_GLOBAL void k_gather_T(int64_t n, const int32_t *__restrict__ pos2cell, const real *__restrict__ x, T *y)
@@ -147,96 +91,6 @@ DNDSB_GLOBAL void k_add_T(int64_t n, const T *__restrict__ a, T *b) // b += a
 {
     DNDSB_KERNEL_LOOP(i, n)
     b[i] += a[i];
-}
-
-// scaled flux-increment Jacobian times dU (EulerEvaluator.hpp:1100-1158 with
-// Gas.hpp:462-513), minus w*lambda*dU; o4 = {w n, w lambda}
-template <typename T, int NV>
-DNDSB_D void jac_du_scaled(const T *U, const T *dU, const typename Vec4<T>::type &o4, T gamma, T *dF)
-{
-    T ir = T(1) / U[0];
-    T v0 = U[1] * ir, v1 = U[2] * ir, v2 = U[3] * ir;
-    T p = (gamma - T(1)) * (U[4] - U[0] * T(0.5) * (v0 * v0 + v1 * v1 + v2 * v2));
-    T dv0 = (dU[1] - U[1] * ir * dU[0]) * ir;
-    T dv1 = (dU[2] - U[2] * ir * dU[0]) * ir;
-    T dv2 = (dU[3] - U[3] * ir * dU[0]) * ir;
-    T dp = (gamma - T(1)) * (dU[4] - T(0.5) * (dU[1] * v0 + dU[2] * v1 + dU[3] * v2 + U[1] * dv0 + U[2] * dv1 + U[3] * dv2));
-    T vn = v0 * o4.x + v1 * o4.y + v2 * o4.z;
-    T dvn = dv0 * o4.x + dv1 * o4.y + dv2 * o4.z;
-    dF[0] = dU[1] * o4.x + dU[2] * o4.y + dU[3] * o4.z;
-    dF[1] = dU[1] * vn + U[1] * dvn + o4.x * dp;
-    dF[2] = dU[2] * vn + U[2] * dvn + o4.y * dp;
-    dF[3] = dU[3] * vn + U[3] * dvn + o4.z * dp;
-    dF[4] = (dU[4] + dp) * vn + (U[4] + p) * dvn;
-    for (int j = 5; j < NV; j++)
-        dF[j] = dU[j] * vn + U[j] * dvn;
-    for (int j = 0; j < NV; j++)
-        dF[j] -= o4.w * dU[j];
-}
-
-// one colour class of a forward / backward sweep (UpdateSGS, EulerEvaluator.hxx:550-693)
-template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_sgs_pos(int64_t pBeg, int64_t pEnd, const int32_t *__restrict__ nbrPos, const typename Vec4<T>::type *__restrict__ op,
-                            const T *__restrict__ jd, const T *__restrict__ uT, const T *__restrict__ rhs, const T *__restrict__ xOld,
-                            T *xNew, T gamma, int forward, int gsUpdate, int uIncIsZero)
-{
-    DNDSB_KERNEL_LOOP(ii, pEnd - pBeg)
-    {
-        int64_t p = pBeg + ii;
-        T buf[NV];
-        for (int v = 0; v < NV; v++)
-            buf[v] = rhs[p * NV + v];
-#pragma unroll
-        for (int k = 0; k < NF; k++)
-        {
-            int q = nbrPos[p * NF + k];
-            if (q < 0 || q == p)
-                continue;
-            bool useNew = gsUpdate && (forward ? q < pBeg : q >= pEnd);
-            if (uIncIsZero && !useNew)
-                continue;
-            typename Vec4<T>::type o4 = op[p * NF + k];
-            const T *dU = (useNew ? xNew : xOld) + (int64_t)q * NV;
-            T dF[NV];
-            jac_du_scaled<T, NV>(uT + (int64_t)q * NV, dU, o4, gamma, dF);
-            for (int v = 0; v < NV; v++)
-                buf[v] -= dF[v];
-        }
-        constexpr int JD = jd_of<T, NV>();
-        for (int v = 0; v < NV; v++)
-            xNew[p * NV + v] = buf[v] * (T(1) / jd[p * JD + (JD > 1 ? v : 0)]);
-    }
-}
-
-// LUSGSMatrixVec (EulerEvaluator.hxx:175-274)
-// xs (may be null): a scale of x (the normalising factor of an unnormalised basis column): Ax = A (xs x)
-template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_matvec_pos(int64_t n, const int32_t *__restrict__ nbrPos, const typename Vec4<T>::type *__restrict__ op,
-                               const T *__restrict__ jd, const T *__restrict__ uT, const T *__restrict__ x, T *Ax, T gamma,
-                               const real *__restrict__ xs)
-{
-    const T sx = xs ? (T)*xs : T(1);
-    DNDSB_KERNEL_LOOP(p, n)
-    {
-        T buf[NV];
-        for (int v = 0; v < NV; v++)
-            buf[v] = 0;
-#pragma unroll
-        for (int k = 0; k < NF; k++)
-        {
-            int q = nbrPos[p * NF + k];
-            if (q < 0)
-                continue;
-            typename Vec4<T>::type o4 = op[p * NF + k];
-            T dF[NV];
-            jac_du_scaled<T, NV>(uT + (int64_t)q * NV, x + (int64_t)q * NV, o4, gamma, dF);
-            for (int v = 0; v < NV; v++)
-                buf[v] -= dF[v];
-        }
-        constexpr int JD = jd_of<T, NV>();
-        for (int v = 0; v < NV; v++)
-            Ax[p * NV + v] = sx * (jd[p * JD + (JD > 1 ? v : 0)] * x[p * NV + v] - buf[v]);
-    }
 }
 
 // block operator build.  Storage is tiled by 32 positions (ilu::BlockLay, s = 5): element k NV NV + e of a position's
@@ -579,8 +433,10 @@ struct LinWs
     int prec = -1, k = 0, nv = 0, nf = 0, jacMode = 0;
     int64_t nCell = 0;
     int32_t *cellPos = nullptr, *nbrPos = nullptr;
-    void *op = nullptr, *jd = nullptr, *uT = nullptr, *rhsT = nullptr, *x = nullptr, *tmp = nullptr, *tmp2 = nullptr, *MLb = nullptr,
-         *V = nullptr;
+    // scalar mode: the packed operator of posop.cuh (opNu: 6 variables)
+    void *op = nullptr, *jd = nullptr, *jdi = nullptr, *vh = nullptr, *opNu = nullptr;
+    int32_t *opCnt = nullptr;
+    void *rhsT = nullptr, *x = nullptr, *tmp = nullptr, *tmp2 = nullptr, *MLb = nullptr, *V = nullptr;
     real *H = nullptr, *sc = nullptr, *s2 = nullptr, *red = nullptr;
     void *opB = nullptr, *jdB = nullptr; // block mode: off-diagonal blocks [nCell][nf][nv][nv], diagonal blocks + inverses [nCell][2][nv][nv]
     void *luB = nullptr, *luD = nullptr, *tmp3 = nullptr; // jacobiCode 2: ILU(0) slot blocks, inverted pivots, scratch
@@ -599,7 +455,7 @@ void linws_free(LinWs *w)
     if (!w)
         return;
     for (void *p : {(void *)w->cellPos, (void *)w->nbrPos, w->op, w->jd, w->opB, w->jdB, w->luB, w->luD, w->tmp3, (void *)w->luNbr,
-                    (void *)w->luNLow, w->uT, w->rhsT, w->x, w->tmp, w->tmp2, w->MLb, w->V, (void *)w->H,
+                    (void *)w->luNLow, w->jdi, w->vh, w->opNu, (void *)w->opCnt, w->rhsT, w->x, w->tmp, w->tmp2, w->MLb, w->V, (void *)w->H,
                     (void *)w->sc, (void *)w->s2, (void *)w->red, (void *)w->colScale, (void *)w->cnt})
         dev_free(p);
     graph_free(w->graph);
@@ -633,10 +489,9 @@ int ws_prepare(const MeshD &m, LinWs *&w, const LinSettings &ls, int nv, int jac
     w = new LinWs();
     w->prec = ls.precision, w->k = k, w->nv = nv, w->nf = m.nf, w->nCell = m.nCell, w->jacMode = jacMode;
     int64_t n = m.nCell * nv;
+    const int64_t nPad = ilu::padded_rows(m.nCell, 5); // the operator arrays are tiled by 32 positions
     bool ok = dev_alloc((void **)&w->cellPos, sizeof(int32_t) * m.nCell) == cudaSuccess &&
-              dev_alloc((void **)&w->nbrPos, sizeof(int32_t) * m.nCell * m.nf) == cudaSuccess &&
-              dev_alloc(&w->op, 4 * es * m.nCell * m.nf) == cudaSuccess && dev_alloc(&w->jd, es * m.nCell * (nv == 6 ? 6 : 1)) == cudaSuccess &&
-              dev_alloc(&w->uT, es * n) == cudaSuccess && dev_alloc(&w->rhsT, es * n) == cudaSuccess &&
+              dev_alloc((void **)&w->nbrPos, sizeof(int32_t) * nPad * m.nf) == cudaSuccess && dev_alloc(&w->rhsT, es * n) == cudaSuccess &&
               dev_alloc(&w->x, es * n) == cudaSuccess && dev_alloc(&w->tmp, es * n) == cudaSuccess &&
               dev_alloc(&w->tmp2, es * n) == cudaSuccess && dev_alloc(&w->MLb, es * n) == cudaSuccess &&
               dev_alloc(&w->V, es * krylov_ld(n) * (k + 1)) == cudaSuccess &&
@@ -645,7 +500,12 @@ int ws_prepare(const MeshD &m, LinWs *&w, const LinSettings &ls, int nv, int jac
               dev_alloc((void **)&w->s2, sizeof(real) * 8) == cudaSuccess &&
               dev_alloc((void **)&w->red, sizeof(real) * kRedBufLenK) == cudaSuccess &&
               dev_alloc((void **)&w->colScale, sizeof(real) * 33) == cudaSuccess && dev_alloc((void **)&w->cnt, sizeof(unsigned)) == cudaSuccess;
-    const int64_t nPad = ilu::padded_rows(m.nCell, 5); // the block arrays are tiled by 32 positions
+    const int64_t jdLen = m.nCell * (nv == 6 ? 6 : 1);
+    if (ok && !jacMode)
+        ok = dev_alloc(&w->op, 4 * es * nPad * m.nf) == cudaSuccess && dev_alloc(&w->jd, es * jdLen) == cudaSuccess &&
+             dev_alloc(&w->jdi, es * jdLen) == cudaSuccess && dev_alloc(&w->vh, 4 * es * m.nCell) == cudaSuccess &&
+             dev_alloc((void **)&w->opCnt, sizeof(int32_t) * m.nCell) == cudaSuccess &&
+             (nv != 6 || dev_alloc(&w->opNu, es * m.nCell) == cudaSuccess);
     if (ok && jacMode)
         ok = dev_alloc(&w->opB, es * nv * nv * nPad * m.nf) == cudaSuccess && dev_alloc(&w->jdB, es * 2 * nv * nv * nPad) == cudaSuccess;
     if (ok && jacMode && ls.jacobiCode == 2)
@@ -680,7 +540,6 @@ struct Solve
     T gamma;
     cudaStream_t st;
     int64_t n() const { return m.nCell * NV; }
-    using T4 = typename Vec4<T>::type;
     int64_t ld() const { return krylov_ld(n()); }
     T *V(int i) const { return (T *)w.V + (int64_t)i * ld(); }
 
@@ -705,21 +564,33 @@ struct Solve
             }
             return;
         }
+        auto kern = posop::k_sweep<T, NV, NF>;
+        const T *old = zeroIn ? nullptr : xOld;
         if (!gs)
         {
-            auto kern = k_sgs_pos<T, NV, NF>;
-            DNDSB_LAUNCH(kern, m.nCell, 128, st, 0, m.nCell, w.nbrPos, (const T4 *)w.op, (const T *)w.jd,
-                         (const T *)w.uT, rhs, xOld, xNew, gamma, (int)forward, 0, (int)zeroIn);
+            DNDSB_LAUNCH(kern, m.nCell, 128, st, 0, m.nCell, A(), rhs, old, old, xNew, gamma - 1);
             return;
         }
-        auto kern = k_sgs_pos<T, NV, NF>;
         for (int ci = 0; ci < m.nColor; ci++)
         {
             int col = forward ? ci : m.nColor - 1 - ci;
             int64_t b = m.colorStart[col], e = m.colorStart[col + 1];
-            DNDSB_LAUNCH(kern, e - b, 128, st, b, e, w.nbrPos, (const T4 *)w.op, (const T *)w.jd, (const T *)w.uT, rhs,
-                         xOld, xNew, gamma, (int)forward, 1, (int)zeroIn);
+            DNDSB_LAUNCH(kern, e - b, 128, st, b, e, A(), rhs, forward ? (const T *)xNew : old, forward ? old : (const T *)xNew, xNew, gamma - 1);
         }
+    }
+
+    posop::Op<T> A() const
+    {
+        using T4 = typename posop::Vec4<T>::type;
+        return posop::Op<T>{w.nbrPos, w.opCnt, (T4 *)w.op, (T *)w.jd, (T *)w.jdi, (T4 *)w.vh, (T *)w.opNu};
+    }
+
+    // the backward half of a scalar-Jacobian pair whose forward half, from zero, is in x (the last colour is done)
+    void back(T *x) const
+    {
+        auto kb = posop::k_back<T, NV, NF>;
+        for (int col = m.nColor - 2; col >= 0; col--)
+            DNDSB_LAUNCH(kb, m.colorStart[col + 1] - m.colorStart[col], 128, st, m.colorStart[col], m.colorStart[col + 1], A(), x, gamma - 1);
     }
 
     // doPrecondition with jacobiCode 2 (EulerSolver.hxx:1642-1657): two LUSGSMatrixSolveJacobianLU steps,
@@ -760,6 +631,12 @@ struct Solve
             return;
         }
         bool gs = ls.jacobiCode == 1;
+        if (gs && zeroIn && !w.jacMode)
+        {
+            sweep(rhs, nullptr, x, true, true, true);
+            back(x);
+            return;
+        }
         sweep(rhs, x, (T *)w.tmp2, true, gs, zeroIn);
         sweep(rhs, (T *)w.tmp2, x, false, gs, false);
     }
@@ -780,9 +657,25 @@ struct Solve
             DNDSB_LAUNCH(kb, m.nCell, 128, st, m.nCell, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, x, Ax, xs);
             return;
         }
-        auto kern = k_matvec_pos<T, NV, NF>;
-        DNDSB_LAUNCH(kern, m.nCell, 128, st, m.nCell, w.nbrPos, (const T4 *)w.op, (const T *)w.jd, (const T *)w.uT, x,
-                     Ax, gamma, xs);
+        auto kern = posop::k_product<T, NV, NF>;
+        DNDSB_LAUNCH(kern, m.nCell, 128, st, m.nCell, A(), x, Ax, gamma - 1, xs);
+    }
+
+    // y = M^-1 A (xs x); one symmetric sweep on the scalar-Jacobian operator takes product and sweep together
+    void MA(const T *x, T *y, const real *xs) const
+    {
+        T *tmp = (T *)w.tmp;
+        if (w.jacMode || ls.jacobiCode != 1 || ls.sgsIter != 0)
+        {
+            FA(x, tmp, xs);
+            FML(tmp, y);
+            return;
+        }
+        auto kf = posop::k_product_forward<T, NV, NF>;
+        for (int col = 0; col < m.nColor; col++)
+            DNDSB_LAUNCH(kf, m.colorStart[col + 1] - m.colorStart[col], 128, st, m.colorStart[col], m.colorStart[col + 1], A(), x, tmp, y, gamma - 1,
+                         xs);
+        back(y);
     }
 
     void body() const
@@ -803,7 +696,7 @@ struct Solve
             return;
         // GMRES_LeftPreconditioned::solve (Linear.hpp:46-133)
         int k = ls.nGmresSpace;
-        T *MLb = (T *)w.MLb, *tmp = (T *)w.tmp;
+        T *MLb = (T *)w.MLb;
         FML(b, MLb);
         krylov_norm(prec(), nn, NV, MLb, w.s2, w.red, w.sc + 0, w.cnt, st); // scale
         for (int r = 0; r < ls.nGmresIter; r++)
@@ -816,8 +709,7 @@ struct Solve
             }
             else
             {
-                FA(x, tmp);
-                FML(tmp, V(0));
+                MA(x, V(0), nullptr);
                 krylov_diff_norm(prec(), nn, NV, V(0), MLb, w.s2, w.red, w.sc + 1, w.cnt, st);
                 DNDSB_LAUNCH(k_gmres_v0<T>, nn, 256, st, nn, V(0), MLb, V(0), w.sc, 0);
             }
@@ -825,8 +717,7 @@ struct Solve
             for (int j = 0; j < k; j++)
             {
                 // the basis columns stay unnormalised: v_j = colScale[j] V(j), the factor applied by each reader
-                FA(V(j), tmp, w.colScale + j);
-                FML(tmp, V(j + 1));
+                MA(V(j), V(j + 1), w.colScale + j);
                 real *hcol = w.H + (int64_t)j * (k + 1);
                 // classical Gram-Schmidt: h = V^T w, w -= V h, h[j+1] = |w|, colScale[j+1] = 1 / h[j+1]
                 krylov_mdot(prec(), nn, ld(), NV, j + 1, w.V, V(j + 1), w.s2, w.red, hcol, w.colScale, w.cnt, st);
@@ -845,17 +736,17 @@ template <typename T, int NV, int NF>
 int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &w, const LinSettings &ls, real alphaDiag, const real *dTau,
         real dt, const real *u, const real *rhs, real *xInc, cudaStream_t st)
 {
-    using T4 = typename Vec4<T>::type;
     // the caller's stream -> the solver's stream
     event_record(w.evIn, st);
     stream_wait(w.cs, w.evIn);
     cudaStream_t cs = w.cs;
     h2d(w.s2, ls.scale2, sizeof(real) * 8, cs);
-    auto kbuild = k_sgsop_build<T, NV>;
+    auto kbuild = posop::k_build<T, NV, NF>;
     auto kgather = k_gather_T<T, NV>;
     auto kscatter = k_scatter_T<T, NV>;
     if (NV == 6 && !ev.jSource)
         return ST_BADARG;
+    Solve<T, NV, NF> S{m, w, ls, (T)ev.s.gamma, cs};
     if (w.jacMode)
     {
         if (w.jacMode == 2 && (!ev.lambdaFace0 || (m.nBndFace > 0 && !bnd.type)))
@@ -874,10 +765,8 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         }
     }
     else
-        DNDSB_LAUNCH(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, u, ev.jSource, w.cellPos, w.nbrPos, (T4 *)w.op,
-                     (T *)w.jd, (T *)w.uT);
+        DNDSB_LAUNCH(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
     DNDSB_LAUNCH(kgather, m.nCell, 256, cs, m.nCell, m.colorCells, rhs, (T *)w.rhsT);
-    Solve<T, NV, NF> S{m, w, ls, (T)ev.s.gamma, cs};
     if (ls.useGraph)
     {
         if (!(w.graph && w.keyValid && same_key(w.key, ls)))
