@@ -2,6 +2,7 @@
 // partition into kRedBlocks chunks, a fixed shared-memory tree per chunk and
 // a single-block final pass, so results do not depend on scheduling.
 #include "solver.cuh"
+#include "krylov_update.cuh"
 
 namespace dndsb
 {
@@ -167,15 +168,15 @@ DNDSB_D real warp_sum(real x)
     return x;
 }
 
-constexpr int kKG = 8; // columns per pass of the multi-dot
+constexpr int kKG = 8; // most columns a block of the multi-dot takes
 
-// Called by every block after it has written its partials [block][ncol]: the block that arrives last
+// Called by every block after it has written its partials [nb][ncol]: the block that arrives last
 // (a ticket on *cnt, which it resets for the next launch) sums them per column in a fixed order (lanes
 // over a fixed stride of the blocks, then a fixed xor tree, lane 0's value), the order the separate
 // final pass used, so the result does not depend on which block finishes last.  out[col] = the sum
 // (its square root with takeSqrt) times colScale[col] (when given).  Returns true in that block
 // (uniformly over its threads).
-DNDSB_D bool last_block_final(int ncol, const real *partial, real *out, const real *colScale, int takeSqrt, unsigned *cnt)
+DNDSB_D bool last_block_final(int nb, int ncol, const real *partial, real *out, const real *colScale, int takeSqrt, unsigned *cnt)
 {
     __shared__ unsigned ticket;
     __threadfence();
@@ -190,7 +191,7 @@ DNDSB_D bool last_block_final(int ncol, const real *partial, real *out, const re
     for (int col = wid; col < ncol; col += nw)
     {
         real a = 0;
-        for (int i = lane; i < (int)gridDim.x; i += 32)
+        for (int i = lane; i < nb; i += 32)
             a += __ldcg(partial + (int64_t)i * ncol + col);
         a = warp_sum(a);
         if (lane == 0)
@@ -205,12 +206,54 @@ DNDSB_D bool last_block_final(int ncol, const real *partial, real *out, const re
     return true;
 }
 
-// partial[block][col] = sum_i V[col][i] w[i] s2[i % NV] over the block's chunk of quads.  Columns are
-// ld apart (ld a multiple of 4, the pad beyond n zero); all columns of a pass share one read of w.
-// out[col] = partial sums reduced by the last block, times colScale[col] (the basis columns are stored
-// unnormalised; colScale holds their normalising factors)
+// sums of NK columns from V against w over the quads [q0, q1): warp sums into sh[column][warp]
+template <typename T, int NV, int NK>
+DNDSB_D void mdot_group(int64_t q0, int64_t q1, int64_t ld, const T *__restrict__ V, const T *__restrict__ w, const real *ss,
+                        real (*sh)[kRedBlock / 32])
+{
+    real a[NK];
+#pragma unroll
+    for (int k = 0; k < NK; k++)
+        a[k] = 0;
+    // r = (4 q) % NV, advanced incrementally with q
+    const int dr = (int)((4 * (int64_t)blockDim.x) % NV);
+    int r = (int)((4 * (q0 + threadIdx.x)) % NV);
+    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x)
+    {
+        // every load issued (in its storage type) before the first use
+        typename Quad<T>::raw v[NK];
+#pragma unroll
+        for (int k = 0; k < NK; k++)
+            v[k] = Quad<T>::load_raw(V + k * ld + 4 * q);
+        real wv[4];
+        Quad<T>::load(w + 4 * q, wv);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            wv[e] *= ss[r + e < NV ? r + e : r + e - NV];
+        r += dr;
+        r = r >= NV ? r - NV : r;
+#pragma unroll
+        for (int k = 0; k < NK; k++)
+            a[k] += Quad<T>::dot(v[k], wv);
+    }
+#pragma unroll
+    for (int k = 0; k < NK; k++)
+    {
+        const real x = warp_sum(a[k]);
+        if ((threadIdx.x & 31) == 0)
+            sh[k][threadIdx.x >> 5] = x;
+    }
+}
+
+// out[col] = colScale[col] sum_i V[col][i] w[i] s2[i % NV] (the basis columns are stored unnormalised; colScale holds
+// their normalising factors).  Columns are ld apart (ld a multiple of 4, the pad beyond n zero).
+// HBM bound on the basis.  The kRedBlocks blocks split into nG groups of at most kKG columns (their widths differ by
+// at most one) times chunks of quads, block = chunk nG + group, so the blocks of a chunk share its w in L2 and every
+// block makes one pass: 592 blocks that each walked all column groups over a chunk of 592 paid a block reduction per
+// group for one or two quads per thread (30 steps of 249,600 tets in FP64: 1.30 -> 1.08 ms).  partial [chunks][ncol]; the
+// last block to finish sums the chunks.
 template <typename T, int NV>
-DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld, int ncol, const T *__restrict__ V, const T *__restrict__ w,
+DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld, int ncol, int nG, const T *__restrict__ V, const T *__restrict__ w,
                                                        const real *__restrict__ s2, real *partial, real *out, const real *colScale,
                                                        unsigned *cnt)
 {
@@ -219,70 +262,32 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
     if (threadIdx.x < NV)
         ss[threadIdx.x] = s2[threadIdx.x];
     __syncthreads();
-    const int64_t nq = (n + 3) >> 2, cq = (nq + gridDim.x - 1) / gridDim.x;
-    const int64_t q0 = blockIdx.x * cq, q1 = q0 + cq < nq ? q0 + cq : nq;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c0 = 0; c0 < ncol; c0 += kKG)
+    const int grp = blockIdx.x % nG, chunk = blockIdx.x / nG, nChunk = gridDim.x / nG;
+    const int base = ncol / nG, extra = ncol - base * nG; // the first `extra` groups have one column more
+    const int c0 = grp * base + (grp < extra ? grp : extra), nk = base + (grp < extra ? 1 : 0);
+    const int64_t nq = (n + 3) >> 2, cq = (nq + nChunk - 1) / nChunk;
+    const int64_t q0 = chunk * cq, q1 = q0 + cq < nq ? q0 + cq : nq;
+    const T *Vc = V + (int64_t)c0 * ld;
+    switch (nk)
     {
-        real a[kKG];
-#pragma unroll
-        for (int k = 0; k < kKG; k++)
-            a[k] = 0;
-        // r = (4 q) % NV, advanced incrementally with q
-        const int dr = (int)((4 * (int64_t)blockDim.x) % NV);
-        int r = (int)((4 * (q0 + threadIdx.x)) % NV);
-        const T *Vc = V + (int64_t)c0 * ld;
-        for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x)
-        {
-            real wv[4];
-            Quad<T>::load(w + 4 * q, wv);
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                wv[e] *= ss[r + e < NV ? r + e : r + e - NV];
-            r += dr;
-            r = r >= NV ? r - NV : r;
-            const T *pv = Vc + 4 * q;
-            if (c0 + kKG <= ncol)
-            {
-                // a full group: every load issued (in its storage type) before the first use
-                typename Quad<T>::raw v[kKG];
-#pragma unroll
-                for (int k = 0; k < kKG; k++)
-                    v[k] = Quad<T>::load_raw(pv + k * ld);
-#pragma unroll
-                for (int k = 0; k < kKG; k++)
-                    a[k] += Quad<T>::dot(v[k], wv);
-            }
-            else
-            {
-#pragma unroll
-                for (int k = 0; k < kKG; k++)
-                    if (c0 + k < ncol)
-                    {
-                        real v[4];
-                        Quad<T>::load(pv + k * ld, v);
-                        a[k] += v[0] * wv[0] + v[1] * wv[1] + v[2] * wv[2] + v[3] * wv[3];
-                    }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kKG; k++)
-        {
-            real x = warp_sum(a[k]);
-            if (lane == 0)
-                sh[k][wid] = x;
-        }
-        __syncthreads();
-        if (threadIdx.x < kKG && c0 + (int)threadIdx.x < ncol)
-        {
-            real t = 0;
-            for (int q = 0; q < nw; q++)
-                t += sh[threadIdx.x][q];
-            partial[blockIdx.x * ncol + c0 + threadIdx.x] = t;
-        }
-        __syncthreads();
+    case 1: mdot_group<T, NV, 1>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 2: mdot_group<T, NV, 2>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 3: mdot_group<T, NV, 3>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 4: mdot_group<T, NV, 4>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 5: mdot_group<T, NV, 5>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 6: mdot_group<T, NV, 6>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 7: mdot_group<T, NV, 7>(q0, q1, ld, Vc, w, ss, sh); break;
+    default: mdot_group<T, NV, 8>(q0, q1, ld, Vc, w, ss, sh); break;
     }
-    last_block_final(ncol, partial, out, colScale, 0, cnt);
+    __syncthreads();
+    if ((int)threadIdx.x < nk)
+    {
+        real t = 0;
+        for (int q = 0; q < (int)(blockDim.x >> 5); q++)
+            t += sh[threadIdx.x][q];
+        partial[(int64_t)chunk * ncol + c0 + threadIdx.x] = t;
+    }
+    last_block_final(nChunk, ncol, partial, out, colScale, 0, cnt);
 }
 
 // w -= sum_c h[c] colScale[c] V[c] (columns subtracted in index order); the last block writes
@@ -356,13 +361,60 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
             t += sh[q];
         partial[blockIdx.x] = t;
     }
-    if (last_block_final(1, partial, outNorm, nullptr, 1, cnt) && gsc && threadIdx.x == 0)
+    if (last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt) && gsc && threadIdx.x == 0)
     {
         real hn = *outNorm;
         bool broken = !(hn > gsc[0] * 1e-32) || gsc[2] <= j;
         *scaleNext = broken ? 0.0 : 1.0 / hn;
         if (broken && gsc[2] > j)
             gsc[2] = j;
+    }
+}
+
+// x += sum_c y_c colScale_c V_c over the valid columns (gsc[2], at most k), y = gsc[yOff ...].  HBM bound on the
+// basis: quads of a column as in the multi-dot, four columns in flight (one element per thread and column at a time
+// took 371 us at 2 million cells, FP32; now 185).  x needs no alignment or pad: its ragged end goes by elements.
+template <typename T>
+DNDSB_GLOBAL void __launch_bounds__(kRedBlock) k_kupdate(int64_t n, int64_t ld, int k, const T *__restrict__ V, const real *__restrict__ gsc, int yOff,
+                                                        const real *__restrict__ colScale, T *x)
+{
+    __shared__ real hs[32];
+    const int nv = dmin(gsc[2], k);
+    if ((int)threadIdx.x < nv)
+        hs[threadIdx.x] = gsc[yOff + threadIdx.x] * colScale[threadIdx.x];
+    __syncthreads();
+    DNDSB_KERNEL_LOOP(q, (n + 3) >> 2)
+    {
+        const int m = n - 4 * q < 4 ? (int)(n - 4 * q) : 4;
+        real a[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            a[e] = e < m ? (real)x[4 * q + e] : 0.0;
+        int c = 0;
+        for (; c + 4 <= nv; c += 4)
+        {
+            real v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                Quad<T>::load(V + (int64_t)(c + i) * ld + 4 * q, v[i]);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    a[e] += hs[c + i] * v[i][e];
+        }
+        for (; c < nv; c++)
+        {
+            real v[4];
+            Quad<T>::load(V + (int64_t)c * ld + 4 * q, v);
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                a[e] += hs[c] * v[e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (e < m)
+                x[4 * q + e] = (T)a[e];
     }
 }
 
@@ -382,7 +434,7 @@ DNDSB_GLOBAL void k_knorm2(int64_t n, const T *__restrict__ x, const real *__res
     block_sum4(sh, a, 0, 0, 0);
     if (threadIdx.x == 0)
         partial[blockIdx.x] = sh[0][0];
-    last_block_final(1, partial, outNorm, nullptr, 1, cnt);
+    last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt);
 }
 
 // partial[block] = sum_i (a_i - b_i)^2 s2[i % NV]
@@ -402,14 +454,15 @@ DNDSB_GLOBAL void k_kdiff_norm(int64_t n, const T *__restrict__ x, const T *__re
     block_sum4(sh, a, 0, 0, 0);
     if (threadIdx.x == 0)
         partial[blockIdx.x] = sh[0][0];
-    last_block_final(1, partial, outNorm, nullptr, 1, cnt);
+    last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt);
 }
 
 template <typename T, int NV>
 void kmdot(int64_t n, int64_t ld, int ncol, const void *V, const void *w, const real *s2, real *red, real *out, const real *colScale,
            unsigned *cnt, cudaStream_t st)
 {
-    k_kmdot<T, NV><<<kRedBlocks, kRedBlock, 0, st>>>(n, ld, ncol, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
+    const int nG = (ncol + kKG - 1) / kKG;
+    k_kmdot<T, NV><<<kRedBlocks / nG * nG, kRedBlock, 0, st>>>(n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
 }
 
 template <typename T, int NV>
@@ -457,6 +510,15 @@ void krylov_maxpy_norm(int prec, int64_t n, int64_t ld, int nv, int ncol, const 
                        const real *s2, real *red, real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st)
 {
     DNDSB_KDISPATCH(kmaxpy, n, ld, ncol, V, h, colScale, w, s2, red, outNorm, cnt, gsc, j, scaleNext, st);
+}
+
+void krylov_update_x(int prec, int64_t n, int k, const void *V, const real *gsc, int yOff, const real *colScale, void *x, cudaStream_t st)
+{
+    const int64_t nq = (n + 3) >> 2;
+    if (prec)
+        DNDSB_LAUNCH(k_kupdate<float>, nq, kRedBlock, st, n, krylov_ld(n), k, (const float *)V, gsc, yOff, colScale, (float *)x);
+    else
+        DNDSB_LAUNCH(k_kupdate<double>, nq, kRedBlock, st, n, krylov_ld(n), k, (const double *)V, gsc, yOff, colScale, (double *)x);
 }
 
 void krylov_norm(int prec, int64_t n, int nv, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st)
