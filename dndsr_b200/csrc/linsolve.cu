@@ -73,27 +73,6 @@ DNDSB_GLOBAL void k_zero_T(int64_t n, T *x)
     x[i] = (T)0;
 }
 
-template <typename T>
-DNDSB_GLOBAL void k_copy_T(int64_t n, const T *__restrict__ a, T *b)
-{
-    DNDSB_KERNEL_LOOP(i, n)
-    b[i] = a[i];
-}
-
-template <typename T>
-DNDSB_GLOBAL void k_sub_T(int64_t n, const T *__restrict__ a, const T *__restrict__ b, T *c) // c = a - b
-{
-    DNDSB_KERNEL_LOOP(i, n)
-    c[i] = a[i] - b[i];
-}
-
-template <typename T>
-DNDSB_GLOBAL void k_add_T(int64_t n, const T *__restrict__ a, T *b) // b += a
-{
-    DNDSB_KERNEL_LOOP(i, n)
-    b[i] += a[i];
-}
-
 // block operator build.  Storage is tiled by 32 positions (ilu::BlockLay, s = 5): element k NV NV + e of a position's
 // row of opB is element e of slot k's off-diagonal block (zero on boundaries); elements e and NV NV + e of jdB are
 // the diagonal block and its inverse.  A warp reads one element of its 32 positions as one 256-byte line
@@ -273,47 +252,6 @@ DNDSB_GLOBAL void k_sgs_pos_blk(int64_t n, int64_t pBeg, int64_t pEnd, const int
     }
 }
 
-template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_matvec_pos_blk(int64_t n, const int32_t *__restrict__ nbrPos, const T *__restrict__ opB, const T *__restrict__ jdB,
-                                   const T *__restrict__ x, T *Ax, const real *__restrict__ xs)
-{
-    constexpr int NN = NV * NV;
-    const ilu::BlockLay oL{NF * NN, 5}, dL{2 * NN, 5};
-    const T sx = xs ? (T)*xs : T(1);
-    DNDSB_KERNEL_LOOP(p, n)
-    {
-        T xp[NV], y[NV];
-        for (int l = 0; l < NV; l++)
-            xp[l] = x[p * NV + l];
-        for (int r = 0; r < NV; r++)
-        {
-            T acc = 0;
-            for (int l = 0; l < NV; l++)
-                acc += jdB[dL.at(p, r * NV + l)] * xp[l];
-            y[r] = acc;
-        }
-#pragma unroll
-        for (int k = 0; k < NF; k++)
-        {
-            int q = nbrPos[p * NF + k];
-            if (q < 0)
-                continue;
-            T xq[NV];
-            for (int l = 0; l < NV; l++)
-                xq[l] = x[(int64_t)q * NV + l];
-            for (int r = 0; r < NV; r++)
-            {
-                T acc = 0;
-                for (int l = 0; l < NV; l++)
-                    acc += opB[oL.at(p, k * NN + r * NV + l)] * xq[l];
-                y[r] += acc;
-            }
-        }
-        for (int v = 0; v < NV; v++)
-            Ax[p * NV + v] = sx * y[v];
-    }
-}
-
 // GMRES bookkeeping kernels on device scalars.  sc layout: [0] scale = |M b|,
 // [1] beta, [2] number of valid Arnoldi columns, [8 ...] least-squares y.
 constexpr int kScY = 8;
@@ -432,7 +370,7 @@ struct LinWs
     void *rhsT = nullptr, *x = nullptr, *tmp = nullptr, *tmp2 = nullptr, *MLb = nullptr, *V = nullptr;
     real *H = nullptr, *sc = nullptr, *s2 = nullptr, *red = nullptr;
     void *opB = nullptr, *jdB = nullptr; // block mode: off-diagonal blocks [nCell][nf][nv][nv], diagonal blocks + inverses [nCell][2][nv][nv]
-    void *luB = nullptr, *luD = nullptr, *tmp3 = nullptr; // jacobiCode 2: ILU(0) slot blocks, inverted pivots, scratch
+    void *luB = nullptr, *luD = nullptr; // jacobiCode 2: ILU(0) slot blocks, inverted pivots
     int32_t *luNbr = nullptr, *luNLow = nullptr;          // the factors' compact slot order: neighbour positions, lower count
     real *colScale = nullptr; // [33] normalising factors of the stored (unnormalised) Krylov columns
     unsigned *cnt = nullptr;  // ticket counter of the one-launch reductions (zero between launches)
@@ -447,7 +385,7 @@ void linws_free(LinWs *w)
 {
     if (!w)
         return;
-    for (void *p : {(void *)w->cellPos, (void *)w->nbrPos, w->op, w->jd, w->opB, w->jdB, w->luB, w->luD, w->tmp3, (void *)w->luNbr,
+    for (void *p : {(void *)w->cellPos, (void *)w->nbrPos, w->op, w->jd, w->opB, w->jdB, w->luB, w->luD, (void *)w->luNbr,
                     (void *)w->luNLow, w->jdi, w->vh, w->opNu, (void *)w->opCnt, w->rhsT, w->x, w->tmp, w->tmp2, w->MLb, w->V, (void *)w->H,
                     (void *)w->sc, (void *)w->s2, (void *)w->red, (void *)w->colScale, (void *)w->cnt})
         dev_free(p);
@@ -503,7 +441,7 @@ int ws_prepare(const MeshD &m, LinWs *&w, const LinSettings &ls, int nv, int jac
         ok = dev_alloc(&w->opB, es * nv * nv * nPad * m.nf) == cudaSuccess && dev_alloc(&w->jdB, es * 2 * nv * nv * nPad) == cudaSuccess;
     if (ok && jacMode && ls.jacobiCode == 2)
         ok = dev_alloc(&w->luB, es * nv * nv * nPad * m.nf) == cudaSuccess && dev_alloc(&w->luD, es * nv * nv * nPad) == cudaSuccess &&
-             dev_alloc(&w->tmp3, es * n) == cudaSuccess && dev_alloc((void **)&w->luNbr, sizeof(int32_t) * m.nCell * m.nf) == cudaSuccess &&
+             dev_alloc((void **)&w->luNbr, sizeof(int32_t) * m.nCell * m.nf) == cudaSuccess &&
              dev_alloc((void **)&w->luNLow, sizeof(int32_t) * m.nCell) == cudaSuccess;
     ok = ok && dev_zero(w->V, es * krylov_ld(n) * (k + 1), nullptr) == cudaSuccess; // the column pads stay zero
     ok = ok && dev_zero(w->cnt, sizeof(unsigned), nullptr) == cudaSuccess && dev_zero(w->colScale, sizeof(real) * 33, nullptr) == cudaSuccess;
@@ -590,29 +528,37 @@ struct Solve
     // x += (LU)^-1 (rhs - A x) (x = (LU)^-1 rhs from a zero input)
     void ilu_pair(const T *rhs, T *x, bool zeroIn) const
     {
-        int64_t nn = n();
-        T *r = (T *)w.tmp2, *ax = (T *)w.tmp3;
+        T *r = (T *)w.tmp2;
+        auto kl = ilu::k_ilu_lower_c<T, NV, NF>;
+        auto ku = ilu::k_ilu_upper_c<T, NV, NF>;
+        const ilu::BlockLay lay{NF * NV * NV, 5}, dlay{NV * NV, 5};
         for (int it = 0; it < 2; it++)
         {
-            bool zero = zeroIn && it == 0;
+            const bool zero = zeroIn && it == 0;
             T *y = zero ? x : r;
             if (!zero)
-            {
-                FA(x, ax);
-                DNDSB_LAUNCH(k_sub_T<T>, nn, 256, st, nn, rhs, (const T *)ax, r);
-            }
-            auto kl = ilu::k_ilu_lower_c<T, NV, NF>;
-            auto ku = ilu::k_ilu_upper_c<T, NV, NF>;
-            const ilu::BlockLay lay{NF * NV * NV, 5}, dlay{NV * NV, 5};
+                product_blk(x, r, nullptr, rhs);
             for (int ci = 0; ci < m.nColor; ci++)
-                DNDSB_LAUNCH(kl, m.colorStart[ci + 1] - m.colorStart[ci], 128, st, m.colorStart[ci], m.colorStart[ci + 1], (const int32_t *)w.luNbr,
-                             (const int32_t *)w.luNLow, (const T *)w.luB, lay, zero ? rhs : (const T *)r, y);
+            {
+                const int64_t b = m.colorStart[ci], e = m.colorStart[ci + 1];
+                if (e > b)
+                    kl<<<ilu::tile_blocks(b, e), 32 * NV, 0, st>>>(b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, zero ? rhs : (const T *)r, y);
+            }
             for (int ci = m.nColor - 1; ci >= 0; ci--)
-                DNDSB_LAUNCH(ku, m.colorStart[ci + 1] - m.colorStart[ci], 128, st, m.colorStart[ci], m.colorStart[ci + 1], (const int32_t *)w.luNbr,
-                             (const int32_t *)w.luNLow, (const T *)w.luB, lay, (const T *)w.luD, dlay, y);
-            if (!zero)
-                DNDSB_LAUNCH(k_add_T<T>, nn, 256, st, nn, (const T *)r, x);
+            {
+                const int64_t b = m.colorStart[ci], e = m.colorStart[ci + 1];
+                if (e > b)
+                    ku<<<ilu::tile_blocks(b, e), 32 * NV, 0, st>>>(b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, (const T *)w.luD, dlay, y,
+                                                                  zero ? (T *)nullptr : x);
+            }
         }
+    }
+
+    // y = A (xs x) of the block operator, or rhs - A x
+    void product_blk(const T *x, T *y, const real *xs, const T *rhs) const
+    {
+        ilu::k_block_product<T, NV, NF><<<ilu::tile_blocks(0, m.nCell), 32 * NV, 0, st>>>(m.nCell, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, x, y,
+                                                                                        xs, rhs);
     }
 
     // doPrecondition (EulerSolver.hxx:1605-1635): forward then backward sweep; x in, x out (ping-pong through tmp2)
@@ -646,8 +592,7 @@ struct Solve
     {
         if (w.jacMode)
         {
-            auto kb = k_matvec_pos_blk<T, NV, NF>;
-            DNDSB_LAUNCH(kb, m.nCell, 128, st, m.nCell, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, x, Ax, xs);
+            product_blk(x, Ax, xs, nullptr);
             return;
         }
         auto kern = posop::k_product<T, NV, NF>;
