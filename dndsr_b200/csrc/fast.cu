@@ -1,4 +1,4 @@
-// Tuned kernels of the two dominant operators.
+// Tuned face kernel of the right-hand side.
 //
 // RHS face flux: one thread per (face, Gauss point), 32 faces per block.  The
 // reconstruction data of the 64 cells adjacent to the block's faces (uRec,
@@ -8,11 +8,6 @@
 // summed in a fixed order, so results are deterministic.  The basis and its
 // first derivatives are generated from compile-time exponent tables, so the
 // sparse derivative rows cost only their non-zero terms.
-//
-// VR Jacobi sweep: R threads per cell (one output row each), 32 cells per
-// block.  Each thread streams its rows of the A^-1 B_k blocks once (coalesced
-// across the cell's threads) while the neighbour reconstructions are staged
-// in shared memory face by face.
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "sa.cuh"
@@ -262,79 +257,6 @@ DNDSB_GLOBAL void k_cell_par(int64_t nCell, int aniso, const real *__restrict__ 
     }
 }
 
-// VR Jacobi sweep, R threads per cell (VariationalReconstruction_Reconstruction.hxx:485-615).
-// Coefficients come from the packed, transposed stream coefT[cell][face][j][i] (j < R: A^-1 B
-// entry (i, j); j = R: A^-1 b entry i), so for each j the R threads of a cell read R consecutive
-// values (one or two L1 lines per cell instead of a strided row each).  The neighbour's uRec
-// block and mean are read as broadcasts: the R threads of a cell share each line through L1.
-// No barriers; the next face's coefficients are loaded while the current face is applied.
-template <int R, int NV, typename TC>
-__global__ void __launch_bounds__(32 * R, 2) k_vr_jacobi_fast(int64_t nCell, int nf, const int32_t *__restrict__ nbr, const TC *__restrict__ coefT,
-                                                           const real *__restrict__ uRec, real *__restrict__ uRecNew, const real *__restrict__ u,
-                                                           real relax, int recordInc, int uRecIsZero)
-{
-    const int tid = threadIdx.x;
-    const int cl = tid / R, i = tid - cl * R;
-    const int64_t c = (int64_t)blockIdx.x * 32 + cl;
-    if (c >= nCell)
-        return;
-    real acc[NV], ui[NV];
-#pragma unroll
-    for (int v = 0; v < NV; v++)
-    {
-        real x = uRec[(c * R + i) * NV + v];
-        acc[v] = recordInc ? (uRecIsZero ? 0.0 : x) : x * (1 - relax);
-        ui[v] = u[c * NV + v];
-    }
-    const real sgn = recordInc ? -1.0 : relax;
-    const bool useRec = !(recordInc && uRecIsZero);
-    const TC *cb = coefT + c * nf * (R + 1) * R + i; // entry (face k, j) at cb[(k (R+1) + j) R]
-    TC Mcur[R + 1], Mnext[R + 1];
-#pragma unroll
-    for (int j = 0; j <= R; j++)
-        Mcur[j] = (useRec || j == R) ? cb[j * R] : TC(0);
-    for (int k = 0; k < nf; k++)
-    {
-        if (k + 1 < nf)
-        {
-#pragma unroll
-            for (int j = 0; j <= R; j++)
-                Mnext[j] = (useRec || j == R) ? cb[((k + 1) * (R + 1) + j) * R] : TC(0);
-        }
-        int o = nbr[c * nf + k];
-        if (o >= 0)
-        {
-            real t[NV];
-            const real *rr = uRec + (int64_t)o * R * NV;
-            const real *uo = u + (int64_t)o * NV;
-            const real bi = (real)Mcur[R];
-#pragma unroll
-            for (int v = 0; v < NV; v++)
-                t[v] = bi * (uo[v] - ui[v]);
-            if (useRec)
-            {
-#pragma unroll
-                for (int j = 0; j < R; j++)
-                {
-                    const real mij = (real)Mcur[j];
-#pragma unroll
-                    for (int v = 0; v < NV; v++)
-                        t[v] += mij * rr[j * NV + v];
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < NV; v++)
-                acc[v] += sgn * t[v];
-        }
-#pragma unroll
-        for (int j = 0; j <= R; j++)
-            Mcur[j] = Mnext[j];
-    }
-#pragma unroll
-    for (int v = 0; v < NV; v++)
-        uRecNew[(c * R + i) * NV + v] = acc[v];
-}
-
 template <int DIM, int P, int NV, int NG>
 int launch_rhs_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, const real *u, const real *uRec, real *ff, cudaStream_t st)
 {
@@ -445,57 +367,5 @@ int rhs_face_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev
     if (vr.P == 2)
         return dispatch_ng<3, 2>(g.nGf, m, g, vr, ev, u, uRec, ff, st);
     return dispatch_ng<3, 3>(g.nGf, m, g, vr, ev, u, uRec, ff, st);
-}
-
-int vr_iter_fast(const MeshD &m, const VRD &vr, int nv, const real *uRec, real *uRecNew, const real *u, int recordInc, int uRecIsZero,
-                 int useFP32, cudaStream_t st)
-{
-    if ((nv != 5 && nv != 6) || !vr.sweepCoef)
-        return ST_UNSUPPORTED;
-    if (nv == 6)
-    {
-        // the SA model at degree 1 in 3-D (R = 3)
-        if (vr.R != 3)
-            return ST_UNSUPPORTED;
-        unsigned nb6 = (unsigned)((m.nCell + 31) / 32);
-        if (useFP32)
-            k_vr_jacobi_fast<3, 6, float><<<nb6, 32 * 3, 0, st>>>(m.nCell, m.nf, m.cellNbr, vr.sweepCoef32, uRec, uRecNew, u, vr.s.jacobiRelax,
-                                                                 recordInc, uRecIsZero);
-        else
-            k_vr_jacobi_fast<3, 6, real><<<nb6, 32 * 3, 0, st>>>(m.nCell, m.nf, m.cellNbr, vr.sweepCoef, uRec, uRecNew, u, vr.s.jacobiRelax,
-                                                                recordInc, uRecIsZero);
-        return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
-    }
-    unsigned nb = (unsigned)((m.nCell + 31) / 32);
-    real relax = vr.s.jacobiRelax;
-#define DNDSB_VRF(RR)                                                                                                                       \
-    do                                                                                                                                      \
-    {                                                                                                                                       \
-        if (useFP32)                                                                                                                        \
-            k_vr_jacobi_fast<RR, 5, float><<<nb, 32 * RR, 0, st>>>(m.nCell, m.nf, m.cellNbr, vr.sweepCoef32, uRec, uRecNew, u, relax,      \
-                                                                   recordInc, uRecIsZero);                                                  \
-        else                                                                                                                                \
-            k_vr_jacobi_fast<RR, 5, real><<<nb, 32 * RR, 0, st>>>(m.nCell, m.nf, m.cellNbr, vr.sweepCoef, uRec, uRecNew, u, relax,         \
-                                                                  recordInc, uRecIsZero);                                                   \
-    } while (0)
-    switch (vr.R)
-    {
-    case 2:
-        DNDSB_VRF(2);
-        break;
-    case 3:
-        DNDSB_VRF(3);
-        break;
-    case 5:
-        DNDSB_VRF(5);
-        break;
-    case 9:
-        DNDSB_VRF(9);
-        break;
-    default:
-        return ST_UNSUPPORTED;
-    }
-#undef DNDSB_VRF
-    return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 } // namespace dndsb

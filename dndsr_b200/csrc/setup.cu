@@ -5,6 +5,7 @@
 // Follows CFV/FiniteVolume.cpp:22-648 (metrics), VariationalReconstruction.cpp
 // :56-498 (ConstructBaseAndWeight) and :507-872 (ConstructRecCoeff).
 #include "solver.cuh"
+#include "sweep_layout.cuh"
 #include "basis_eval.cuh"
 
 namespace dndsb
@@ -477,20 +478,22 @@ DNDSB_GLOBAL void k_vr_coeff(MeshD m, GeomD g, VRD vr, int *err)
     }
 }
 
-// packed sweep coefficients [cell][face k][j][i]: entry (i, j) of A^-1 B_k for j < R, (A^-1 b_k)_i for j = R
-DNDSB_GLOBAL void k_pack_sweep(int64_t nCell, int nf, int R, const real *__restrict__ AAInvB, const real *__restrict__ AInvb, real *out,
-                               float *out32)
+// packed sweep coefficients in the layout of sweep_layout.cuh
+DNDSB_GLOBAL void k_pack_sweep(int64_t nCell, int64_t nPad, int tiled, int nf, int R, const real *__restrict__ AAInvB, const real *__restrict__ AInvb,
+                               real *out, float *out32)
 {
     const int64_t per = (int64_t)nf * R * (R + 1);
-    DNDSB_KERNEL_LOOP(e, nCell * per)
+    DNDSB_KERNEL_LOOP(e, nPad * per)
     {
-        int64_t c = e / per;
-        int r = (int)(e - c * per);
-        // layout [cell][face k][j][i]: j < R is column j of A^-1 B_k, j = R is A^-1 b_k
+        const int64_t t = tiled ? e >> 5 : e;
+        const int64_t c = tiled ? t / per * 32 + (e & 31) : t / per;
+        const int r = (int)(t % per);
         int k = r / (R * (R + 1));
         int rem = r - k * R * (R + 1);
         int j = rem / R, i = rem - j * R;
-        real v = j < R ? AAInvB[((c * (nf + 1) + 1 + k) * R + i) * R + j] : AInvb[(c * nf + k) * R + i];
+        real v = 0;
+        if (c < nCell)
+            v = j < R ? AAInvB[((c * (nf + 1) + 1 + k) * R + i) * R + j] : AInvb[(c * nf + k) * R + i];
         out[e] = v;
         out32[e] = (float)v;
     }
@@ -629,12 +632,14 @@ int vr_construct_rec_coeff(const MeshD &m, const GeomD &g, VRD &vr, int *errWord
     DNDSB_LAUNCH(k_to_f32, nA, 256, st, nA, vr.AAInvB, vr.AAInvB32);
     DNDSB_LAUNCH(k_to_f32, nb, 256, st, nb, vr.AInvb, vr.AInvb32);
     {
-        int64_t nS = m.nCell * m.nf * R * (R + 1);
+        const bool tiled = sweep_tiled(R, m.nCell);
+        const int64_t nPad = tiled ? (m.nCell + 31) / 32 * 32 : m.nCell;
+        int64_t nS = nPad * m.nf * R * (R + 1);
         dev_free(vr.sweepCoef), dev_free(vr.sweepCoef32);
         vr.sweepCoef = nullptr, vr.sweepCoef32 = nullptr;
         if (alloc_real(&vr.sweepCoef, nS) || dev_alloc((void **)&vr.sweepCoef32, sizeof(float) * nS) != cudaSuccess)
             return ST_CUDA;
-        DNDSB_LAUNCH(k_pack_sweep, nS, 256, st, m.nCell, m.nf, R, vr.AAInvB, vr.AInvb, vr.sweepCoef, vr.sweepCoef32);
+        DNDSB_LAUNCH(k_pack_sweep, nS, 256, st, m.nCell, nPad, (int)tiled, m.nf, R, vr.AAInvB, vr.AInvb, vr.sweepCoef, vr.sweepCoef32);
     }
     int e = 0;
     d2h(&e, errWord, sizeof(int), st);
