@@ -16,7 +16,7 @@ extern template void coords_lanes_launch<2>(const MeshD &, const GeomD &, const 
 
 namespace
 {
-// dX[n] = sum of the shares of node n, in (cell, slot) order
+// dX[n] = sum of the shares of node n, in (face, slot) order
 DNDSB_GLOBAL void k_node_gather(int64_t nNode, const int64_t *__restrict__ start, const int64_t *__restrict__ ent, const real *__restrict__ share,
                                 real *__restrict__ dX)
 {
@@ -45,50 +45,48 @@ int geo_status(cudaStream_t st, int *errWord)
 }
 } // namespace
 
-// the patch of every cell (its nodes, then its face neighbours' nodes, first occurrence kept) and
-// the node-to-share map of the gather; built once per mesh from the device topology
-int coords_ws_build(const MeshD &m, CoordAdjWs &ws)
+// the patch of every face (its first cell's nodes, then its second cell's, first occurrence kept) and the
+// node-to-share map of the gather; built once per mesh from the device topology.  The share array is followed by two
+// arrays [nCell][R][5] of the VJP's sweep part.
+int face_patches(const MeshD &m, int R, CoordAdjWs &ws)
 {
     if (ws.patch)
         return ST_OK;
-    std::vector<int32_t> c2n((size_t)m.nCell * m.nvert), nbr((size_t)m.nCell * m.nf);
+    std::vector<int32_t> c2n((size_t)m.nCell * m.nvert), f2c((size_t)m.nFace * 2);
     if (cudaMemcpy(c2n.data(), m.cell2node, sizeof(int32_t) * c2n.size(), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(nbr.data(), m.cellNbr, sizeof(int32_t) * nbr.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+        cudaMemcpy(f2c.data(), m.face2cell, sizeof(int32_t) * f2c.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
         return ST_CUDA;
-    const int cap = m.nvert * (m.nf + 1);
-    std::vector<int32_t> lists((size_t)m.nCell * cap);
-    std::vector<int> cnt(m.nCell);
+    const int cap = 2 * m.nvert;
+    std::vector<int32_t> lists((size_t)m.nFace * cap);
+    std::vector<int> cnt(m.nFace);
     int maxSlot = 1;
-    for (int64_t c = 0; c < m.nCell; c++)
+    for (int64_t f = 0; f < m.nFace; f++)
     {
-        int32_t *L = &lists[(size_t)c * cap];
+        int32_t *L = &lists[(size_t)f * cap];
         int n = 0;
-        auto add = [&](int64_t cell)
+        for (int sd = 0; sd < 2; sd++)
         {
-            for (int v = 0; v < m.nvert; v++)
+            const int64_t c = f2c[(size_t)f * 2 + sd];
+            for (int v = 0; c >= 0 && v < m.nvert; v++)
             {
-                int32_t nd = c2n[(size_t)cell * m.nvert + v];
+                const int32_t nd = c2n[(size_t)c * m.nvert + v];
                 bool seen = false;
                 for (int i = 0; i < n && !seen; i++)
                     seen = L[i] == nd;
                 if (!seen)
                     L[n++] = nd;
             }
-        };
-        add(c);
-        for (int k = 0; k < m.nf; k++)
-            if (nbr[(size_t)c * m.nf + k] >= 0)
-                add(nbr[(size_t)c * m.nf + k]);
-        cnt[c] = n;
+        }
+        cnt[f] = n;
         maxSlot = n > maxSlot ? n : maxSlot;
     }
-    std::vector<int32_t> patch((size_t)m.nCell * maxSlot, -1);
+    std::vector<int32_t> patch((size_t)m.nFace * maxSlot, -1);
     std::vector<int64_t> start(m.nNode + 1, 0);
-    for (int64_t c = 0; c < m.nCell; c++)
-        for (int i = 0; i < cnt[c]; i++)
+    for (int64_t f = 0; f < m.nFace; f++)
+        for (int i = 0; i < cnt[f]; i++)
         {
-            int32_t nd = lists[(size_t)c * cap + i];
-            patch[(size_t)c * maxSlot + i] = nd;
+            int32_t nd = lists[(size_t)f * cap + i];
+            patch[(size_t)f * maxSlot + i] = nd;
             start[nd + 1]++;
         }
     for (int64_t n = 0; n < m.nNode; n++)
@@ -100,7 +98,7 @@ int coords_ws_build(const MeshD &m, CoordAdjWs &ws)
     if (dev_alloc((void **)&ws.patch, sizeof(int32_t) * patch.size()) != cudaSuccess ||
         dev_alloc((void **)&ws.start, sizeof(int64_t) * start.size()) != cudaSuccess ||
         dev_alloc((void **)&ws.ent, sizeof(int64_t) * ent.size()) != cudaSuccess ||
-        dev_alloc((void **)&ws.share, sizeof(real) * 3 * patch.size()) != cudaSuccess ||
+        dev_alloc((void **)&ws.share, sizeof(real) * (3 * patch.size() + 2 * (size_t)m.nCell * R * 5)) != cudaSuccess ||
         cudaMemcpy(ws.patch, patch.data(), sizeof(int32_t) * patch.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(ws.start, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(ws.ent, ent.data(), sizeof(int64_t) * ent.size(), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -142,7 +140,7 @@ int coords_vjp(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSetting
 {
     if (!geo_supported(m, vr) || (s && (s->nVars != 5 || !s->ignoreVis)))
         return ST_UNSUPPORTED;
-    int rc = coords_ws_build(m, ws);
+    int rc = face_patches(m, vr.R, ws);
     if (rc != ST_OK)
         return rc;
     coords_lanes_build(m, g, vr, ws, st);
@@ -161,10 +159,10 @@ int pressure_force_coords(const MeshD &m, const GeomD &g, const VRD &vr, real ga
 {
     if (!geo_supported(m, vr))
         return ST_UNSUPPORTED;
-    int rc = coords_ws_build(m, ws);
+    int rc = face_patches(m, vr.R, ws);
     if (rc != ST_OK)
         return rc;
-    dev_zero(ws.share, sizeof(real) * 3 * m.nCell * ws.maxSlot, st);
+    dev_zero(ws.share, sizeof(real) * 3 * m.nFace * ws.maxSlot, st);
     if (m.dim == 2)
         pressure_force_coords_launch<2>(m, g, vr, gamma, zone, dir, u, uRec, ws, st);
     else

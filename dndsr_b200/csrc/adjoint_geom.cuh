@@ -9,9 +9,9 @@
 // neighbours (centres, barycentres, half boxes and basis moments of both sides of each face; the
 // face points, normals, Jacobians and weights).  These kernels recompute that chain for one cell
 // in dual numbers, in the order the setup kernels use:
-//   * VJP: one thread per (cell, patch node) with the node's three coordinates seeded
-//     (Dual<3>); the cell's residual derivatives contracted with the cotangent give the node's
-//     share, and a gather in node order sums the shares (deterministic, no atomics);
+//   * VJP: the contracted derivatives as a sum over faces (k_coords_vjp_face), one thread per (face,
+//     node of its cells) with the node's three coordinates seeded (Dual<3>); a gather in node order
+//     sums the shares (deterministic, no atomics);
 //   * JVP: one thread per cell with a coordinate direction seeded on every node (Dual<1>).
 // The cell means u, the reconstruction uRec and deltaLambdaCell are held fixed.  A^-1 is
 // differentiated as d(A^-1) = -A^-1 dA A^-1 (A is symmetric positive definite, where the
@@ -21,6 +21,7 @@
 #include "basis_eval.cuh"
 #include "bc.cuh"
 #include "dual.cuh"
+#include "fast_common.cuh"
 
 namespace dndsb
 {
@@ -556,40 +557,312 @@ DNDSB_D void cell_local(const MeshD &m, const GeomD &g, const VRD &vr, const Eul
     }
 }
 
-// VJP share of one (cell, patch node): the derivatives of cell c's residual entries with respect to
-// the node's coordinates, contracted with the cotangents w (EvaluateRHS) and relax * cot (sweep)
-template <int DIM, int P>
-DNDSB_GLOBAL void __launch_bounds__(kGeoBlock) k_coords_vjp(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ dLamCell,
-                                                            const real *__restrict__ u, const real *__restrict__ uRec, const real *__restrict__ w,
-                                                            const real *__restrict__ cot, real relax, const int32_t *__restrict__ patch,
-                                                            int maxSlot, real *__restrict__ share, int *err, const real *__restrict__ lanes)
+// ---- VJP, face by face ----
+// With the cotangents w (EvaluateRHS) and relax cot (sweep), J = sum_c w_c . flux_c / V_c + sum_c relax cot_c : S_c.
+// S = A^-1 s, so dS = A^-1 (ds - dA S) and, with lambda_c = relax A_c^-1 cot_c (A symmetric),
+//   d(relax cot : S) = lambda : ds - sum_ij dA_ij sum_v lambda_iv S_jv
+// where s and A are sums over the cell's faces and their points.  Holding lambda, S, u and uRec, J is therefore a sum
+// over faces of scalars that depend on the nodes of the face's two cells only; with rows a_k = D_k phi at a point seen
+// from side 0 and b_k from side 1 (k over the derivatives, c_k the functional's weight of order |k|),
+//   sum_k c_k sum_v [h0_v (g1_v - s0_v) + h1_v (g0_v - s1_v)] - |J| w F . (w_0 / V_0 - w_1 / V_1),
+//   h0 = a_k lambda_0, g0 = a_k uRec_0, s0 = a_k S_0, h1, g1, s1 the same from b_k (k = 0 adds u_1 - u_0 to g1 and
+// subtracts it from g0: the functional against the constant).
+// One thread per (face, node of its cells), the node's coordinates seeded (Dual<3>); the rows are generated one at a
+// time from compile-time exponents, so nothing but zeros-free rows of one derivative is live.  Bound by FP64 latency in
+// dual numbers.  The recomputation of a whole cell per (cell, patch node) that this replaces carried A and s as arrays
+// of dual numbers (7 KB of stack a thread, 14 GB of spill traffic) and evaluated every face of the cell for every node
+// of the patch and every flux twice: 9.8 ms on 38,400 tetrahedra, against 1.6 ms.
+template <int DIM, int K>
+struct Mono // exponents of basis function K
 {
-    constexpr int NV = 5, NDOF = ndof_of<DIM>(P), R = NDOF - 1;
-    DNDSB_KERNEL_LOOP(e, m.nCell * maxSlot)
+    static constexpr int c = fastc::mcode(DIM, K), x = c & 3, y = (c >> 2) & 3, z = (c >> 4) & 3, order = x + y + z;
+};
+// whether derivative K of function J does not vanish identically
+template <int DIM, int K, int J>
+constexpr bool row_nz() { return Mono<DIM, J>::x >= Mono<DIM, K>::x && Mono<DIM, J>::y >= Mono<DIM, K>::y && Mono<DIM, J>::z >= Mono<DIM, K>::z; }
+constexpr int falling_i(int p, int d) { return d == 0 ? 1 : p * falling_i(p - 1, d - 1); }
+
+template <int E, typename T>
+DNDSB_D void mul_pow(const T &x, T &r)
+{
+    if constexpr (E > 0)
     {
-        const int64_t c = e / maxSlot;
-        const int32_t node = patch[e];
-        real out[3] = {0, 0, 0};
-        if (node >= 0)
+        r = r * x;
+        mul_pow<E - 1>(x, r);
+    }
+}
+
+// D_K phi_J at the scaled point x; sK = the product of the 1 / L of derivative K
+template <int DIM, int K, int J, typename T>
+DNDSB_D T row_entry(const T *x, const T &sK)
+{
+    using A = Mono<DIM, J>;
+    using B = Mono<DIM, K>;
+    constexpr int cf = falling_i(A::x, B::x) * falling_i(A::y, B::y) * falling_i(A::z, B::z);
+    T r = K == 0 ? T((real)cf) : sK * (real)cf;
+    mul_pow<A::x - B::x>(x[0], r);
+    mul_pow<A::y - B::y>(x[1], r);
+    if constexpr (DIM == 3)
+        mul_pow<A::z - B::z>(x[2], r);
+    return r;
+}
+
+// one side of a face point: scaled coordinates and 1 / L of the cell
+template <int DIM, typename T>
+struct SideG
+{
+    T x[3], iL[3];
+    DNDSB_D void set(const T *cent, const T *scale, bool aniso, const T *p)
+    {
+        T L[3];
+        cell_lengths<DIM>(scale, aniso, L);
+        for (int d = 0; d < DIM; d++)
+            iL[d] = 1.0 / L[d], x[d] = (p[d] - cent[d]) * iL[d];
+    }
+};
+
+// h += sum_{j >= J} row_j lam_jv, g and t the same with rec and S, for derivative K of one side
+template <int DIM, int P, int K, int J, typename T>
+DNDSB_D void side_rows(const SideG<DIM, T> &sg, const T &sK, const T *moment, const real *lam, const real *rec, const real *S, T *h, T *g, T *t)
+{
+    constexpr int NV = 5;
+    if constexpr (J < ndof_of<DIM>(P))
+    {
+        if constexpr (row_nz<DIM, K, J>())
         {
-            SeedNode sd{node};
-            Dual<3> rhs[NV], S[R * NV];
-            int bad = 0;
-            cell_local<DIM, P>(m, g, vr, s, dLamCell, u, uRec, c, sd, w != nullptr, cot != nullptr, rhs, S, bad, lanes);
-            Dual<3> acc = 0.0;
-            if (w)
+            T r = row_entry<DIM, K, J>(sg.x, sK);
+            if constexpr (K == 0)
+            {
+                r = r - moment[J];
+            }
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+            {
+                if (lam)
+                    h[v] += r * lam[(J - 1) * NV + v], t[v] += r * S[(J - 1) * NV + v];
+                g[v] += r * rec[(J - 1) * NV + v];
+            }
+        }
+        side_rows<DIM, P, K, J + 1>(sg, sK, moment, lam, rec, S, h, g, t);
+    }
+}
+
+template <int DIM, int P, int K, typename T>
+DNDSB_D void side_sums(const SideG<DIM, T> &sg, const T *moment, const real *lam, const real *rec, const real *S, T *h, T *g, T *t)
+{
+    T sK = 1.0;
+    mul_pow<Mono<DIM, K>::x>(sg.iL[0], sK);
+    mul_pow<Mono<DIM, K>::y>(sg.iL[1], sK);
+    if constexpr (DIM == 3)
+    {
+        mul_pow<Mono<DIM, K>::z>(sg.iL[2], sK);
+    }
+    for (int v = 0; v < 5; v++)
+        h[v] = g[v] = t[v] = 0.0;
+    side_rows<DIM, P, K, 1>(sg, sK, moment, lam, rec, S, h, g, t);
+}
+
+// what the terms of one face point read (l, r, S: lambda, uRec and S rows of the two cells; l0 null: no sweep part)
+template <int DIM, int P>
+struct FacePoint
+{
+    using T = Dual<3>;
+    SideG<DIM, T> s0, s1;
+    const T *m0, *m1, *w2L; // moments of the cells, functional weights
+    T JW;
+    const real *l0, *r0, *S0, *l1, *r1, *S1, *u0, *u1;
+};
+
+// the sweep's terms of the derivatives K .. NDOF - 1 into acc; K = 0 also gives the point states UL, UR and, on a
+// boundary face, h0 (for the boundary term)
+template <int DIM, int P, bool BND, int K>
+DNDSB_D void face_terms(const FacePoint<DIM, P> &c, Dual<3> &acc, Dual<3> *UL, Dual<3> *UR, Dual<3> *hb)
+{
+    using T = Dual<3>;
+    constexpr int NV = 5, NDOF = ndof_of<DIM>(P);
+    if constexpr (K < NDOF)
+    {
+        if (K > 0 && !c.l0)
+            return;
+        T h0[NV], G0[NV], t0[NV], h1[NV], G1[NV], t1[NV];
+        side_sums<DIM, P, K>(c.s0, c.m0, c.l0, c.r0, c.S0, h0, G0, t0);
+        if constexpr (!BND)
+        {
+            side_sums<DIM, P, K>(c.s1, c.m1, c.l1, c.r1, c.S1, h1, G1, t1);
+        }
+        if constexpr (K == 0)
+        {
+            for (int v = 0; v < NV; v++)
+                UL[v] = G0[v] + c.u0[v];
+            if constexpr (BND)
+            {
                 for (int v = 0; v < NV; v++)
-                    acc += rhs[v] * w[c * NV + v];
-            if (cot)
-                for (int i = 0; i < R * NV; i++)
-                    acc += S[i] * (relax * cot[c * R * NV + i]);
+                    hb[v] = h0[v];
+            }
+            else
+            {
+                for (int v = 0; v < NV; v++)
+                {
+                    UR[v] = G1[v] + c.u1[v];
+                    G1[v] += c.u1[v] - c.u0[v], G0[v] += c.u0[v] - c.u1[v];
+                }
+            }
+        }
+        if (c.l0)
+        {
+            T sum = 0.0;
+            for (int v = 0; v < NV; v++)
+            {
+                if constexpr (BND)
+                {
+                    sum -= h0[v] * t0[v];
+                }
+                else
+                {
+                    sum += h0[v] * (G1[v] - t0[v]) + h1[v] * (G0[v] - t1[v]);
+                }
+            }
+            acc += c.w2L[Mono<DIM, K>::order] * c.JW * ((real)Basis<DIM>::ncomb(K) * sum);
+        }
+        face_terms<DIM, P, BND, K + 1>(c, acc, UL, UR, hb);
+    }
+}
+
+// lam [nCell][R][NV] = relax A^-1 cot; on entry S holds uRec - S_c (the sweep's recordInc), on exit S_c
+template <int R>
+DNDSB_GLOBAL void k_coords_prep(int64_t nCell, int nf, const real *__restrict__ AAInvB, const real *__restrict__ cot, const real *__restrict__ uRec,
+                                real relax, real *lam, real *S)
+{
+    constexpr int NV = 5;
+    DNDSB_KERNEL_LOOP(e, nCell * (R * NV))
+    {
+        const int64_t c = e / (R * NV);
+        const int r = (int)(e - c * (R * NV)), i = r / NV, v = r - i * NV;
+        real a = 0;
+        for (int j = 0; j < R; j++)
+            a += AAInvB[c * (nf + 1) * R * R + i * R + j] * cot[(c * R + j) * NV + v];
+        lam[e] = relax * a;
+        S[e] = uRec[e] - S[e];
+    }
+}
+
+// share[f][slot][3] of the faces with two cells (BND false) or of the boundary faces (BND true); lam null: no sweep part,
+// w null: no EvaluateRHS part
+template <int DIM, int P, bool BND>
+DNDSB_GLOBAL void __launch_bounds__(kGeoBlock) k_coords_vjp_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ dLamCell,
+                                                                 const real *__restrict__ u, const real *__restrict__ uRec,
+                                                                 const real *__restrict__ w, const real *__restrict__ lam,
+                                                                 const real *__restrict__ Sc, const int32_t *__restrict__ patch, int maxSlot,
+                                                                 real *__restrict__ share, int *err, const real *__restrict__ lanes)
+{
+    using T = Dual<3>;
+    constexpr int NV = 5, NDOF = ndof_of<DIM>(P), R = NDOF - 1;
+    const int intOrder = vr.s.intOrder;
+    const bool aniso = vr.s.anisotropicLengths;
+    DNDSB_KERNEL_LOOP(e, (BND ? m.nBndFace : m.nFace) * maxSlot)
+    {
+        const int64_t ii = e / maxSlot, f = BND ? (int64_t)m.bndFace[ii] : ii;
+        const int slot = (int)(e - ii * maxSlot);
+        const int64_t c0 = m.face2cell[f * 2], c1 = m.face2cell[f * 2 + 1];
+        if (!BND && c1 < 0)
+            continue;
+        real *out = share + (f * maxSlot + slot) * 3;
+        const int32_t node = patch[f * maxSlot + slot];
+        if (node < 0)
+        {
             for (int d = 0; d < 3; d++)
-                out[d] = acc.d[d];
-            if (bad)
-                atomicOr(err, (int)DE_NONPHYSICAL);
+                out[d] = 0;
+            continue;
+        }
+        const SeedNode sd{node};
+        CellG<T, NDOF> g0, g1;
+        FaceG<T> fg;
+        face_geo(m, intOrder, g.nGf, f, sd, fg);
+        cell_geo_or_lanes<DIM, NDOF>(lanes, m, intOrder, g.nGc, aniso, c0, sd, g0);
+        if constexpr (!BND)
+            cell_geo_or_lanes<DIM, NDOF>(lanes, m, intOrder, g.nGc, aniso, c1, sd, g1);
+        T w2L[P + 1], w0 = 0.0;
+        if (lam)
+            face_weights<DIM, P>(m, vr, f, fg, g0.bary, BND ? nullptr : g1.bary, g0.scale, BND ? nullptr : g1.scale, w2L, w0);
+        const real *u0 = u + c0 * NV, *u1 = BND ? nullptr : u + c1 * NV, *r0 = uRec + c0 * R * NV, *r1 = BND ? nullptr : uRec + c1 * R * NV;
+        const real *l0 = lam ? lam + c0 * R * NV : nullptr, *S0 = lam ? Sc + c0 * R * NV : nullptr;
+        const real *l1 = lam && !BND ? lam + c1 * R * NV : nullptr, *S1 = lam && !BND ? Sc + c1 * R * NV : nullptr;
+        T gbar[NV];
+        if (w)
+        {
+            const T iv0 = 1.0 / g0.vol;
+            for (int v = 0; v < NV; v++)
+                gbar[v] = iv0 * w[c0 * NV + v];
+            if constexpr (!BND)
+            {
+                const T iv1 = 1.0 / g1.vol;
+                for (int v = 0; v < NV; v++)
+                    gbar[v] -= iv1 * w[c1 * NV + v];
+            }
+        }
+        const int zone = BND ? m.faceZone[f] : 0;
+        T ULm[NV], URm[NV];
+        for (int v = 0; v < NV; v++)
+        {
+            ULm[v] = u0[v];
+            if constexpr (!BND)
+                URm[v] = u1[v];
+        }
+        if (BND && w && !bc_value<NV>(vr.bnd, zone, ULm, fg.meanNorm, URm))
+            for (int v = 0; v < NV; v++)
+                URm[v] = ULm[v];
+        T acc = 0.0;
+        bool bad = false;
+#pragma unroll 1
+        for (int q = 0; q < g.nGf; q++)
+        {
+            T p0[3], nrm[3];
+            FacePoint<DIM, P> c{{}, {}, g0.moment, g1.moment, w2L, T(0.0), l0, r0, S0, l1, r1, S1, u0, u1};
+            face_point(m, intOrder, fg, q, g.faceQw[q], p0, nrm, c.JW);
+            c.s0.set(g0.cent, g0.scale, aniso, p0);
+            if constexpr (!BND)
+            {
+                T p1[3];
+                for (int d = 0; d < 3; d++)
+                    p1[d] = p0[d] + m.facePShift[f * 3 + d];
+                c.s1.set(g1.cent, g1.scale, aniso, p1);
+            }
+            T UL[NV], UR[NV], hb[NV];
+            face_terms<DIM, P, BND, 0>(c, acc, UL, UR, hb);
+            if (BND && lam && value_of(w0) != 0)
+            {
+                // GetBoundaryRHS (_Reconstruction.hxx:19-176) as k_vr_bc
+                T uc[NV], ULf[NV], UB[NV], sum = 0.0;
+                for (int v = 0; v < NV; v++)
+                    uc[v] = u0[v];
+                compress_rec<NV>(uc, UL, ULf);
+                if (!bc_value_fix<NV>(vr.bnd, zone, ULf, nrm, UB))
+                    for (int v = 0; v < NV; v++)
+                        UB[v] = ULf[v];
+                for (int v = 0; v < NV; v++)
+                    sum += hb[v] * (UB[v] - u0[v]);
+                acc += sum * c.JW * w0 * w0;
+            }
+            if (w)
+            {
+                T F[NV], e0, e1, e4;
+                for (int v = 0; v < NV; v++)
+                    F[v] = 0.0;
+                if (BND && !bc_value_fix<NV>(vr.bnd, zone, UL, nrm, UR))
+                    for (int v = 0; v < NV; v++)
+                        UR[v] = UL[v];
+                const real dLambda = BND ? dLamCell[c0] : dmax(dLamCell[c0], dLamCell[BND ? c0 : c1]);
+                bad |= !riemann_flux(s.rsType, UL, UR, ULm, URm, nrm, s.gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, e0, e1, e4);
+                T sum = 0.0;
+                for (int v = 0; v < NV; v++)
+                    sum += F[v] * gbar[v];
+                acc -= c.JW * sum;
+            }
         }
         for (int d = 0; d < 3; d++)
-            share[e * 3 + d] = out[d];
+            out[d] = acc.d[d];
+        if (bad)
+            atomicOr(err, (int)DE_NONPHYSICAL);
     }
 }
 
@@ -645,69 +918,50 @@ DNDSB_GLOBAL void __launch_bounds__(kGeoBlock) k_cell_lanes(MeshD m, GeomD g, VR
     }
 }
 
-// Share of one (boundary cell, cell vertex) in the derivative of the pressure force
+// Share of one (boundary face, node of its cell) in the derivative of the pressure force
 // J = sum over the zone's faces and points of p(U) (n . dir) |J| w (k_pressure_force) with respect to
-// the vertex coordinates: the cell's basis and its faces' geometry depend on its own nodes only.
-// Written into the patch slot of that node in the cell's own patch (a node met twice in a cell, as
-// periodic images, is seeded once).
+// the node's coordinates: the cell's basis and the face's geometry depend on the cell's own nodes only.
 template <int DIM, int P>
 DNDSB_GLOBAL void __launch_bounds__(kGeoBlock) k_pressure_force_coords(MeshD m, GeomD g, VRD vr, real gamma, int zone, real d0, real d1, real d2,
                                                                        const real *__restrict__ u, const real *__restrict__ uRec,
                                                                        const int32_t *__restrict__ patch, int maxSlot, real *__restrict__ share)
 {
     constexpr int NV = 5, NDOF = ndof_of<DIM>(P), R = NDOF - 1;
-    DNDSB_KERNEL_LOOP(e, m.nBndCell * m.nvert)
+    DNDSB_KERNEL_LOOP(e, m.nBndFace * maxSlot)
     {
-        const int64_t ii = e / m.nvert;
-        const int v = (int)(e - ii * m.nvert);
-        const int64_t c = m.bndCell[ii];
-        const int32_t node = m.cell2node[c * m.nvert + v];
-        bool dup = false;
-        for (int v2 = 0; v2 < v; v2++)
-            dup = dup || m.cell2node[c * m.nvert + v2] == node;
-        int slot = 0;
-        while (slot < maxSlot && patch[c * maxSlot + slot] != node)
-            slot++;
-        if (dup || slot == maxSlot)
+        const int64_t f = m.bndFace[e / maxSlot];
+        const int slot = (int)(e - e / maxSlot * maxSlot);
+        const int32_t node = patch[f * maxSlot + slot];
+        if (node < 0 || m.faceZone[f] != zone)
             continue;
+        const int64_t c = m.face2cell[f * 2];
         SeedNode sd{node};
         const bool aniso = vr.s.anisotropicLengths;
         CellG<Dual<3>, NDOF> gc;
-        bool any = false;
         Dual<3> J = 0.0;
-        for (int k = 0; k < m.nf; k++)
+        cell_geo<DIM, NDOF>(m, vr.s.intOrder, g.nGc, aniso, c, sd, gc);
+        FaceG<Dual<3>> fg;
+        face_geo(m, vr.s.intOrder, g.nGf, f, sd, fg);
+        for (int q = 0; q < g.nGf; q++)
         {
-            if (m.cellNbr[c * m.nf + k] >= 0)
-                continue;
-            const int64_t f = m.cell2face[c * m.nf + k] >> 1;
-            if (m.faceZone[f] != zone)
-                continue;
-            if (!any)
-                cell_geo<DIM, NDOF>(m, vr.s.intOrder, g.nGc, aniso, c, sd, gc);
-            any = true;
-            FaceG<Dual<3>> fg;
-            face_geo(m, vr.s.intOrder, g.nGf, f, sd, fg);
-            for (int q = 0; q < g.nGf; q++)
+            Dual<3> pp[3], nrm[3], JW, T0[NDOF];
+            face_point(m, vr.s.intOrder, fg, q, g.faceQw[q], pp, nrm, JW);
+            cell_basis<DIM, NDOF>(gc.cent, gc.scale, gc.moment, aniso, pp, 1, T0);
+            Dual<3> UL[NV];
+            for (int w = 0; w < NV; w++)
             {
-                Dual<3> pp[3], nrm[3], JW, T0[NDOF];
-                face_point(m, vr.s.intOrder, fg, q, g.faceQw[q], pp, nrm, JW);
-                cell_basis<DIM, NDOF>(gc.cent, gc.scale, gc.moment, aniso, pp, 1, T0);
-                Dual<3> UL[NV];
-                for (int w = 0; w < NV; w++)
-                {
-                    Dual<3> a = 0.0;
-                    for (int j = 0; j < R; j++)
-                        a += T0[1 + j] * uRec[(c * R + j) * NV + w];
-                    UL[w] = u[c * NV + w] + a;
-                }
-                Dual<3> vel[3] = {UL[1] / UL[0], UL[2] / UL[0], UL[3] / UL[0]};
-                Dual<3> pr = (gamma - 1) * (UL[4] - 0.5 * UL[0] * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]));
-                Dual<3> wt = JW * (nrm[0] * d0 + nrm[1] * d1 + nrm[2] * d2);
-                J += wt * pr;
+                Dual<3> a = 0.0;
+                for (int j = 0; j < R; j++)
+                    a += T0[1 + j] * uRec[(c * R + j) * NV + w];
+                UL[w] = u[c * NV + w] + a;
             }
+            Dual<3> vel[3] = {UL[1] / UL[0], UL[2] / UL[0], UL[3] / UL[0]};
+            Dual<3> pr = (gamma - 1) * (UL[4] - 0.5 * UL[0] * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]));
+            Dual<3> wt = JW * (nrm[0] * d0 + nrm[1] * d1 + nrm[2] * d2);
+            J += wt * pr;
         }
         for (int d = 0; d < 3; d++)
-            share[(c * maxSlot + slot) * 3 + d] = J.d[d];
+            share[(f * maxSlot + slot) * 3 + d] = J.d[d];
     }
 }
 } // namespace
@@ -717,7 +971,7 @@ void pressure_force_coords_launch(const MeshD &m, const GeomD &g, const VRD &vr,
                                   const real *uRec, const CoordAdjWs &ws, cudaStream_t st)
 {
     constexpr int PTop = DIM == 2 ? 3 : 2;
-    const int64_t n = m.nBndCell * m.nvert;
+    const int64_t n = m.nBndFace * ws.maxSlot;
     if (vr.P == 1)
         DNDSB_LAUNCH((k_pressure_force_coords<DIM, 1>), n, kGeoBlock, st, m, g, vr, gamma, zone, dir[0], dir[1], dir[2], u, uRec, ws.patch, ws.maxSlot, ws.share);
     else if (vr.P == 2)
@@ -728,22 +982,36 @@ void pressure_force_coords_launch(const MeshD &m, const GeomD &g, const VRD &vr,
 }
 
 // launches for one dimension; P = 1, 2 (and 3 in 2-D)
+template <int DIM, int P>
+void coords_vjp_launch_p(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
+                         const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
+{
+    constexpr int R = ndof_of<DIM>(P) - 1;
+    real *lam = nullptr, *S = nullptr;
+    if (cot)
+    {
+        lam = ws.share + 3 * m.nFace * ws.maxSlot, S = lam + m.nCell * R * 5; // see face_patches
+        vr_iter(m, g, vr, 5, uRec, S, u, 1, 0, 0, st);
+        DNDSB_LAUNCH(k_coords_prep<R>, m.nCell * R * 5, 256, st, m.nCell, m.nf, vr.AAInvB, cot, uRec, vr.s.jacobiRelax, lam, S);
+    }
+    auto kf = k_coords_vjp_face<DIM, P, false>;
+    auto kb = k_coords_vjp_face<DIM, P, true>;
+    DNDSB_LAUNCH(kf, m.nFace * ws.maxSlot, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, lam, S, ws.patch, ws.maxSlot, ws.share, err, ws.lanes);
+    DNDSB_LAUNCH(kb, m.nBndFace * ws.maxSlot, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, lam, S, ws.patch, ws.maxSlot, ws.share, err,
+                 ws.lanes);
+}
+
 template <int DIM>
 void coords_vjp_launch(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
                        const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
 {
     constexpr int PTop = DIM == 2 ? 3 : 2;
-    const int64_t n = m.nCell * ws.maxSlot;
-    const real relax = vr.s.jacobiRelax;
     if (vr.P == 1)
-        DNDSB_LAUNCH((k_coords_vjp<DIM, 1>), n, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, cot, relax, ws.patch, ws.maxSlot, ws.share, err,
-                     ws.lanes);
+        coords_vjp_launch_p<DIM, 1>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
     else if (vr.P == 2)
-        DNDSB_LAUNCH((k_coords_vjp<DIM, 2>), n, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, cot, relax, ws.patch, ws.maxSlot, ws.share, err,
-                     ws.lanes);
+        coords_vjp_launch_p<DIM, 2>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
     else
-        DNDSB_LAUNCH((k_coords_vjp<DIM, PTop>), n, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, cot, relax, ws.patch, ws.maxSlot, ws.share,
-                     err, ws.lanes);
+        coords_vjp_launch_p<DIM, PTop>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
 }
 
 template <int DIM>
