@@ -100,6 +100,7 @@ SIGNATURES = {
     "dndsb_eval_cell_rhs_alpha_expansion": [_P, _P, _P, _P, _d, _d, _d, _P],
     "dndsb_eval_add_fixed_increment": [_P, _P, _P, _d, _d, _d, _i, _P, _P],
     "dndsb_eval_evaluate_norm": [_P, _P, _i, _i, _D, _P],
+    "dndsb_eval_pseudo_iteration": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _D, _P],
     "dndsb_eval_solve_linear": [_P, _P, _d, _P, _d, _P, _P, _P, _P],
     "dndsb_vr_set_boundary": [_P, _i, _I32, _D, _i, _d, _d],
     "dndsb_eval_set_bc": [_P, _i, _I32, _D],

@@ -4,6 +4,7 @@
 #include "../../include/dndsb.h"
 #include "solver.cuh"
 #include "wall_flux.cuh"
+#include "pseudo.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -38,6 +39,7 @@ struct dndsb_eval
     dndsb_vr *vr = nullptr;
     EvalD e;
     LinWs *lin = nullptr; // workspace of dndsb_eval_solve_linear
+    double *pinned = nullptr; // [9] page-locked: the norm and the error word of dndsb_eval_pseudo_iteration
 };
 
 namespace
@@ -606,6 +608,8 @@ extern "C"
                         (void *)e->e.luDinv, (void *)e->e.luDiag})
             dev_free(p);
         linws_free(e->lin);
+        if (e->pinned)
+            cudaFreeHost(e->pinned);
         delete e;
         return DNDSB_OK;
     }
@@ -1054,6 +1058,53 @@ extern "C"
         if (rc == ST_BADARG)
             return fail(DNDSB_E_BADARG, "dndsb_eval_solve_linear: gmresCode 0..2, jacobiCode 0..2, nGmresSpace 1..32, precision 0..1");
         return status_msg(rc, "dndsb_eval_solve_linear");
+    }
+
+    int dndsb_eval_pseudo_iteration(dndsb_eval *e, const dndsb_pseudo_settings *s, double *u, double *uRec, double *uRecNew,
+                                    const double *resOther, double *rhs, double *res, double *dTau, double *xInc, double *resNorm,
+                                    void *stream)
+    {
+        if (!e || !s || !u || !uRec || !uRecNew || !resOther || !rhs || !res || !dTau || !xInc || !resNorm)
+            return fail(DNDSB_E_BADARG, "dndsb_eval_pseudo_iteration: null argument");
+        if (s->nSweep < 0 || s->normOrd < 1 || !(s->alphaDiag > 0))
+            return fail(DNDSB_E_BADARG, "dndsb_eval_pseudo_iteration: nSweep >= 0, normOrd >= 1, alphaDiag > 0");
+        const int nv = e->e.s.nVars;
+        const int64_t nCell = e->vr->mesh->d.nCell;
+        cudaStream_t st = S(stream);
+        if (!e->pinned && cudaMallocHost((void **)&e->pinned, sizeof(double) * 9) != cudaSuccess)
+            return cuda_fail("dndsb_eval_pseudo_iteration");
+        int rc = dndsb_eval_evaluate_dt(e, u, s->CFL, 1e100, 1, dTau, nullptr, stream);
+        for (int i = 0; rc == DNDSB_OK && i < s->nSweep; i++)
+            rc = dndsb_vr_do_reconstruction_iter(e->vr, uRec, uRecNew, u, nv, 0, 0, 0, s->sweepPrecision, stream);
+        if (rc == DNDSB_OK)
+            rc = dndsb_eval_evaluate_rhs(e, rhs, u, uRec, stream);
+        if (rc == DNDSB_OK)
+            rc = status_msg(unsteady_residual(nCell, nv, resOther, u, rhs, s->dt, s->alphaDiag, res, dTau, st), "dndsb_eval_pseudo_iteration");
+        if (rc == DNDSB_OK)
+            rc = dndsb_eval_solve_linear(e, &s->linear, s->alphaDiag, dTau, s->dt, u, res, xInc, stream);
+        if (rc != DNDSB_OK)
+            return rc;
+        if (add_increment(nCell * nv, xInc, u, st) != ST_OK)
+            return cuda_fail("dndsb_eval_pseudo_iteration");
+        const bool sum = s->normOrd < 3;
+        const real *nrm = reduce_cols(sum ? 0 : 2, nCell, nv, res, sum && s->normVolWise ? e->vr->g.vol : nullptr, sum ? s->normOrd : 1, e->e.redBuf, st);
+        int *word = (int *)(e->pinned + 8);
+        *word = 0;
+        d2h(e->pinned, nrm, sizeof(double) * nv, st);
+        if (e->e.deferErr)
+            d2h(word, e->e.errDeferred, sizeof(int), st);
+        if (dev_sync(st) != cudaSuccess)
+            return cuda_fail("dndsb_eval_pseudo_iteration");
+        for (int v = 0; v < nv; v++)
+            resNorm[v] = s->normOrd == 2 ? std::sqrt(e->pinned[v]) : e->pinned[v];
+        if (*word)
+        {
+            const int w = *word;
+            dev_zero(e->e.errDeferred, sizeof(int), st);
+            if (w & (DE_NONPHYSICAL | DE_NONFINITE))
+                return status_msg(w & DE_NONPHYSICAL ? ST_NONPHYSICAL : ST_NONFINITE, "dndsb_eval_pseudo_iteration");
+        }
+        return DNDSB_OK;
     }
 
     int64_t dndsb_krylov_ld(int64_t n) { return krylov_ld(n); }

@@ -6,6 +6,7 @@
 #include "sa.cuh"
 #include "wall_flux.cuh"
 #include "basis_rows.cuh"
+#include "pseudo.cuh"
 
 namespace dndsb
 {
@@ -928,6 +929,46 @@ int init_field(const MeshD &m, const GeomD &g, const EvalD &ev, int kind, real c
     if (ev.s.nVars != 5)
         return ST_UNSUPPORTED;
     DNDSB_LAUNCH(k_init_field<5>, m.nCell, 128, st, m, g, ev.s.gamma, kind, chi, u);
+    return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
+}
+
+namespace
+{
+// res = resOther - u / dt + alphaDiag rhs and dTau *= 1 / alphaDiag (ODE.hpp:300-330 with EulerSolver.hxx:674-694)
+template <int NV>
+DNDSB_GLOBAL void k_unsteady_residual(int64_t nCell, const real *__restrict__ other, const real *__restrict__ u, const real *__restrict__ rhs,
+                                      real mInvDt, real alphaDiag, real *__restrict__ res, real *__restrict__ dTau)
+{
+    DNDSB_KERNEL_LOOP(e, nCell * NV)
+    {
+        res[e] = (other[e] + mInvDt * u[e]) + alphaDiag * rhs[e];
+        if (e < nCell)
+            dTau[e] *= 1.0 / alphaDiag;
+    }
+}
+
+DNDSB_GLOBAL void k_add(int64_t n, const real *__restrict__ a, real *__restrict__ x)
+{
+    DNDSB_KERNEL_LOOP(i, n)
+    x[i] += a[i];
+}
+} // namespace
+
+int unsteady_residual(int64_t nCell, int nv, const real *other, const real *u, const real *rhs, real dt, real alphaDiag, real *res, real *dTau,
+                      cudaStream_t st)
+{
+    if (nv == 5)
+        DNDSB_LAUNCH(k_unsteady_residual<5>, nCell * 5, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
+    else if (nv == 6)
+        DNDSB_LAUNCH(k_unsteady_residual<6>, nCell * 6, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
+    else
+        return ST_UNSUPPORTED;
+    return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
+}
+
+int add_increment(int64_t n, const real *inc, real *u, cudaStream_t st)
+{
+    DNDSB_LAUNCH(k_add, n, 256, st, n, inc, u);
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 

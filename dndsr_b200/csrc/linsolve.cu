@@ -621,7 +621,8 @@ struct Solve
         T *x = (T *)w.x;
         const T *b = (const T *)w.rhsT;
         int64_t nn = n();
-        DNDSB_LAUNCH(k_zero_T<T>, nn, 256, st, nn, x);
+        if (ls.gmresCode == 1) // otherwise the pairs from zero write x
+            DNDSB_LAUNCH(k_zero_T<T>, nn, 256, st, nn, x);
         bool xZero = true;
         if (ls.gmresCode == 0 || ls.gmresCode == 2)
         {
@@ -670,15 +671,23 @@ struct Solve
     static int prec() { return sizeof(T) == 4 ? 1 : 0; }
 };
 
+constexpr int kDirectLaunches = 24;
+
 template <typename T, int NV, int NF>
 int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &w, const LinSettings &ls, real alphaDiag, const real *dTau,
         real dt, const real *u, const real *rhs, real *xInc, cudaStream_t st)
 {
-    // the caller's stream -> the solver's stream
-    event_record(w.evIn, st);
-    stream_wait(w.cs, w.evIn);
-    cudaStream_t cs = w.cs;
-    h2d(w.s2, ls.scale2, sizeof(real) * 8, cs);
+    // A few sweeps alone go straight onto the caller's stream: replaying a graph of them and handing over between the
+    // streams costs more than their launches.  Everything else runs on the solver's stream, captured once.
+    const bool direct = ls.gmresCode == 0 && (int64_t)(1 + ls.sgsIter) * 2 * m.nColor * (ls.jacobiCode == 2 ? 2 : 1) <= kDirectLaunches;
+    cudaStream_t cs = direct ? st : w.cs;
+    if (!direct)
+    {
+        event_record(w.evIn, st);
+        stream_wait(cs, w.evIn);
+    }
+    if (ls.gmresCode != 0)
+        h2d(w.s2, ls.scale2, sizeof(real) * 8, cs);
     auto kbuild = posop::k_build<T, NV, NF>;
     auto kgather = k_gather_T<T, NV>;
     auto kscatter = k_scatter_T<T, NV>;
@@ -705,7 +714,9 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
     else
         DNDSB_LAUNCH(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
     DNDSB_LAUNCH(kgather, m.nCell, 256, cs, m.nCell, m.colorCells, rhs, (T *)w.rhsT);
-    if (ls.useGraph)
+    if (direct)
+        S.body();
+    else if (ls.useGraph)
     {
         if (!(w.graph && w.keyValid && same_key(w.key, ls)))
         {
@@ -735,8 +746,11 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         S.body();
     }
     DNDSB_LAUNCH(kscatter, m.nCell, 256, cs, m.nCell, m.colorCells, (const T *)w.x, xInc);
-    event_record(w.evOut, cs);
-    stream_wait(st, w.evOut);
+    if (!direct)
+    {
+        event_record(w.evOut, cs);
+        stream_wait(st, w.evOut);
+    }
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 

@@ -34,6 +34,46 @@ inline void ck(int rc)
         raise_status(rc);
 }
 
+// attribute names and torch objects the argument checks use, made once: a check is then a handful of slot lookups
+struct Names
+{
+    py::str data_ptr{intern("data_ptr")}, is_cuda{intern("is_cuda")}, dtype{intern("dtype")}, is_contiguous{intern("is_contiguous")};
+    py::object f64 = py::module_::import("torch").attr("float64"), f32 = py::module_::import("torch").attr("float32");
+    static py::object intern(const char *s) { return py::reinterpret_steal<py::object>(PyUnicode_InternFromString(s)); }
+    static const Names &get()
+    {
+        static const Names *n = new Names; // never freed: it may outlive the interpreter's own teardown
+        return *n;
+    }
+};
+
+py::object attr_or_null(const py::object &t, const py::str &name)
+{
+    PyObject *r = PyObject_GetAttr(t.ptr(), name.ptr());
+    if (!r)
+        PyErr_Clear();
+    return py::reinterpret_steal<py::object>(r);
+}
+
+bool attr_is_true(const py::object &t, const py::str &name, bool call)
+{
+    py::object a = attr_or_null(t, name);
+    if (a && call)
+        a = py::reinterpret_steal<py::object>(PyObject_CallNoArgs(a.ptr()));
+    if (!a)
+        PyErr_Clear();
+    return a && a.ptr() == Py_True;
+}
+
+// the data pointer, or nullptr with *ok false when t is not a contiguous CUDA tensor (of dtype want, if any)
+void *tensor_ptr(const py::object &t, const py::object *want, bool *ok)
+{
+    const Names &n = Names::get();
+    py::object get = attr_or_null(t, n.data_ptr);
+    *ok = get && attr_is_true(t, n.is_cuda, false) && (!want || attr_or_null(t, n.dtype).is(*want)) && attr_is_true(t, n.is_contiguous, true);
+    return *ok ? reinterpret_cast<void *>(get().cast<uintptr_t>()) : nullptr;
+}
+
 // data pointer of a contiguous CUDA tensor of dtype float64 (or float32); None gives nullptr when allowed
 void *dptr(const py::object &t, const char *name, bool fp32 = false, bool nullable = false)
 {
@@ -43,11 +83,11 @@ void *dptr(const py::object &t, const char *name, bool fp32 = false, bool nullab
             return nullptr;
         throw py::value_error(std::string(name) + " must be a CUDA tensor, not None");
     }
-    const char *want = fp32 ? "torch.float32" : "torch.float64";
-    if (!py::hasattr(t, "data_ptr") || !t.attr("is_cuda").cast<bool>() || py::str(t.attr("dtype")).cast<std::string>() != want ||
-        !t.attr("is_contiguous")().cast<bool>())
+    bool ok;
+    void *p = tensor_ptr(t, fp32 ? &Names::get().f32 : &Names::get().f64, &ok);
+    if (!ok)
         throw py::value_error(std::string(name) + " must be a contiguous " + (fp32 ? "float32" : "float64") + " CUDA tensor");
-    return reinterpret_cast<void *>(t.attr("data_ptr")().cast<uintptr_t>());
+    return p;
 }
 double *dp(const py::object &t, const char *name) { return static_cast<double *>(dptr(t, name)); }
 double *dpn(const py::object &t, const char *name) { return static_cast<double *>(dptr(t, name, false, true)); }
@@ -55,9 +95,11 @@ double *dpn(const py::object &t, const char *name) { return static_cast<double *
 // data pointer of any contiguous CUDA tensor
 void *anyptr(const py::object &t, const char *name)
 {
-    if (t.is_none() || !py::hasattr(t, "data_ptr") || !t.attr("is_cuda").cast<bool>() || !t.attr("is_contiguous")().cast<bool>())
+    bool ok = false;
+    void *p = t.is_none() ? nullptr : tensor_ptr(t, nullptr, &ok);
+    if (!ok)
         throw py::value_error(std::string(name) + " must be a contiguous CUDA tensor");
-    return reinterpret_cast<void *>(t.attr("data_ptr")().cast<uintptr_t>());
+    return p;
 }
 
 // 0 for a float64 tensor, 1 for float32
@@ -71,10 +113,25 @@ int precision_of(const py::object &t)
     throw py::value_error("Krylov vectors must be float64 or float32");
 }
 
+// torch's current stream on the current device (by the raw lookup where this torch has it)
 void *stream()
 {
-    static py::object cur = py::module_::import("torch").attr("cuda").attr("current_stream");
-    return reinterpret_cast<void *>(cur().attr("cuda_stream").cast<uintptr_t>());
+    struct Lookup
+    {
+        py::object raw, device, cur;
+        Lookup()
+        {
+            py::module_ c = py::module_::import("torch._C"), torch = py::module_::import("torch");
+            if (py::hasattr(c, "_cuda_getCurrentRawStream") && py::hasattr(c, "_cuda_getDevice"))
+                raw = c.attr("_cuda_getCurrentRawStream"), device = c.attr("_cuda_getDevice");
+            torch.attr("cuda").attr("init")();
+            cur = torch.attr("cuda").attr("current_stream");
+        }
+    };
+    static const Lookup *l = new Lookup;
+    if (l->raw)
+        return reinterpret_cast<void *>(l->raw(l->device()).cast<uintptr_t>());
+    return reinterpret_cast<void *>(l->cur().attr("cuda_stream").cast<uintptr_t>());
 }
 
 template <class T>
@@ -358,8 +415,7 @@ struct Eval
         ck(dndsb_eval_add_fixed_increment(h, dp(u, "u"), dp(inc, "inc"), alpha, refRho, refP, ppEpsIsRelaxed, &amin, stream()));
         return amin;
     }
-    // EulerSolver.hxx:1407-1658 with Solver/Linear.hpp:46-133
-    void SolveLinear(const py::dict &ls, double alphaDiag, py::object dTau, double dt, py::object u, py::object rhs, py::object xInc)
+    static dndsb_linear_settings linear_settings(const py::dict &ls)
     {
         dndsb_linear_settings s{};
         s.gmresCode = ls["gmresCode"].cast<int>(), s.jacobiCode = ls["jacobiCode"].cast<int>(), s.sgsIter = ls["sgsIter"].cast<int>();
@@ -368,7 +424,24 @@ struct Eval
         auto ms = ls["meanScale"].cast<std::vector<double>>();
         for (int i = 0; i < 8 && i < (int)ms.size(); i++)
             s.meanScale[i] = ms[i];
+        return s;
+    }
+    // EulerSolver.hxx:1407-1658 with Solver/Linear.hpp:46-133
+    void SolveLinear(const py::dict &ls, double alphaDiag, py::object dTau, double dt, py::object u, py::object rhs, py::object xInc)
+    {
+        dndsb_linear_settings s = linear_settings(ls);
         ck(dndsb_eval_solve_linear(h, &s, alphaDiag, dp(dTau, "dTau"), dt, dp(u, "u"), dp(rhs, "rhs"), dp(xInc, "xInc"), stream()));
+    }
+    // one pseudo-time iteration of a stage (EulerSolver.hxx:147-997)
+    Arr<double> PseudoIteration(const py::dict &ls, double CFL, double alphaDiag, double dt, int nSweep, int sweepPrecision, int normOrd,
+                                bool normVolWise, py::object u, py::object uRec, py::object uRecNew, py::object resOther, py::object rhs,
+                                py::object res, py::object dTau, py::object xInc)
+    {
+        dndsb_pseudo_settings s{linear_settings(ls), CFL, alphaDiag, dt, nSweep, sweepPrecision, normOrd, (int)normVolWise};
+        Arr<double> out(nVars);
+        ck(dndsb_eval_pseudo_iteration(h, &s, dp(u, "u"), dp(uRec, "uRec"), dp(uRecNew, "uRecNew"), dp(resOther, "resOther"), dp(rhs, "rhs"),
+                                       dp(res, "res"), dp(dTau, "dTau"), dp(xInc, "xInc"), out.mutable_data(), stream()));
+        return out;
     }
     // EulerEvaluator.hxx:1394-1439
     Arr<double> EvaluateNorm(py::object x, int P, bool volWise)
@@ -478,6 +551,7 @@ PYBIND11_MODULE(_C, m)
         .def("EvaluateCellRHSAlphaExpansion", &Eval::EvaluateCellRHSAlphaExpansion)
         .def("AddFixedIncrement", &Eval::AddFixedIncrement)
         .def("SolveLinear", &Eval::SolveLinear)
+        .def("PseudoIteration", &Eval::PseudoIteration)
         .def("EvaluateNorm", &Eval::EvaluateNorm)
         .def("get", &Eval::get)
         .def("SetDeltaLambda", &Eval::SetDeltaLambda);

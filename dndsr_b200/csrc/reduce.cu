@@ -16,59 +16,64 @@ template <int OP /*0 sum, 1 min, 2 max*/>
 DNDSB_D real red_op(real a, real b) { return OP == 0 ? a + b : OP == 1 ? dmin(a, b) : dmax(a, b); }
 
 template <int OP>
+DNDSB_D real warp_red(real x)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        x = red_op<OP>(x, __shfl_xor_sync(0xffffffffu, x, o));
+    return x;
+}
+
+// partial[block][col] over the block's rows; x is [n][ncol], ncol at most 8, optional row weight w.  One pass for all
+// columns, a thread per row: a tree per column over 592 blocks took 6.3 us for 8,192 rows of 5 and the final one 5.6.
+template <int OP>
 DNDSB_GLOBAL void k_reduce_cols(int64_t n, int ncol, const real *__restrict__ x, const real *__restrict__ w, int powP, real *partial)
 {
-    // partial[block][col] over rows [chunk) ; x is [n][ncol], optional row weight w
-    __shared__ real sh[kRedBlock];
-    real init = OP == 0 ? 0.0 : OP == 1 ? kVeryLarge : -kVeryLarge;
-    int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    int64_t b0 = blockIdx.x * chunk, b1 = b0 + chunk < n ? b0 + chunk : n;
-    for (int col = 0; col < ncol; col++)
+    __shared__ real sh[kRedBlock / 32][8];
+    real a[8];
+#pragma unroll
+    for (int v = 0; v < 8; v++)
+        a[v] = OP == 0 ? 0.0 : OP == 1 ? kVeryLarge : -kVeryLarge;
+    DNDSB_KERNEL_LOOP(i, n)
     {
-        real a = init;
-        for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x)
-        {
-            real xv = x[i * ncol + col];
-            xv = powP == 1 ? fabs(xv) : powP == 2 ? xv * xv : xv;
-            real val = xv * (w ? w[i] : 1.0);
-            a = red_op<OP>(a, val);
-        }
-        sh[threadIdx.x] = a;
-        __syncthreads();
-        for (int st = blockDim.x / 2; st > 0; st >>= 1)
-        {
-            if (threadIdx.x < st)
-                sh[threadIdx.x] = red_op<OP>(sh[threadIdx.x], sh[threadIdx.x + st]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0)
-            partial[blockIdx.x * ncol + col] = sh[0];
-        __syncthreads();
+        const real wi = w ? w[i] : 1.0;
+#pragma unroll
+        for (int v = 0; v < 8; v++)
+            if (v < ncol)
+            {
+                real xv = x[i * ncol + v];
+                xv = powP == 1 ? fabs(xv) : powP == 2 ? xv * xv : xv;
+                a[v] = red_op<OP>(a[v], xv * wi);
+            }
+    }
+#pragma unroll
+    for (int v = 0; v < 8; v++)
+    {
+        const real r = warp_red<OP>(a[v]);
+        if ((threadIdx.x & 31) == 0)
+            sh[threadIdx.x >> 5][v] = r;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < ncol)
+    {
+        real r = sh[0][threadIdx.x];
+        for (int k = 1; k < kRedBlock / 32; k++)
+            r = red_op<OP>(r, sh[k][threadIdx.x]);
+        partial[blockIdx.x * ncol + threadIdx.x] = r;
     }
 }
 
+// one warp per column
 template <int OP>
 DNDSB_GLOBAL void k_reduce_final(int nb, int ncol, const real *__restrict__ partial, real *out)
 {
-    __shared__ real sh[kRedBlock];
-    real init = OP == 0 ? 0.0 : OP == 1 ? kVeryLarge : -kVeryLarge;
-    for (int col = 0; col < ncol; col++)
-    {
-        real a = init;
-        for (int i = threadIdx.x; i < nb; i += blockDim.x)
-            a = red_op<OP>(a, partial[i * ncol + col]);
-        sh[threadIdx.x] = a;
-        __syncthreads();
-        for (int st = blockDim.x / 2; st > 0; st >>= 1)
-        {
-            if (threadIdx.x < st)
-                sh[threadIdx.x] = red_op<OP>(sh[threadIdx.x], sh[threadIdx.x + st]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0)
-            out[col] = sh[0];
-        __syncthreads();
-    }
+    const int col = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    real a = OP == 0 ? 0.0 : OP == 1 ? kVeryLarge : -kVeryLarge;
+    for (int i = lane; i < nb; i += 32)
+        a = red_op<OP>(a, partial[i * ncol + col]);
+    a = warp_red<OP>(a);
+    if (lane == 0)
+        out[col] = a;
 }
 
 } // namespace
@@ -76,20 +81,22 @@ DNDSB_GLOBAL void k_reduce_final(int nb, int ncol, const real *__restrict__ part
 real *reduce_cols(int op, int64_t n, int ncol, const real *x, const real *w, int powP, real *redBuf, cudaStream_t st)
 {
     real *out = redBuf + kRedBlocks * 8;
+    const int64_t want = (n + kRedBlock - 1) / kRedBlock;
+    const int nb = want < 1 ? 1 : want < kRedBlocks ? (int)want : kRedBlocks;
     if (op == 0)
     {
-        k_reduce_cols<0><<<kRedBlocks, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<0><<<1, kRedBlock, 0, st>>>(kRedBlocks, ncol, redBuf, out);
+        k_reduce_cols<0><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
+        k_reduce_final<0><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
     }
     else if (op == 1)
     {
-        k_reduce_cols<1><<<kRedBlocks, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<1><<<1, kRedBlock, 0, st>>>(kRedBlocks, ncol, redBuf, out);
+        k_reduce_cols<1><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
+        k_reduce_final<1><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
     }
     else
     {
-        k_reduce_cols<2><<<kRedBlocks, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<2><<<1, kRedBlock, 0, st>>>(kRedBlocks, ncol, redBuf, out);
+        k_reduce_cols<2><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
+        k_reduce_final<2><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
     }
     return out;
 }

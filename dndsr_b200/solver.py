@@ -387,10 +387,24 @@ class EulerEvaluator:
         """EulerSolver::solveLinear with LUSGSMatrixInit (EulerSolver.hxx:1407-1579, EulerEvaluator.hxx:37-159):
         xInc = M^-1 rhs by LU-SGS pairs (gmresCode 0), GMRES preconditioned by SGS pairs (1), or both (2),
         in FP64 or FP32; all on the device, no host synchronisation."""
-        ls = dict(gmresCode=int(gmresCode), jacobiCode=int(jacobiCode), sgsIter=int(sgsIter), nGmresSpace=int(nGmresSpace),
-                  nGmresIter=int(nGmresIter), precision=1 if precision == "fp32" else 0, useGraph=int(bool(useGraph)),
-                  meanScale=[float(x) for x in (meanScale if meanScale is not None else [])])
-        self._c.SolveLinear(ls, float(alphaDiag), dTau, float(dt), u, rhs, xInc)
+        self._c.SolveLinear(self.LinearSettings(gmresCode, jacobiCode, sgsIter, nGmresSpace, nGmresIter, precision, meanScale, useGraph),
+                            float(alphaDiag), dTau, float(dt), u, rhs, xInc)
+
+    @staticmethod
+    def LinearSettings(gmresCode=0, jacobiCode=1, sgsIter=0, nGmresSpace=5, nGmresIter=1, precision="fp64", meanScale=None, useGraph=True):
+        """linearSolverControl as SolveLinear and PseudoIteration take it."""
+        return dict(gmresCode=int(gmresCode), jacobiCode=int(jacobiCode), sgsIter=int(sgsIter), nGmresSpace=int(nGmresSpace),
+                    nGmresIter=int(nGmresIter), precision=1 if precision == "fp32" else 0, useGraph=int(bool(useGraph)),
+                    meanScale=[float(x) for x in (meanScale if meanScale is not None else [])])
+
+    def PseudoIteration(self, linear, CFL, alphaDiag, dt, u, uRec, uRecNew, resOther, rhs, res, dTau, xInc, nSweep=1, sweepPrecision="fp64",
+                        normOrd=1, normVolWise=False):
+        """One pseudo-time iteration of an implicit stage in one call (EulerSolver.hxx:147-997): local time step over
+        alphaDiag into dTau, nSweep sweeps of uRec, rhs = EvaluateRHS, res = resOther - u / dt + alphaDiag rhs, xInc =
+        SolveLinear (linear: LinearSettings), u += xInc; returns EvaluateNorm(res) and raises on a non-physical or
+        non-finite state, the call's one synchronisation."""
+        return self._c.PseudoIteration(linear, float(CFL), float(alphaDiag), float(dt), int(nSweep), 1 if sweepPrecision == "fp32" else 0,
+                                       int(normOrd), bool(normVolWise), u, uRec, uRecNew, resOther, rhs, res, dTau, xInc)
 
     def EvaluateNorm(self, x, P=1, volWise=True):
         return self._c.EvaluateNorm(x, int(P), bool(volWise))

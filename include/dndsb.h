@@ -368,6 +368,24 @@ typedef struct dndsb_linear_settings
  * zero, as the reference's fsolve does).  No host synchronisation. */
 int dndsb_eval_solve_linear(dndsb_eval *ev, const dndsb_linear_settings *ls, double alphaDiag, const double *dTau, double dt,
                             const double *u, const double *rhs, double *xInc, void *stream);
+/* One pseudo-time iteration of an implicit stage (EulerSolver.hxx:147-997: fdtau, frhs, fsolve, fincrement and the
+ * residual norm that fstop reads, without limiter, positivity fix or reconstruction GMRES) in one call:
+ *   dTau = local time step / alphaDiag; nSweep reconstruction sweeps of uRec (Jacobi, or SOR); rhs = EvaluateRHS;
+ *   res = resOther - u / dt + alphaDiag rhs; xInc = solve_linear(res); u += xInc; resNorm[nVars] = norm of res.
+ * Only the norm and the error word of the residual come back (one synchronisation); a non-physical or non-finite
+ * state gives the error that evaluate_rhs reports. */
+typedef struct dndsb_pseudo_settings
+{
+    dndsb_linear_settings linear;
+    double CFL, alphaDiag, dt;
+    int nSweep;         /* reconstruction sweeps (nInternalRecStep) */
+    int sweepPrecision; /* their coefficients: 0 FP64, 1 FP32 */
+    int normOrd;        /* 1, 2 or >= 3 (max norm) */
+    int normVolWise;
+} dndsb_pseudo_settings;
+int dndsb_eval_pseudo_iteration(dndsb_eval *ev, const dndsb_pseudo_settings *s, double *u, double *uRec, double *uRecNew,
+                                const double *resOther, double *rhs, double *res, double *dTau, double *xInc, double *resNorm,
+                                void *stream);
 /* EvaluateNorm(res, rhs, P, volWise), EulerEvaluator.hxx:1394-1439; P = 1, 2 or >= 3 (max norm) */
 int dndsb_eval_evaluate_norm(dndsb_eval *ev, const double *x, int P, int volWise, double *resHost, void *stream);
 /* named evaluator arrays to host: "lambdaFace", "lambdaFaceC", "lambdaFaceVis", "deltaLambdaCell" */
