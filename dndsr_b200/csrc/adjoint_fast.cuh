@@ -168,8 +168,7 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
     real p0[3] = {0, 0, 0}, n[3] = {0, 0, 0}, JW = 0;
     if (f < m.nFace)
     {
-        const real *pt = facePt + ((int64_t)q * m.nFace + f) * 7;
-        p0[0] = pt[0], p0[1] = pt[1], p0[2] = pt[2], n[0] = pt[3], n[1] = pt[4], n[2] = pt[5], JW = pt[6];
+        face_point(facePt, m.nFace, q, f, p0, n, JW);
     }
     __syncthreads();
     for (int e = tid; e < 64 * CS; e += nthr)

@@ -8,6 +8,14 @@
 // summed in a fixed order, so results are deterministic.  The basis and its
 // first derivatives are generated from compile-time exponent tables, so the
 // sparse derivative rows cost only their non-zero terms.
+//
+// Bound: FP64 and its latency at degree 2 (38 % of the pipe, 1.9 instructions per cycle at 9 points), the staging below
+// that.  A warp copies a cell's row with one or two asynchronous copies per lane and the point data lie in planes of
+// faces; filling the rows element by element (a division to find the element's cell, a register and a store each) and
+// reading 7-value point records took 898 us instead of 723 for 786,432 faces of degree 2 with 9 points and the viscous
+// flux, 526 us instead of 414 for the SA plate's 304,515 hexahedra.  One thread per face, its points in turn, was slower
+// than one per point at every size (inviscid flux of 221,400 faces: 93 against 75 us at degree 1, 265 against 147 us at
+// degree 2).
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "sa.cuh"
@@ -19,14 +27,16 @@ namespace
 {
 using namespace fastc;
 
-// resident blocks per SM the register budget is sized for (about 27 warps per SM: at 9 points per
-// face, 3 blocks of 288 threads with 72 registers each and some spilling beat 2 blocks with 96 by
-// 18 % on the TGV workload at 64^3)
-#ifndef DNDSB_RHS_WARPS_PER_SM
-#define DNDSB_RHS_WARPS_PER_SM 27
-#endif
-template <int NG>
-constexpr int min_blocks() { return (DNDSB_RHS_WARPS_PER_SM / NG) > 0 ? (DNDSB_RHS_WARPS_PER_SM / NG) : 1; }
+// resident blocks per SM the register budget is sized for: about 27 warps per SM (at 9 points per face, 3 blocks of 288
+// threads with 72 registers each and some spilling take 312 us against 332 us for 2 blocks with 96, 331,776 faces of
+// degree 2); 18 with few points above degree 1 (64 against 71 us for 196,608 edges of degree 2, 86 against 96 us at
+// degree 3, where degree 1 takes 60 against 58 us)
+template <int P, int NG>
+constexpr int min_blocks()
+{
+    constexpr int warps = P > 1 && NG <= 3 ? 18 : 27;
+    return warps / NG > 0 ? warps / NG : 1;
+}
 
 // MODE 0: the whole integrand; 1: the inviscid flux only, from point values without their gradients (the
 // evaluators that ignore viscosity).  Splitting a viscous evaluation into an inviscid and a viscous launch
@@ -35,63 +45,45 @@ constexpr int min_blocks() { return (DNDSB_RHS_WARPS_PER_SM / NG) > 0 ? (DNDSB_R
 // LAM: also record the face integrals of the Riemann eigenvalues divided by the area into lam [3][nFace]
 // (EvaluateRHS.hxx:527-545, for useRoeJacobian); a separate instantiation, so the default one is unchanged
 template <int DIM, int P, int NV, int NG, int MODE, bool LAM>
-__global__ void __launch_bounds__(32 * NG, min_blocks<NG>())
+__global__ void __launch_bounds__(32 * NG, min_blocks<P, NG>())
     k_rhs_face_fast(MeshD m, GeomD g, const real *__restrict__ facePt, const real *__restrict__ cellPar, const real *__restrict__ moment,
                     EulerSettingsD s, const real *__restrict__ u, const real *__restrict__ uRec, const real *__restrict__ dLamCell,
                     real *__restrict__ faceFlux, int *err, real *__restrict__ lam)
 {
     using Lt = Layout<DIM, P, NV>;
-    constexpr int CS = Lt::CS, R = Lt::R, NDOF = Lt::NDOF;
+    constexpr int CS = Lt::CS;
     extern __shared__ real sm[];
     real *sCell = sm;                                 // [64][CS]: slots 0..31 side-0 cells, 32..63 side-1 cells
     FaceData *sFace = (FaceData *)(sCell + 64 * CS);  // [32]
     real *sFlux = (real *)(sFace + 32);               // [NG][32][NV]
-    __shared__ int sC[64];
     const int tid = threadIdx.x;
     const int64_t f0 = (int64_t)blockIdx.x * 32;
     const real gamma = s.gamma, cp = s.Rgas * gamma / (gamma - 1);
-    if (tid < 32)
-    {
-        int64_t f = f0 + tid;
-        sC[tid] = f < m.nFace ? m.face2cell[f * 2] : -1;
-        sC[32 + tid] = f < m.nFace ? m.face2cell[f * 2 + 1] : -1;
-    }
-    // this thread's Gauss point (issued before the staging barriers so the loads overlap them)
     const int fl = tid & 31, q = tid >> 5;
     const int64_t f = f0 + fl;
+    // every warp holds the cells of the block's 32 faces and stages its share of their rows
+    const int c0 = f < m.nFace ? m.face2cell[f * 2] : -1, c1 = f < m.nFace ? m.face2cell[f * 2 + 1] : -1;
+#pragma unroll 4
+    for (int t = q; t < 64; t += NG)
+    {
+        const int c = __shfl_sync(0xffffffffu, t < 32 ? c0 : c1, t & 31);
+        if (c >= 0)
+            stage_cell<DIM, P, NV>(sCell + t * CS, c, fl, uRec, u, cellPar, moment);
+    }
+    copies_commit();
+    // this thread's Gauss point (its loads overlap the copies)
     real p0[3] = {0, 0, 0}, n[3] = {0, 0, 0}, JW = 0;
     if (f < m.nFace)
-    {
-        const real *pt = facePt + ((int64_t)q * m.nFace + f) * 7;
-        p0[0] = pt[0], p0[1] = pt[1], p0[2] = pt[2], n[0] = pt[3], n[1] = pt[4], n[2] = pt[5], JW = pt[6];
-    }
-    __syncthreads();
-    for (int e = tid; e < 64 * CS; e += blockDim.x)
-    {
-        int slot = e / CS, off = e - slot * CS;
-        int c = sC[slot];
-        real val = 0;
-        if (c >= 0)
-        {
-            if (off < Lt::OC)
-                val = off < Lt::OU ? uRec[(int64_t)c * (R * NV) + off] : u[(int64_t)c * NV + off - Lt::OU];
-            else if (off < Lt::OM)
-                val = cellPar[(int64_t)c * 6 + off - Lt::OC];
-            else if (off < Lt::OM + NDOF)
-                val = moment[(int64_t)c * NDOF + off - Lt::OM];
-            // off == OM + NDOF is the padding slot of an odd stride: nothing to read
-        }
-        sCell[e] = val;
-    }
+        face_point(facePt, m.nFace, q, f, p0, n, JW);
+    copies_wait<0>();
     __syncthreads();
     if (tid < 64)
     {
         // warp 0: Roe averages of the cell means; warp 1: dLambda and face geometry
-        int t = tid & 31;
-        int64_t ff = f0 + t;
-        int c0 = sC[t], c1 = sC[32 + t];
+        const int t = fl;
+        const int64_t ff = f;
         FaceData *fd = sFace + t;
-        if (ff < m.nFace && c1 >= 0)
+        if (c1 >= 0)
         {
             if (tid < 32)
             {
@@ -117,7 +109,7 @@ __global__ void __launch_bounds__(32 * NG, min_blocks<NG>())
 #pragma unroll
     for (int v = 0; v < NV; v++)
         out[v] = 0;
-    if (f < m.nFace && sC[32 + fl] >= 0)
+    if (c1 >= 0)
     {
         const FaceData *fd = sFace + fl;
         real p1[3] = {p0[0] + fd->shift[0], p0[1] + fd->shift[1], p0[2] + fd->shift[2]};
@@ -138,7 +130,6 @@ __global__ void __launch_bounds__(32 * NG, min_blocks<NG>())
         for (int v = 0; v < NV; v++)
             Fv[v] = 0;
         if constexpr (MODE != 1)
-            if (!s.ignoreVis)
         {
             real distGRP = fd->gbase;
             distGRP = dmax(dmin(fabs(fd->db[0] * n[0] + fd->db[1] * n[1] + fd->db[2] * n[2]), distGRP * 2), distGRP * 0.25);
@@ -218,7 +209,7 @@ __global__ void __launch_bounds__(32 * NG, min_blocks<NG>())
         {
             int fi = e / 3, i = e - fi * 3;
             int64_t ff = f0 + fi;
-            if (ff < m.nFace && sC[32 + fi] >= 0) // boundary faces are recorded by the boundary kernel
+            if (ff < m.nFace && m.face2cell[ff * 2 + 1] >= 0) // boundary faces are recorded by the boundary kernel
             {
                 real acc = 0;
 #pragma unroll
@@ -230,7 +221,7 @@ __global__ void __launch_bounds__(32 * NG, min_blocks<NG>())
     }
 }
 
-// facePt [NG][nFace][7] = point, unit normal, |J| w   and cellPar [nCell][6] = centre, 1/L
+// facePt [NG][7][nFace] = point, unit normal, |J| w   and cellPar [nCell][6] = centre, 1/L
 DNDSB_GLOBAL void k_face_points(int64_t nFace, int nG, const real *__restrict__ pp, const real *__restrict__ nrm, const real *__restrict__ jd,
                                 const real *__restrict__ qw, real *out)
 {
@@ -238,10 +229,10 @@ DNDSB_GLOBAL void k_face_points(int64_t nFace, int nG, const real *__restrict__ 
     {
         int64_t f = i / nG;
         int q = (int)(i - f * nG);
-        real *o = out + ((int64_t)q * nFace + f) * 7;
+        real *o = out + (int64_t)q * 7 * nFace + f;
         for (int d = 0; d < 3; d++)
-            o[d] = pp[i * 3 + d], o[3 + d] = nrm[i * 3 + d];
-        o[6] = jd[i] * qw[q];
+            o[d * nFace] = pp[i * 3 + d], o[(3 + d) * nFace] = nrm[i * 3 + d];
+        o[6 * nFace] = jd[i] * qw[q];
     }
 }
 

@@ -26,6 +26,44 @@ struct Layout
     static constexpr int CS = (OM + NDOF) | 1; // odd stride: lanes of a warp (different faces) hit different banks
 };
 
+// asynchronous copy of one double to shared memory, and its group bookkeeping
+DNDSB_D void copy8_async(void *smem, const void *g)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g));
+}
+DNDSB_D void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+DNDSB_D void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// point, unit normal and |J| w of Gauss point q of face f: facePt is [nGf][7][nFace], so the faces of a warp read lines
+DNDSB_D void face_point(const real *__restrict__ facePt, int64_t nFace, int q, int64_t f, real *p, real *n, real &JW)
+{
+    const real *pt = facePt + (int64_t)q * 7 * nFace + f;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        p[d] = pt[d * nFace], n[d] = pt[(3 + d) * nFace];
+    JW = pt[6 * nFace];
+}
+
+// the lanes of a warp start copying the row of cell c (uRec, u, centre, 1/L, moments) to dst: the copies run along the
+// row, so a row costs a few cache lines and no register
+template <int DIM, int P, int NV>
+DNDSB_D void stage_cell(real *dst, int64_t c, int lane, const real *uRec, const real *u, const real *cellPar, const real *moment)
+{
+    using Lt = Layout<DIM, P, NV>;
+    constexpr int LEN = Lt::OM + Lt::NDOF;
+#pragma unroll
+    for (int e0 = 0; e0 < LEN; e0 += 32)
+    {
+        const int e = e0 + lane;
+        if (e < LEN)
+            copy8_async(dst + e, e < Lt::OU   ? uRec + c * (Lt::R * NV) + e
+                                 : e < Lt::OC ? u + c * NV + (e - Lt::OU)
+                                 : e < Lt::OM ? cellPar + c * 6 + (e - Lt::OC)
+                                              : moment + c * Lt::NDOF + (e - Lt::OM));
+    }
+}
+
 // per-face data shared by the Gauss points of a face (29 doubles: an odd stride in shared memory)
 struct FaceData
 {
@@ -38,7 +76,6 @@ struct FaceData
 };
 static_assert(sizeof(FaceData) == 29 * sizeof(real), "FaceData layout");
 
-// u + phi . uRec and the gradient D1 phi . uRec of one cell at point p (VariationalReconstruction.hpp:378-442 rows 0..dim)
 // u + phi . uRec of one cell at point p, without the gradient
 template <int DIM, int P, int NV>
 DNDSB_D void recon_value(const real *cell, const real *p, real *U)
@@ -62,6 +99,7 @@ DNDSB_D void recon_value(const real *cell, const real *p, real *U)
     }
 }
 
+// u + phi . uRec and the gradient D1 phi . uRec of one cell at point p (VariationalReconstruction.hpp:378-442 rows 0..dim)
 template <int DIM, int P, int NV, bool ACC>
 DNDSB_D void recon_point(const real *cell, const real *p, real *U, real *G)
 {

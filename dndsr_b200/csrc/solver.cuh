@@ -144,7 +144,7 @@ struct EvalD
     real *lambdaFace = nullptr, *lambdaFaceC = nullptr, *lambdaFaceVis = nullptr, *lambdaConv = nullptr, *deltaLambdaFace = nullptr;
     real *deltaLambdaCell = nullptr;
     real *faceFlux = nullptr; // scratch [nFace][nv]
-    real *facePt = nullptr;   // [nGf][nFace][7]: point, unit normal, |J| w (layout of the tuned face kernel)
+    real *facePt = nullptr;   // [nGf][7][nFace]: point, unit normal, |J| w (layout of the tuned face kernels)
     real *cellPar = nullptr;  // [nCell][6]: centre, 1/L
     real *redBuf = nullptr;   // scratch for reductions
     real *adjBuf = nullptr;   // scratch of the derivative kernels [nFace][2][(R+1) nv], allocated on first use

@@ -18,18 +18,15 @@
 // of the neighbour and the lanes exchange rows by shuffles, so a row costs NV loads instead of R NV broadcasts.
 #include "solver.cuh"
 #include "sweep_layout.cuh"
+#include "fast_common.cuh"
 
 namespace dndsb
 {
 namespace
 {
-DNDSB_D void copy8_async(void *smem, const void *g)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g));
-}
-DNDSB_D void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-DNDSB_D void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+using fastc::copies_commit;
+using fastc::copies_wait;
+using fastc::copy8_async;
 
 template <int R, int NV>
 struct Stage
