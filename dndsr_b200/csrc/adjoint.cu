@@ -16,6 +16,7 @@
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "bc.cuh"
+#include "vr_vjp.cuh"
 
 namespace dndsb
 {
@@ -38,31 +39,28 @@ DNDSB_D void recon_value(const real *T, const real *u, const real *rec, real *U)
     }
 }
 
-// cotangent of one interior or boundary face: faceAdj[f][side][(R+1)][NV], entry 0 = d/du, 1+j = d/duRec_j
+// cotangent of the interior faces: faceAdj[f][side][(R+1)][NV], entry 0 = d/du, 1+j = d/duRec_j
 template <int DIM, int P>
 DNDSB_GLOBAL void k_rhs_vjp_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w, const real *__restrict__ u,
-                                 const real *__restrict__ uRec, const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err,
-                                 int boundaryOnly)
+                                 const real *__restrict__ uRec, const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV;
     const real gamma = s.gamma;
-    // boundaryOnly: the boundary faces of the list m.bndFace (the reverse-mode Roe kernel writes the others)
-    DNDSB_KERNEL_LOOP(ii, boundaryOnly ? m.nBndFace : m.nFace)
+    DNDSB_KERNEL_LOOP(f, m.nFace)
     {
-        const int64_t f = boundaryOnly ? (int64_t)m.bndFace[ii] : ii;
         const real *nMV = s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr; // batched mean-value eigenvalues
         int64_t c0 = m.face2cell[f * 2], c1 = m.face2cell[f * 2 + 1];
-        bool bnd = c1 < 0;
-        int zone = m.faceZone[f];
+        if (c1 < 0)
+            continue; // k_rhs_vjp_bnd
         real *o0 = faceAdj + (f * 2) * W, *o1 = faceAdj + (f * 2 + 1) * W;
         for (int i = 0; i < W; i++)
             o0[i] = 0, o1[i] = 0;
         real gbar[NV];
         for (int v = 0; v < NV; v++)
-            gbar[v] = w[c0 * NV + v] / g.vol[c0] - (bnd ? 0.0 : w[c1 * NV + v] / g.vol[c1]);
+            gbar[v] = w[c0 * NV + v] / g.vol[c0] - w[c1 * NV + v] / g.vol[c1];
         const real *ULm = u + c0 * NV;
-        const real *URm = bnd ? nullptr : u + c1 * NV;
-        real dLambda = bnd ? dLamCell[c0] : dmax(dLamCell[c0], dLamCell[c1]);
+        const real *URm = u + c1 * NV;
+        real dLambda = dmax(dLamCell[c0], dLamCell[c1]);
         real ULmbar[NV] = {0, 0, 0, 0, 0}, URmbar[NV] = {0, 0, 0, 0, 0};
         bool bad = false;
         for (int q = 0; q < g.nGf; q++)
@@ -84,54 +82,31 @@ DNDSB_GLOBAL void k_rhs_vjp_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, con
             recon_value<R>(T0, u + c0 * NV, uRec + c0 * R * NV, UL);
             real ULbar[NV] = {0, 0, 0, 0, 0}, URbar[NV] = {0, 0, 0, 0, 0};
             D10 F[NV], l0, l1, l4;
-            if (!bnd)
-            {
-                cell_basis<DIM, NDOF>(&g.cellCent[c1 * 3], &g.cellScale[c1 * 3], &vr.baseMoment[c1 * NDOF], vr.s.anisotropicLengths, p1, 1, T1);
-                recon_value<R>(T1, u + c1 * NV, uRec + c1 * R * NV, UR);
-                // pass 1: point states UL (0..4), UR (5..9)
-                D10 ULd[NV], URd[NV], ULmd[NV], URmd[NV];
-                for (int v = 0; v < NV; v++)
-                    ULd[v] = D10::var(UL[v], v), URd[v] = D10::var(UR[v], 5 + v), ULmd[v] = D10(ULm[v]), URmd[v] = D10(URm[v]);
-                bad |= !riemann_flux(s.rsType, ULd, URd, ULmd, URmd, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4, nMV);
-                for (int v = 0; v < NV; v++)
-                    for (int i = 0; i < NV; i++)
-                        ULbar[i] += F[v].d[i] * Fbar[v], URbar[i] += F[v].d[5 + i] * Fbar[v];
-                // pass 2: cell means ULm (0..4), URm (5..9) through the Roe averages
-                for (int v = 0; v < NV; v++)
-                    ULd[v] = D10(UL[v]), URd[v] = D10(UR[v]), ULmd[v] = D10::var(ULm[v], v), URmd[v] = D10::var(URm[v], 5 + v);
-                bad |= !riemann_flux(s.rsType, ULd, URd, ULmd, URmd, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4, nMV);
-                for (int v = 0; v < NV; v++)
-                    for (int i = 0; i < NV; i++)
-                        ULmbar[i] += F[v].d[i] * Fbar[v], URmbar[i] += F[v].d[5 + i] * Fbar[v];
-            }
-            else
-            {
-                // boundary: UR = ghost(UL) at this point, URm = ghost(ULm) at the face centre
-                D10 ULd[NV], URd[NV], ULmd[NV], URmd[NV];
-                for (int v = 0; v < NV; v++)
-                    ULd[v] = D10::var(UL[v], v), ULmd[v] = D10::var(ULm[v], 5 + v);
-                if (!bc_value<NV>(vr.bnd, zone, ULd, n, URd))
-                    for (int v = 0; v < NV; v++)
-                        URd[v] = ULd[v];
-                if (!bc_value<NV>(vr.bnd, zone, ULmd, &g.faceMeanNorm[f * 3], URmd))
-                    for (int v = 0; v < NV; v++)
-                        URmd[v] = ULmd[v];
-                bad |= !riemann_flux(s.rsType, ULd, URd, ULmd, URmd, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4, nMV);
-                for (int v = 0; v < NV; v++)
-                    for (int i = 0; i < NV; i++)
-                        ULbar[i] += F[v].d[i] * Fbar[v], ULmbar[i] += F[v].d[5 + i] * Fbar[v];
-            }
+            cell_basis<DIM, NDOF>(&g.cellCent[c1 * 3], &g.cellScale[c1 * 3], &vr.baseMoment[c1 * NDOF], vr.s.anisotropicLengths, p1, 1, T1);
+            recon_value<R>(T1, u + c1 * NV, uRec + c1 * R * NV, UR);
+            // pass 1: point states UL (0..4), UR (5..9)
+            D10 ULd[NV], URd[NV], ULmd[NV], URmd[NV];
+            for (int v = 0; v < NV; v++)
+                ULd[v] = D10::var(UL[v], v), URd[v] = D10::var(UR[v], 5 + v), ULmd[v] = D10(ULm[v]), URmd[v] = D10(URm[v]);
+            bad |= !riemann_flux(s.rsType, ULd, URd, ULmd, URmd, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4, nMV);
+            for (int v = 0; v < NV; v++)
+                for (int i = 0; i < NV; i++)
+                    ULbar[i] += F[v].d[i] * Fbar[v], URbar[i] += F[v].d[5 + i] * Fbar[v];
+            // pass 2: cell means ULm (0..4), URm (5..9) through the Roe averages
+            for (int v = 0; v < NV; v++)
+                ULd[v] = D10(UL[v]), URd[v] = D10(UR[v]), ULmd[v] = D10::var(ULm[v], v), URmd[v] = D10::var(URm[v], 5 + v);
+            bad |= !riemann_flux(s.rsType, ULd, URd, ULmd, URmd, n, gamma, dLambda, s.rsFixScale, s.rsIncFScale, F, l0, l1, l4, nMV);
+            for (int v = 0; v < NV; v++)
+                for (int i = 0; i < NV; i++)
+                    ULmbar[i] += F[v].d[i] * Fbar[v], URmbar[i] += F[v].d[5 + i] * Fbar[v];
             for (int v = 0; v < NV; v++)
             {
                 o0[v] += ULbar[v];
                 for (int j = 0; j < R; j++)
                     o0[NV + j * NV + v] += T0[1 + j] * ULbar[v];
-                if (!bnd)
-                {
-                    o1[v] += URbar[v];
-                    for (int j = 0; j < R; j++)
-                        o1[NV + j * NV + v] += T1[1 + j] * URbar[v];
-                }
+                o1[v] += URbar[v];
+                for (int j = 0; j < R; j++)
+                    o1[NV + j * NV + v] += T1[1 + j] * URbar[v];
             }
         }
         for (int v = 0; v < NV; v++)
@@ -141,26 +116,74 @@ DNDSB_GLOBAL void k_rhs_vjp_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, con
     }
 }
 
-// du_c = sum over the cell's faces of the face cotangents of its side (fixed face order)
-template <int W>
-DNDSB_GLOBAL void k_adj_gather(int64_t nCell, int nf, const int32_t *__restrict__ c2f, const real *__restrict__ faceAdj, real *du, real *duRec)
+// The same for the boundary faces (side 0): the ghost states are differentiated with the flux, with respect to the point
+// state (pass 0) and to the cell mean at the face centre (pass 1), five seeds each.  Thread (pass, face, point), one
+// warp per pass, the sums over the points shared out in point order: a thread that walked both passes and the points of a
+// face took 103 us for 19,040 faces of 3 points, this 87 us.
+template <int DIM, int P>
+DNDSB_GLOBAL void __launch_bounds__(64) k_rhs_vjp_bnd(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w,
+                                                      const real *__restrict__ u, const real *__restrict__ uRec,
+                                                      const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
 {
-    DNDSB_KERNEL_LOOP(c, nCell)
+    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV, ROW = (2 * NV + R) | 1;
+    using D5 = Dual<NV>;
+    __shared__ real sm[32][ROW]; // per point: d/dU, d/du (the mean), phi
+    const int nG = g.nGf, rows = 32 / nG, lane = threadIdx.x & 31, pass = threadIdx.x >> 5;
+    const int fl = lane / nG, q = lane - fl * nG;
+    const int64_t ii = (int64_t)blockIdx.x * rows + fl;
+    if (fl < rows && ii < m.nBndFace)
     {
-        real acc[W];
-        for (int i = 0; i < W; i++)
-            acc[i] = 0;
-        for (int k = 0; k < nf; k++)
-        {
-            int fp = c2f[c * nf + k];
-            const real *src = faceAdj + ((int64_t)(fp >> 1) * 2 + (fp & 1)) * W;
-            for (int i = 0; i < W; i++)
-                acc[i] += src[i];
-        }
+        const int64_t f = m.bndFace[ii], c0 = m.face2cell[f * 2];
+        const int zone = m.faceZone[f];
+        const real *n = &g.faceNorm[(f * nG + q) * 3];
+        const real JW = g.faceJDet[f * nG + q] * g.faceQw[q], iv = 1.0 / g.vol[c0];
+        real phi[R];
+        basis_rows<DIM, P, false>(g, vr, c0, &g.facePP[(f * nG + q) * 3], phi, nullptr);
+        D5 UL[NV], UR[NV], ULm[NV], URm[NV], F[NV], l0, l1, l4;
+#pragma unroll
         for (int v = 0; v < NV; v++)
-            du[c * NV + v] = acc[v];
-        for (int i = NV; i < W; i++)
-            duRec[c * (W - NV) + i - NV] = acc[i];
+        {
+            real a = u[c0 * NV + v];
+            ULm[v] = D5::var(a, pass == 1 ? v : -1);
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                a += phi[j] * uRec[(c0 * R + j) * NV + v];
+            UL[v] = D5::var(a, pass == 0 ? v : -1);
+        }
+        if (!bc_value<NV>(vr.bnd, zone, UL, n, UR))
+            for (int v = 0; v < NV; v++)
+                UR[v] = UL[v];
+        if (!bc_value<NV>(vr.bnd, zone, ULm, &g.faceMeanNorm[f * 3], URm))
+            for (int v = 0; v < NV; v++)
+                URm[v] = ULm[v];
+        if (!riemann_flux(s.rsType, UL, UR, ULm, URm, n, s.gamma, dLamCell[c0], s.rsFixScale, s.rsIncFScale, F, l0, l1, l4,
+                          s.rsMeanValueEig ? &g.faceMeanNorm[f * 3] : nullptr))
+            atomicOr(err, (int)DE_NONPHYSICAL);
+        for (int i = 0; i < NV; i++)
+        {
+            real a = 0;
+            for (int v = 0; v < NV; v++)
+                a -= F[v].d[i] * (JW * (w[c0 * NV + v] * iv));
+            sm[lane][pass * NV + i] = a;
+        }
+        if (pass == 0)
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                sm[lane][2 * NV + j] = phi[j];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < rows * W; e += 64)
+    {
+        const int fi = e / W, i = e - fi * W, j = i / NV - 1, v = i - (j + 1) * NV;
+        if ((int64_t)blockIdx.x * rows + fi >= m.nBndFace)
+            break;
+        real acc = 0;
+        for (int p = 0; p < nG; p++)
+        {
+            const real *r = sm[fi * nG + p];
+            acc += j < 0 ? r[v] + r[NV + v] : r[2 * NV + j] * r[v];
+        }
+        faceAdj[(int64_t)m.bndFace[(int64_t)blockIdx.x * rows + fi] * 2 * W + i] = acc;
     }
 }
 
@@ -275,12 +298,11 @@ DNDSB_GLOBAL void k_flux_gather(int64_t nCell, int nf, const int32_t *__restrict
 // one Jacobi sweep uRecNew = S(uRec, u) (VariationalReconstruction_Reconstruction.hxx:485-615):
 //   uRecNew_i = (1-w) uRec_i + w sum_k [M_ik uRec_k + b_ik (u_k - u_i)] + w A_i^-1 BCC_i(u_i, uRec_i)
 // ---------------------------------------------------------------------------
-// derivative of the boundary term of cell c: BCC = sum_q w0^2 |J| w phi_q (UB_q - u_c) with
-// UB_q = ghost(compress(u_c, u_c + phi_q . uRec_c)); mode 0: VJP of t (R x NV cotangent of BCC)
-// into (vRec, vU); mode 1: JVP (dRec, du) -> dBCC
+// tangent of the boundary term of cell c along (dRec, du): BCC = sum_q w0^2 |J| w phi_q (UB_q - u_c) with
+// UB_q = ghost(compress(u_c, u_c + phi_q . uRec_c)); its transpose is k_vr_vjp_bnd
 template <int DIM, int P>
-DNDSB_D void bcc_derivative(const MeshD &m, const GeomD &g, const VRD &vr, int64_t c, const real *u, const real *uRec, int mode, const real *t,
-                            real *vRec, real *vU, const real *dRec, const real *duc, real *dBCC)
+DNDSB_D void bcc_tangent(const MeshD &m, const GeomD &g, const VRD &vr, int64_t c, const real *u, const real *uRec, const real *dRec,
+                         const real *duc, real *dBCC)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
     const real *uc = u + c * NV, *rc = uRec + c * R * NV;
@@ -310,116 +332,24 @@ DNDSB_D void bcc_derivative(const MeshD &m, const GeomD &g, const VRD &vr, int64
             if (!bc_value<NV>(vr.bnd, zone, ULf, n, UB))
                 for (int v = 0; v < NV; v++)
                     UB[v] = ULf[v];
-            if (mode == 0)
+            real dUL[NV];
+            for (int v = 0; v < NV; v++)
             {
-                real UBbar[NV];
-                for (int v = 0; v < NV; v++)
-                {
-                    real a = 0;
-                    for (int i = 0; i < R; i++)
-                        a += T[1 + i] * t[i * NV + v];
-                    UBbar[v] = a * JW;
-                    vU[v] -= UBbar[v];
-                }
+                real a = duc[v];
+                for (int j = 0; j < R; j++)
+                    a += T[1 + j] * dRec[j * NV + v];
+                dUL[v] = a;
+            }
+            for (int v = 0; v < NV; v++)
+            {
+                real dUB = 0;
                 for (int i = 0; i < NV; i++)
-                {
-                    real gl = 0, gm = 0;
-                    for (int v = 0; v < NV; v++)
-                        gl += UB[v].d[i] * UBbar[v], gm += UB[v].d[5 + i] * UBbar[v];
-                    vU[i] += gl + gm;
-                    for (int j = 0; j < R; j++)
-                        vRec[j * NV + i] += T[1 + j] * gl;
-                }
-            }
-            else
-            {
-                real dUL[NV];
-                for (int v = 0; v < NV; v++)
-                {
-                    real a = duc[v];
-                    for (int j = 0; j < R; j++)
-                        a += T[1 + j] * dRec[j * NV + v];
-                    dUL[v] = a;
-                }
-                for (int v = 0; v < NV; v++)
-                {
-                    real dUB = 0;
-                    for (int i = 0; i < NV; i++)
-                        dUB += UB[v].d[i] * dUL[i] + UB[v].d[5 + i] * duc[i];
-                    real dd = (dUB - duc[v]) * JW;
-                    for (int i = 0; i < R; i++)
-                        dBCC[i * NV + v] += T[1 + i] * dd;
-                }
+                    dUB += UB[v].d[i] * dUL[i] + UB[v].d[5 + i] * duc[i];
+                real dd = (dUB - duc[v]) * JW;
+                for (int i = 0; i < R; i++)
+                    dBCC[i * NV + v] += T[1 + i] * dd;
             }
         }
-    }
-}
-
-// VJP of the sweep: v = cotangent of uRecNew -> vRec (of uRec), vU (of u); gathered per cell o
-template <int DIM, int P>
-DNDSB_GLOBAL void k_vr_vjp(MeshD m, GeomD g, VRD vr, const real *__restrict__ v, const real *__restrict__ uRec, const real *__restrict__ u,
-                           real *vRec, real *vU)
-{
-    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
-    const real om = vr.s.jacobiRelax;
-    const int nf = m.nf;
-    DNDSB_KERNEL_LOOP(o, m.nCell)
-    {
-        real aRec[R * NV], aU[NV] = {0, 0, 0, 0, 0};
-        const real *vo = v + o * R * NV;
-        for (int i = 0; i < R * NV; i++)
-            aRec[i] = (1 - om) * vo[i];
-        bool hasBnd = false;
-        for (int j = 0; j < nf; j++)
-        {
-            int i = m.cellNbr[o * nf + j];
-            if (i < 0)
-            {
-                hasBnd = true;
-                continue;
-            }
-            int k = m.nbrSlot[o * nf + j];
-            const real *M = vr.AAInvB + ((int64_t)i * (nf + 1) + 1 + k) * R * R;
-            const real *b = vr.AInvb + ((int64_t)i * nf + k) * R;
-            const real *vi = v + (int64_t)i * R * NV;
-            // neighbour i's row k reads uRec_o and u_o: transpose into o
-            for (int r = 0; r < R; r++)
-                for (int x = 0; x < NV; x++)
-                {
-                    real a = 0;
-                    for (int l = 0; l < R; l++)
-                        a += M[l * R + r] * vi[l * NV + x];
-                    aRec[r * NV + x] += om * a;
-                }
-            // b_ik (u_o - u_i): + into o, and o's own row: - b_oj (u_o) for its own slot j
-            const real *bo = vr.AInvb + (o * nf + j) * R;
-            for (int x = 0; x < NV; x++)
-            {
-                real a = 0, a2 = 0;
-                for (int l = 0; l < R; l++)
-                    a += b[l] * vi[l * NV + x], a2 += bo[l] * vo[l * NV + x];
-                aU[x] += om * (a - a2);
-            }
-        }
-        if (hasBnd && vr.bnd.nZone > 0)
-        {
-            // t = w A_o^-T v_o, the cotangent of BCC_o
-            const real *Ai = vr.AAInvB + (o * (nf + 1)) * R * R;
-            real t[R * NV];
-            for (int r = 0; r < R; r++)
-                for (int x = 0; x < NV; x++)
-                {
-                    real a = 0;
-                    for (int l = 0; l < R; l++)
-                        a += Ai[l * R + r] * vo[l * NV + x];
-                    t[r * NV + x] = om * a;
-                }
-            bcc_derivative<DIM, P>(m, g, vr, o, u, uRec, 0, t, aRec, aU, nullptr, nullptr, nullptr);
-        }
-        for (int i = 0; i < R * NV; i++)
-            vRec[o * R * NV + i] = aRec[i];
-        for (int x = 0; x < NV; x++)
-            vU[o * NV + x] = aU[x];
     }
 }
 
@@ -461,7 +391,7 @@ DNDSB_GLOBAL void k_vr_jvp(MeshD m, GeomD g, VRD vr, const real *__restrict__ dR
             real dB[R * NV];
             for (int i = 0; i < R * NV; i++)
                 dB[i] = 0;
-            bcc_derivative<DIM, P>(m, g, vr, c, u, uRec, 1, nullptr, nullptr, nullptr, dRec + c * R * NV, du + c * NV, dB);
+            bcc_tangent<DIM, P>(m, g, vr, c, u, uRec, dRec + c * R * NV, du + c * NV, dB);
             const real *Ai = vr.AAInvB + (c * (nf + 1)) * R * R;
             for (int r = 0; r < R; r++)
                 for (int x = 0; x < NV; x++)
@@ -486,7 +416,14 @@ int rhs_vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const r
     // the hand-reversed Roe kernel takes the point-normal eigenvalues; the batched mean-value variant
     // (rsMeanValueEig with Roe_M1..M5) runs through the forward-mode face kernel on every face
     const int roe = roe_scheme_of(ev.s.rsType) >= 0 && !(ev.s.rsMeanValueEig && ev.s.rsType >= RS_Roe_M1 && ev.s.rsType <= RS_Roe_M1 + 4);
-    DNDSB_LAUNCH(kf, roe ? m.nBndFace : m.nFace, 64, st, m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord, roe);
+    if (!roe)
+        DNDSB_LAUNCH(kf, m.nFace, 64, st, m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
+    if (m.nBndFace > 0)
+    {
+        const int rows = 32 / g.nGf; // at most 16 points per face
+        k_rhs_vjp_bnd<DIM, P><<<(unsigned)((m.nBndFace + rows - 1) / rows), 64, 0, st>>>(m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf,
+                                                                                       ev.errWord);
+    }
     bool viscDone = false;
     if (roe)
     {
@@ -500,8 +437,8 @@ int rhs_vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const r
         if (rc != ST_OK)
             return rc;
     }
-    auto kg = k_adj_gather<W>;
-    DNDSB_LAUNCH(kg, m.nCell, 128, st, m.nCell, m.nf, m.cell2face, ev.adjBuf, du, duRec);
+    auto kg = k_adj_gather<W, NV>;
+    DNDSB_LAUNCH(kg, m.nCell * W, 256, st, m.nCell, m.nf, m.cell2face, ev.adjBuf, du, duRec);
     return ST_OK;
 }
 
@@ -546,8 +483,7 @@ template <int DIM, int P>
 int vr_vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, const real *v, const real *uRec, const real *u, real *vRec, real *vU,
               cudaStream_t st)
 {
-    auto k = k_vr_vjp<DIM, P>;
-    DNDSB_LAUNCH(k, m.nCell, 64, st, m, g, vr, v, uRec, u, vRec, vU);
+    launch_vr_vjp<DIM, P, NV>(m, g, vr, v, uRec, u, vRec, vU, st);
     return ST_OK;
 }
 

@@ -12,9 +12,11 @@
 //     row_j,v = sum_q [phi_j(p_q) Ub_q,v + sum_d dphi_j/dx_d(p_q) GMb_q,d,v],
 // are summed over the points in point order through shared memory, all rows in one round (or half of them
 // per round where the shares would not fit).  The Roe-average cotangents are summed the same way and
-// carried to the two cell means by a
-// Dual<1> evaluation of the averages per mean component (one thread each).  The block's face records
-// [32][2][(R+1) NV] are assembled in shared memory and stored row-contiguously.
+// carried to the two cell means by the
+// reverse of the averages, one thread per side.  The block's face records [32][2][(R+1) NV] are assembled in shared
+// memory and stored row-contiguously.
+//
+// The inviscid flux at degree 1 takes k_rhs_vjp_inviscid below, one thread per face.
 #pragma once
 #include "solver.cuh"
 #include "fast_common.cuh"
@@ -26,7 +28,6 @@ namespace dndsb
 namespace
 {
 using namespace fastc;
-using D1 = Dual<1>;
 
 // resident blocks per SM the register budget is sized for (two blocks of 9 warps at 9 points per face)
 template <int NG>
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
 {
     using Lt = Layout<DIM, P, NV>;
     using Rows = VjpRows<DIM, P, NV, NG, VISC>;
-    constexpr int CS = Lt::CS, R = Lt::R, NDOF = Lt::NDOF, W = Rows::W, CH = Rows::CH;
+    constexpr int CS = Lt::CS, W = Rows::W, CH = Rows::CH;
     extern __shared__ real sm[];
     real *sCell = sm;                                // [64][CS]: slots 0..31 side-0 cells, 32..63 side-1 cells
     FaceData *sFace = (FaceData *)(sCell + 64 * CS); // [32]
@@ -171,24 +172,13 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
         face_point(facePt, m.nFace, q, f, p0, n, JW);
     }
     __syncthreads();
-    for (int e = tid; e < 64 * CS; e += nthr)
-    {
-        int slot = e / CS, off = e - slot * CS;
-        int c = sC[slot];
-        real val = 0;
-        if (c >= 0)
-        {
-            if (off < Lt::OC)
-                val = off < Lt::OU ? uRec[(int64_t)c * (R * NV) + off] : u[(int64_t)c * NV + off - Lt::OU];
-            else if (off < Lt::OM)
-                val = cellPar[(int64_t)c * 6 + off - Lt::OC];
-            else if (off < Lt::OM + NDOF)
-                val = moment[(int64_t)c * NDOF + off - Lt::OM];
-        }
-        sCell[e] = val;
-    }
+    for (int t = tid >> 5; t < 64; t += NG)
+        if (sC[t] >= 0)
+            stage_cell<DIM, P, NV>(sCell + t * CS, sC[t], tid & 31, uRec, u, cellPar, moment);
+    copies_commit();
     for (int e = tid; e < 32 * 2 * W; e += nthr)
         sOut[e] = 0;
+    copies_wait<0>();
     __syncthreads();
     if (tid < 64)
     {
@@ -330,26 +320,23 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
         }
         __syncthreads();
     }
-    // ... carried to the cell means: thread e -> face e % 32, mean component e / 32 (side (e / 32) / NV)
-    for (int e = tid; e < 32 * 2 * NV; e += nthr)
+    // ... carried to the cell means: one thread per (face, side)
+    for (int e = tid; e < 64; e += nthr)
     {
-        const int fi = e & 31, i = e >> 5;
+        const int fi = e & 31, side = e >> 5;
         if (f0 + fi < m.nFace && sC[32 + fi] >= 0)
         {
-            const real *m0 = sCell + fi * CS + Lt::OU, *m1 = sCell + (32 + fi) * CS + Lt::OU;
-            RoeAvgT<D1> rD;
-            D1 a[NV], b[NV];
-#pragma unroll
-            for (int v = 0; v < NV; v++)
-                a[v] = D1::var(m0[v], i == v ? 0 : -1), b[v] = D1::var(m1[v], i == NV + v ? 0 : -1);
-            roe_average(a, b, gamma, rD);
             const real *t = sT + fi;
-            real x = t[9 * 32] * rD.aL.d[0] + t[10 * 32] * rD.aR.d[0] + t[11 * 32] * rD.vsqr.d[0] + t[12 * 32] * rD.H.d[0] +
-                     t[13 * 32] * rD.asqr.d[0] + t[14 * 32] * rD.a.d[0];
+            roe_rev::RoeBar b;
 #pragma unroll
             for (int d = 0; d < 3; d++)
-                x += t[d * 32] * rD.v[d].d[0] + t[(3 + d) * 32] * rD.vL[d].d[0] + t[(6 + d) * 32] * rD.vR[d].d[0];
-            sOut[fi * 2 * W + (i / NV) * W + i % NV] = x;
+                b.v[d] = t[d * 32], b.vL[d] = t[(3 + d) * 32], b.vR[d] = t[(6 + d) * 32];
+            b.aL = t[9 * 32], b.aR = t[10 * 32], b.vsqr = t[11 * 32], b.H = t[12 * 32], b.asqr = t[13 * 32], b.a = t[14 * 32];
+            real Ub[5];
+            roe_rev::roe_average_rev(side, sCell + fi * CS + Lt::OU, sCell + (32 + fi) * CS + Lt::OU, sFace[fi].r, gamma, b, Ub);
+#pragma unroll
+            for (int v = 0; v < 5; v++)
+                sOut[fi * 2 * W + side * W + v] = Ub[v];
         }
     }
     __syncthreads();
@@ -364,15 +351,161 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
     }
 }
 
+// VJP of the interior faces at degree 1 without the viscous flux: one thread per face, 32 faces per warp.  The rows of
+// the 64 cells are staged by the warp and the face records leave through the same shared memory, so both run along
+// memory; the points accumulate in registers (sum_q Ub and sum_q x_d Ub, of which the rows of the linear basis are
+// combinations).  A thread that read and wrote its rows in place touched a line per lane and access
+// (668 us for 508,720 faces of 3 points, now 355; one thread per point, k_rhs_vjp_fast, 512 us, and 13 against 21 us at
+// 5,008 faces, where it no longer matters).
+template <int DIM, int NG, bool HLLEP>
+__global__ void __launch_bounds__(64, 4)
+    k_rhs_vjp_inviscid(MeshD m, GeomD g, const real *__restrict__ facePt, const real *__restrict__ cellPar, const real *__restrict__ moment,
+                       EulerSettingsD s, const real *__restrict__ w, const real *__restrict__ u, const real *__restrict__ uRec,
+                       const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
+{
+    constexpr int NV = 5, P = 1;
+    using Lt = Layout<DIM, P, NV>;
+    constexpr int CS = Lt::CS, W = (Lt::R + 1) * NV, OS = (2 * W) | 1;
+    static_assert(Lt::R == DIM && 32 * OS <= 64 * CS, "the face records take the place of the cells' rows");
+    extern __shared__ real sm[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    real *sCell = sm + wid * 64 * CS; // slots 0..31 side-0 cells, 32..63 side-1 cells
+    const int64_t f0 = ((int64_t)blockIdx.x * 2 + wid) * 32, f = f0 + lane;
+    const int c0 = f < m.nFace ? m.face2cell[f * 2] : -1, c1 = f < m.nFace ? m.face2cell[f * 2 + 1] : -1;
+#pragma unroll 4
+    for (int t = 0; t < 64; t++)
+    {
+        const int c = __shfl_sync(0xffffffffu, t < 32 ? c0 : c1, t & 31);
+        if (c >= 0)
+            stage_cell<DIM, P, NV>(sCell + t * CS, c, lane, uRec, u, cellPar, moment);
+    }
+    copies_commit();
+    const bool on = c1 >= 0; // boundary faces belong to the boundary kernel
+    real sh[3] = {0, 0, 0}, dLambda = 0, gb[NV];
+    if (on)
+    {
+        dLambda = dmax(dLamCell[c0], dLamCell[c1]);
+        const real iv0 = 1.0 / g.vol[c0], iv1 = 1.0 / g.vol[c1];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            sh[d] = m.facePShift[f * 3 + d];
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+            gb[v] = w[(int64_t)c0 * NV + v] * iv0 - w[(int64_t)c1 * NV + v] * iv1;
+    }
+    copies_wait<0>();
+    __syncwarp();
+    real acc[2][DIM + 1][NV]; // per side: sum_q Ub, sum_q x_d Ub; then the rows
+#pragma unroll
+    for (int i = 0; i < 2 * (DIM + 1) * NV; i++)
+        (&acc[0][0][0])[i] = 0;
+    if (on)
+    {
+        RoeAvg r;
+        roe_average(sCell + lane * CS + Lt::OU, sCell + (32 + lane) * CS + Lt::OU, s.gamma, r);
+        roe_rev::RoeBar rb;
+        roe_rev::roebar_zero(rb);
+        bool ok = r.asqr > 0;
+#pragma unroll 1
+        for (int q = 0; q < NG; q++)
+        {
+            // the rows stay in shared memory: read ahead of the loop they would fill the registers
+            int off = lane * CS;
+            asm volatile("" : "+r"(off));
+            const real *cell0 = sCell + off, *cell1 = cell0 + 32 * CS;
+            real p0[3], n[3], JW;
+            face_point(facePt, m.nFace, q, f, p0, n, JW);
+            const real p1[3] = {p0[0] + sh[0], p0[1] + sh[1], p0[2] + sh[2]};
+            real UL[NV], UR[NV], Ub0[NV], Ub1[NV], Fbar[NV];
+            recon_value<DIM, P, NV>(cell0, p0, UL);
+            recon_value<DIM, P, NV>(cell1, p1, UR);
+            ok = ok && UL[0] > 0 && UR[0] > 0;
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                Fbar[v] = -JW * gb[v];
+            if constexpr (HLLEP)
+                roe_rev::hllep_rev(UL, UR, n, r, s.gamma, dLambda, s.rsFixScale, Fbar, Ub0, Ub1, rb);
+            else
+            {
+                real incU[NV], incFb[NV], incUb[NV];
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    incU[v] = UR[v] - UL[v], incFb[v] = -0.5 * Fbar[v];
+                roe_rev::roe0_diss_rev(incU, n, r, s.gamma, dLambda, s.rsFixScale, s.rsIncFScale, incFb, incUb, rb);
+                flux_jac_du_t<NV>(UL, n, Fbar, 0.0, s.gamma, Ub0);
+                flux_jac_du_t<NV>(UR, n, Fbar, 0.0, s.gamma, Ub1);
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    Ub0[v] = 0.5 * Ub0[v] - incUb[v], Ub1[v] = 0.5 * Ub1[v] + incUb[v];
+            }
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                acc[0][0][v] += Ub0[v], acc[1][0][v] += Ub1[v];
+#pragma unroll
+            for (int d = 0; d < DIM; d++)
+            {
+                const real x0 = (p0[d] - cell0[Lt::OC + d]) * cell0[Lt::OL + d] - cell0[Lt::OM + 1 + d];
+                const real x1 = (p1[d] - cell1[Lt::OC + d]) * cell1[Lt::OL + d] - cell1[Lt::OM + 1 + d];
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    acc[0][1 + d][v] += x0 * Ub0[v], acc[1][1 + d][v] += x1 * Ub1[v];
+            }
+        }
+        if (!ok)
+            atomicOr(err, (int)DE_NONPHYSICAL);
+#pragma unroll
+        for (int side = 0; side < 2; side++)
+        {
+            real Ub[NV];
+            roe_rev::roe_average_rev(side, sCell + lane * CS + Lt::OU, sCell + (32 + lane) * CS + Lt::OU, r, s.gamma, rb, Ub);
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                acc[side][0][v] += Ub[v];
+        }
+    }
+    __syncwarp(); // all rows read
+    real *sOut = sCell;
+#pragma unroll
+    for (int i = 0; i < 2 * W; i++)
+        sOut[lane * OS + i] = (&acc[0][0][0])[i];
+    __syncwarp();
+    const unsigned in = __ballot_sync(0xffffffffu, on);
+    for (int e = lane; e < 32 * 2 * W; e += 32)
+    {
+        const int fi = e / (2 * W);
+        if ((in >> fi) & 1)
+            faceAdj[f0 * 2 * W + e] = sOut[fi * OS + e - fi * 2 * W];
+    }
+}
+
+template <int DIM, int NG>
+int launch_vjp_inviscid(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, bool hllep, const real *w, const real *u,
+                        const real *uRec, real *faceAdj, cudaStream_t st)
+{
+    constexpr int smem = sizeof(real) * 2 * 64 * Layout<DIM, 1, 5>::CS; // 31 KB at most
+    auto kern = hllep ? k_rhs_vjp_inviscid<DIM, NG, true> : k_rhs_vjp_inviscid<DIM, NG, false>;
+    kern<<<(unsigned)((m.nFace + 63) / 64), 64, smem, st>>>(m, g, ev.facePt, ev.cellPar, vr.baseMoment, ev.s, w, u, uRec, ev.deltaLambdaCell,
+                                                            faceAdj, ev.errWord);
+    return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
+}
+
 template <int DIM, int P, int NV, int NG>
 int launch_vjp_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &ev, bool hllep, bool visc, const real *w, const real *u,
                     const real *uRec, real *faceAdj, cudaStream_t st)
 {
     using Lt = Layout<DIM, P, NV>;
+    if constexpr (P == 1 && NV == 5)
+    {
+        if (!visc)
+            return launch_vjp_inviscid<DIM, NG>(m, g, vr, ev, hllep, w, u, uRec, faceAdj, st);
+    }
     constexpr int W = (Lt::R + 1) * NV, CH = VjpRows<DIM, P, NV, NG, true>::CH;
     constexpr size_t smem = sizeof(real) * (64 * Lt::CS + 32 * NV + 15 * 32 + CH * NG * 32 + 32 * 2 * W) + sizeof(FaceData) * 32;
     static_assert(smem <= 227 * 1024, "shared memory of k_rhs_vjp_fast above the 227 KB a block may hold");
-    auto kern = visc ? k_rhs_vjp_fast<DIM, P, NV, NG, true> : k_rhs_vjp_fast<DIM, P, NV, NG, false>;
+    auto kern = k_rhs_vjp_fast<DIM, P, NV, NG, true>;
+    if constexpr (P > 1 && NV == 5)
+        if (!visc)
+            kern = k_rhs_vjp_fast<DIM, P, NV, NG, false>;
     static unsigned long long attrSet[2] = {0, 0}; // per variant, one bit per device: dynamic shared memory limit raised
     int dev = 0;
     cudaGetDevice(&dev);

@@ -24,6 +24,7 @@
 #include "bc.cuh"
 #include "sa.cuh"
 #include "basis_rows.cuh"
+#include "vr_vjp.cuh"
 
 namespace dndsb
 {
@@ -485,28 +486,6 @@ DNDSB_GLOBAL void k_rhs_jvp_face_g(MeshD m, GeomD g, VRD vr, EulerSettingsD s, c
     }
 }
 
-template <int W, int NV>
-DNDSB_GLOBAL void k_adj_gather_g(int64_t nCell, int nf, const int32_t *__restrict__ c2f, const real *__restrict__ faceAdj, real *du, real *duRec)
-{
-    DNDSB_KERNEL_LOOP(c, nCell)
-    {
-        real acc[W];
-        for (int i = 0; i < W; i++)
-            acc[i] = 0;
-        for (int k = 0; k < nf; k++)
-        {
-            int fp = c2f[c * nf + k];
-            const real *src = faceAdj + ((int64_t)(fp >> 1) * 2 + (fp & 1)) * W;
-            for (int i = 0; i < W; i++)
-                acc[i] += src[i];
-        }
-        for (int v = 0; v < NV; v++)
-            du[c * NV + v] = acc[v];
-        for (int i = NV; i < W; i++)
-            duRec[c * (W - NV) + i - NV] = acc[i];
-    }
-}
-
 template <int NV>
 DNDSB_GLOBAL void k_flux_gather_g(int64_t nCell, int nf, const int32_t *__restrict__ c2f, const real *__restrict__ vol, const real *__restrict__ ff,
                                   real *rhs)
@@ -718,11 +697,11 @@ DNDSB_D void recon_value_g(const real *T, const real *u, const real *rec, real *
     }
 }
 
-// the boundary term BCC = sum_q w0^2 |J| w phi_q (UB_q - u_c), UB_q = ghost(compress(u_c, u_c + phi_q . uRec_c)):
-// mode 0: VJP of its cotangent t into (vRec, vU); mode 1: JVP (dRec, du) -> dBCC
+// tangent of the boundary term BCC = sum_q w0^2 |J| w phi_q (UB_q - u_c), UB_q = ghost(compress(u_c, u_c + phi_q . uRec_c)),
+// along (dRec, du); its transpose is k_vr_vjp_bnd
 template <int DIM, int P, int NV>
-DNDSB_D void bcc_derivative_g(const MeshD &m, const GeomD &g, const VRD &vr, int64_t c, const real *u, const real *uRec, int mode,
-                              const real *t, real *vRec, real *vU, const real *dRec, const real *duc, real *dBCC)
+DNDSB_D void bcc_tangent_g(const MeshD &m, const GeomD &g, const VRD &vr, int64_t c, const real *u, const real *uRec, const real *dRec,
+                           const real *duc, real *dBCC)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
     using DV = Dual<2 * NV>;
@@ -752,114 +731,24 @@ DNDSB_D void bcc_derivative_g(const MeshD &m, const GeomD &g, const VRD &vr, int
             if (!bc_value_fix<NV>(vr.bnd, zone, ULf, n, UB))
                 for (int v = 0; v < NV; v++)
                     UB[v] = ULf[v];
-            if (mode == 0)
+            real dUL[NV];
+            for (int v = 0; v < NV; v++)
             {
-                real UBbar[NV];
-                for (int v = 0; v < NV; v++)
-                {
-                    real a = 0;
-                    for (int i = 0; i < R; i++)
-                        a += T[1 + i] * t[i * NV + v];
-                    UBbar[v] = a * JW;
-                    vU[v] -= UBbar[v];
-                }
+                real a = duc[v];
+                for (int j = 0; j < R; j++)
+                    a += T[1 + j] * dRec[j * NV + v];
+                dUL[v] = a;
+            }
+            for (int v = 0; v < NV; v++)
+            {
+                real dUB = 0;
                 for (int i = 0; i < NV; i++)
-                {
-                    real gl = 0, gm = 0;
-                    for (int v = 0; v < NV; v++)
-                        gl += UB[v].d[i] * UBbar[v], gm += UB[v].d[NV + i] * UBbar[v];
-                    vU[i] += gl + gm;
-                    for (int j = 0; j < R; j++)
-                        vRec[j * NV + i] += T[1 + j] * gl;
-                }
-            }
-            else
-            {
-                real dUL[NV];
-                for (int v = 0; v < NV; v++)
-                {
-                    real a = duc[v];
-                    for (int j = 0; j < R; j++)
-                        a += T[1 + j] * dRec[j * NV + v];
-                    dUL[v] = a;
-                }
-                for (int v = 0; v < NV; v++)
-                {
-                    real dUB = 0;
-                    for (int i = 0; i < NV; i++)
-                        dUB += UB[v].d[i] * dUL[i] + UB[v].d[NV + i] * duc[i];
-                    real dd = (dUB - duc[v]) * JW;
-                    for (int i = 0; i < R; i++)
-                        dBCC[i * NV + v] += T[1 + i] * dd;
-                }
+                    dUB += UB[v].d[i] * dUL[i] + UB[v].d[NV + i] * duc[i];
+                real dd = (dUB - duc[v]) * JW;
+                for (int i = 0; i < R; i++)
+                    dBCC[i * NV + v] += T[1 + i] * dd;
             }
         }
-    }
-}
-
-template <int DIM, int P, int NV>
-DNDSB_GLOBAL void k_vr_vjp_g(MeshD m, GeomD g, VRD vr, const real *__restrict__ v, const real *__restrict__ uRec, const real *__restrict__ u,
-                             real *vRec, real *vU)
-{
-    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1;
-    const real om = vr.s.jacobiRelax;
-    const int nf = m.nf;
-    DNDSB_KERNEL_LOOP(o, m.nCell)
-    {
-        real aRec[R * NV], aU[NV];
-        const real *vo = v + o * R * NV;
-        for (int i = 0; i < R * NV; i++)
-            aRec[i] = (1 - om) * vo[i];
-        for (int x = 0; x < NV; x++)
-            aU[x] = 0;
-        bool hasBnd = false;
-        for (int j = 0; j < nf; j++)
-        {
-            int i = m.cellNbr[o * nf + j];
-            if (i < 0)
-            {
-                hasBnd = true;
-                continue;
-            }
-            int k = m.nbrSlot[o * nf + j];
-            const real *M = vr.AAInvB + ((int64_t)i * (nf + 1) + 1 + k) * R * R;
-            const real *b = vr.AInvb + ((int64_t)i * nf + k) * R;
-            const real *vi = v + (int64_t)i * R * NV;
-            for (int r = 0; r < R; r++)
-                for (int x = 0; x < NV; x++)
-                {
-                    real a = 0;
-                    for (int l = 0; l < R; l++)
-                        a += M[l * R + r] * vi[l * NV + x];
-                    aRec[r * NV + x] += om * a;
-                }
-            const real *bo = vr.AInvb + (o * nf + j) * R;
-            for (int x = 0; x < NV; x++)
-            {
-                real a = 0, a2 = 0;
-                for (int l = 0; l < R; l++)
-                    a += b[l] * vi[l * NV + x], a2 += bo[l] * vo[l * NV + x];
-                aU[x] += om * (a - a2);
-            }
-        }
-        if (hasBnd && vr.bnd.nZone > 0)
-        {
-            const real *Ai = vr.AAInvB + (o * (nf + 1)) * R * R;
-            real t[R * NV];
-            for (int r = 0; r < R; r++)
-                for (int x = 0; x < NV; x++)
-                {
-                    real a = 0;
-                    for (int l = 0; l < R; l++)
-                        a += Ai[l * R + r] * vo[l * NV + x];
-                    t[r * NV + x] = om * a;
-                }
-            bcc_derivative_g<DIM, P, NV>(m, g, vr, o, u, uRec, 0, t, aRec, aU, nullptr, nullptr, nullptr);
-        }
-        for (int i = 0; i < R * NV; i++)
-            vRec[o * R * NV + i] = aRec[i];
-        for (int x = 0; x < NV; x++)
-            vU[o * NV + x] = aU[x];
     }
 }
 
@@ -900,7 +789,7 @@ DNDSB_GLOBAL void k_vr_jvp_g(MeshD m, GeomD g, VRD vr, const real *__restrict__ 
             real dB[R * NV];
             for (int i = 0; i < R * NV; i++)
                 dB[i] = 0;
-            bcc_derivative_g<DIM, P, NV>(m, g, vr, c, u, uRec, 1, nullptr, nullptr, nullptr, dRec + c * R * NV, du + c * NV, dB);
+            bcc_tangent_g<DIM, P, NV>(m, g, vr, c, u, uRec, dRec + c * R * NV, du + c * NV, dB);
             const real *Ai = vr.AAInvB + (c * (nf + 1)) * R * R;
             for (int r = 0; r < R; r++)
                 for (int x = 0; x < NV; x++)
@@ -948,8 +837,8 @@ int vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real 
         k_rhs_vjp_bnd_g<DIM, P, NV><<<(unsigned)((m.nBndFace + rows - 1) / rows), 32 * (DIM + 2), 0, st>>>(
             m, g, vr, ev.s, w, objDir, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
     }
-    auto kg = k_adj_gather_g<W, NV>;
-    DNDSB_LAUNCH(kg, m.nCell, 128, st, m.nCell, m.nf, m.cell2face, ev.adjBuf, du, duRec);
+    auto kg = k_adj_gather<W, NV>;
+    DNDSB_LAUNCH(kg, m.nCell * W, 256, st, m.nCell, m.nf, m.cell2face, ev.adjBuf, du, duRec);
     if constexpr (NV == 6)
         if (!objDir)
         {
@@ -979,8 +868,7 @@ int jvp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real 
 template <int DIM, int P, int NV>
 int vr_vjp_dp_g(const MeshD &m, const GeomD &g, const VRD &vr, const real *v, const real *uRec, const real *u, real *vRec, real *vU, cudaStream_t st)
 {
-    auto k = k_vr_vjp_g<DIM, P, NV>;
-    DNDSB_LAUNCH(k, m.nCell, 64, st, m, g, vr, v, uRec, u, vRec, vU);
+    launch_vr_vjp<DIM, P, NV>(m, g, vr, v, uRec, u, vRec, vU, st);
     return ST_OK;
 }
 

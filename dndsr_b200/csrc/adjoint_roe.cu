@@ -11,11 +11,11 @@
 //     the five unit jumps in real arithmetic;
 //   * cell means: only D depends on them.  For plain Roe a hand-written reverse sweep of the
 //     eigenvalues, wave strengths and dissipation gives, per Gauss point, D^T Fbar and the
-//     cotangents of the Roe-average fields, and one Dual<10> evaluation of the averages per face
-//     carries those to the means; the other schemes take the eigenvalues and D (U_R - U_L) in
+//     cotangents of the Roe-average fields, carried to the means by the reverse of the averages
+//     (roe_average_rev), once per face; the other schemes take the eigenvalues and D (U_R - U_L) in
 //     Dual<10> per Gauss point.
 // HLLEPFlux_IdealGas (Gas.hpp:601-714) mixes the point states into its wave-speed bounds, so it is
-// reversed as a whole (hllep_rev), with the same per-face Dual<10> Roe averages for the means.
+// reversed as a whole (hllep_rev), with the same reverse of the averages.
 // This replaces two 10-wide forward passes through the whole flux.  Boundary faces keep the
 // generic derivative kernel (ghost states).
 #include "solver.cuh"
@@ -30,7 +30,6 @@ namespace
 constexpr int NV = 5;
 constexpr int kHLLEP = 100; // flux mode of HLLE+ (Roe schemes use their eigScheme 0..8)
 using D10 = Dual<10>;
-using D1 = Dual<1>;
 using roe_rev::RoeBar;
 using roe_rev::roebar_zero;
 using roe_rev::roe0_diss_rev;
@@ -86,6 +85,7 @@ DNDSB_GLOBAL void k_rhs_vjp_face_roe(MeshD m, GeomD g, VRD vr, EulerSettingsD s,
         RoeAvg r;
         roe_average(ULm, URm, gamma, r);
         RoeAvgT<D10> rD;
+        if (es != 0 && es != kHLLEP)
         {
             D10 a[NV], b[NV];
             for (int v = 0; v < NV; v++)
@@ -209,15 +209,9 @@ DNDSB_GLOBAL void k_rhs_vjp_face_roe(MeshD m, GeomD g, VRD vr, EulerSettingsD s,
         }
         if (es == 0 || es == kHLLEP)
         {
-            // Roe-average cotangents -> cell means through the per-face Dual<10> averages
-            for (int i = 0; i < 2 * NV; i++)
-            {
-                real a = rbar.aL * rD.aL.d[i] + rbar.aR * rD.aR.d[i] + rbar.vsqr * rD.vsqr.d[i] + rbar.H * rD.H.d[i] + rbar.asqr * rD.asqr.d[i] +
-                         rbar.a * rD.a.d[i];
-                for (int d = 0; d < 3; d++)
-                    a += rbar.v[d] * rD.v[d].d[i] + rbar.vL[d] * rD.vL[d].d[i] + rbar.vR[d] * rD.vR[d].d[i];
-                mbar[i] = a;
-            }
+            // Roe-average cotangents -> cell means
+            for (int side = 0; side < 2; side++)
+                roe_rev::roe_average_rev(side, ULm, URm, r, gamma, rbar, mbar + side * NV);
         }
         for (int v = 0; v < NV; v++)
             acc0[v] += mbar[v], acc1[v] += mbar[NV + v];
@@ -245,10 +239,9 @@ int rhs_vjp_roe_interior(const MeshD &m, const GeomD &g, const VRD &vr, const Ev
     if (es < 0 || ev.s.nVars != NV)
         return ST_UNSUPPORTED;
     *viscDone = false;
-    // plain Roe and HLLE+ with the viscous flux: the Gauss-point-parallel kernel of adjoint_fast.cu (the
-    // inviscid flux alone is as fast or faster in the thread-per-face kernel below: 1.06 against 1.88 ms for
-    // plain Roe on 249,600 tets at degree 1, 3.7 ms either way for HLLE+ on the 64^3 TGV at degree 2)
-    if ((es == 0 || es == kHLLEP) && !ev.s.ignoreVis)
+    // plain Roe and HLLE+: the kernels of adjoint_fast.cuh (508,720 inviscid faces of degree 2: 1.39 against 2.23 ms in
+    // the thread-per-face kernel below, which takes the other schemes and the quadratures those do not cover)
+    if (es == 0 || es == kHLLEP)
     {
         int rc = rhs_vjp_interior_fast(m, g, vr, ev, es == kHLLEP, w, u, uRec, faceAdj, st);
         if (rc != ST_UNSUPPORTED)

@@ -22,6 +22,35 @@ DNDSB_D void roebar_zero(RoeBar &b)
     b.aL = b.aR = b.vsqr = b.H = b.asqr = b.a = 0;
 }
 
+// reverse of roe_average (Gas.hpp:229-259) for the mean of one side (side 0: the left one): the cotangents b of the
+// averages carried to that mean, Ub
+DNDSB_D void roe_average_rev(int side, const real *UL, const real *UR, const RoeAvg &r, real gamma, const RoeBar &b, real *Ub)
+{
+    const real asqrb = b.asqr + b.a * r.inv2a, Hb = b.H + (gamma - 1) * asqrb, vsqrb = b.vsqr - 0.5 * (gamma - 1) * asqrb;
+    const real *U = side ? UR : UL, *vS = side ? r.vR : r.vL, *vSbIn = side ? b.vR : b.vL;
+    const real sL = sqrt(UL[0]), sR = sqrt(UR[0]), is = 1.0 / (sL + sR), sS = side ? sR : sL;
+    const real i = 1.0 / U[0], p = side ? r.pRm : r.pLm, H = (U[4] + p) * i, w = sS * is;
+    real vSb[3], sSb = (H - r.H) * Hb, ib = 0, v2 = 0;
+    for (int d = 0; d < 3; d++)
+    {
+        const real vb = b.v[d] + 2 * vsqrb * r.v[d];
+        vSb[d] = vSbIn[d] + w * vb;
+        sSb += (vS[d] - r.v[d]) * vb;
+        v2 += vS[d] * vS[d];
+    }
+    const real HSb = w * Hb, a2b = (side ? b.aR : b.aL) * 0.5 / (side ? r.aR : r.aL);
+    const real pb = gamma * i * a2b + HSb * i;
+    ib += gamma * p * a2b + HSb * (U[4] + p);
+    for (int d = 0; d < 3; d++)
+    {
+        vSb[d] -= (gamma - 1) * U[0] * vS[d] * pb;
+        Ub[1 + d] = vSb[d] * i;
+        ib += vSb[d] * U[1 + d];
+    }
+    Ub[0] = is * sSb * 0.5 / sS - (gamma - 1) * 0.5 * v2 * pb - ib * i * i;
+    Ub[4] = HSb * i + (gamma - 1) * pb;
+}
+
 // reverse of one Harten-Yee limiter application of Roe_EntropyFixer scheme 0 (Gas.hpp:878-930):
 //   th = max(max(0, lam - lamL), lamR - lam) sHY,  out = v < th ? (v^2 / th + th) / 2 : v
 DNDSB_D void flim_rev(real v, real lam, real lamL, real lamR, real sHY, real ob, real &vb, real &lamb, real &lamLb, real &lamRb)
@@ -78,9 +107,10 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
         a23T[d] = a23[d] - n[d] * a23n;
     real incU4b = incU[4] - dot3(a23T, r.v);
     real X = incU[0] * (r.H - vN * vN) + vN * incU123N - incU4b;
-    real wa1 = (gamma - 1) / r.asqr * X;
+    real wa1 = r.gOverA2 * X;
     real num = incU[0] * (vN + r.a) - incU123N - r.a * wa1;
-    real wa0 = num / (2 * r.a);
+    const real ia = 2 * r.inv2a;
+    real wa0 = num * r.inv2a;
     real wa4 = incU[0] - (wa0 + wa1);
     // forward: dissipation products
     real A0 = wa0 * l0, A1 = wa1 * l123, A4 = wa4 * l4;
@@ -116,15 +146,15 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
     incUb[0] += wa4b;
     wa0b -= wa4b;
     wa1b -= wa4b;
-    real numb = wa0b / (2 * r.a);
-    rb.a += -wa0 / r.a * wa0b;
+    real numb = wa0b * r.inv2a;
+    rb.a += -wa0 * ia * wa0b;
     incUb[0] += (vN + r.a) * numb;
     vNb += incU[0] * numb;
     rb.a += (incU[0] - wa1) * numb;
     real incU123Nb = -numb;
     wa1b -= r.a * numb;
-    real Xb = (gamma - 1) / r.asqr * wa1b;
-    rb.asqr += -wa1 / r.asqr * wa1b;
+    real Xb = r.gOverA2 * wa1b;
+    rb.asqr += -wa1 * ia * ia * wa1b;
     incUb[0] += (r.H - vN * vN) * Xb;
     rb.H += incU[0] * Xb;
     vNb += (-2 * vN * incU[0] + incU123N) * Xb;

@@ -1,6 +1,5 @@
-"""The inviscid face kernels (one thread per face, rows staged by the warp) at ragged face counts and each quadrature size
-that they cover, with periodic, interior and boundary faces: the residual against the oracle, its spectral radii, and the
-transpose against the tangent."""
+"""The inviscid face kernels (cell rows staged by the warps) at ragged face counts and each quadrature size that they cover,
+with periodic, interior and boundary faces: the residual against the oracle, the transpose against the tangent."""
 import numpy as np
 import pytest
 import torch
