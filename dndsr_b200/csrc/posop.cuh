@@ -6,8 +6,8 @@
 // (in the product, in no sweep); slots of boundary faces are dropped.  Per slot {w n, w lambda} with
 // w = alpha A_f / (2 V_c) and the neighbour's position, both in tiles of 32 positions (the 32 lanes of a warp read one
 // slot of their positions as one contiguous line).  The flux Jacobian of a cell needs only its velocity and total
-// enthalpy, kept as one aligned 4-vector per cell (and U5 / rho for the SA variable), so a product takes two vector
-// loads and five scalar ones per neighbour and no division:
+// enthalpy, kept as one aligned 4-vector per cell (and U5 / rho for the SA variable), and the vectors are split as in
+// vec_split.cuh, so a product takes three vector loads and a scalar one per neighbour and no division:
 //   A(U) dU . n:  q = dm.n - (v.n) drho, dp = (gamma - 1)(dE - v.dm + v^2 drho / 2);
 //   {dm.n, dm (v.n) + v q + n dp, (dE + dp)(v.n) + H q, dU5 (v.n) + (U5 / rho) q}.
 //
@@ -20,26 +20,17 @@
 //
 // Bound by the operator stream and the neighbour gathers.  GMRES(30) preconditioned by one pair, per solve: 249,600
 // tets in FP64 2.57 ms of sweeps and products before (248 + 30 launches, neighbours' conservative states gathered and
-// divided, all slots tested in each sweep); 1,996,800 tets in FP32 8.28 ms.  This form: 1.92 ms and 5.44 ms.
+// divided, all slots tested in each sweep); 1,996,800 tets in FP32 8.28 ms.  This form: 1.69 ms and 5.15 ms, with
+// the vectors as cell rows 1.89 ms and 5.36 ms.
 #pragma once
 #include "solver.cuh"
+#include "vec_split.cuh"
 
 namespace dndsb
 {
 namespace posop
 {
-template <typename T>
-struct Vec4;
-template <>
-struct Vec4<float>
-{
-    using type = float4;
-};
-template <>
-struct Vec4<double>
-{
-    using type = double4;
-};
+using vsplit::Vec4;
 
 // diagonals per cell: 1, or NV with the SA source Jacobian
 template <int NV>
@@ -53,6 +44,7 @@ template <typename T>
 struct Op
 {
     using T4 = typename Vec4<T>::type;
+    int64_t n = 0;            // positions
     int32_t *nbr = nullptr;   // [tiles][NF][32] neighbour positions
     int32_t *cnt = nullptr;   // [n] lower | (lower + upper) << 8 | all << 16
     T4 *op = nullptr;         // [tiles][NF][32] {w n, w lambda}
@@ -164,10 +156,7 @@ DNDSB_D void add_slots(const Op<T> &A, int64_t p, int j0, int j1, int ja, const 
                 o[k] = A.op[slot_at<NF>(p, b + k)];
                 s[k] = A.vh[q[b + k]];
                 nu[k] = NV == 6 ? A.nu[q[b + k]] : T(0);
-                const T *src = (b + k < ja ? xa : xb) + (int64_t)q[b + k] * NV;
-#pragma unroll
-                for (int v = 0; v < NV; v++)
-                    d[k][v] = src[v];
+                vsplit::load<T, NV>(b + k < ja ? xa : xb, A.n, q[b + k], d[k]);
             }
 #pragma unroll
         for (int k = 0; k < G; k++)
@@ -187,13 +176,15 @@ DNDSB_GLOBAL void k_sweep(int64_t pBeg, int64_t pEnd, Op<T> A, const T *__restri
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, nu = (cnt >> 8) & 255;
         T buf[NV], r[NV];
+        vsplit::load<T, NV>(rhs, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            buf[v] = 0, r[v] = rhs[p * NV + v];
+            buf[v] = 0;
         add_slots<T, NV, NF>(A, p, xLow ? 0 : nl, xUp ? nu : nl, nl, xLow, T(1), xUp, T(1), g1, buf);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            xNew[p * NV + v] = (r[v] - buf[v]) * A.jdi[p * JD + (JD > 1 ? v : 0)];
+            r[v] = (r[v] - buf[v]) * A.jdi[p * JD + (JD > 1 ? v : 0)];
+        vsplit::store<T, NV>(xNew, A.n, p, r);
     }
 }
 
@@ -207,13 +198,15 @@ DNDSB_GLOBAL void k_back(int64_t pBeg, int64_t pEnd, Op<T> A, T *x, T g1)
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, nu = (cnt >> 8) & 255;
         T buf[NV], r[NV];
+        vsplit::load<T, NV>(x, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            buf[v] = 0, r[v] = x[p * NV + v];
+            buf[v] = 0;
         add_slots<T, NV, NF>(A, p, nl, nu, nl, (const T *)x, T(1), (const T *)x, T(1), g1, buf);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            x[p * NV + v] = r[v] - buf[v] * A.jdi[p * JD + (JD > 1 ? v : 0)];
+            r[v] -= buf[v] * A.jdi[p * JD + (JD > 1 ? v : 0)];
+        vsplit::store<T, NV>(x, A.n, p, r);
     }
 }
 
@@ -229,17 +222,19 @@ DNDSB_GLOBAL void k_product_forward(int64_t pBeg, int64_t pEnd, Op<T> A, const T
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, na = cnt >> 16;
         T buf[NV], r[NV];
+        vsplit::load<T, NV>(x, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            buf[v] = 0, r[v] = x[p * NV + v];
+            buf[v] = 0;
         add_slots<T, NV, NF>(A, p, 0, na, nl, (const T *)t, T(-1), x, sx, g1, buf);
 #pragma unroll
         for (int v = 0; v < NV; v++)
         {
-            const T tv = buf[v] * A.jdi[p * JD + (JD > 1 ? v : 0)];
-            t[p * NV + v] = tv;
-            y[p * NV + v] = sx * r[v] + tv;
+            buf[v] *= A.jdi[p * JD + (JD > 1 ? v : 0)];
+            r[v] = sx * r[v] + buf[v];
         }
+        vsplit::store<T, NV>(t, A.n, p, buf);
+        vsplit::store<T, NV>(y, A.n, p, r);
     }
 }
 
@@ -253,13 +248,15 @@ DNDSB_GLOBAL void k_product(int64_t n, Op<T> A, const T *__restrict__ x, T *__re
     {
         const int cnt = A.cnt[p];
         T buf[NV];
+        vsplit::load<T, NV>(x, A.n, p, buf);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            buf[v] = A.jd[p * JD + (JD > 1 ? v : 0)] * x[p * NV + v];
+            buf[v] *= A.jd[p * JD + (JD > 1 ? v : 0)];
         add_slots<T, NV, NF>(A, p, 0, cnt >> 16, NF, x, T(1), x, T(1), g1, buf);
 #pragma unroll
         for (int v = 0; v < NV; v++)
-            Ax[p * NV + v] = sx * buf[v];
+            buf[v] *= sx;
+        vsplit::store<T, NV>(Ax, A.n, p, buf);
     }
 }
 } // namespace posop

@@ -3,6 +3,8 @@
 // a single-block final pass, so results do not depend on scheduling.
 #include "solver.cuh"
 #include "krylov_update.cuh"
+#include "vec_split.cuh"
+#include <type_traits>
 
 namespace dndsb
 {
@@ -102,8 +104,8 @@ real *reduce_cols(int op, int64_t n, int ncol, const real *x, const real *w, int
 }
 // ---------------------------------------------------------------------------
 // Krylov reductions for the native GMRES (weighted dots, Gram-Schmidt).
-// Vectors are flat [n] arrays of T whose element i carries the variable
-// weight s2[i % NV]; sums accumulate in FP64 over the same fixed partition.
+// Vectors are flat [n] arrays of T, cell rows of NV variables or (SPLIT) laid out as in vec_split.cuh;
+// element i carries the weight s2 of its variable; sums accumulate in FP64 over the same fixed partition.
 // ---------------------------------------------------------------------------
 namespace
 {
@@ -213,19 +215,43 @@ DNDSB_D bool last_block_final(int nb, int ncol, const real *partial, real *out, 
     return true;
 }
 
+// weights of the four elements of quad q, for quads q0, q0 + dq, ...: split vectors hold a quad within the first four
+// variables of a cell or within the rest, plain ones start it at variable (4 q) % NV
+template <int NV, bool SPLIT>
+struct QuadWeights
+{
+    const real *ss;
+    int64_t nCell;
+    int r, dr;
+    DNDSB_D QuadWeights(const real *ss_, int64_t n, int64_t q0, int dq)
+        : ss(ss_), nCell(n / NV), r(SPLIT ? 0 : (int)((4 * q0) % NV)), dr(SPLIT ? 0 : (4 * dq) % NV)
+    {
+    }
+    DNDSB_D real at(int64_t q, int e) const
+    {
+        if constexpr (SPLIT)
+            return ss[q < nCell ? e : NV == 5 ? 4 : 4 + (e & 1)];
+        else
+            return ss[r + e < NV ? r + e : r + e - NV];
+    }
+    DNDSB_D void next()
+    {
+        if constexpr (!SPLIT)
+            r = r + dr >= NV ? r + dr - NV : r + dr;
+    }
+};
+
 // sums of NK columns from V against w over the quads [q0, q1): warp sums into sh[column][warp]
-template <typename T, int NV, int NK>
-DNDSB_D void mdot_group(int64_t q0, int64_t q1, int64_t ld, const T *__restrict__ V, const T *__restrict__ w, const real *ss,
+template <typename T, int NV, bool SPLIT, int NK>
+DNDSB_D void mdot_group(int64_t n, int64_t q0, int64_t q1, int64_t ld, const T *V, const T *w, const real *ss,
                         real (*sh)[kRedBlock / 32])
 {
     real a[NK];
 #pragma unroll
     for (int k = 0; k < NK; k++)
         a[k] = 0;
-    // r = (4 q) % NV, advanced incrementally with q
-    const int dr = (int)((4 * (int64_t)blockDim.x) % NV);
-    int r = (int)((4 * (q0 + threadIdx.x)) % NV);
-    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x)
+    QuadWeights<NV, SPLIT> qw(ss, n, q0 + threadIdx.x, (int)blockDim.x);
+    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x, qw.next())
     {
         // every load issued (in its storage type) before the first use
         typename Quad<T>::raw v[NK];
@@ -236,9 +262,7 @@ DNDSB_D void mdot_group(int64_t q0, int64_t q1, int64_t ld, const T *__restrict_
         Quad<T>::load(w + 4 * q, wv);
 #pragma unroll
         for (int e = 0; e < 4; e++)
-            wv[e] *= ss[r + e < NV ? r + e : r + e - NV];
-        r += dr;
-        r = r >= NV ? r - NV : r;
+            wv[e] *= qw.at(q, e);
 #pragma unroll
         for (int k = 0; k < NK; k++)
             a[k] += Quad<T>::dot(v[k], wv);
@@ -252,15 +276,15 @@ DNDSB_D void mdot_group(int64_t q0, int64_t q1, int64_t ld, const T *__restrict_
     }
 }
 
-// out[col] = colScale[col] sum_i V[col][i] w[i] s2[i % NV] (the basis columns are stored unnormalised; colScale holds
+// out[col] = colScale[col] sum_i V[col][i] w[i] s2[var(i)] (the basis columns are stored unnormalised; colScale holds
 // their normalising factors).  Columns are ld apart (ld a multiple of 4, the pad beyond n zero).
 // HBM bound on the basis.  The kRedBlocks blocks split into nG groups of at most kKG columns (their widths differ by
 // at most one) times chunks of quads, block = chunk nG + group, so the blocks of a chunk share its w in L2 and every
 // block makes one pass: 592 blocks that each walked all column groups over a chunk of 592 paid a block reduction per
 // group for one or two quads per thread (30 steps of 249,600 tets in FP64: 1.30 -> 1.08 ms).  partial [chunks][ncol]; the
 // last block to finish sums the chunks.
-template <typename T, int NV>
-DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld, int ncol, int nG, const T *__restrict__ V, const T *__restrict__ w,
+template <typename T, int NV, bool SPLIT>
+DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld, int ncol, int nG, const T *V, const T *w,
                                                        const real *__restrict__ s2, real *partial, real *out, const real *colScale,
                                                        unsigned *cnt)
 {
@@ -277,14 +301,14 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
     const T *Vc = V + (int64_t)c0 * ld;
     switch (nk)
     {
-    case 1: mdot_group<T, NV, 1>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 2: mdot_group<T, NV, 2>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 3: mdot_group<T, NV, 3>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 4: mdot_group<T, NV, 4>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 5: mdot_group<T, NV, 5>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 6: mdot_group<T, NV, 6>(q0, q1, ld, Vc, w, ss, sh); break;
-    case 7: mdot_group<T, NV, 7>(q0, q1, ld, Vc, w, ss, sh); break;
-    default: mdot_group<T, NV, 8>(q0, q1, ld, Vc, w, ss, sh); break;
+    case 1: mdot_group<T, NV, SPLIT, 1>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 2: mdot_group<T, NV, SPLIT, 2>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 3: mdot_group<T, NV, SPLIT, 3>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 4: mdot_group<T, NV, SPLIT, 4>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 5: mdot_group<T, NV, SPLIT, 5>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 6: mdot_group<T, NV, SPLIT, 6>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 7: mdot_group<T, NV, SPLIT, 7>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    default: mdot_group<T, NV, SPLIT, 8>(n, q0, q1, ld, Vc, w, ss, sh); break;
     }
     __syncthreads();
     if ((int)threadIdx.x < nk)
@@ -298,13 +322,13 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
 }
 
 // w -= sum_c h[c] colScale[c] V[c] (columns subtracted in index order); the last block writes
-// *outNorm = sqrt(sum_i w_i^2 s2[i % NV]) of the stored w.  w is column ncol of the same basis (not read
+// *outNorm = sqrt(sum_i w_i^2 s2[var(i)]) of the stored w.  w is column ncol of the same basis (not read
 // through V).  With gsc (the GMRES scalars: [0] scale, [2] valid columns) it also sets the normalising
 // factor of the new column, *scaleNext = 1 / norm, or 0 at a breakdown (norm <= 1e-32 scale), which it
 // records in gsc[2] = j (GMRES_LeftPreconditioned::solve, Linear.hpp:100-108).
-template <typename T, int NV>
-DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64_t ld, int ncol, const T *__restrict__ V, const real *__restrict__ h,
-                                                             const real *__restrict__ colScale, T *w, const real *__restrict__ s2, real *partial,
+template <typename T, int NV, bool SPLIT>
+DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64_t ld, int ncol, const T *V, const real *h,
+                                                             const real *colScale, T *w, const real *__restrict__ s2, real *partial,
                                                              real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext)
 {
     __shared__ real hs[32];
@@ -318,9 +342,8 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
     const int64_t nq = (n + 3) >> 2, cq = (nq + gridDim.x - 1) / gridDim.x;
     const int64_t q0 = blockIdx.x * cq, q1 = q0 + cq < nq ? q0 + cq : nq;
     real a = 0;
-    const int dr = (int)((4 * (int64_t)blockDim.x) % NV);
-    int r = (int)((4 * (q0 + threadIdx.x)) % NV);
-    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x)
+    QuadWeights<NV, SPLIT> qw(ss, n, q0 + threadIdx.x, (int)blockDim.x);
+    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x, qw.next())
     {
         real x[4];
         Quad<T>::load(w + 4 * q, x);
@@ -353,9 +376,7 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
         Quad<T>::store(w + 4 * q, x, xr);
 #pragma unroll
         for (int e = 0; e < 4; e++)
-            a += xr[e] * xr[e] * ss[r + e < NV ? r + e : r + e - NV];
-        r += dr;
-        r = r >= NV ? r - NV : r;
+            a += xr[e] * xr[e] * qw.at(q, e);
     }
     const real x = warp_sum(a);
     if ((threadIdx.x & 31) == 0)
@@ -425,8 +446,8 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock) k_kupdate(int64_t n, int64_t ld, 
     }
 }
 
-// partial[block] = sum_i x_i^2 s2[i % NV] (any length, any alignment)
-template <typename T, int NV>
+// partial[block] = sum_i x_i^2 s2[var(i)] (any length, any alignment)
+template <typename T, int NV, bool SPLIT>
 DNDSB_GLOBAL void k_knorm2(int64_t n, const T *__restrict__ x, const real *__restrict__ s2, real *partial, real *outNorm, unsigned *cnt)
 {
     __shared__ real sh[4][kRedBlock];
@@ -436,7 +457,7 @@ DNDSB_GLOBAL void k_knorm2(int64_t n, const T *__restrict__ x, const real *__res
     for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x)
     {
         real d = (real)x[i];
-        a += d * d * s2[i % NV];
+        a += d * d * s2[SPLIT ? vsplit::var_of<NV>(n / NV, i) : (int)(i % NV)];
     }
     block_sum4(sh, a, 0, 0, 0);
     if (threadIdx.x == 0)
@@ -444,8 +465,8 @@ DNDSB_GLOBAL void k_knorm2(int64_t n, const T *__restrict__ x, const real *__res
     last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt);
 }
 
-// partial[block] = sum_i (a_i - b_i)^2 s2[i % NV]
-template <typename T, int NV>
+// partial[block] = sum_i (a_i - b_i)^2 s2[var(i)]
+template <typename T, int NV, bool SPLIT>
 DNDSB_GLOBAL void k_kdiff_norm(int64_t n, const T *__restrict__ x, const T *__restrict__ y, const real *__restrict__ s2, real *partial,
                                real *outNorm, unsigned *cnt)
 {
@@ -456,7 +477,7 @@ DNDSB_GLOBAL void k_kdiff_norm(int64_t n, const T *__restrict__ x, const T *__re
     for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x)
     {
         real d = (real)x[i] - (real)y[i];
-        a += d * d * s2[i % NV];
+        a += d * d * s2[SPLIT ? vsplit::var_of<NV>(n / NV, i) : (int)(i % NV)];
     }
     block_sum4(sh, a, 0, 0, 0);
     if (threadIdx.x == 0)
@@ -464,56 +485,54 @@ DNDSB_GLOBAL void k_kdiff_norm(int64_t n, const T *__restrict__ x, const T *__re
     last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt);
 }
 
-template <typename T, int NV>
+template <typename T, int NV, bool SPLIT>
 void kmdot(int64_t n, int64_t ld, int ncol, const void *V, const void *w, const real *s2, real *red, real *out, const real *colScale,
            unsigned *cnt, cudaStream_t st)
 {
     const int nG = (ncol + kKG - 1) / kKG;
-    k_kmdot<T, NV><<<kRedBlocks / nG * nG, kRedBlock, 0, st>>>(n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
+    k_kmdot<T, NV, SPLIT><<<kRedBlocks / nG * nG, kRedBlock, 0, st>>>(n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
 }
 
-template <typename T, int NV>
+template <typename T, int NV, bool SPLIT>
 void kmaxpy(int64_t n, int64_t ld, int ncol, const void *V, const real *h, const real *colScale, void *w, const real *s2, real *red,
             real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st)
 {
-    k_kmaxpy_norm<T, NV><<<kRedBlocks, kRedBlock, 0, st>>>(n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
+    k_kmaxpy_norm<T, NV, SPLIT><<<kRedBlocks, kRedBlock, 0, st>>>(n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
                                                            scaleNext);
 }
 
-template <typename T, int NV>
+template <typename T, int NV, bool SPLIT>
 void knorm(int64_t n, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st)
 {
-    k_knorm2<T, NV><<<kRedBlocks, kRedBlock, 0, st>>>(n, (const T *)x, s2, red, outNorm, cnt);
+    k_knorm2<T, NV, SPLIT><<<kRedBlocks, kRedBlock, 0, st>>>(n, (const T *)x, s2, red, outNorm, cnt);
 }
 
-template <typename T, int NV>
+template <typename T, int NV, bool SPLIT>
 void kdiff(int64_t n, const void *x, const void *y, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st)
 {
-    k_kdiff_norm<T, NV><<<kRedBlocks, kRedBlock, 0, st>>>(n, (const T *)x, (const T *)y, s2, red, outNorm, cnt);
+    k_kdiff_norm<T, NV, SPLIT><<<kRedBlocks, kRedBlock, 0, st>>>(n, (const T *)x, (const T *)y, s2, red, outNorm, cnt);
 }
 
-#define DNDSB_KDISPATCH(FN, ...)                      \
-    do                                                \
-    {                                                 \
-        if (prec == 0 && nv == 5)                     \
-            FN<double, 5>(__VA_ARGS__);               \
-        else if (prec == 0)                           \
-            FN<double, 6>(__VA_ARGS__);               \
-        else if (nv == 5)                             \
-            FN<float, 5>(__VA_ARGS__);                \
-        else                                          \
-            FN<float, 6>(__VA_ARGS__);                \
-    } while (0)
+template <typename F>
+void for_kind(int prec, int nv, bool split, F f)
+{
+    using std::integral_constant;
+    auto nvs = [&](auto t, auto sp) { nv == 5 ? f(t, integral_constant<int, 5>(), sp) : f(t, integral_constant<int, 6>(), sp); };
+    auto sps = [&](auto t) { split ? nvs(t, std::true_type()) : nvs(t, std::false_type()); };
+    prec ? sps(float()) : sps(double());
+}
+#define DNDSB_KDISPATCH(FN, ...) \
+    for_kind(prec, nv, split, [&](auto t, auto v, auto sp) { FN<decltype(t), decltype(v)::value, decltype(sp)::value>(__VA_ARGS__); })
 } // namespace
 
 // V: ncol columns ld apart (ld a multiple of 4, 16-byte aligned, zero beyond n); w: a column of the same storage
-void krylov_mdot(int prec, int64_t n, int64_t ld, int nv, int ncol, const void *V, const void *w, const real *s2, real *red, real *out,
+void krylov_mdot(int prec, int64_t n, int64_t ld, int nv, bool split, int ncol, const void *V, const void *w, const real *s2, real *red, real *out,
                  const real *colScale, unsigned *cnt, cudaStream_t st)
 {
     DNDSB_KDISPATCH(kmdot, n, ld, ncol, V, w, s2, red, out, colScale, cnt, st);
 }
 
-void krylov_maxpy_norm(int prec, int64_t n, int64_t ld, int nv, int ncol, const void *V, const real *h, const real *colScale, void *w,
+void krylov_maxpy_norm(int prec, int64_t n, int64_t ld, int nv, bool split, int ncol, const void *V, const real *h, const real *colScale, void *w,
                        const real *s2, real *red, real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st)
 {
     DNDSB_KDISPATCH(kmaxpy, n, ld, ncol, V, h, colScale, w, s2, red, outNorm, cnt, gsc, j, scaleNext, st);
@@ -528,12 +547,12 @@ void krylov_update_x(int prec, int64_t n, int k, const void *V, const real *gsc,
         DNDSB_LAUNCH(k_kupdate<double>, nq, kRedBlock, st, n, krylov_ld(n), k, (const double *)V, gsc, yOff, colScale, (double *)x);
 }
 
-void krylov_norm(int prec, int64_t n, int nv, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st)
+void krylov_norm(int prec, int64_t n, int nv, bool split, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st)
 {
     DNDSB_KDISPATCH(knorm, n, x, s2, red, outNorm, cnt, st);
 }
 
-void krylov_diff_norm(int prec, int64_t n, int nv, const void *x, const void *y, const real *s2, real *red, real *outNorm, unsigned *cnt,
+void krylov_diff_norm(int prec, int64_t n, int nv, bool split, const void *x, const void *y, const real *s2, real *red, real *outNorm, unsigned *cnt,
                       cudaStream_t st)
 {
     DNDSB_KDISPATCH(kdiff, n, x, y, s2, red, outNorm, cnt, st);

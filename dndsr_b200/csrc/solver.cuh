@@ -117,8 +117,7 @@ struct VRD
     real *baseMoment = nullptr, *faceWeight = nullptr, *faceL = nullptr;
     real *AAInvB = nullptr, *AInvb = nullptr, *matA = nullptr;
     float *AAInvB32 = nullptr, *AInvb32 = nullptr;
-    // the sweep's coefficients packed per cell as [nf][R][R+1] (row i of A^-1 B_k, then (A^-1 b_k)_i):
-    // one contiguous, 16-byte aligned range per cell, staged into shared memory by bulk async copies
+    // the sweep's coefficients, A^-1 B_k and A^-1 b_k of every slot, in the layout of sweep_layout.cuh
     real *sweepCoef = nullptr;
     float *sweepCoef32 = nullptr;
     BoundaryD bnd;           // boundary values for the BC faces of the sweep
@@ -285,13 +284,12 @@ int add_fixed_increment(const MeshD &m, EvalD &ev, real *u, const real *inc, rea
 struct CoordAdjWs
 {
     int maxSlot = 0;
-    int32_t *patch = nullptr;                 // [nCell][maxSlot] patch nodes of each cell, -1 padded
-    int64_t *start = nullptr, *ent = nullptr; // node -> (cell, slot) entries, CSR in entry order
-    real *share = nullptr;                    // [nCell][maxSlot][3]
+    int32_t *patch = nullptr;                 // [nFace][maxSlot] nodes of each face's cells, -1 padded
+    int64_t *start = nullptr, *ent = nullptr; // node -> (face, slot) entries, CSR in entry order
+    real *share = nullptr;                    // [nFace][maxSlot][3], then the sweep's two cell vectors (face_patches)
     real *lanes = nullptr;                    // [nCell][10 + NDOF][1 + 3 nvert] cell geometry and its vertex derivatives
     bool noLanes = false;                     // no memory for the lanes: geometry recomputed per use
 };
-int coords_ws_build(const MeshD &m, CoordAdjWs &ws);
 void coords_ws_free(CoordAdjWs &ws);
 // s == nullptr: the VR sweep only (w unused); otherwise EvaluateRHS (w) and/or the sweep (cot)
 int coords_vjp(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD *s, const real *dLamCell, CoordAdjWs &ws, const real *w,
@@ -337,19 +335,20 @@ struct LinWs;
 int linear_solve(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs *&ws, const LinSettings &ls, real alphaDiag,
                  const real *dTau, real dt, const real *u, const real *rhs, real *xInc, cudaStream_t st);
 void linws_free(LinWs *w);
-// prec 0: double vectors, 1: float vectors; nv 5 or 6; FP64 accumulation, deterministic
+// prec 0: double vectors, 1: float vectors; nv 5 or 6; split: laid out as in vec_split.cuh, else cell rows; FP64
+// accumulation, deterministic
 // Krylov basis columns are ld apart: ld = n rounded up to a multiple of 4, storage 16-byte aligned, pad zero
 inline int64_t krylov_ld(int64_t n) { return (n + 3) & ~(int64_t)3; }
 // Each is one launch: the last block to finish reduces the per-block partials (cnt: a zeroed device counter
 // the kernels share; it is reset after each use).  colScale (may be null): normalising factors of the
 // basis columns, which are stored unnormalised.
-void krylov_mdot(int prec, int64_t n, int64_t ld, int nv, int ncol, const void *V, const void *w, const real *s2, real *red, real *out,
+void krylov_mdot(int prec, int64_t n, int64_t ld, int nv, bool split, int ncol, const void *V, const void *w, const real *s2, real *red, real *out,
                  const real *colScale, unsigned *cnt, cudaStream_t st);
 // w -= V (h colScale); *outNorm = |w|; with gsc (GMRES scalars) also *scaleNext = 1 / |w| or 0 at a breakdown
-void krylov_maxpy_norm(int prec, int64_t n, int64_t ld, int nv, int ncol, const void *V, const real *h, const real *colScale, void *w,
+void krylov_maxpy_norm(int prec, int64_t n, int64_t ld, int nv, bool split, int ncol, const void *V, const real *h, const real *colScale, void *w,
                        const real *s2, real *red, real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st);
-void krylov_norm(int prec, int64_t n, int nv, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st);
-void krylov_diff_norm(int prec, int64_t n, int nv, const void *x, const void *y, const real *s2, real *red, real *outNorm, unsigned *cnt,
+void krylov_norm(int prec, int64_t n, int nv, bool split, const void *x, const real *s2, real *red, real *outNorm, unsigned *cnt, cudaStream_t st);
+void krylov_diff_norm(int prec, int64_t n, int nv, bool split, const void *x, const void *y, const real *s2, real *red, real *outNorm, unsigned *cnt,
                       cudaStream_t st);
 // A caller-driven Arnoldi process (linsolve.cu): V holds k + 1 columns krylov_ld(n) apart (zero beyond n),
 // H k columns of k + 1, gsc the GMRES scalars ([0] breakdown scale, [1] beta, [2] valid columns, [8...] y),
