@@ -12,6 +12,7 @@
 // ([row][E]).  nbr [r][NF] holds the neighbour row of each slot (-1: none).
 #pragma once
 #include "roejac.cuh"
+#include "chain.cuh"
 
 namespace dndsb
 {
@@ -213,16 +214,23 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_ilu_lower_c(int64_t beg, int64_t 
     const int64_t r = (((beg >> 5) + blockIdx.x) << 5) + lane;
     const bool on = r >= beg && r < end;
     const int nl = on ? cnlow[r] : 0;
-    T f[NF][NV], acc = on ? b[r * NV + i] : T(0);
+    T f[NF][NV];
+    int q[NF];
 #pragma unroll
     for (int j = 0; j < NF; j++)
         if (j < nl)
         {
+            q[j] = cnbr[r * NF + j];
 #pragma unroll
             for (int l = 0; l < NV; l++)
                 f[j][l] = off[offL.at(r, j * NN + i * NV + l)];
-            sx[j][i][lane] = x[(int64_t)cnbr[r * NF + j] * NV + i];
         }
+    chain_step();
+    T acc = on ? b[r * NV + i] : T(0);
+#pragma unroll
+    for (int j = 0; j < NF; j++)
+        if (j < nl)
+            sx[j][i][lane] = x[(int64_t)q[j] * NV + i];
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < NF; j++)
@@ -249,29 +257,33 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_ilu_upper_c(int64_t beg, int64_t 
     const int64_t r = (((beg >> 5) + blockIdx.x) << 5) + lane;
     const bool on = r >= beg && r < end;
     const int nl = on ? cnlow[r] : NF;
-    T f[NF][NV], d[NV], acc = on ? x[r * NV + i] : T(0);
-    bool use[NF];
+    T f[NF][NV], d[NV];
+    int q[NF];
 #pragma unroll
     for (int j = 0; j < NF; j++)
     {
-        const int64_t q = j >= nl ? (int64_t)cnbr[r * NF + j] : -1;
-        use[j] = q >= 0;
-        if (use[j])
+        q[j] = j >= nl ? cnbr[r * NF + j] : -1;
+        if (q[j] >= 0)
         {
 #pragma unroll
             for (int l = 0; l < NV; l++)
                 f[j][l] = off[offL.at(r, j * NN + i * NV + l)];
-            sx[j][i][lane] = x[q * NV + i];
         }
     }
     if (on)
 #pragma unroll
         for (int l = 0; l < NV; l++)
             d[l] = dinv[dL.at(r, i * NV + l)];
+    chain_step();
+    T acc = on ? x[r * NV + i] : T(0);
+#pragma unroll
+    for (int j = 0; j < NF; j++)
+        if (q[j] >= 0)
+            sx[j][i][lane] = x[(int64_t)q[j] * NV + i];
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < NF; j++)
-        if (use[j])
+        if (q[j] >= 0)
         {
             T s = 0;
 #pragma unroll
@@ -296,8 +308,7 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_ilu_upper_c(int64_t beg, int64_t 
 // with rhs: y = rhs - A x
 template <typename T, int NV, int NF>
 DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_block_product(int64_t n, const int32_t *__restrict__ nbr, const T *__restrict__ opB,
-                                                            const T *__restrict__ jdB, const T *__restrict__ x, T *__restrict__ y,
-                                                            const real *__restrict__ xs, const T *__restrict__ rhs)
+                                                            const T *__restrict__ jdB, const T *x, T *y, const real *xs, const T *rhs)
 {
     constexpr int NN = NV * NV;
     const BlockLay oL{NF * NN, 5}, dL{2 * NN, 5};
@@ -305,20 +316,17 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_block_product(int64_t n, const in
     const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
     const int64_t r = ((int64_t)blockIdx.x << 5) + lane;
     const bool on = r < n;
-    const T sc = xs ? (T)*xs : T(1);
     T f[NF][NV], d[NV];
-    bool use[NF];
+    int q[NF];
 #pragma unroll
     for (int j = 0; j < NF; j++)
     {
-        const int64_t q = on ? (int64_t)nbr[r * NF + j] : -1;
-        use[j] = q >= 0;
-        if (use[j])
+        q[j] = on ? nbr[r * NF + j] : -1;
+        if (q[j] >= 0)
         {
 #pragma unroll
             for (int l = 0; l < NV; l++)
                 f[j][l] = opB[oL.at(r, j * NN + i * NV + l)];
-            sx[j][i][lane] = x[q * NV + i];
         }
     }
     if (on)
@@ -326,8 +334,15 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_block_product(int64_t n, const in
 #pragma unroll
         for (int l = 0; l < NV; l++)
             d[l] = jdB[dL.at(r, i * NV + l)];
-        sx[NF][i][lane] = x[r * NV + i];
     }
+    chain_step();
+    const T sc = xs ? (T)*xs : T(1);
+#pragma unroll
+    for (int j = 0; j < NF; j++)
+        if (q[j] >= 0)
+            sx[j][i][lane] = x[(int64_t)q[j] * NV + i];
+    if (on)
+        sx[NF][i][lane] = x[r * NV + i];
     __syncthreads();
     if (!on)
         return;
@@ -337,7 +352,7 @@ DNDSB_GLOBAL void __launch_bounds__(32 * NV) k_block_product(int64_t n, const in
         acc += d[l] * sx[NF][l][lane];
 #pragma unroll
     for (int j = 0; j < NF; j++)
-        if (use[j])
+        if (q[j] >= 0)
         {
             T s = 0;
 #pragma unroll

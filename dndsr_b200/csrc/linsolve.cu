@@ -514,7 +514,7 @@ struct Solve
         const T *old = zeroIn ? nullptr : xOld;
         if (!gs)
         {
-            kern<<<grid_for(m.nCell, 128), 128, 0, st>>>(0, m.nCell, A(), rhs, old, old, xNew, gamma - 1);
+            launch_chained(kern, grid_for(m.nCell, 128), 128, st, 0, m.nCell, A(), rhs, old, old, xNew, gamma - 1);
             return;
         }
         for (int ci = 0; ci < m.nColor; ci++)
@@ -522,7 +522,7 @@ struct Solve
             int col = forward ? ci : m.nColor - 1 - ci;
             int64_t b = m.colorStart[col], e = m.colorStart[col + 1];
             if (e > b)
-                kern<<<grid_for(e - b, 128), 128, 0, st>>>(b, e, A(), rhs, forward ? (const T *)xNew : old, forward ? old : (const T *)xNew, xNew, gamma - 1);
+                launch_chained(kern, grid_for(e - b, 128), 128, st, b, e, A(), rhs, forward ? (const T *)xNew : old, forward ? old : (const T *)xNew, xNew, gamma - 1);
         }
     }
 
@@ -540,7 +540,7 @@ struct Solve
         {
             const int64_t b = m.colorStart[col], e = m.colorStart[col + 1];
             if (e > b)
-                kb<<<grid_for(e - b, 128), 128, 0, st>>>(b, e, A(), x, gamma - 1);
+                launch_chained(kb, grid_for(e - b, 128), 128, st, b, e, A(), x, gamma - 1);
         }
     }
 
@@ -562,13 +562,13 @@ struct Solve
             {
                 const int64_t b = m.colorStart[ci], e = m.colorStart[ci + 1];
                 if (e > b)
-                    kl<<<ilu::tile_blocks(b, e), 32 * NV, 0, st>>>(b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, zero ? rhs : (const T *)r, y);
+                    launch_chained(kl, ilu::tile_blocks(b, e), 32 * NV, st, b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, zero ? rhs : (const T *)r, y);
             }
             for (int ci = m.nColor - 1; ci >= 0; ci--)
             {
                 const int64_t b = m.colorStart[ci], e = m.colorStart[ci + 1];
                 if (e > b)
-                    ku<<<ilu::tile_blocks(b, e), 32 * NV, 0, st>>>(b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, (const T *)w.luD, dlay, y,
+                    launch_chained(ku, ilu::tile_blocks(b, e), 32 * NV, st, b, e, w.luNbr, w.luNLow, (const T *)w.luB, lay, (const T *)w.luD, dlay, y,
                                                                   zero ? (T *)nullptr : x);
             }
         }
@@ -577,7 +577,7 @@ struct Solve
     // y = A (xs x) of the block operator, or rhs - A x
     void product_blk(const T *x, T *y, const real *xs, const T *rhs) const
     {
-        ilu::k_block_product<T, NV, NF><<<ilu::tile_blocks(0, m.nCell), 32 * NV, 0, st>>>(m.nCell, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, x, y,
+        launch_chained(ilu::k_block_product<T, NV, NF>, ilu::tile_blocks(0, m.nCell), 32 * NV, st, m.nCell, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, x, y,
                                                                                         xs, rhs);
     }
 
@@ -616,7 +616,7 @@ struct Solve
             return;
         }
         auto kern = posop::k_product<T, NV, NF>;
-        kern<<<grid_for(m.nCell, 128), 128, 0, st>>>(m.nCell, A(), x, Ax, gamma - 1, xs);
+        launch_chained(kern, grid_for(m.nCell, 128), 128, st, m.nCell, A(), x, Ax, gamma - 1, xs);
     }
 
     // y = M^-1 A (xs x); one symmetric sweep on the scalar-Jacobian operator takes product and sweep together
@@ -634,7 +634,7 @@ struct Solve
         {
             const int64_t b = m.colorStart[col], e = m.colorStart[col + 1];
             if (e > b)
-                kf<<<grid_for(e - b, 128), 128, 0, st>>>(b, e, A(), x, tmp, y, gamma - 1, xs);
+                launch_chained(kf, grid_for(e - b, 128), 128, st, b, e, A(), x, tmp, y, gamma - 1, xs);
         }
         back(y);
     }

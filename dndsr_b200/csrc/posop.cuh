@@ -25,6 +25,7 @@
 #pragma once
 #include "solver.cuh"
 #include "vec_split.cuh"
+#include "chain.cuh"
 
 namespace dndsb
 {
@@ -134,9 +135,11 @@ DNDSB_D void add_jac(const typename Vec4<T>::type &o, const typename Vec4<T>::ty
 }
 
 // buf += sum over the slots [j0, j1) of f (w A - w lambda) x_q, with x = xa, f = fa for slots below ja and xb, fb from
-// there; a group's loads are all issued before the first use
-template <typename T, int NV, int NF>
-DNDSB_D void add_slots(const Op<T> &A, int64_t p, int j0, int j1, int ja, const T *xa, T fa, const T *xb, T fb, T g1, T *buf)
+// there; a group's loads are all issued before the first use.  The first group's coefficients are read ahead of the
+// chain's wait; own() reads the row's own values (and may set fb) right
+// after it.  What the sequence writes is passed without __restrict__, so that no load moves ahead of the wait.
+template <typename T, int NV, int NF, typename F>
+DNDSB_D void add_slots(const Op<T> &A, int64_t p, int j0, int j1, int ja, const T *xa, T fa, const T *xb, const T &fb, T g1, T *buf, F own)
 {
     using T4 = typename Vec4<T>::type;
     constexpr int G = NF <= 4 ? NF : 3;
@@ -156,8 +159,16 @@ DNDSB_D void add_slots(const Op<T> &A, int64_t p, int j0, int j1, int ja, const 
                 o[k] = A.op[slot_at<NF>(p, b + k)];
                 s[k] = A.vh[q[b + k]];
                 nu[k] = NV == 6 ? A.nu[q[b + k]] : T(0);
-                vsplit::load<T, NV>(b + k < ja ? xa : xb, A.n, q[b + k], d[k]);
             }
+        if (b == 0)
+        {
+            chain_step();
+            own();
+        }
+#pragma unroll
+        for (int k = 0; k < G; k++)
+            if (q[b + k] >= 0)
+                vsplit::load<T, NV>(b + k < ja ? xa : xb, A.n, q[b + k], d[k]);
 #pragma unroll
         for (int k = 0; k < G; k++)
             if (q[b + k] >= 0)
@@ -168,7 +179,7 @@ DNDSB_D void add_slots(const Op<T> &A, int64_t p, int j0, int j1, int ja, const 
 // x_p = D_p^-1 (rhs_p - sum_lower xLow - sum_upper xUp) over positions [pBeg, pEnd); a null xLow or xUp is a zero
 // vector whose slots are skipped.  xNew may be xLow or xUp (other colours' rows are read, the own row written).
 template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_sweep(int64_t pBeg, int64_t pEnd, Op<T> A, const T *__restrict__ rhs, const T *xLow, const T *xUp, T *xNew, T g1)
+DNDSB_GLOBAL void k_sweep(int64_t pBeg, int64_t pEnd, Op<T> A, const T *rhs, const T *xLow, const T *xUp, T *xNew, T g1)
 {
     constexpr int JD = jd_of<NV>();
     DNDSB_KERNEL_LOOP(ii, pEnd - pBeg)
@@ -176,11 +187,11 @@ DNDSB_GLOBAL void k_sweep(int64_t pBeg, int64_t pEnd, Op<T> A, const T *__restri
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, nu = (cnt >> 8) & 255;
         T buf[NV], r[NV];
-        vsplit::load<T, NV>(rhs, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
             buf[v] = 0;
-        add_slots<T, NV, NF>(A, p, xLow ? 0 : nl, xUp ? nu : nl, nl, xLow, T(1), xUp, T(1), g1, buf);
+        add_slots<T, NV, NF>(A, p, xLow ? 0 : nl, xUp ? nu : nl, nl, xLow, T(1), xUp, T(1), g1, buf,
+                             [&] { vsplit::load<T, NV>(rhs, A.n, p, r); });
 #pragma unroll
         for (int v = 0; v < NV; v++)
             r[v] = (r[v] - buf[v]) * A.jdi[p * JD + (JD > 1 ? v : 0)];
@@ -198,11 +209,10 @@ DNDSB_GLOBAL void k_back(int64_t pBeg, int64_t pEnd, Op<T> A, T *x, T g1)
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, nu = (cnt >> 8) & 255;
         T buf[NV], r[NV];
-        vsplit::load<T, NV>(x, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
             buf[v] = 0;
-        add_slots<T, NV, NF>(A, p, nl, nu, nl, (const T *)x, T(1), (const T *)x, T(1), g1, buf);
+        add_slots<T, NV, NF>(A, p, nl, nu, nl, (const T *)x, T(1), (const T *)x, T(1), g1, buf, [&] { vsplit::load<T, NV>(x, A.n, p, r); });
 #pragma unroll
         for (int v = 0; v < NV; v++)
             r[v] -= buf[v] * A.jdi[p * JD + (JD > 1 ? v : 0)];
@@ -212,21 +222,24 @@ DNDSB_GLOBAL void k_back(int64_t pBeg, int64_t pEnd, Op<T> A, T *x, T g1)
 
 // the forward half of M^-1 A (s x), s = *xs (null: 1): t_p = D_p^-1 (s sum_{upper, self} x - sum_lower t), y_p = s x_p + t_p
 template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_product_forward(int64_t pBeg, int64_t pEnd, Op<T> A, const T *__restrict__ x, T *t, T *__restrict__ y, T g1,
-                                    const real *__restrict__ xs)
+DNDSB_GLOBAL void k_product_forward(int64_t pBeg, int64_t pEnd, Op<T> A, const T *x, T *t, T *y, T g1, const real *xs)
 {
     constexpr int JD = jd_of<NV>();
-    const T sx = xs ? (T)*xs : T(1);
+    T sx = 1;
     DNDSB_KERNEL_LOOP(ii, pEnd - pBeg)
     {
         const int64_t p = pBeg + ii;
         const int cnt = A.cnt[p], nl = cnt & 255, na = cnt >> 16;
         T buf[NV], r[NV];
-        vsplit::load<T, NV>(x, A.n, p, r);
 #pragma unroll
         for (int v = 0; v < NV; v++)
             buf[v] = 0;
-        add_slots<T, NV, NF>(A, p, 0, na, nl, (const T *)t, T(-1), x, sx, g1, buf);
+        add_slots<T, NV, NF>(A, p, 0, na, nl, (const T *)t, T(-1), x, sx, g1, buf,
+                             [&]
+                             {
+                                 sx = xs ? (T)*xs : T(1);
+                                 vsplit::load<T, NV>(x, A.n, p, r);
+                             });
 #pragma unroll
         for (int v = 0; v < NV; v++)
         {
@@ -240,19 +253,23 @@ DNDSB_GLOBAL void k_product_forward(int64_t pBeg, int64_t pEnd, Op<T> A, const T
 
 // Ax = A (s x), s = *xs (null: 1)
 template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_product(int64_t n, Op<T> A, const T *__restrict__ x, T *__restrict__ Ax, T g1, const real *__restrict__ xs)
+DNDSB_GLOBAL void k_product(int64_t n, Op<T> A, const T *x, T *Ax, T g1, const real *xs)
 {
     constexpr int JD = jd_of<NV>();
-    const T sx = xs ? (T)*xs : T(1);
+    T sx = 1;
     DNDSB_KERNEL_LOOP(p, n)
     {
         const int cnt = A.cnt[p];
         T buf[NV];
-        vsplit::load<T, NV>(x, A.n, p, buf);
+        add_slots<T, NV, NF>(A, p, 0, cnt >> 16, NF, x, T(1), x, T(1), g1, buf,
+                             [&]
+                             {
+                                 sx = xs ? (T)*xs : T(1);
+                                 vsplit::load<T, NV>(x, A.n, p, buf);
 #pragma unroll
-        for (int v = 0; v < NV; v++)
-            buf[v] *= A.jd[p * JD + (JD > 1 ? v : 0)];
-        add_slots<T, NV, NF>(A, p, 0, cnt >> 16, NF, x, T(1), x, T(1), g1, buf);
+                                 for (int v = 0; v < NV; v++)
+                                     buf[v] *= A.jd[p * JD + (JD > 1 ? v : 0)];
+                             });
 #pragma unroll
         for (int v = 0; v < NV; v++)
             buf[v] *= sx;

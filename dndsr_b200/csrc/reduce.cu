@@ -4,6 +4,7 @@
 #include "solver.cuh"
 #include "krylov_update.cuh"
 #include "vec_split.cuh"
+#include "chain.cuh"
 #include <type_traits>
 
 namespace dndsb
@@ -288,6 +289,7 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
                                                        const real *__restrict__ s2, real *partial, real *out, const real *colScale,
                                                        unsigned *cnt)
 {
+    chain_step();
     __shared__ real sh[kKG][kRedBlock / 32];
     __shared__ real ss[8];
     if (threadIdx.x < NV)
@@ -331,6 +333,7 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
                                                              const real *colScale, T *w, const real *__restrict__ s2, real *partial,
                                                              real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext)
 {
+    chain_step();
     __shared__ real hs[32];
     __shared__ real ss[8];
     __shared__ real sh[kRedBlock / 32];
@@ -490,14 +493,14 @@ void kmdot(int64_t n, int64_t ld, int ncol, const void *V, const void *w, const 
            unsigned *cnt, cudaStream_t st)
 {
     const int nG = (ncol + kKG - 1) / kKG;
-    k_kmdot<T, NV, SPLIT><<<kRedBlocks / nG * nG, kRedBlock, 0, st>>>(n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
+    launch_chained(k_kmdot<T, NV, SPLIT>, kRedBlocks / nG * nG, kRedBlock, st, n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
 }
 
 template <typename T, int NV, bool SPLIT>
 void kmaxpy(int64_t n, int64_t ld, int ncol, const void *V, const real *h, const real *colScale, void *w, const real *s2, real *red,
             real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st)
 {
-    k_kmaxpy_norm<T, NV, SPLIT><<<kRedBlocks, kRedBlock, 0, st>>>(n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
+    launch_chained(k_kmaxpy_norm<T, NV, SPLIT>, kRedBlocks, kRedBlock, st, n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
                                                            scaleNext);
 }
 
