@@ -727,12 +727,14 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
                      (T *)w.jdB, ev.errWord);
         if (ls.jacobiCode == 2) // LUSGSMatrixToJacobianLU + InPlaceDecompose, colour by colour
         {
-            auto kf = ilu::k_ilu_factor<T, NV, NF>;
             const ilu::BlockLay lay{NF * NV * NV, 5}, dlay{NV * NV, 5}, jlay{2 * NV * NV, 5};
             for (int ci = 0; ci < m.nColor; ci++)
-                DNDSB_LAUNCH(kf, m.colorStart[ci + 1] - m.colorStart[ci], 64, cs, m.colorStart[ci], m.colorStart[ci + 1], (const int32_t *)nullptr,
-                             w.nbrPos, (const int32_t *)nullptr, (const T *)w.opB, (const T *)w.jdB, lay, dlay, jlay, (T *)w.luB, (T *)w.luD,
-                             ev.errWord, w.luNbr, w.luNLow);
+            {
+                const int64_t b = m.colorStart[ci], e = m.colorStart[ci + 1];
+                if (e > b)
+                    ilu::k_ilu_factor_c<T, NV, NF><<<ilu::tile_blocks(b, e), 32 * NV, 0, cs>>>(
+                        b, e, w.nbrPos, (const T *)w.opB, (const T *)w.jdB, lay, dlay, jlay, (T *)w.luB, (T *)w.luD, ev.errWord, w.luNbr, w.luNLow);
+            }
         }
     }
     else

@@ -217,8 +217,7 @@ void lu_factor_colors(const MeshD &m, EvalD &ev, const real *jd, cudaStream_t st
     const ilu::BlockLay DL{ev.jacMode ? 2 * NN : NN, 0};
     for (int ci = 0; ci < m.nColor; ci++)
         DNDSB_LAUNCH(kf, m.colorStart[ci + 1] - m.colorStart[ci], 64, st, m.colorStart[ci], m.colorStart[ci + 1], m.colorCells, m.cellNbr,
-                     m.cellColor, (const real *)ev.luOff, jd, ilu::BlockLay{NF * NN, 0}, ilu::BlockLay{NN, 0}, DL, ev.luOff, ev.luDinv, ev.errWord,
-                     (int32_t *)nullptr, (int32_t *)nullptr);
+                     m.cellColor, (const real *)ev.luOff, jd, ilu::BlockLay{NF * NN, 0}, ilu::BlockLay{NN, 0}, DL, ev.luOff, ev.luDinv, ev.errWord);
 }
 
 template <int NV, int NF>

@@ -65,3 +65,27 @@ def test_six_variables(nx, kw):
     ev.EvaluateRHS(rhs, u, torch.tensor(rec, device="cuda"))  # also the source Jacobian of the diagonal
     r0 = o.eval_rhs(a, rec)
     _compare(ev, oe, u0, torch.tensor(r0), dTau0, kw, [1.0, 1.2, 1.3, 1.4, 2.5, 1.1], (True,))
+
+
+@pytest.mark.parametrize("name,mk,kind,rs", FIVE, ids=[c[0] for c in FIVE])
+def test_block_ilu(name, mk, kind, rs):
+    """The tiled block ILU(0): rows in partly filled tiles of 32 and tiles shared by two colours."""
+    from tests.test_gpu_roe_jacobian import _reference_solve as reference
+    m, o, vr, ev = _setup(mk, 1, rs, 0.0)
+    oe, u0 = OracleEval(o), _init(o, kind)
+    oe.SetJacobianMode(False, True)
+    ev.SetJacobianMode(False, True)
+    dTau0 = torch.zeros(m.n_cell, dtype=torch.float64)
+    oe.EvaluateDt(dTau0, u0, 5.0)
+    u = u0.cuda()
+    ev.EvaluateDt(torch.zeros(m.n_cell, dtype=torch.float64, device="cuda"), u, 5.0)
+    rec0 = np.zeros((m.n_cell, o.R, 5))
+    rhs = torch.zeros_like(u)
+    ev.EvaluateRHS(rhs, u, torch.tensor(rec0, device="cuda"))  # also the eigenvalues of the Roe term
+    r0 = torch.tensor(o.eval_rhs(u0.numpy(), rec0)) + torch.tensor(np.random.default_rng(5).normal(size=(m.n_cell, 5)))
+    for k in (0, 6):  # two ILU steps alone, and as the preconditioner
+        ref = reference(oe, u0, r0, dTau0, 0.1, 0.5, int(k > 0), 0, max(k, 1), 1, 2)
+        for prec, tol in (("fp64", 1e-10), ("fp32", 1e-5)):  # the bounds of the block solve's parity tests
+            x = torch.zeros_like(rhs)
+            ev.SolveLinear(0.5, dTau0.cuda(), 0.1, u, r0.cuda(), x, gmresCode=int(k > 0), nGmresSpace=max(k, 1), jacobiCode=2, precision=prec)
+            assert relerr(x.cpu().numpy(), ref.numpy()) < tol, (k, prec)
