@@ -216,7 +216,7 @@ DNDSB_D bool last_block_final(int nb, int ncol, const real *partial, real *out, 
     return true;
 }
 
-// weights of the four elements of quad q, for quads q0, q0 + dq, ...: split vectors hold a quad within the first four
+// weights of the four elements of quad q, for quads q0, q0 + dq, ... (dq of either sign): split vectors hold a quad within the first four
 // variables of a cell or within the rest, plain ones start it at variable (4 q) % NV
 template <int NV, bool SPLIT>
 struct QuadWeights
@@ -225,7 +225,7 @@ struct QuadWeights
     int64_t nCell;
     int r, dr;
     DNDSB_D QuadWeights(const real *ss_, int64_t n, int64_t q0, int dq)
-        : ss(ss_), nCell(n / NV), r(SPLIT ? 0 : (int)((4 * q0) % NV)), dr(SPLIT ? 0 : (4 * dq) % NV)
+        : ss(ss_), nCell(n / NV), r(SPLIT ? 0 : (int)((4 * q0) % NV)), dr(SPLIT ? 0 : ((4 * dq) % NV + NV) % NV)
     {
     }
     DNDSB_D real at(int64_t q, int e) const
@@ -242,17 +242,18 @@ struct QuadWeights
     }
 };
 
-// sums of NK columns from V against w over the quads [q0, q1): warp sums into sh[column][warp]
+// sums of NK columns from V against w over the quads q0, q0 + dq, ...: warp sums into sh[column][warp]
 template <typename T, int NV, bool SPLIT, int NK>
-DNDSB_D void mdot_group(int64_t n, int64_t q0, int64_t q1, int64_t ld, const T *V, const T *w, const real *ss,
+DNDSB_D void mdot_group(int64_t n, int64_t q0, int dq, int64_t ld, const T *V, const T *w, const real *ss,
                         real (*sh)[kRedBlock / 32])
 {
     real a[NK];
 #pragma unroll
     for (int k = 0; k < NK; k++)
         a[k] = 0;
-    QuadWeights<NV, SPLIT> qw(ss, n, q0 + threadIdx.x, (int)blockDim.x);
-    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x, qw.next())
+    const int64_t nq = (n + 3) >> 2;
+    QuadWeights<NV, SPLIT> qw(ss, n, q0, dq);
+    for (int64_t q = q0; q < nq; q += dq, qw.next())
     {
         // every load issued (in its storage type) before the first use
         typename Quad<T>::raw v[NK];
@@ -284,6 +285,10 @@ DNDSB_D void mdot_group(int64_t n, int64_t q0, int64_t q1, int64_t ld, const T *
 // block makes one pass: 592 blocks that each walked all column groups over a chunk of 592 paid a block reduction per
 // group for one or two quads per thread (30 steps of 249,600 tets in FP64: 1.30 -> 1.08 ms).  partial [chunks][ncol]; the
 // last block to finish sums the chunks.
+// All chunks advance together through the vector (a chunk's threads take every nChunk-th group of 256 quads), so what the
+// caches hold at the end is the end of every column: k_kmaxpy_norm walks back from there.  With each block on a range of
+// its own and both kernels forwards, GMRES(30) took 3.49 ms for 249,600 tets in FP64 and 12.45 ms for 1,996,800 in FP32,
+// now 3.30 and 12.10.
 template <typename T, int NV, bool SPLIT>
 DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld, int ncol, int nG, const T *V, const T *w,
                                                        const real *__restrict__ s2, real *partial, real *out, const real *colScale,
@@ -298,19 +303,19 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
     const int grp = blockIdx.x % nG, chunk = blockIdx.x / nG, nChunk = gridDim.x / nG;
     const int base = ncol / nG, extra = ncol - base * nG; // the first `extra` groups have one column more
     const int c0 = grp * base + (grp < extra ? grp : extra), nk = base + (grp < extra ? 1 : 0);
-    const int64_t nq = (n + 3) >> 2, cq = (nq + nChunk - 1) / nChunk;
-    const int64_t q0 = chunk * cq, q1 = q0 + cq < nq ? q0 + cq : nq;
+    const int64_t q0 = (int64_t)chunk * blockDim.x + threadIdx.x;
+    const int dq = nChunk * (int)blockDim.x;
     const T *Vc = V + (int64_t)c0 * ld;
     switch (nk)
     {
-    case 1: mdot_group<T, NV, SPLIT, 1>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 2: mdot_group<T, NV, SPLIT, 2>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 3: mdot_group<T, NV, SPLIT, 3>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 4: mdot_group<T, NV, SPLIT, 4>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 5: mdot_group<T, NV, SPLIT, 5>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 6: mdot_group<T, NV, SPLIT, 6>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    case 7: mdot_group<T, NV, SPLIT, 7>(n, q0, q1, ld, Vc, w, ss, sh); break;
-    default: mdot_group<T, NV, SPLIT, 8>(n, q0, q1, ld, Vc, w, ss, sh); break;
+    case 1: mdot_group<T, NV, SPLIT, 1>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 2: mdot_group<T, NV, SPLIT, 2>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 3: mdot_group<T, NV, SPLIT, 3>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 4: mdot_group<T, NV, SPLIT, 4>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 5: mdot_group<T, NV, SPLIT, 5>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 6: mdot_group<T, NV, SPLIT, 6>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    case 7: mdot_group<T, NV, SPLIT, 7>(n, q0, dq, ld, Vc, w, ss, sh); break;
+    default: mdot_group<T, NV, SPLIT, 8>(n, q0, dq, ld, Vc, w, ss, sh); break;
     }
     __syncthreads();
     if ((int)threadIdx.x < nk)
@@ -323,7 +328,8 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmdot(int64_t n, int64_t ld,
     last_block_final(nChunk, ncol, partial, out, colScale, 0, cnt);
 }
 
-// w -= sum_c h[c] colScale[c] V[c] (columns subtracted in index order); the last block writes
+// w -= sum_c h[c] colScale[c] V[c] (columns subtracted in index order), the quads from the last to the first (see k_kmdot);
+// the last block writes
 // *outNorm = sqrt(sum_i w_i^2 s2[var(i)]) of the stored w.  w is column ncol of the same basis (not read
 // through V).  With gsc (the GMRES scalars: [0] scale, [2] valid columns) it also sets the normalising
 // factor of the new column, *scaleNext = 1 / norm, or 0 at a breakdown (norm <= 1e-32 scale), which it
@@ -342,12 +348,14 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
     if (threadIdx.x < NV)
         ss[threadIdx.x] = s2[threadIdx.x];
     __syncthreads();
-    const int64_t nq = (n + 3) >> 2, cq = (nq + gridDim.x - 1) / gridDim.x;
-    const int64_t q0 = blockIdx.x * cq, q1 = q0 + cq < nq ? q0 + cq : nq;
+    const int64_t nq = (n + 3) >> 2, dq = (int64_t)gridDim.x * blockDim.x, at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t q1 = at + (nq - 1) / dq * dq; // the thread's last quad, or one dq beyond
     real a = 0;
-    QuadWeights<NV, SPLIT> qw(ss, n, q0 + threadIdx.x, (int)blockDim.x);
-    for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x, qw.next())
+    QuadWeights<NV, SPLIT> qw(ss, n, q1, -(int)dq);
+    for (int64_t q = q1; q >= 0; q -= dq, qw.next())
     {
+        if (q >= nq)
+            continue;
         real x[4];
         Quad<T>::load(w + 4 * q, x);
         int c = 0;
@@ -488,19 +496,26 @@ DNDSB_GLOBAL void k_kdiff_norm(int64_t n, const T *__restrict__ x, const T *__re
     last_block_final(gridDim.x, 1, partial, outNorm, nullptr, 1, cnt);
 }
 
+// blocks of kRedBlock threads for n elements, at most `most`, each thread with the same number of quads where it can be
+unsigned even_blocks(int64_t n, int most)
+{
+    const int64_t nq = (n + 3) >> 2, rounds = (nq + (int64_t)most * kRedBlock - 1) / ((int64_t)most * kRedBlock);
+    return (unsigned)((nq + rounds * kRedBlock - 1) / (rounds * kRedBlock));
+}
+
 template <typename T, int NV, bool SPLIT>
 void kmdot(int64_t n, int64_t ld, int ncol, const void *V, const void *w, const real *s2, real *red, real *out, const real *colScale,
            unsigned *cnt, cudaStream_t st)
 {
     const int nG = (ncol + kKG - 1) / kKG;
-    launch_chained(k_kmdot<T, NV, SPLIT>, kRedBlocks / nG * nG, kRedBlock, st, n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
+    launch_chained(k_kmdot<T, NV, SPLIT>, even_blocks(n, kRedBlocks / nG) * nG, kRedBlock, st, n, ld, ncol, nG, (const T *)V, (const T *)w, s2, red, out, colScale, cnt);
 }
 
 template <typename T, int NV, bool SPLIT>
 void kmaxpy(int64_t n, int64_t ld, int ncol, const void *V, const real *h, const real *colScale, void *w, const real *s2, real *red,
             real *outNorm, unsigned *cnt, real *gsc, int j, real *scaleNext, cudaStream_t st)
 {
-    launch_chained(k_kmaxpy_norm<T, NV, SPLIT>, kRedBlocks, kRedBlock, st, n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
+    launch_chained(k_kmaxpy_norm<T, NV, SPLIT>, even_blocks(n, kRedBlocks), kRedBlock, st, n, ld, ncol, (const T *)V, h, colScale, (T *)w, s2, red, outNorm, cnt, gsc, j,
                                                            scaleNext);
 }
 
