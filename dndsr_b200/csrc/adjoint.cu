@@ -17,6 +17,7 @@
 #include "basis_eval.cuh"
 #include "bc.cuh"
 #include "vr_vjp.cuh"
+#include "roe_rev.cuh"
 
 namespace dndsb
 {
@@ -116,7 +117,7 @@ DNDSB_GLOBAL void k_rhs_vjp_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, con
     }
 }
 
-// The same for the boundary faces (side 0): the ghost states are differentiated with the flux, with respect to the point
+// The same for the boundary faces (side 0), any flux: the ghost states are differentiated with the flux, with respect to the point
 // state (pass 0) and to the cell mean at the face centre (pass 1), five seeds each.  Thread (pass, face, point), one
 // warp per pass, the sums over the points shared out in point order: a thread that walked both passes and the points of a
 // face took 103 us for 19,040 faces of 3 points, this 87 us.
@@ -173,6 +174,110 @@ DNDSB_GLOBAL void __launch_bounds__(64) k_rhs_vjp_bnd(MeshD m, GeomD g, VRD vr, 
     }
     __syncthreads();
     for (int e = threadIdx.x; e < rows * W; e += 64)
+    {
+        const int fi = e / W, i = e - fi * W, j = i / NV - 1, v = i - (j + 1) * NV;
+        if ((int64_t)blockIdx.x * rows + fi >= m.nBndFace)
+            break;
+        real acc = 0;
+        for (int p = 0; p < nG; p++)
+        {
+            const real *r = sm[fi * nG + p];
+            acc += j < 0 ? r[v] + r[NV + v] : r[2 * NV + j] * r[v];
+        }
+        faceAdj[(int64_t)m.bndFace[(int64_t)blockIdx.x * rows + fi] * 2 * W + i] = acc;
+    }
+}
+
+// The boundary faces under plain Roe or HLLE+: the flux reversed by hand (roe_rev.cuh) with respect to both point states
+// and, through the Roe averages, both means; only the ghost states are differentiated by dual numbers, at the point and at
+// the face centre.  One thread per (face, point), 32 threads, the sums over the points shared out in point order.  For 19,040
+// faces of 3 points 27 us, with k_rhs_vjp_bnd 87 us (1.3 KB stack per thread).
+template <int DIM, int P, bool HLLEP>
+DNDSB_GLOBAL void __launch_bounds__(32) k_rhs_vjp_bnd_rev(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const real *__restrict__ w,
+                                                          const real *__restrict__ u, const real *__restrict__ uRec,
+                                                          const real *__restrict__ dLamCell, real *__restrict__ faceAdj, int *err)
+{
+    constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, W = (R + 1) * NV, ROW = (2 * NV + R) | 1;
+    using D5 = Dual<NV>;
+    __shared__ real sm[32][ROW]; // per point: d/dU, d/du (the mean), phi
+    const int nG = g.nGf, rows = 32 / nG, lane = threadIdx.x, fl = lane / nG, q = lane - fl * nG;
+    const int64_t ii = (int64_t)blockIdx.x * rows + fl;
+    if (fl < rows && ii < m.nBndFace)
+    {
+        const int64_t f = m.bndFace[ii], c0 = m.face2cell[f * 2];
+        const int zone = m.faceZone[f];
+        const real *n = &g.faceNorm[(f * nG + q) * 3], *nm = &g.faceMeanNorm[f * 3];
+        const real JW = g.faceJDet[f * nG + q] * g.faceQw[q], iv = 1.0 / g.vol[c0], dLambda = dLamCell[c0];
+        real phi[R], UL[NV], UR[NV], ULm[NV], URm[NV], Fbar[NV], Ub0[NV], Ub1[NV], mb0[NV], mb1[NV];
+        basis_rows<DIM, P, false>(g, vr, c0, &g.facePP[(f * nG + q) * 3], phi, nullptr);
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+        {
+            real a = u[c0 * NV + v];
+            ULm[v] = a;
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                a += phi[j] * uRec[(c0 * R + j) * NV + v];
+            UL[v] = a;
+            Fbar[v] = -(JW * (w[c0 * NV + v] * iv));
+        }
+        // Ub += (dghost(U) / dU)^T Ugb
+        auto ghost_rev = [&](const real *U, const real *nn, const real *Ugb, real *Ub)
+        {
+            D5 a[NV], b[NV];
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                a[v] = D5::var(U[v], v);
+            if (!bc_value<NV>(vr.bnd, zone, a, nn, b))
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    b[v] = a[v];
+#pragma unroll
+            for (int i = 0; i < NV; i++)
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    Ub[i] += b[v].d[i] * Ugb[v];
+        };
+        if (!bc_value<NV>(vr.bnd, zone, UL, n, UR))
+            for (int v = 0; v < NV; v++)
+                UR[v] = UL[v];
+        if (!bc_value<NV>(vr.bnd, zone, ULm, nm, URm))
+            for (int v = 0; v < NV; v++)
+                URm[v] = ULm[v];
+        RoeAvg r;
+        roe_average(ULm, URm, s.gamma, r);
+        if (!(r.asqr > 0 && UL[0] > 0 && UR[0] > 0))
+            atomicOr(err, (int)DE_NONPHYSICAL);
+        roe_rev::RoeBar rb;
+        roe_rev::roebar_zero(rb);
+        if constexpr (HLLEP)
+            roe_rev::hllep_rev(UL, UR, n, r, s.gamma, dLambda, s.rsFixScale, Fbar, Ub0, Ub1, rb);
+        else
+        {
+            real incU[NV], incFb[NV], incUb[NV];
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                incU[v] = UR[v] - UL[v], incFb[v] = -0.5 * Fbar[v];
+            roe_rev::roe0_diss_rev(incU, n, r, s.gamma, dLambda, s.rsFixScale, s.rsIncFScale, incFb, incUb, rb);
+            flux_jac_du_t<NV>(UL, n, Fbar, 0.0, s.gamma, Ub0);
+            flux_jac_du_t<NV>(UR, n, Fbar, 0.0, s.gamma, Ub1);
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+                Ub0[v] = 0.5 * Ub0[v] - incUb[v], Ub1[v] = 0.5 * Ub1[v] + incUb[v];
+        }
+        roe_rev::roe_average_rev(0, ULm, URm, r, s.gamma, rb, mb0);
+        roe_rev::roe_average_rev(1, ULm, URm, r, s.gamma, rb, mb1);
+        ghost_rev(UL, n, Ub1, Ub0);
+        ghost_rev(ULm, nm, mb1, mb0);
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+            sm[lane][v] = Ub0[v], sm[lane][NV + v] = mb0[v];
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            sm[lane][2 * NV + j] = phi[j];
+    }
+    __syncwarp();
+    for (int e = lane; e < rows * W; e += 32)
     {
         const int fi = e / W, i = e - fi * W, j = i / NV - 1, v = i - (j + 1) * NV;
         if ((int64_t)blockIdx.x * rows + fi >= m.nBndFace)
@@ -421,8 +526,13 @@ int rhs_vjp_dp(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const r
     if (m.nBndFace > 0)
     {
         const int rows = 32 / g.nGf; // at most 16 points per face
-        k_rhs_vjp_bnd<DIM, P><<<(unsigned)((m.nBndFace + rows - 1) / rows), 64, 0, st>>>(m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf,
-                                                                                       ev.errWord);
+        const unsigned nb = (unsigned)((m.nBndFace + rows - 1) / rows);
+        if (ev.s.rsType == RS_Roe)
+            k_rhs_vjp_bnd_rev<DIM, P, false><<<nb, 32, 0, st>>>(m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
+        else if (ev.s.rsType == RS_HLLEP)
+            k_rhs_vjp_bnd_rev<DIM, P, true><<<nb, 32, 0, st>>>(m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
+        else
+            k_rhs_vjp_bnd<DIM, P><<<nb, 64, 0, st>>>(m, g, vr, ev.s, w, u, uRec, ev.deltaLambdaCell, ev.adjBuf, ev.errWord);
     }
     bool viscDone = false;
     if (roe)

@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(32 * NG, vjp_min_blocks<NG>())
 // the 64 cells are staged by the warp and the face records leave through the same shared memory, so both run along
 // memory; the points accumulate in registers (sum_q Ub and sum_q x_d Ub, of which the rows of the linear basis are
 // combinations).  A thread that read and wrote its rows in place touched a line per lane and access
-// (668 us for 508,720 faces of 3 points, now 355; one thread per point, k_rhs_vjp_fast, 512 us, and 13 against 21 us at
+// (564 us for 508,720 faces of 3 points, now 355; one thread per point, k_rhs_vjp_fast, 512 us, and 13 against 21 us at
 // 5,008 faces, where it no longer matters).
 template <int DIM, int NG, bool HLLEP>
 __global__ void __launch_bounds__(64, 4)

@@ -239,8 +239,9 @@ int rhs_vjp_roe_interior(const MeshD &m, const GeomD &g, const VRD &vr, const Ev
     if (es < 0 || ev.s.nVars != NV)
         return ST_UNSUPPORTED;
     *viscDone = false;
-    // plain Roe and HLLE+: the kernels of adjoint_fast.cuh (508,720 inviscid faces of degree 2: 1.39 against 2.23 ms in
-    // the thread-per-face kernel below, which takes the other schemes and the quadratures those do not cover)
+    // plain Roe and HLLE+: the kernels of adjoint_fast.cuh (508,720 faces of degree 2 without the viscous flux: 1.39 ms;
+    // the thread-per-face kernel below with the boundary faces 2.23 ms; it takes the other schemes and the quadratures that
+    // those do not cover)
     if (es == 0 || es == kHLLEP)
     {
         int rc = rhs_vjp_interior_fast(m, g, vr, ev, es == kHLLEP, w, u, uRec, faceAdj, st);
