@@ -21,13 +21,25 @@ DNDSB_D void chain_step()
 }
 
 template <typename... P, typename... A>
-void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A &&...args)
+void launch_chained_shared(void (*kernel)(P...), unsigned grid, unsigned block, size_t shared, cudaStream_t st, A &&...args)
 {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(block), cfg.stream = st, cfg.attrs = &at, cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = shared, cfg.stream = st, cfg.attrs = &at, cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A &&...args)
+{
+    launch_chained_shared(kernel, grid, block, 0, st, std::forward<A>(args)...);
+}
+// DNDSB_LAUNCH, chained
+#define DNDSB_CHAIN(kernel, n, block, stream, ...)                                                           \
+    do                                                                                                       \
+    {                                                                                                        \
+        if ((n) > 0)                                                                                         \
+            ::dndsb::launch_chained(kernel, ::dndsb::grid_for((n), (block)), (block), (stream), __VA_ARGS__); \
+    } while (0)
 } // namespace dndsb

@@ -20,6 +20,7 @@
 #include "basis_eval.cuh"
 #include "sa.cuh"
 #include "fast_common.cuh"
+#include "chain.cuh"
 
 namespace dndsb
 {
@@ -47,8 +48,7 @@ constexpr int min_blocks()
 template <int DIM, int P, int NV, int NG, int MODE, bool LAM>
 __global__ void __launch_bounds__(32 * NG, min_blocks<P, NG>())
     k_rhs_face_fast(MeshD m, GeomD g, const real *__restrict__ facePt, const real *__restrict__ cellPar, const real *__restrict__ moment,
-                    EulerSettingsD s, const real *__restrict__ u, const real *__restrict__ uRec, const real *__restrict__ dLamCell,
-                    real *__restrict__ faceFlux, int *err, real *__restrict__ lam)
+                    EulerSettingsD s, const real *u, const real *uRec, const real *dLamCell, real *faceFlux, int *err, real *lam)
 {
     using Lt = Layout<DIM, P, NV>;
     constexpr int CS = Lt::CS;
@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(32 * NG, min_blocks<P, NG>())
     const int64_t f = f0 + fl;
     // every warp holds the cells of the block's 32 faces and stages its share of their rows
     const int c0 = f < m.nFace ? m.face2cell[f * 2] : -1, c1 = f < m.nFace ? m.face2cell[f * 2 + 1] : -1;
+    chain_step();
 #pragma unroll 4
     for (int t = q; t < 64; t += NG)
     {
@@ -268,8 +269,8 @@ int launch_rhs_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &
     unsigned nb = (unsigned)((m.nFace + 31) / 32);
     real *lam = ev.jacMode == 2 ? ev.lambdaFace0 : nullptr;
 #define DNDSB_RFF(MODE, LAM)                                                                                                                  \
-    k_rhs_face_fast<DIM, P, NV, NG, MODE, LAM><<<nb, 32 * NG, smem, st>>>(m, g, ev.facePt, ev.cellPar, vr.baseMoment, ev.s, u, uRec,            \
-                                                                          ev.deltaLambdaCell, ff, ev.errWord, lam)
+    launch_chained_shared(k_rhs_face_fast<DIM, P, NV, NG, MODE, LAM>, nb, 32 * NG, smem, st, m, g, ev.facePt, ev.cellPar, vr.baseMoment, ev.s, u,  \
+                          uRec, ev.deltaLambdaCell, ff, ev.errWord, lam)
     if (ev.s.ignoreVis)
     {
         if (lam)

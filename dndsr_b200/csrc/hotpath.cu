@@ -7,6 +7,7 @@
 #include "wall_flux.cuh"
 #include "basis_rows.cuh"
 #include "pseudo.cuh"
+#include "chain.cuh"
 
 namespace dndsb
 {
@@ -84,6 +85,7 @@ DNDSB_GLOBAL void k_fill_from(int64_t n, const real *src, real *out)
 
 DNDSB_GLOBAL void k_swap(int64_t n, real *a, real *b)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(i, n)
     {
         real t = a[i];
@@ -203,8 +205,9 @@ DNDSB_GLOBAL void k_rhs_face(MeshD m, GeomD g, VRD vr, EulerSettingsD s, const r
 // per-cell gather of the face fluxes (deterministic, replaces the reference's face scatter)
 template <int NV>
 DNDSB_GLOBAL void k_rhs_gather(int64_t nCell, int nf, const int32_t *__restrict__ c2f, const real *__restrict__ vol,
-                               const real *__restrict__ faceFlux, real *__restrict__ rhs)
+                               const real *faceFlux, real *rhs)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(c, nCell)
     {
         real acc[NV];
@@ -228,9 +231,10 @@ DNDSB_GLOBAL void k_rhs_gather(int64_t nCell, int nf, const int32_t *__restrict_
 // Local time step: EulerEvaluator_EvaluateDt.hxx:875-1039
 // ---------------------------------------------------------------------------
 template <int NV>
-DNDSB_GLOBAL void k_dt_face(MeshD m, GeomD g, EulerSettingsD s, const real *__restrict__ u, real *lamFace, real *lamFaceC,
+DNDSB_GLOBAL void k_dt_face(MeshD m, GeomD g, EulerSettingsD s, const real *u, real *lamFace, real *lamFaceC,
                             real *lamFaceVis, real *lamConv, real *dLamFace)
 {
+    chain_step();
     const real gamma = s.gamma, cp = s.Rgas * gamma / (gamma - 1);
     DNDSB_KERNEL_LOOP(f, m.nFace)
     {
@@ -276,9 +280,10 @@ DNDSB_GLOBAL void k_dt_face(MeshD m, GeomD g, EulerSettingsD s, const real *__re
     }
 }
 
-DNDSB_GLOBAL void k_dt_cell(MeshD m, GeomD g, const real *__restrict__ lamFace, const real *__restrict__ dLamFace, real CFL, real MaxDt,
+DNDSB_GLOBAL void k_dt_cell(MeshD m, GeomD g, const real *lamFace, const real *dLamFace, real CFL, real MaxDt,
                             real *dt, real *dLamCell)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(c, m.nCell)
     {
         real lc = 0, dl = 0;
@@ -640,7 +645,7 @@ int vr_iter(const MeshD &m, const GeomD &g, const VRD &vr, int nv, const real *u
 
 int vr_swap(int64_t n, real *a, real *b, cudaStream_t st)
 {
-    DNDSB_LAUNCH(k_swap, n, 256, st, n, a, b);
+    DNDSB_CHAIN(k_swap, n, 256, st, n, a, b);
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 
@@ -772,10 +777,10 @@ int eval_rhs_ex(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const 
     if (brc != ST_OK)
         return brc;
     if (nv == 5)
-        DNDSB_LAUNCH(k_rhs_gather<5>, m.nCell, 256, st, m.nCell, m.nf, m.cell2face, g.vol, ff, rhs);
+        DNDSB_CHAIN(k_rhs_gather<5>, m.nCell, 256, st, m.nCell, m.nf, m.cell2face, g.vol, ff, rhs);
     else
     {
-        DNDSB_LAUNCH(k_rhs_gather<6>, m.nCell, 256, st, m.nCell, m.nf, m.cell2face, g.vol, ff, rhs);
+        DNDSB_CHAIN(k_rhs_gather<6>, m.nCell, 256, st, m.nCell, m.nf, m.cell2face, g.vol, ff, rhs);
         // SA source (EvaluateRHS.hxx:665-801) and its Jacobian diagonal JSource
         if (!ev.dWall)
             return ST_BADARG;
@@ -824,14 +829,14 @@ int eval_dt(const MeshD &m, const GeomD &g, EvalD &ev, const real *u, real CFL, 
             cudaStream_t st)
 {
     if (ev.s.nVars == 5)
-        DNDSB_LAUNCH(k_dt_face<5>, m.nFace, 256, st, m, g, ev.s, u, ev.lambdaFace, ev.lambdaFaceC, ev.lambdaFaceVis, ev.lambdaConv,
+        DNDSB_CHAIN(k_dt_face<5>, m.nFace, 256, st, m, g, ev.s, u, ev.lambdaFace, ev.lambdaFaceC, ev.lambdaFaceVis, ev.lambdaConv,
                      ev.deltaLambdaFace);
     else if (ev.s.nVars == 6)
-        DNDSB_LAUNCH(k_dt_face<6>, m.nFace, 256, st, m, g, ev.s, u, ev.lambdaFace, ev.lambdaFaceC, ev.lambdaFaceVis, ev.lambdaConv,
+        DNDSB_CHAIN(k_dt_face<6>, m.nFace, 256, st, m, g, ev.s, u, ev.lambdaFace, ev.lambdaFaceC, ev.lambdaFaceVis, ev.lambdaConv,
                      ev.deltaLambdaFace);
     else
         return ST_UNSUPPORTED;
-    DNDSB_LAUNCH(k_dt_cell, m.nCell, 256, st, m, g, ev.lambdaFace, ev.deltaLambdaFace, CFL, MaxDt, dt, ev.deltaLambdaCell);
+    DNDSB_CHAIN(k_dt_cell, m.nCell, 256, st, m, g, ev.lambdaFace, ev.deltaLambdaFace, CFL, MaxDt, dt, ev.deltaLambdaCell);
     if (ev.lambdaFace0) // lambdaFace0 = lambdaFace123 = lambdaFace4 = the convective speed (EvaluateDt.hxx:995-996)
         for (real *l : {ev.lambdaFace0, ev.lambdaFace123, ev.lambdaFace4})
             d2d(l, ev.lambdaConv, sizeof(real) * m.nFace, st);
@@ -936,9 +941,10 @@ namespace
 {
 // res = resOther - u / dt + alphaDiag rhs and dTau *= 1 / alphaDiag (ODE.hpp:300-330 with EulerSolver.hxx:674-694)
 template <int NV>
-DNDSB_GLOBAL void k_unsteady_residual(int64_t nCell, const real *__restrict__ other, const real *__restrict__ u, const real *__restrict__ rhs,
-                                      real mInvDt, real alphaDiag, real *__restrict__ res, real *__restrict__ dTau)
+DNDSB_GLOBAL void k_unsteady_residual(int64_t nCell, const real *other, const real *u, const real *rhs, real mInvDt, real alphaDiag, real *res,
+                                      real *dTau)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(e, nCell * NV)
     {
         res[e] = (other[e] + mInvDt * u[e]) + alphaDiag * rhs[e];
@@ -947,8 +953,9 @@ DNDSB_GLOBAL void k_unsteady_residual(int64_t nCell, const real *__restrict__ ot
     }
 }
 
-DNDSB_GLOBAL void k_add(int64_t n, const real *__restrict__ a, real *__restrict__ x)
+DNDSB_GLOBAL void k_add(int64_t n, const real *a, real *x)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(i, n)
     x[i] += a[i];
 }
@@ -958,9 +965,9 @@ int unsteady_residual(int64_t nCell, int nv, const real *other, const real *u, c
                       cudaStream_t st)
 {
     if (nv == 5)
-        DNDSB_LAUNCH(k_unsteady_residual<5>, nCell * 5, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
+        DNDSB_CHAIN(k_unsteady_residual<5>, nCell * 5, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
     else if (nv == 6)
-        DNDSB_LAUNCH(k_unsteady_residual<6>, nCell * 6, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
+        DNDSB_CHAIN(k_unsteady_residual<6>, nCell * 6, 256, st, nCell, other, u, rhs, -1.0 / dt, alphaDiag, res, dTau);
     else
         return ST_UNSUPPORTED;
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
@@ -968,7 +975,7 @@ int unsteady_residual(int64_t nCell, int nv, const real *other, const real *u, c
 
 int add_increment(int64_t n, const real *inc, real *u, cudaStream_t st)
 {
-    DNDSB_LAUNCH(k_add, n, 256, st, n, inc, u);
+    DNDSB_CHAIN(k_add, n, 256, st, n, inc, u);
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 

@@ -48,8 +48,9 @@ namespace
 {
 // natural order FP64 -> position order T, and back
 template <typename T, int NV>
-DNDSB_GLOBAL void k_gather_T(int64_t n, bool split, const int32_t *__restrict__ pos2cell, const real *__restrict__ x, T *y)
+DNDSB_GLOBAL void k_gather_T(int64_t n, bool split, const int32_t *__restrict__ pos2cell, const real *x, T *y)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(p, n)
     {
         int64_t c = pos2cell[p];
@@ -65,8 +66,9 @@ DNDSB_GLOBAL void k_gather_T(int64_t n, bool split, const int32_t *__restrict__ 
 }
 
 template <typename T, int NV>
-DNDSB_GLOBAL void k_scatter_T(int64_t n, bool split, const int32_t *__restrict__ pos2cell, const T *__restrict__ y, real *x)
+DNDSB_GLOBAL void k_scatter_T(int64_t n, bool split, const int32_t *__restrict__ pos2cell, const T *y, real *x)
 {
+    chain_step();
     DNDSB_KERNEL_LOOP(p, n)
     {
         int64_t c = pos2cell[p];
@@ -738,8 +740,8 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         }
     }
     else
-        DNDSB_LAUNCH(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
-    DNDSB_LAUNCH(kgather, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, rhs, (T *)w.rhsT);
+        DNDSB_CHAIN(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
+    DNDSB_CHAIN(kgather, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, rhs, (T *)w.rhsT);
     if (direct)
         S.body();
     else if (ls.useGraph)
@@ -771,7 +773,7 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         w.key = ls, w.keyValid = true;
         S.body();
     }
-    DNDSB_LAUNCH(kscatter, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, (const T *)w.x, xInc);
+    DNDSB_CHAIN(kscatter, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, (const T *)w.x, xInc);
     if (!direct)
     {
         event_record(w.evOut, cs);

@@ -56,9 +56,10 @@ struct Op
 };
 
 template <typename T, int NV, int NF>
-DNDSB_GLOBAL void k_build(MeshD m, GeomD g, const real *__restrict__ lamFace, const real *__restrict__ dTau, real dt, real alphaDiag,
-                          real gamma, const real *__restrict__ u, const real *__restrict__ jSource, const int32_t *__restrict__ cellPos, Op<T> A)
+DNDSB_GLOBAL void k_build(MeshD m, GeomD g, const real *lamFace, const real *dTau, real dt, real alphaDiag, real gamma, const real *u,
+                          const real *jSource, const int32_t *__restrict__ cellPos, Op<T> A)
 {
+    chain_step();
     using T4 = typename Vec4<T>::type;
     DNDSB_KERNEL_LOOP(p, m.nCell)
     {

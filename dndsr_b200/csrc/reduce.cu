@@ -30,8 +30,9 @@ DNDSB_D real warp_red(real x)
 // partial[block][col] over the block's rows; x is [n][ncol], ncol at most 8, optional row weight w.  One pass for all
 // columns, a thread per row: a tree per column over 592 blocks took 6.3 us for 8,192 rows of 5 and the final one 5.6.
 template <int OP>
-DNDSB_GLOBAL void k_reduce_cols(int64_t n, int ncol, const real *__restrict__ x, const real *__restrict__ w, int powP, real *partial)
+DNDSB_GLOBAL void k_reduce_cols(int64_t n, int ncol, const real *x, const real *__restrict__ w, int powP, real *partial)
 {
+    chain_step();
     __shared__ real sh[kRedBlock / 32][8];
     real a[8];
 #pragma unroll
@@ -68,8 +69,9 @@ DNDSB_GLOBAL void k_reduce_cols(int64_t n, int ncol, const real *__restrict__ x,
 
 // one warp per column
 template <int OP>
-DNDSB_GLOBAL void k_reduce_final(int nb, int ncol, const real *__restrict__ partial, real *out)
+DNDSB_GLOBAL void k_reduce_final(int nb, int ncol, const real *partial, real *out)
 {
+    chain_step();
     const int col = threadIdx.x >> 5, lane = threadIdx.x & 31;
     real a = OP == 0 ? 0.0 : OP == 1 ? kVeryLarge : -kVeryLarge;
     for (int i = lane; i < nb; i += 32)
@@ -88,18 +90,18 @@ real *reduce_cols(int op, int64_t n, int ncol, const real *x, const real *w, int
     const int nb = want < 1 ? 1 : want < kRedBlocks ? (int)want : kRedBlocks;
     if (op == 0)
     {
-        k_reduce_cols<0><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<0><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
+        launch_chained(k_reduce_cols<0>, nb, kRedBlock, st, n, ncol, x, w, powP, redBuf);
+        launch_chained(k_reduce_final<0>, 1, 32 * ncol, st, nb, ncol, redBuf, out);
     }
     else if (op == 1)
     {
-        k_reduce_cols<1><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<1><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
+        launch_chained(k_reduce_cols<1>, nb, kRedBlock, st, n, ncol, x, w, powP, redBuf);
+        launch_chained(k_reduce_final<1>, 1, 32 * ncol, st, nb, ncol, redBuf, out);
     }
     else
     {
-        k_reduce_cols<2><<<nb, kRedBlock, 0, st>>>(n, ncol, x, w, powP, redBuf);
-        k_reduce_final<2><<<1, 32 * ncol, 0, st>>>(nb, ncol, redBuf, out);
+        launch_chained(k_reduce_cols<2>, nb, kRedBlock, st, n, ncol, x, w, powP, redBuf);
+        launch_chained(k_reduce_final<2>, 1, 32 * ncol, st, nb, ncol, redBuf, out);
     }
     return out;
 }

@@ -19,6 +19,7 @@
 #include "solver.cuh"
 #include "sweep_layout.cuh"
 #include "fast_common.cuh"
+#include "chain.cuh"
 
 namespace dndsb
 {
@@ -39,9 +40,10 @@ constexpr int kStagedRows = 3; // rows a thread of the staged kernel takes
 
 template <int R, int NV, int NF, typename TC>
 __global__ void __launch_bounds__(32 * (R / kStagedRows))
-    k_vr_sweep_staged(int64_t nCell, const int32_t *__restrict__ nbr, const TC *__restrict__ coef, const real *__restrict__ uRec,
-                      real *__restrict__ uRecNew, const real *__restrict__ u, real relax, int recordInc, int uRecIsZero)
+    k_vr_sweep_staged(int64_t nCell, const int32_t *__restrict__ nbr, const TC *__restrict__ coef, const real *uRec,
+                      real *uRecNew, const real *u, real relax, int recordInc, int uRecIsZero)
 {
+    chain_step();
     using St = Stage<R, NV>;
     constexpr int RT = kStagedRows, G = R / RT;
     extern __shared__ real sb[]; // three stages
@@ -172,9 +174,10 @@ constexpr int kRowWarps = 4;
 
 template <int R, int NV, int NF, typename TC>
 __global__ void __launch_bounds__(32 * kRowWarps)
-    k_vr_sweep_rows(int64_t nCell, const int32_t *__restrict__ nbr, const TC *__restrict__ coef, const real *__restrict__ uRec,
-                    real *__restrict__ uRecNew, const real *__restrict__ u, real relax, int recordInc, int uRecIsZero)
+    k_vr_sweep_rows(int64_t nCell, const int32_t *__restrict__ nbr, const TC *__restrict__ coef, const real *uRec,
+                    real *uRecNew, const real *u, real relax, int recordInc, int uRecIsZero)
 {
+    chain_step();
     constexpr int CW = warp_cells<R>();
     const int lane = threadIdx.x & 31, cl = lane / R, i = lane - cl * R, lane0 = lane - i;
     const int64_t c = ((int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5)) * CW + cl;
@@ -254,12 +257,12 @@ int launch(int64_t nCell, const int32_t *nbr, const TC *coef, const real *uRec, 
                 if (dev < 64)
                     attrSet |= 1ULL << dev;
             }
-            k_vr_sweep_staged<R, NV, NF, TC><<<(unsigned)((nCell + 31) / 32), 32 * (R / kStagedRows), sh, st>>>(nCell, nbr, coef, uRec, uRecNew, u, relax,
+            launch_chained_shared(k_vr_sweep_staged<R, NV, NF, TC>, (unsigned)((nCell + 31) / 32), 32 * (R / kStagedRows), sh, st, nCell, nbr, coef, uRec, uRecNew, u, relax,
                                                                                                              recordInc, uRecIsZero);
             return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
         }
     const int64_t warps = (nCell + warp_cells<R>() - 1) / warp_cells<R>();
-    k_vr_sweep_rows<R, NV, NF, TC><<<(unsigned)((warps + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(nCell, nbr, coef, uRec, uRecNew, u, relax,
+    launch_chained(k_vr_sweep_rows<R, NV, NF, TC>, (unsigned)((warps + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, st, nCell, nbr, coef, uRec, uRecNew, u, relax,
                                                                                                             recordInc, uRecIsZero);
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
 }
