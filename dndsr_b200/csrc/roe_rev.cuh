@@ -79,9 +79,10 @@ DNDSB_D void flim_rev(real v, real lam, real lamL, real lamR, real sHY, real ob,
 // and of the Roe-average fields (rb, accumulated), recomputing the forward intermediates of
 // roe_eigen / roe_waves / roe_dissipation statement by statement
 // (l123bIn: an extra cotangent of the fixed eigenvalue l123, which the SA convective flux also uses; l123Out,
-// when given, receives l123)
+// when given, receives l123; incFOut and nb, when given, receive D incU and, added, the cotangent of the normal)
 DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, real gamma, real dLambda, real fixScale, real incFScale,
-                           const real *incFb, real *incUb, RoeBar &rb, real l123bIn = 0, real *l123Out = nullptr)
+                           const real *incFb, real *incUb, RoeBar &rb, real l123bIn = 0, real *l123Out = nullptr, real *incFOut = nullptr,
+                           real *nb = nullptr)
 {
     // forward: eigenvalues
     const real sHY = 0.05 * fixScale;
@@ -115,6 +116,13 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
     // forward: dissipation products
     real A0 = wa0 * l0, A1 = wa1 * l123, A4 = wa4 * l4;
     real t[3] = {a23T[0] * l123, a23T[1] * l123, a23T[2] * l123};
+    if (incFOut)
+    {
+        incFOut[0] = A0 + A1 + A4;
+        for (int d = 0; d < 3; d++)
+            incFOut[1 + d] = (A0 + A1 + A4) * r.v[d] + (A4 - A0) * r.a * n[d] + t[d];
+        incFOut[4] = A0 * (r.H - vN * r.a) + 0.5 * A1 * r.vsqr + A4 * (r.H + vN * r.a) + dot3(t, r.v);
+    }
     // reverse: dissipation
     const real *Fb = incFb;
     real A0b = Fb[0] + (r.H - vN * r.a) * Fb[4], A1b = Fb[0] + 0.5 * r.vsqr * Fb[4], A4b = Fb[0] + (r.H + vN * r.a) * Fb[4];
@@ -131,6 +139,8 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
         tb[d] = r.v[d] * Fb[4] + Fb[1 + d];
         rb.a += n[d] * (A4 - A0) * Fb[1 + d];
         rb.v[d] += t[d] * Fb[4] + (A0 + A4 + A1) * Fb[1 + d];
+        if (nb)
+            nb[d] += r.a * (A4 - A0) * Fb[1 + d];
     }
     real l0b = wa0 * A0b, l123b = wa1 * A1b + l123bIn, l4b = wa4 * A4b;
     real wa0b = l0 * A0b, wa1b = l123 * A1b, wa4b = l4 * A4b;
@@ -175,6 +185,8 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
         incUb[1 + d] += a23b[d] + n[d] * incU123Nb;
         incUb[0] += -r.v[d] * a23b[d];
         rb.v[d] += -incU[0] * a23b[d];
+        if (nb)
+            nb[d] += incU[1 + d] * incU123Nb + a23[d] * a23nb - a23Tb[d] * a23n;
     }
     // reverse: eigenvalues (the three limiter applications and the |.| of their inputs; at a kink
     // |x| takes the slope of x >= 0, as the forward-mode dual numbers do)
@@ -204,6 +216,41 @@ DNDSB_D void roe0_diss_rev(const real *incU, const real *n, const RoeAvg &r, rea
         rb.v[d] += n[d] * vNb;
         rb.vL[d] += n[d] * vLm0b;
         rb.vR[d] += n[d] * vRm0b;
+        if (nb)
+            nb[d] += r.v[d] * vNb + r.vL[d] * vLm0b + r.vR[d] * vRm0b;
+    }
+}
+
+// nb += the cotangent of the normal of F_phys(U, n) under y
+DNDSB_D void phys_flux_nbar(const real *U, const real *y, real gamma, real c, real *nb)
+{
+    const real i = 1.0 / U[0], p = (gamma - 1) * (U[4] - 0.5 * (U[1] * U[1] + U[2] * U[2] + U[3] * U[3]) * i);
+    const real a = (U[1] * y[1] + U[2] * y[2] + U[3] * y[3] + (U[4] + p) * y[4]) * i;
+    for (int d = 0; d < 3; d++)
+        nb[d] += c * (U[1 + d] * (y[0] + a) + p * y[1 + d]);
+}
+
+// Plain Roe at one point under the cotangent y: the flux F, the cotangents of both states and of the normal (set) and of the
+// Roe-average fields (rb, accumulated)
+DNDSB_D void roe0_face_rev(const real *UL, const real *UR, const real *n, const RoeAvg &r, real gamma, real dLambda, real fixScale, real incFScale,
+                           const real *y, real *F, real *ULb, real *URb, real *nb, RoeBar &rb)
+{
+    real incU[5], incFb[5], incUb[5], incF[5], FR[5], p, a2;
+    for (int v = 0; v < 5; v++)
+        incU[v] = UR[v] - UL[v], incFb[v] = -0.5 * y[v];
+    for (int d = 0; d < 3; d++)
+        nb[d] = 0;
+    roe0_diss_rev(incU, n, r, gamma, dLambda, fixScale, incFScale, incFb, incUb, rb, 0, nullptr, incF, nb);
+    phys_flux(UL, n, gamma, F, p, a2);
+    phys_flux(UR, n, gamma, FR, p, a2);
+    phys_flux_nbar(UL, y, gamma, 0.5, nb);
+    phys_flux_nbar(UR, y, gamma, 0.5, nb);
+    flux_jac_du_t<5>(UL, n, y, 0.0, gamma, ULb);
+    flux_jac_du_t<5>(UR, n, y, 0.0, gamma, URb);
+    for (int v = 0; v < 5; v++)
+    {
+        F[v] = 0.5 * (F[v] + FR[v]) - 0.5 * incF[v];
+        ULb[v] = 0.5 * ULb[v] - incUb[v], URb[v] = 0.5 * URb[v] + incUb[v];
     }
 }
 
