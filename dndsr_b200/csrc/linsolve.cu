@@ -326,15 +326,16 @@ DNDSB_GLOBAL void k_gmres_lsq(int k, const real *H, real *sc, int ncolMax, real 
         }
         __syncwarp();
     }
-    real rmax = lane < nv ? fabs(R[lane][lane]) : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        rmax = dmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    // the same chain in every lane: a maximum through an exchange differs between lanes where an entry is not a number,
+    // and the lanes of the substitution must take one way
+    real rmax = 0;
+    for (int jj = 0; jj < nv; jj++)
+        rmax = dmax(rmax, fabs(R[jj][jj]));
     real acc = lane < nv ? gv[lane] : 0.0, y = 0;
     for (int jj = nv - 1; jj >= 0; jj--)
     {
-        const real d = R[jj][jj];
-        const real yj = fabs(d) > 1e-14 * rmax ? __shfl_sync(0xffffffffu, acc, jj) / d : 0.0;
+        const real d = R[jj][jj], a = __shfl_sync(0xffffffffu, acc, jj);
+        const real yj = fabs(d) > 1e-14 * rmax ? a / d : 0.0;
         if (lane == jj)
             y = yj;
         if (lane < jj)
