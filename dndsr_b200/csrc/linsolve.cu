@@ -376,6 +376,26 @@ DNDSB_GLOBAL void k_copy_scalar(const real *a, real *b)
 }
 } // namespace
 
+// The end of the last solve on a workspace.  A solve on another stream waits for it before it writes the workspace.
+struct SolveEnd
+{
+    cudaEvent_t done = nullptr;
+    bool any = false;
+    unsigned long long stream = 0, capture = 0;
+    // a capture cannot outlive its streams, so that there the handle is identity enough
+    static unsigned long long id(cudaStream_t s, unsigned long long cap) { return cap ? (unsigned long long)(uintptr_t)s : stream_id(s); }
+    void order(cudaStream_t s, unsigned long long cap) const
+    {
+        if (any && capture == cap && stream != id(s, cap))
+            stream_wait(s, done);
+    }
+    void record(cudaStream_t s, unsigned long long cap)
+    {
+        event_record(done, s);
+        any = true, stream = id(s, cap), capture = cap;
+    }
+};
+
 // workspace owned by an evaluator handle
 struct LinWs
 {
@@ -393,7 +413,8 @@ struct LinWs
     real *colScale = nullptr; // [33] normalising factors of the stored (unnormalised) Krylov columns
     unsigned *cnt = nullptr;  // ticket counter of the one-launch reductions (zero between launches)
     cudaStream_t cs = nullptr;
-    cudaEvent_t evIn = nullptr, evOut = nullptr;
+    cudaEvent_t evIn = nullptr;
+    SolveEnd end[2]; // [0] outside stream captures, [1] within one: neither may wait for an event of the other
     cudaGraphExec_t graph = nullptr;
     LinSettings key{};
     bool keyValid = false;
@@ -410,7 +431,8 @@ void linws_free(LinWs *w)
     graph_free(w->graph);
     stream_free(w->cs);
     event_free(w->evIn);
-    event_free(w->evOut);
+    for (SolveEnd &e : w->end)
+        event_free(e.done);
     delete w;
 }
 
@@ -463,7 +485,8 @@ int ws_prepare(const MeshD &m, LinWs *&w, const LinSettings &ls, int nv, int jac
              dev_alloc((void **)&w->luNLow, sizeof(int32_t) * m.nCell) == cudaSuccess;
     ok = ok && dev_zero(w->V, es * krylov_ld(n) * (k + 1), nullptr) == cudaSuccess; // the column pads stay zero
     ok = ok && dev_zero(w->cnt, sizeof(unsigned), nullptr) == cudaSuccess && dev_zero(w->colScale, sizeof(real) * 33, nullptr) == cudaSuccess;
-    if (!ok || stream_create(&w->cs) != cudaSuccess || event_create(&w->evIn) != cudaSuccess || event_create(&w->evOut) != cudaSuccess)
+    if (!ok || stream_create(&w->cs) != cudaSuccess || event_create(&w->evIn) != cudaSuccess ||
+        event_create(&w->end[0].done) != cudaSuccess || event_create(&w->end[1].done) != cudaSuccess)
     {
         linws_free(w);
         w = nullptr;
@@ -705,7 +728,12 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         real dt, const real *u, const real *rhs, real *xInc, cudaStream_t st)
 {
     // A few sweeps alone go straight onto the caller's stream: replaying a graph of them and handing over between the
-    // streams costs more than their launches.  Everything else runs on the solver's stream, captured once.
+    // streams costs more than their launches.  Everything else runs on the solver's stream, captured once.  The callers'
+    // streams share the workspace, so each solve waits for the last one where that ran on another stream.
+    if (NV == 6 && !ev.jSource)
+        return ST_BADARG;
+    if (w.jacMode == 2 && (!ev.lambdaFace0 || (m.nBndFace > 0 && !bnd.type)))
+        return ST_BADARG;
     const bool direct = ls.gmresCode == 0 && (int64_t)(1 + ls.sgsIter) * 2 * m.nColor * (ls.jacobiCode == 2 ? 2 : 1) <= kDirectLaunches;
     cudaStream_t cs = direct ? st : w.cs;
     if (!direct)
@@ -713,18 +741,17 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         event_record(w.evIn, st);
         stream_wait(cs, w.evIn);
     }
+    const unsigned long long cap = capture_id(cs);
+    SolveEnd &end = w.end[cap != 0];
+    end.order(cs, cap);
     if (ls.gmresCode != 0)
         h2d(w.s2, ls.scale2, sizeof(real) * 8, cs);
     auto kbuild = posop::k_build<T, NV, NF>;
     auto kgather = k_gather_T<T, NV>;
     auto kscatter = k_scatter_T<T, NV>;
-    if (NV == 6 && !ev.jSource)
-        return ST_BADARG;
     Solve<T, NV, NF> S{m, w, ls, (T)ev.s.gamma, cs};
     if (w.jacMode)
     {
-        if (w.jacMode == 2 && (!ev.lambdaFace0 || (m.nBndFace > 0 && !bnd.type)))
-            return ST_BADARG;
         auto kb = k_sgsop_build_blk<T, NV, NF>;
         DNDSB_LAUNCH(kb, m.nCell, 128, cs, m, g, bnd, ev, (int)(w.jacMode == 2), dTau, dt, alphaDiag, u, w.cellPos, w.nbrPos, (T *)w.opB,
                      (T *)w.jdB, ev.errWord);
@@ -743,6 +770,7 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
     else
         DNDSB_CHAIN(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
     DNDSB_CHAIN(kgather, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, rhs, (T *)w.rhsT);
+    bool launched = true;
     if (direct)
         S.body();
     else if (ls.useGraph)
@@ -763,8 +791,7 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         if (w.graph)
         {
             w.key = ls, w.keyValid = true;
-            if (graph_launch(w.graph, cs) != cudaSuccess)
-                return ST_CUDA;
+            launched = graph_launch(w.graph, cs) == cudaSuccess;
         }
         else
             S.body();
@@ -775,12 +802,10 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         S.body();
     }
     DNDSB_CHAIN(kscatter, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, (const T *)w.x, xInc);
+    end.record(cs, cap);
     if (!direct)
-    {
-        event_record(w.evOut, cs);
-        stream_wait(st, w.evOut);
-    }
-    return last_error() == cudaSuccess ? ST_OK : ST_CUDA;
+        stream_wait(st, end.done);
+    return last_error() == cudaSuccess && launched ? ST_OK : ST_CUDA;
 }
 
 template <typename T, int NV>

@@ -63,6 +63,19 @@ inline void event_free(cudaEvent_t e)
 }
 inline cudaError_t event_record(cudaEvent_t e, cudaStream_t s) { return cudaEventRecord(e, s); }
 inline cudaError_t stream_wait(cudaStream_t s, cudaEvent_t e) { return cudaStreamWaitEvent(s, e, 0); }
+// the identity of a stream, unique in the process (its handle is reused; asking for it ends a capture), and of the capture it is in (0: none)
+inline unsigned long long stream_id(cudaStream_t s)
+{
+    unsigned long long id = 0;
+    cudaStreamGetId(s, &id);
+    return id;
+}
+inline unsigned long long capture_id(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    return cudaStreamGetCaptureInfo(s, &st, &id) == cudaSuccess && st == cudaStreamCaptureStatusActive ? id + 1 : 0;
+}
 inline cudaError_t graph_begin(cudaStream_t s) { return cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal); }
 inline cudaError_t graph_end(cudaStream_t s, cudaGraphExec_t *exec)
 {

@@ -6,6 +6,26 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+def _box(n=7):
+    """n^2 quadrilaterals, 5 n^2 unknowns: with n odd a vector ends within a group of four."""
+    from dndsr_b200 import mesh as M
+    from dndsr_b200.solver import EulerEvaluator, VariationalReconstruction
+    from tests.util import VR_HQM_PY
+    vr = VariationalReconstruction(M.periodic_quad_2d(n, jitter=0.1), dict(VR_HQM_PY, maxOrder=1)).construct()
+    ev = EulerEvaluator(vr, dict(nVars=5, riemannSolverType="Roe", muGas=0.0, ignoreVis=True))
+    u = vr.BuildUDof(5)
+    ev.InitializeUDOF(u, 2)
+    dTau = torch.zeros(vr.mesh.n_cell, dtype=torch.float64, device="cuda")
+    ev.EvaluateDt(dTau, u, 5.0)
+    return ev, u, dTau, torch.tensor(np.random.default_rng(5).normal(size=(vr.mesh.n_cell, 5)), device="cuda")
+
+
+def _solve(ev, u, dTau, rhs, **kw):
+    x = torch.zeros_like(rhs)
+    ev.SolveLinear(0.5, dTau, 0.1, u, rhs, x, **kw)
+    return x
+
+
 def _least_squares(H, beta, k):
     """min |beta e1 - H y| by Givens rotations in the order of the device's chain; H[j] is column j."""
     dmax = lambda a, b: a if a > b else b  # noqa: E731  the device's maximum, which is not symmetric in a NaN
@@ -61,3 +81,56 @@ def test_least_squares_with_an_infinite_entry(k, at):
     got = gsc[8:8 + k].cpu().numpy()
     # a chain of k rotations and substitutions of a matrix of condition below 1e3
     assert np.allclose(got, y, rtol=1e-10, atol=1e-12, equal_nan=True), (got, y)
+
+
+DIRECT, SWEEPS, GMRES = dict(gmresCode=0), dict(gmresCode=0, sgsIter=8), dict(gmresCode=1, nGmresSpace=6)
+
+
+@pytest.mark.parametrize("first,second", [(DIRECT, DIRECT), (DIRECT, GMRES), (GMRES, DIRECT), (DIRECT, SWEEPS), (GMRES, GMRES)])
+def test_solves_on_two_streams_follow_each_other(first, second):
+    """Two callers' streams, one workspace: the second solve waits until the first is done (held back here by other work
+    on its stream), and both give what they give in turn."""
+    ev, u, dTau, rhs = _box(41)
+    rhs2 = torch.flip(rhs, [0]) * 2
+    want = [_solve(ev, u, dTau, r, **k).clone() for r, k in ((rhs, first), (rhs2, second))]
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    big = torch.ones((4096, 4096), device="cuda")
+    x1, x2, held = torch.zeros_like(rhs), torch.zeros_like(rhs), torch.empty_like(big)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        done1 = torch.cuda.Event()
+        x1.zero_(), x2.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s1):
+            for _ in range(20):
+                torch.mm(big, big, out=held)
+            ev.SolveLinear(0.5, dTau, 0.1, u, rhs, x1, **first)
+            done1.record()
+        with torch.cuda.stream(s2):
+            ev.SolveLinear(0.5, dTau, 0.1, u, rhs2, x2, **second)
+        s2.synchronize()
+        assert done1.query()
+        torch.cuda.synchronize()
+        assert torch.equal(x1, want[0]) and torch.equal(x2, want[1])
+
+
+def test_solve_on_two_streams_of_a_capture():
+    """The same order inside a captured graph; solves before and after it, and its replay, give the same."""
+    ev, u, dTau, rhs = _box(41)
+    want = _solve(ev, u, dTau, rhs).clone()
+    x1, x2 = torch.zeros_like(rhs), torch.zeros_like(rhs)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        side.wait_stream(torch.cuda.current_stream())
+        ev.SolveLinear(0.5, dTau, 0.1, u, rhs, x1)
+        with torch.cuda.stream(side):
+            ev.SolveLinear(0.5, dTau, 0.1, u, rhs, x2)
+        torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(_solve(ev, u, dTau, rhs), want)  # outside the capture again
+    torch.cuda.synchronize()
+    for _ in range(2):
+        x1.zero_(), x2.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(x1, want) and torch.equal(x2, want)
