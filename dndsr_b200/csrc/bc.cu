@@ -21,6 +21,13 @@ namespace
 // 74 -> 24 us (VR term) and 102 -> 12 us (RHS) for the 5,180 faces of a 36k-tet bump at degree 2 (7 points), 31 -> 21
 // and 33 -> 22 us for the 19,040 faces of a 250k-tet one at degree 1 (3 points).
 inline int bc_rows(int nGf) { return nGf < 64 ? 64 / nGf : 1; }
+// the same where a row takes `bytes` of dynamic shared memory: as many as the 48 KB that a launch has without asking hold
+// (at degree 3 with one point per face 51 of the 64 rows)
+inline int bc_rows(int nGf, size_t bytes)
+{
+    const int fit = (int)(48 * 1024 / bytes), rows = bc_rows(nGf);
+    return rows < fit ? rows : fit;
+}
 
 // VariationalReconstruction_Reconstruction.hxx:19-176 GetBoundaryRHS with the Euler FBoundary of
 // EulerSolver.hxx:163-175, applied as in :568-586:
@@ -331,9 +338,10 @@ void launch_vr_bc(const MeshD &m, const GeomD &g, const VRD &vr, const real *uRe
                   cudaStream_t st)
 {
     constexpr int R = ndof_of<DIM>(P) - 1;
-    const int rows = bc_rows(g.nGf);
+    const size_t rowBytes = sizeof(real) * (g.nGf * (R + NV) + R * NV);
+    const int rows = bc_rows(g.nGf, rowBytes);
     const unsigned nb = (unsigned)((m.nBndCell + rows - 1) / rows);
-    const size_t sh = sizeof(real) * rows * (g.nGf * (R + NV) + R * NV);
+    const size_t sh = rows * rowBytes;
     if (useFP32)
         k_vr_bc<DIM, P, NV, float><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, vr.AAInvB32, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
     else

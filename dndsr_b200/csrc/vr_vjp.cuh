@@ -205,8 +205,10 @@ void launch_vr_vjp(const MeshD &m, const GeomD &g, const VRD &vr, const real *v,
     k_vr_vjp_rows<R, NV><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(m, vr, v, vRec, vU);
     if (m.nBndCell > 0 && vr.bnd.nZone > 0)
     {
-        const int rows = g.nGf < 32 ? 32 / g.nGf : 1;
-        const size_t sh = sizeof(real) * rows * (2 * R * NV + NV + g.nGf * (R + 2 * NV));
+        // about 32 threads, and no more rows than the 48 KB of shared memory that a launch has without asking hold
+        const size_t rowBytes = sizeof(real) * (2 * R * NV + NV + g.nGf * (R + 2 * NV));
+        const int want = g.nGf < 32 ? 32 / g.nGf : 1, fit = (int)(48 * 1024 / rowBytes), rows = want < fit ? want : fit;
+        const size_t sh = rows * rowBytes;
         k_vr_vjp_bnd<DIM, P, NV><<<(unsigned)((m.nBndCell + rows - 1) / rows), rows * g.nGf, sh, st>>>(m, g, vr, v, uRec, u, vRec, vU);
     }
 }

@@ -6,7 +6,7 @@ import torch
 
 from dndsr_b200 import mesh as M
 from tests.bump_case import bump_bc, bump_oracle, perturbed_state
-from tests.util import VR_HQM_PY, relerr
+from tests.util import VR_HQM, VR_HQM_PY, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,41 @@ def test_points_per_face_against_the_oracle(p, intOrder):
     o.eval_dt(u0, 5.0)
     ev.EvaluateRHS(rhs, u, rec)
     assert relerr(rhs.cpu().numpy(), o.eval_rhs(u0, rec0)) < 1e-12
+
+
+@pytest.mark.parametrize("mk,nv,intOrder", [("tet", 5, 1), ("tet", 5, 0), ("hex", 5, 1), ("hex", 6, 1)])
+def test_one_point_per_face_at_degree_3(mk, nv, intOrder):
+    """The longest rows of the boundary reconstruction, R = 19, with the most rows to a block: VR boundary term against the
+    oracle, and its transpose against the tangent."""
+    import oracle
+    from dndsr_b200.solver import EulerEvaluator, VariationalReconstruction
+    from tests.plate_case import plate_oracle, plate_perturbed
+    if mk == "tet":
+        m = M.renumber_by_color(M.bump_channel_tet(3, 2, 2))  # 64 boundary faces
+        o, far, types, vals, w = bump_oracle(m, 3, "Roe", 0.0, 1, intOrder=intOrder)
+        u0, rec0 = perturbed_state(m, far, R=o.R)
+    else:
+        m = M.renumber_by_color(M.flat_plate_hex(8, 6, 3, y1=1e-2, growth=1.3))
+        o, far, mu, types, vals, w = plate_oracle(m, 3, "Roe", intOrder)
+        u0, rec0 = plate_perturbed(m, far, R=o.R)
+        if nv == 5:
+            far, vals, u0, rec0 = far[:5], vals[:, :5].copy(), u0[:, :5].copy(), rec0[:, :, :5].copy()
+            o = oracle.Oracle(m, dict(VR_HQM, maxOrder=3, intOrder=intOrder), dict(nVars=5, rsType=oracle.RS["Roe"], rsFixScale=1.0, rsIncFScale=1.0,
+                              gamma=1.4, Rgas=1.0, muGas=0.0, prGas=0.72, TRef=273.15, CSutherland=110.4, muModel=0, ignoreVis=1))
+            assert o.construct(w) == 0
+            o.set_bc(types, vals)
+    vr = VariationalReconstruction(m, dict(VR_HQM_PY, maxOrder=3, intOrder=intOrder)).construct(w)
+    EulerEvaluator(vr, dict(nVars=nv, riemannSolverType="Roe", muGas=1e-3)).SetBC(types, vals)  # the sweep's boundary table too
+    u, rec = torch.tensor(u0, device="cuda"), torch.tensor(rec0, device="cuda")
+    new = torch.zeros_like(rec)
+    vr.DoReconstructionIter(rec, new, u, putIntoNew=True)
+    # both sides invert A in FP64: its condition number times a few roundings
+    tol = 8 * np.finfo(float).eps * np.linalg.cond(o.get("matrixA").reshape(m.n_cell, o.R, o.R)).max()
+    assert relerr(new.cpu().numpy(), o.vr_iter(rec0, u0)) < max(tol, 1e-12)
+    if nv == 5:
+        g = torch.Generator("cuda").manual_seed(1)
+        cot, dRec, du = (torch.randn(t.shape, generator=g, dtype=torch.float64, device="cuda") for t in (rec, rec, u))
+        vRec, vU = vr.DoReconstructionIterVJP(cot, rec, u)
+        lhs = float((cot * vr.DoReconstructionIterJVP(dRec, du, rec, u)).sum())
+        terms = torch.cat([(vRec * dRec).flatten(), (vU * du).flatten()])
+        assert abs(lhs - float(terms.sum())) < 1e-12 * float(terms.abs().sum())
