@@ -797,10 +797,7 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
             S.body();
     }
     else
-    {
-        w.key = ls, w.keyValid = true;
-        S.body();
-    }
+        S.body(); // the recorded sequence and its key stay as they are
     DNDSB_CHAIN(kscatter, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, (const T *)w.x, xInc);
     end.record(cs, cap);
     if (!direct)

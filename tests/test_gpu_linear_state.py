@@ -134,3 +134,17 @@ def test_solve_on_two_streams_of_a_capture():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(x1, want) and torch.equal(x2, want)
+
+
+@pytest.mark.parametrize("other", [dict(nGmresSpace=5), dict(nGmresSpace=10, sgsIter=1), dict(nGmresSpace=10, nGmresIter=2),
+                                   dict(nGmresSpace=10, jacobiCode=0), dict(nGmresSpace=10, gmresCode=2)])
+def test_recorded_sequence_is_of_its_settings(other):
+    """A solve that records nothing between two that do: the third replays the second's settings, not the first's."""
+    ev, u, dTau, rhs = _box()
+    first, other = dict(gmresCode=1, nGmresSpace=10), dict(dict(gmresCode=1), **other)
+    a = _solve(ev, u, dTau, rhs, useGraph=True, **first)
+    b = _solve(ev, u, dTau, rhs, useGraph=False, **other)
+    c = _solve(ev, u, dTau, rhs, useGraph=True, **other)
+    assert not torch.equal(a, b)
+    assert torch.equal(b, c)
+    assert torch.equal(a, _solve(ev, u, dTau, rhs, useGraph=True, **first))
