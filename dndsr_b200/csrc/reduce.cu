@@ -385,6 +385,12 @@ DNDSB_GLOBAL void __launch_bounds__(kRedBlock, 4) k_kmaxpy_norm(int64_t n, int64
             for (int e = 0; e < 4; e++)
                 x[e] -= hc * v[e];
         }
+        if (4 * q + 4 > n) // the pad stays zero also where a factor is not finite: later solves read it
+        {
+#pragma unroll
+            for (int e = 1; e < 4; e++)
+                x[e] = 4 * q + e < n ? x[e] : 0.0;
+        }
         real xr[4];
         Quad<T>::store(w + 4 * q, x, xr);
 #pragma unroll

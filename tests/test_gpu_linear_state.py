@@ -148,3 +148,20 @@ def test_recorded_sequence_is_of_its_settings(other):
     assert not torch.equal(a, b)
     assert torch.equal(b, c)
     assert torch.equal(a, _solve(ev, u, dTau, rhs, useGraph=True, **first))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("gmresCode", [1, 2])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_solve_after_a_nonfinite_one(bad, gmresCode, precision):
+    """Nothing of a solve that is not finite stays in the workspace, the Krylov columns' ends included."""
+    kw = dict(gmresCode=gmresCode, nGmresSpace=6, precision=precision)
+    ev, u, dTau, rhs = _box()
+    poisoned = rhs.clone()
+    poisoned[3, 1] = bad
+    _solve(ev, u, dTau, poisoned, **kw)
+    x = _solve(ev, u, dTau, rhs, **kw)
+    fresh = _box()[0]
+    fresh.EvaluateDt(torch.zeros_like(dTau), u, 5.0)
+    assert bool(torch.isfinite(x).all()) and float(x.abs().max()) > 0
+    assert torch.equal(x, _solve(fresh, u, dTau, rhs, **kw))
