@@ -6,7 +6,7 @@
 
 namespace dndsb
 {
-extern template void coords_vjp_launch<2>(const MeshD &, const GeomD &, const VRD &, const EulerSettingsD &, const real *, const real *,
+extern template int coords_vjp_launch<2>(const MeshD &, const GeomD &, const VRD &, const EulerSettingsD &, const real *, const real *,
                                           const real *, const real *, const real *, const CoordAdjWs &, int *, cudaStream_t);
 extern template void pressure_force_coords_launch<2>(const MeshD &, const GeomD &, const VRD &, real, int, const real *, const real *,
                                                      const real *, const CoordAdjWs &, cudaStream_t);
@@ -146,10 +146,10 @@ int coords_vjp(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSetting
     coords_lanes_build(m, g, vr, ws, st);
     const EulerSettingsD es = s ? *s : EulerSettingsD();
     dev_zero(errWord, sizeof(int), st);
-    if (m.dim == 2)
-        coords_vjp_launch<2>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, errWord, st);
-    else
-        coords_vjp_launch<3>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, errWord, st);
+    rc = m.dim == 2 ? coords_vjp_launch<2>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, errWord, st)
+                    : coords_vjp_launch<3>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, errWord, st);
+    if (rc != ST_OK)
+        return rc;
     DNDSB_LAUNCH(k_node_gather, m.nNode, 256, st, m.nNode, ws.start, ws.ent, ws.share, dX);
     return geo_status(st, errWord);
 }

@@ -1014,15 +1014,17 @@ void pressure_force_coords_launch(const MeshD &m, const GeomD &g, const VRD &vr,
 
 // launches for one dimension; P = 1, 2 (and 3 in 2-D)
 template <int DIM, int P>
-void coords_vjp_launch_p(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
-                         const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
+[[nodiscard]] int coords_vjp_launch_p(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
+                                      const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
 {
     constexpr int R = ndof_of<DIM>(P) - 1;
     real *lam = nullptr, *S = nullptr;
     if (cot)
     {
         lam = ws.share + 3 * m.nFace * ws.maxSlot, S = lam + m.nCell * R * 5; // see face_patches
-        vr_iter(m, g, vr, 5, uRec, S, u, 1, 0, 0, st);
+        const int rc = vr_iter(m, g, vr, 5, uRec, S, u, 1, 0, 0, st);
+        if (rc != ST_OK)
+            return rc;
         DNDSB_LAUNCH(k_coords_prep<R>, m.nCell * R * 5, 256, st, m.nCell, m.nf, vr.AAInvB, cot, uRec, vr.s.jacobiRelax, lam, S);
     }
     auto kf = !w || es.rsType == RS_Roe ? k_coords_vjp_face<DIM, P, false, true> : k_coords_vjp_face<DIM, P, false, false>;
@@ -1030,19 +1032,19 @@ void coords_vjp_launch_p(const MeshD &m, const GeomD &g, const VRD &vr, const Eu
     DNDSB_LAUNCH(kf, m.nFace * ws.maxSlot, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, lam, S, ws.patch, ws.maxSlot, ws.share, err, ws.lanes);
     DNDSB_LAUNCH(kb, m.nBndFace * ws.maxSlot, kGeoBlock, st, m, g, vr, es, dLamCell, u, uRec, w, lam, S, ws.patch, ws.maxSlot, ws.share, err,
                  ws.lanes);
+    return ST_OK;
 }
 
 template <int DIM>
-void coords_vjp_launch(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
-                       const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
+[[nodiscard]] int coords_vjp_launch(const MeshD &m, const GeomD &g, const VRD &vr, const EulerSettingsD &es, const real *dLamCell, const real *u,
+                                    const real *uRec, const real *w, const real *cot, const CoordAdjWs &ws, int *err, cudaStream_t st)
 {
     constexpr int PTop = DIM == 2 ? 3 : 2;
     if (vr.P == 1)
-        coords_vjp_launch_p<DIM, 1>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
-    else if (vr.P == 2)
-        coords_vjp_launch_p<DIM, 2>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
-    else
-        coords_vjp_launch_p<DIM, PTop>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
+        return coords_vjp_launch_p<DIM, 1>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
+    if (vr.P == 2)
+        return coords_vjp_launch_p<DIM, 2>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
+    return coords_vjp_launch_p<DIM, PTop>(m, g, vr, es, dLamCell, u, uRec, w, cot, ws, err, st);
 }
 
 template <int DIM>

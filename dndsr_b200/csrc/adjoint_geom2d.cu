@@ -5,7 +5,7 @@
 
 namespace dndsb
 {
-template void coords_vjp_launch<2>(const MeshD &, const GeomD &, const VRD &, const EulerSettingsD &, const real *, const real *, const real *,
+template int coords_vjp_launch<2>(const MeshD &, const GeomD &, const VRD &, const EulerSettingsD &, const real *, const real *, const real *,
                                    const real *, const real *, const CoordAdjWs &, int *, cudaStream_t);
 template void pressure_force_coords_launch<2>(const MeshD &, const GeomD &, const VRD &, real, int, const real *, const real *, const real *,
                                               const CoordAdjWs &, cudaStream_t);

@@ -178,8 +178,8 @@ int vr_construct_base_and_weight(const MeshD &m, const GeomD &g, VRD &vr, const 
 int vr_construct_rec_coeff(const MeshD &m, const GeomD &g, VRD &vr, int *errWord, cudaStream_t st);
 
 // ---- hot path (hotpath.cu) ----
-int vr_iter(const MeshD &m, const GeomD &g, const VRD &vr, int nv, const real *uRec, real *uRecNew, const real *u, int recordInc,
-            int uRecIsZero, int useFP32, cudaStream_t st);
+[[nodiscard]] int vr_iter(const MeshD &m, const GeomD &g, const VRD &vr, int nv, const real *uRec, real *uRecNew, const real *u, int recordInc,
+                          int uRecIsZero, int useFP32, cudaStream_t st);
 int eval_dt(const MeshD &m, const GeomD &g, EvalD &ev, const real *u, real CFL, real MaxDt, int useLocalDt, real *dt, real *dtMin,
             cudaStream_t st);
 int eval_rhs(const MeshD &m, const GeomD &g, const VRD &vr, EvalD &ev, const real *u, const real *uRec, real *rhs, real *faceFlux,
