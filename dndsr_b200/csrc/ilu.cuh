@@ -249,10 +249,15 @@ DNDSB_D bool tile_inv(const real *row, real (*sD)[32], real (*sU)[32], real *inv
 // position): slot j < cnlow[r] holds the j-th lower neighbour in ascending rank, the upper neighbours follow, cnbr
 // [r][NF] their rows (-1 after the last), so the triangular solves read a row's lower (or upper) blocks from consecutive
 // slots.  Row i of L_j, of the diagonal and of the upper blocks depends on row i of the operator's blocks alone, so warp
-// i takes it; the neighbours' factors and the pivot rows go through shared memory.  The sums run in factor_row's order.  One thread per row held its blocks in local memory: 121 us per colour of
-// 249,600 tets in FP64, now 93.
+// i takes it; the neighbours' factors and the pivot rows go through shared memory.  The sums run in factor_row's order.
+// One thread per row held its blocks in local memory: 121 us per colour of 249,600 tets in FP64, now 93.
+// Bound by the gathers of the neighbours' blocks, so three blocks per SM (136 registers a thread with 5 variables, 113
+// with 6) instead of the one or two that the free choice of registers leaves.  Per solve, three blocks against free
+// choice: 249,600 tets 366 and 474 us in FP64, 349 and 460 in FP32; 110,592 hexahedra 223 and 516, 204 and 506; 131,072
+// triangles 132 and 170, 111 and 146; 65,536 quadrilaterals 91 and 112, 81 and 100; 6 variables on 72,000 hexahedra 231
+// and 404, 215 and 383.
 template <typename T, int NV, int NF>
-DNDSB_GLOBAL void __launch_bounds__(32 * NV, NV == 5 && NF == 4 ? 3 : 1) k_ilu_factor_c(int64_t beg, int64_t end, const int32_t *__restrict__ nbr, const T *__restrict__ A,
+DNDSB_GLOBAL void __launch_bounds__(32 * NV, 3) k_ilu_factor_c(int64_t beg, int64_t end, const int32_t *__restrict__ nbr, const T *__restrict__ A,
                                                            const T *__restrict__ D, BlockLay offL, BlockLay dL, BlockLay DL, T *off, T *dinv,
                                                            int *err, int32_t *cnbr, int32_t *cnlow)
 {
