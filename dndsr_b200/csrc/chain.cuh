@@ -7,9 +7,12 @@
 //
 // A kernel launched by launch_chained may start early; it must call chain_wait before it reads what an earlier kernel of
 // the sequence wrote, or writes what one may still read (the wait ends when all earlier kernels have completed and their
-// writes are visible), and chain_release after it, which lets the next one start in turn.  What was written before the
-// sequence began (the operator) may be read ahead of the wait.  Arrays that a sequence writes are not __restrict__
-// parameters, so that the compiler moves no load of them ahead of the wait.
+// writes are visible), and chain_release after it, which lets the next one start in turn.  Ahead of its wait a kernel may
+// read what was written before the sequence began, and what a kernel of the sequence wrote if another one stands between
+// the two: that one releases its successor only after its own wait, so the writer has completed by then.  The solve's
+// sweeps read the operator that way; its builder is part of the sequence, and the gather of the right-hand side stands
+// between them.  A reader that follows its writer directly has to wait first, or be launched unchained.  Arrays that a
+// sequence writes are not __restrict__ parameters, so that the compiler moves no load of them ahead of the wait.
 #pragma once
 #include "platform.cuh"
 #include <utility>

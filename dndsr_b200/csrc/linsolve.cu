@@ -721,6 +721,13 @@ struct Solve
     bool split() const { return w.jacMode == 0; } // vectors laid out as in vec_split.cuh
 };
 
+// Most launches of a solve of sweeps alone that go straight onto the caller's stream.  Handing over to the solver's stream
+// and back costs 7 to 12 us a solve, a launch by the host up to 0.6 us more than one of the recorded sequence where the
+// kernels are short.  Direct against handed over, us a solve in a row: 8,192 triangles 4 launches 17.3 and 18.9, 8 26.8 and
+// 25.9, 20 53.6 and 45.3; 36,162 tets 8 27.2 and 32.2, 24 64.7 and 65.4, 40 101 and 99; 249,600 tets 24 164 and 175, 120
+// 677 and 703; 262,144 hexahedra 20 262 and 266, 60 714 and 711.  With the host waiting for each, as the drivers do, the
+// triangles take 24.8 and 30.4 at 4 launches, 49.7 and 50.7 at 16, 58.2 and 54.7 at 20.  The line lies where meshes of some
+// ten thousand cells cross; smaller ones lose up to 8 us between 8 and 24 launches, larger ones would gain beyond it.
 constexpr int kDirectLaunches = 24;
 
 template <typename T, int NV, int NF>
@@ -769,6 +776,7 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
     }
     else
         DNDSB_CHAIN(kbuild, m.nCell, 128, cs, m, g, ev.lambdaFace, dTau, dt, alphaDiag, ev.s.gamma, u, ev.jSource, w.cellPos, S.A());
+    // also what lets the first sweep read the operator ahead of its wait (chain.cuh): it stays between builder and sweep
     DNDSB_CHAIN(kgather, m.nCell, 256, cs, m.nCell, S.split(), m.colorCells, rhs, (T *)w.rhsT);
     bool launched = true;
     if (direct)

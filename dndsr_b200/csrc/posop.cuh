@@ -55,6 +55,8 @@ struct Op
     T *nu = nullptr;          // [n] U5 / rho (6 variables)
 };
 
+// Releases its successor on entry, so the next kernel of the sequence may not read the operator ahead of its wait; the
+// sweeps and products do, and another kernel that waits (k_gather_T of linsolve.cu) has to stand before the first of them.
 template <typename T, int NV, int NF>
 DNDSB_GLOBAL void k_build(MeshD m, GeomD g, const real *lamFace, const real *dTau, real dt, real alphaDiag, real gamma, const real *u,
                           const real *jSource, const int32_t *__restrict__ cellPos, Op<T> A)
