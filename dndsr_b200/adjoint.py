@@ -43,7 +43,7 @@ def gmres(op, prec, b, restart=30, max_restarts=100, rtol=1e-10, check_every=5, 
 
     The Arnoldi process runs on the device through the library's Krylov primitives (classical Gram-Schmidt
     with the deterministic one-launch reductions of the native linear solver, least squares by Givens
-    rotations in a one-thread kernel), the preconditioned columns z_j are kept (so the preconditioner may vary,
+    rotations in a one-warp kernel), the preconditioned columns z_j are kept (so the preconditioner may vary,
     e.g. FP32 sweeps), and the host reads the least-squares residual only every ``check_every`` Arnoldi steps
     and at each restart.  Returns x and the relative residual norms (the least-squares estimate after every
     Arnoldi step, the true residual at every restart); ``info`` (a dict) receives the number of Arnoldi

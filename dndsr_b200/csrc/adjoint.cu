@@ -2,11 +2,14 @@
 // Jacobian-vector products (forward mode) of EvaluateRHS and of one VR Jacobi
 // sweep, with respect to the cell means u and the reconstruction uRec.
 //
-// Pointwise derivatives of the Riemann flux and of the boundary ghost states
-// come from the templated gas routines instantiated on dual numbers (two
-// 10-wide passes per Gauss point: the point states, then the cell means that
-// feed the Roe averages); the Gauss-point states are recomputed, not stored.
-// The mesh-level reverse sweep is explicit: per-face cotangents are written to
+// Interior faces of the Roe family and HLLE+ are reversed by hand (adjoint_roe.cu,
+// adjoint_fast.cuh); the other fluxes come from the templated gas routines
+// instantiated on dual numbers (two 10-wide passes per Gauss point: the point
+// states, then the cell means that feed the Roe averages).  Boundary faces: the
+// ghost states in dual numbers, and the flux by hand for plain Roe and HLLE+
+// (k_rhs_vjp_bnd_rev), in dual numbers otherwise (k_rhs_vjp_bnd, five seeds for
+// the point state and five for the cell mean).  The Gauss-point states are
+// recomputed, not stored.  The mesh-level reverse sweep is explicit: per-face cotangents are written to
 // a scratch array and gathered per cell in a fixed order (no atomics on data),
 // and the transposed VR sweep gathers A^-1 B blocks of the neighbours through
 // the face-slot map.  The entropy-fix scale deltaLambdaCell is held fixed.

@@ -1,5 +1,5 @@
 #pragma once
-// Kernels of the forward-mode derivatives for the SA model and viscous boundary zones, included by the
+// Derivative kernels for the SA model and viscous boundary zones, included by the
 // instantiation units adjoint_generic_p{1,2}n{5,6}.cu (one VR degree and variable count each, compiled
 // in parallel); the entry points are in adjoint_generic.cu.
 //
@@ -8,17 +8,18 @@
 // diffusion fluxes, the eddy viscosity in the viscous flux, the source term) and boundary zones with
 // a viscous flux (no-slip and isothermal walls, inflow, pressure outflow), for 5 or 6 variables.
 //
-// Forward mode throughout.  Per face Gauss point the integrand of EvaluateRHS (EvaluateRHS.hxx:224-525:
-// F(UL, UR; ULm, URm) minus the viscous flux of the compact gradient) is evaluated in dual numbers
-// with 2 NV seeds per pass: the two point states, the two cell means, then the two point gradients
-// along each axis; on a boundary face the ghost states are formed inside the pass (the point state
-// and the cell mean are seeded together).  The pass results are contracted with the face cotangent
-// and carried through the reconstruction basis to (u, uRec) of both cells; the per-face cotangents
-// are gathered per cell in a fixed order, as in the specialised kernels.  The SA source is
-// differentiated per cell Gauss point in four passes (the point state, then the gradient along each
-// axis).  The JVPs are the same computations with one seed.  The entropy-fix scale deltaLambdaCell
-// is held fixed.  One Jacobi sweep of the reconstruction and its boundary term are differentiated as
-// in adjoint.cu, for NV variables.
+// Faces in forward mode.  Per face Gauss point the integrand of EvaluateRHS (EvaluateRHS.hxx:224-525:
+// F(UL, UR; ULm, URm) minus the viscous flux of the compact gradient) is evaluated in dual numbers.
+// Interior faces, where no reverse kernel covers them (k_rhs_vjp_face_g): 2 NV seeds per pass, the two
+// point states, the two cell means, then the two point gradients along each axis.  Boundary faces
+// (k_rhs_vjp_bnd_g): NV seeds per pass, the point state, the cell mean, then the gradient along each
+// axis, the passes side by side in the warps of a block and the ghost states formed inside them.  The
+// pass results are contracted with the face cotangent and carried through the reconstruction basis to
+// (u, uRec) of the cells; the per-face cotangents are gathered per cell in a fixed order, as in the
+// specialised kernels.  The SA source is reversed by hand around one evaluation of its core in dual
+// numbers with six seeds (sa_source_rev).  The JVPs evaluate with one seed.  The entropy-fix scale
+// deltaLambdaCell is held fixed.  One Jacobi sweep of the reconstruction and its boundary term: the
+// transpose in vr_vjp.cuh, the tangent here, for NV variables.
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "bc.cuh"

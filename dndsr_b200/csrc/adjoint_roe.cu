@@ -16,8 +16,8 @@
 //     Dual<10> per Gauss point.
 // HLLEPFlux_IdealGas (Gas.hpp:601-714) mixes the point states into its wave-speed bounds, so it is
 // reversed as a whole (hllep_rev), with the same reverse of the averages.
-// This replaces two 10-wide forward passes through the whole flux.  Boundary faces keep the
-// generic derivative kernel (ghost states).
+// This replaces two 10-wide forward passes through the whole flux.  Boundary faces are in adjoint.cu (plain
+// Roe and HLLE+ by the same reverse, the ghost states in dual numbers; the other fluxes in dual numbers).
 #include "solver.cuh"
 #include "basis_eval.cuh"
 #include "flux_t.cuh"

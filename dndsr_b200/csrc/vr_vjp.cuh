@@ -35,7 +35,7 @@ DNDSB_GLOBAL void k_adj_gather(int64_t nCell, int nf, const int32_t *__restrict_
 // R neighbouring lanes per cell, lane r on row r of vRec: it reads column r of the neighbour's block (the lanes of a cell
 // read along its rows), row r of the neighbour's cotangent, and takes the other rows from its neighbours by shuffles.
 // A thread per cell read whole blocks and rows in strides and carried the boundary cells' ghost derivatives: 156 us for
-// 249,600 tets at R = 3 and 697 us at R = 9, now 63 and 340 with the boundary kernel.
+// 249,600 tets at R = 3 and 697 us at R = 9, now 75 and 367, and 31 and 70 in the boundary kernel.
 template <int R, int NV>
 DNDSB_GLOBAL void __launch_bounds__(128) k_vr_vjp_rows(MeshD m, VRD vr, const real *__restrict__ v, real *__restrict__ vRec, real *__restrict__ vU)
 {
