@@ -40,11 +40,11 @@ B_RHS = 8 * ((9 + 2) * 5 + (2 * 3 + 1 + 9) + 3 * (9 * (2 * 3 + 1) + 1))
 B_VR = 8 * (6 * 81 + 6 * 9) + 8 * (2 * 9 * 5 + 5)
 FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes per cell of one k_rhs_face_fast launch (the face kernel: 97% of EvaluateRHS; the per-cell
-# gather adds ~4% more bytes), from the ncu capture of the same workload at 48^3 (dram__bytes_read.sum +
-# dram__bytes_write.sum = 273.1 MB for 110,592 cells); traffic grows in proportion to cells and faces, so
-# a 64^3 launch is scaled by the cell count
-RHS_TRAFFIC_PER_CELL = 273.1e6 / 48 ** 3
-RHS_FP64_PIPE_PCT = 30.5  # sm__pipe_fp64_cycles_active of the same capture
+# gather adds ~4% more bytes), from the ncu capture of this workload at 64^3 (dram__bytes_read.sum +
+# dram__bytes_write.sum = 640 MB for 262,144 cells; profiles/k_rhs_face_fast_tgv64_p2.md); other sizes are
+# scaled by the cell count
+RHS_TRAFFIC_PER_CELL = 640e6 / 64 ** 3
+RHS_FP64_PIPE_PCT = 38.5  # sm__inst_executed_pipe_fp64 of the same capture
 # algorithmic flops per cell (F_alg), counted by the op-counting build of the oracle on this workload
 # (python -m oracle.falg: +, -, *, / and sqrt one each; profiles/falg_tgv_p2.md)
 F_RHS = {2: 50310.0, 1: 30546.0}
@@ -868,12 +868,13 @@ def run_ours(args, rank, world, local_rank):
             "config": dict(workload_config(n, p), parallelism=f"replicas{world}" if world > 1 else "single GPU"),
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": 3 * K,
-            "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
+            # "bound" names the axis of achieved and peak, "limited_by" what the kernel waits for (the FP64 figures are under "fp64")
+            "roofline": {"bound": "hbm", "limited_by": "fp64 latency" if dom_name == "evaluate_rhs" else "hbm", "kernel": dom_name, "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "peak_source": f"{src} (MEASURED_PEAKS.json hbm_gbs)" if src == "measured" else "fallback 6650 GB/s",
                          "traffic": RHS_TRAFFIC_PER_CELL * nc if dom_name == "evaluate_rhs" else None,
-                         "traffic_source": "constant copied from the ncu capture of k_rhs_face_fast at 48^3 (profiles/), scaled by cells",
+                         "traffic_source": "constant copied from the ncu capture of k_rhs_face_fast at 64^3 (profiles/), scaled by cells",
                          "fp64_pipe_pct": RHS_FP64_PIPE_PCT if dom_name == "evaluate_rhs" else None,
-                         "fp64_pipe_pct_source": "constant copied from the same 48^3 ncu capture",
+                         "fp64_pipe_pct_source": "constant copied from the same 64^3 ncu capture",
                          "algorithmic_bytes_per_cell": dom_b,
                          "fp64": fp64},
             "kernels_ms": {"vr_jacobi_sweep": t_vr, "evaluate_rhs": t_rhs,
