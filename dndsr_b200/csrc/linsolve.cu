@@ -728,6 +728,8 @@ struct Solve
 // 677 and 703; 262,144 hexahedra 20 262 and 266, 60 714 and 711.  With the host waiting for each, as the drivers do, the
 // triangles take 24.8 and 30.4 at 4 launches, 49.7 and 50.7 at 16, 58.2 and 54.7 at 20.  The line lies where meshes of some
 // ten thousand cells cross; smaller ones lose up to 8 us between 8 and 24 launches, larger ones would gain beyond it.
+// Only where the kernels are chained: the sweeps of the block Jacobian are not, and went from 237 to 278 us (three pairs
+// on 16,200 tets in FP64) and from 97 to 109 (3,600 quadrilaterals in FP32) when they were launched one by one.
 constexpr int kDirectLaunches = 24;
 
 template <typename T, int NV, int NF>
@@ -741,7 +743,8 @@ int run(const MeshD &m, const GeomD &g, const BoundaryD &bnd, EvalD &ev, LinWs &
         return ST_BADARG;
     if (w.jacMode == 2 && (!ev.lambdaFace0 || (m.nBndFace > 0 && !bnd.type)))
         return ST_BADARG;
-    const bool direct = ls.gmresCode == 0 && (int64_t)(1 + ls.sgsIter) * 2 * m.nColor * (ls.jacobiCode == 2 ? 2 : 1) <= kDirectLaunches;
+    const bool chained = !w.jacMode || ls.jacobiCode == 2;
+    const bool direct = ls.gmresCode == 0 && chained && (int64_t)(1 + ls.sgsIter) * 2 * m.nColor * (ls.jacobiCode == 2 ? 2 : 1) <= kDirectLaunches;
     cudaStream_t cs = direct ? st : w.cs;
     if (!direct)
     {
