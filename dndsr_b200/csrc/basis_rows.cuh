@@ -4,6 +4,13 @@
 
 namespace dndsb
 {
+// threads to a row (a boundary cell with its faces' points) of the boundary kernels of the reconstruction and its transpose:
+// one per point, and with one or two points per face more, as the row's sums and its product with A^-1 are shared out over
+// them.  One point per face, degree 2: the sweep of 14,112 tets takes 28 us with eight threads to a cell, 59 with one per
+// point and 41 with one thread per cell and no shared memory; that of 5,760 hexahedra 27, 66 and 34; their transposes 42, 94
+// and 52, and 33, 84 and 40.
+inline int bnd_row_threads(int nGf) { return nGf < 3 ? 8 : nGf; }
+
 // phi_j (moments removed) and, with GRAD, its gradient of the R reconstruction rows of cell c at point p, generated
 // from the compile-time exponent table: a table filled by runtime loops lives in local memory
 template <int DIM, int P, bool GRAD>

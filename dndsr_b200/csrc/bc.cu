@@ -21,11 +21,11 @@ namespace
 // 74 -> 24 us (VR term) and 102 -> 12 us (RHS) for the 5,180 faces of a 36k-tet bump at degree 2 (7 points), 31 -> 21
 // and 33 -> 22 us for the 19,040 faces of a 250k-tet one at degree 1 (3 points).
 inline int bc_rows(int nGf) { return nGf < 64 ? 64 / nGf : 1; }
-// the same where a row takes `bytes` of dynamic shared memory: as many as the 48 KB that a launch has without asking hold
-// (at degree 3 with one point per face 51 of the 64 rows)
-inline int bc_rows(int nGf, size_t bytes)
+// the same for rows of `threads` threads that take `bytes` of dynamic shared memory: no more than the 48 KB that a launch
+// has without asking hold
+inline int bc_rows(int threads, size_t bytes)
 {
-    const int fit = (int)(48 * 1024 / bytes), rows = bc_rows(nGf);
+    const int fit = (int)(48 * 1024 / bytes), rows = bc_rows(threads);
     return rows < fit ? rows : fit;
 }
 
@@ -33,20 +33,21 @@ inline int bc_rows(int nGf, size_t bytes)
 // EulerSolver.hxx:163-175, applied as in :568-586:
 //   BCC = sum_{bc faces} sum_q w0^2 phi(x_q) (uBV(compress(u + phi . uRec)) - u) |J| w_q
 //   uRecNew += relax A^-1 BCC     (recordInc: -= A^-1 BCC, nothing when uRecIsZero)
-// Thread (cl, q) of a block: point q of the boundary faces of the block's cell cl, one face slot at a time; the
-// cell's threads then share out the R NV sums over the points (in point order) and the product with A^-1.
+// Thread (cl, q) of a block, tpr threads to a cell (bnd_row_threads): point q of the boundary faces of the block's cell cl,
+// one face slot at a time; the cell's threads then share out the R NV sums over the points (in point order) and the product
+// with A^-1.
 template <int DIM, int P, int NV, typename TC>
 DNDSB_GLOBAL void k_vr_bc(MeshD m, GeomD g, VRD vr, const TC *__restrict__ AAInvB, const real *__restrict__ uRec, real *uRecNew,
-                          const real *__restrict__ u, real relax, int recordInc)
+                          const real *__restrict__ u, real relax, int recordInc, int tpr)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, RV = R * NV;
     extern __shared__ real smBc[];
-    const int nG = g.nGf, cl = threadIdx.x / nG, q = threadIdx.x - cl * nG, rows = blockDim.x / nG;
+    const int nG = g.nGf, cl = threadIdx.x / tpr, q = threadIdx.x - cl * tpr, rows = blockDim.x / tpr;
     const int64_t ii = (int64_t)blockIdx.x * rows + cl;
     const int64_t c = ii < m.nBndCell ? m.bndCell[ii] : -1;
     real *sP = smBc + cl * (nG * (R + NV) + RV); // [nG][R + NV]: phi, (uBV - u) |J| w w0^2
     real *sB = sP + nG * (R + NV);               // [R][NV]: BCC
-    for (int e = q; e < RV; e += nG)
+    for (int e = q; e < RV; e += tpr)
         sB[e] = 0;
     for (int k = 0; k < m.nf; k++)
     {
@@ -59,7 +60,7 @@ DNDSB_GLOBAL void k_vr_bc(MeshD m, GeomD g, VRD vr, const TC *__restrict__ AAInv
         }
         if (!__syncthreads_or(w0 != 0)) // also keeps the last slot's sums apart from this slot's points
             continue;
-        if (w0 != 0)
+        if (w0 != 0 && q < nG)
         {
             const real *uc = u + c * NV, *rc = uRec + c * RV;
             const real *n = &g.faceNorm[(f * nG + q) * 3];
@@ -89,7 +90,7 @@ DNDSB_GLOBAL void k_vr_bc(MeshD m, GeomD g, VRD vr, const TC *__restrict__ AAInv
         }
         __syncthreads();
         if (w0 != 0)
-            for (int e = q; e < RV; e += nG)
+            for (int e = q; e < RV; e += tpr)
             {
                 const int i = e / NV, v = e - i * NV;
                 real a = sB[e];
@@ -103,7 +104,7 @@ DNDSB_GLOBAL void k_vr_bc(MeshD m, GeomD g, VRD vr, const TC *__restrict__ AAInv
         return;
     const TC *Ai = AAInvB + c * (m.nf + 1) * R * R;
     const real sgn = recordInc ? -1.0 : relax;
-    for (int e = q; e < RV; e += nG)
+    for (int e = q; e < RV; e += tpr)
     {
         const int i = e / NV, v = e - i * NV;
         real acc = 0;
@@ -339,13 +340,13 @@ void launch_vr_bc(const MeshD &m, const GeomD &g, const VRD &vr, const real *uRe
 {
     constexpr int R = ndof_of<DIM>(P) - 1;
     const size_t rowBytes = sizeof(real) * (g.nGf * (R + NV) + R * NV);
-    const int rows = bc_rows(g.nGf, rowBytes);
+    const int tpr = bnd_row_threads(g.nGf), rows = bc_rows(tpr, rowBytes);
     const unsigned nb = (unsigned)((m.nBndCell + rows - 1) / rows);
     const size_t sh = rows * rowBytes;
     if (useFP32)
-        k_vr_bc<DIM, P, NV, float><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, vr.AAInvB32, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
+        k_vr_bc<DIM, P, NV, float><<<nb, rows * tpr, sh, st>>>(m, g, vr, vr.AAInvB32, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc, tpr);
     else
-        k_vr_bc<DIM, P, NV, real><<<nb, rows * g.nGf, sh, st>>>(m, g, vr, vr.AAInvB, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc);
+        k_vr_bc<DIM, P, NV, real><<<nb, rows * tpr, sh, st>>>(m, g, vr, vr.AAInvB, uRec, uRecNew, u, vr.s.jacobiRelax, recordInc, tpr);
 }
 
 template <int DIM, int NV>

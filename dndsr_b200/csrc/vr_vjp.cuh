@@ -93,15 +93,16 @@ DNDSB_GLOBAL void __launch_bounds__(128) k_vr_vjp_rows(MeshD m, VRD vr, const re
 
 // adds the boundary term's share: t = w A_c^-T v_c is the cotangent of BCC = sum_q w0^2 |J| w phi_q (UB_q - u_c) with
 // UB_q = ghost(compress(u_c, u_c + phi_q . uRec_c)); the ghost is differentiated in dual numbers with respect to the
-// point state and the mean.  One thread per (boundary cell, point), the block's sums in point order (as k_vr_bc).
+// point state and the mean.  One thread per (boundary cell, point), more where the points are few (bnd_row_threads), the
+// block's sums in point order (as k_vr_bc).
 template <int DIM, int P, int NV>
 DNDSB_GLOBAL void k_vr_vjp_bnd(MeshD m, GeomD g, VRD vr, const real *__restrict__ v, const real *__restrict__ uRec, const real *__restrict__ u,
-                               real *vRec, real *vU)
+                               real *vRec, real *vU, int tpr)
 {
     constexpr int NDOF = ndof_of<DIM>(P), R = NDOF - 1, RV = R * NV, ROW = R + 2 * NV;
     using DV = Dual<NV>;
     extern __shared__ real smVb[];
-    const int nG = g.nGf, cl = threadIdx.x / nG, q = threadIdx.x - cl * nG, rows = blockDim.x / nG;
+    const int nG = g.nGf, cl = threadIdx.x / tpr, q = threadIdx.x - cl * tpr, rows = blockDim.x / tpr;
     const int64_t ii = (int64_t)blockIdx.x * rows + cl;
     const int64_t c = ii < m.nBndCell ? m.bndCell[ii] : -1;
     real *sT = smVb + cl * (RV + RV + NV + nG * ROW); // [R][NV] the cotangent of BCC
@@ -111,7 +112,7 @@ DNDSB_GLOBAL void k_vr_vjp_bnd(MeshD m, GeomD g, VRD vr, const real *__restrict_
     if (c >= 0)
     {
         const real *Ai = vr.AAInvB + c * (m.nf + 1) * R * R, *vc = v + c * RV;
-        for (int e = q; e < RV + NV; e += nG)
+        for (int e = q; e < RV + NV; e += tpr)
         {
             sA[e] = 0;
             if (e < RV)
@@ -135,7 +136,7 @@ DNDSB_GLOBAL void k_vr_vjp_bnd(MeshD m, GeomD g, VRD vr, const real *__restrict_
         }
         if (!__syncthreads_or(w0 != 0)) // also orders the sums of the last slot and the points of this one
             continue;
-        if (w0 != 0)
+        if (w0 != 0 && q < nG)
         {
             const real *uc = u + c * NV, *rc = uRec + c * RV, *n = &g.faceNorm[(f * nG + q) * 3];
             const int zone = m.faceZone[f];
@@ -175,7 +176,7 @@ DNDSB_GLOBAL void k_vr_vjp_bnd(MeshD m, GeomD g, VRD vr, const real *__restrict_
         }
         __syncthreads();
         if (w0 != 0)
-            for (int e = q; e < RV + NV; e += nG)
+            for (int e = q; e < RV + NV; e += tpr)
             {
                 const int j = e / NV, x = e - j * NV; // j = R: vU
                 real a = sA[e];
@@ -190,7 +191,7 @@ DNDSB_GLOBAL void k_vr_vjp_bnd(MeshD m, GeomD g, VRD vr, const real *__restrict_
     __syncthreads();
     if (c < 0)
         return;
-    for (int e = q; e < RV + NV; e += nG)
+    for (int e = q; e < RV + NV; e += tpr)
         if (e < RV)
             vRec[c * RV + e] += sA[e];
         else
@@ -207,9 +208,9 @@ void launch_vr_vjp(const MeshD &m, const GeomD &g, const VRD &vr, const real *v,
     {
         // about 32 threads, and no more rows than the 48 KB of shared memory that a launch has without asking hold
         const size_t rowBytes = sizeof(real) * (2 * R * NV + NV + g.nGf * (R + 2 * NV));
-        const int want = g.nGf < 32 ? 32 / g.nGf : 1, fit = (int)(48 * 1024 / rowBytes), rows = want < fit ? want : fit;
+        const int tpr = bnd_row_threads(g.nGf), want = tpr < 32 ? 32 / tpr : 1, fit = (int)(48 * 1024 / rowBytes), rows = want < fit ? want : fit;
         const size_t sh = rows * rowBytes;
-        k_vr_vjp_bnd<DIM, P, NV><<<(unsigned)((m.nBndCell + rows - 1) / rows), rows * g.nGf, sh, st>>>(m, g, vr, v, uRec, u, vRec, vU);
+        k_vr_vjp_bnd<DIM, P, NV><<<(unsigned)((m.nBndCell + rows - 1) / rows), rows * tpr, sh, st>>>(m, g, vr, v, uRec, u, vRec, vU, tpr);
     }
 }
 } // namespace
