@@ -59,6 +59,15 @@ __global__ void __launch_bounds__(32 * (R / kStagedRows))
     auto stage = [&](int s, int mine)
     {
         real *dst = sb + (s % 3) * St::LEN;
+        if (!useRec)
+        {
+            // from a zero reconstruction the sweep reads the means alone: each lane's row by the threads of its cell
+            if (mine >= 0)
+                for (int v = g; v < NV; v += G)
+                    copy8_async(dst + lane * St::SW + St::W + v, u + (int64_t)mine * NV + v);
+            copies_commit();
+            return;
+        }
 #pragma unroll 4
         for (int m = g; m < 32; m += G)
         {
