@@ -502,6 +502,20 @@ int launch_vjp_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &
     constexpr int W = (Lt::R + 1) * NV, CH = VjpRows<DIM, P, NV, NG, true>::CH;
     constexpr size_t smem = sizeof(real) * (64 * Lt::CS + 32 * NV + 15 * 32 + CH * NG * 32 + 32 * 2 * W) + sizeof(FaceData) * 32;
     static_assert(smem <= 227 * 1024, "shared memory of k_rhs_vjp_fast above the 227 KB a block may hold");
+    const unsigned nb = (unsigned)((m.nFace + 31) / 32);
+    if constexpr (DIM == 2 && NV == 5 && (P == 3 || (P == 2 && NG == 2)))
+    {
+        // In 2-D with few points per face a block is two or three warps, of which shared memory lets one (degree 3) or two
+        // blocks on an SM: the kernel is the faster one while all blocks are resident at once.  Without the viscous flux the
+        // caller's thread-per-face kernel takes the larger meshes.  VJP of EvaluateRHS, per point and per face, us: degree 3,
+        // 3 points, quadrilaterals with 4,608 faces 46.7 and 55.0, 6,272 62.2 and 55.2, 33,800 154 and 129, 156,800 607 and
+        // 413; 2 points, 4,608 50.4 and 52.0, 156,800 720 and 362; triangles 3,072 47.9 and 55.2, 4,800 65.4 and 55.6; degree
+        // 2, 2 points, 8,192 42.9 and 51.0, 10,368 57.3 and 51.5, 156,800 300 and 237.  With 3 points at degree 2 they differ
+        // by a tenth at most at every size.
+        constexpr unsigned resident = 228 * 1024 / (smem + 1024);
+        if (!visc && nb > 148 * resident)
+            return ST_UNSUPPORTED;
+    }
     auto kern = k_rhs_vjp_fast<DIM, P, NV, NG, true>;
     if constexpr (P > 1 && NV == 5)
         if (!visc)
@@ -515,7 +529,6 @@ int launch_vjp_fast(const MeshD &m, const GeomD &g, const VRD &vr, const EvalD &
             return ST_CUDA;
         attrSet[visc] |= 1ULL << dev;
     }
-    const unsigned nb = (unsigned)((m.nFace + 31) / 32);
     kern<<<nb, 32 * NG, smem, st>>>(m, g, ev.facePt, ev.cellPar, vr.baseMoment, ev.s, hllep ? 1 : 0, w, u, uRec, ev.deltaLambdaCell, faceAdj,
                                     ev.errWord);
     return last_error() == cudaSuccess ? ST_OK : ST_CUDA;

@@ -240,8 +240,8 @@ int rhs_vjp_roe_interior(const MeshD &m, const GeomD &g, const VRD &vr, const Ev
         return ST_UNSUPPORTED;
     *viscDone = false;
     // plain Roe and HLLE+: the kernels of adjoint_fast.cuh (508,720 faces of degree 2 without the viscous flux: 1.39 ms;
-    // the thread-per-face kernel below with the boundary faces 2.23 ms; it takes the other schemes and the quadratures that
-    // those do not cover)
+    // the thread-per-face kernel below with the boundary faces 2.23 ms; it takes the other schemes, and the quadratures and
+    // sizes that those leave to it)
     if (es == 0 || es == kHLLEP)
     {
         int rc = rhs_vjp_interior_fast(m, g, vr, ev, es == kHLLEP, w, u, uRec, faceAdj, st);

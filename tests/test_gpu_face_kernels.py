@@ -76,3 +76,27 @@ def test_transpose(name, mk, p, order, rs):
     # two sums of the same products in another order: each entry carries some 1e3 rounded operations
     size = float((w * t).abs().sum() + (a * du).abs().sum() + (b * drec).abs().sum())
     assert abs(float((w * t).sum() - (a * du).sum() - (b * drec).sum())) < 1e3 * np.finfo(float).eps * size
+
+
+@pytest.mark.parametrize("rs", ["Roe", "HLLEP"])
+@pytest.mark.parametrize("p,order,n", [(3, 5, 47), (3, 5, 49), (3, 3, 47), (3, 3, 49), (2, 3, 68), (2, 3, 69)])
+def test_transpose_on_both_sides_of_the_line_in_2d(p, order, n, rs):
+    """The point-parallel kernel up to one wave of blocks (4,736 faces at degree 3, 9,472 at degree 2 with two points), the
+    thread-per-face kernel beyond: <w, J v> = <J^T w, v> to the rounding of the sums."""
+    from dndsr_b200.solver import EulerEvaluator, VariationalReconstruction
+    m = M.periodic_quad_2d(n, jitter=0.1)
+    assert ((m.n_face + 31) // 32 > 148 * (4 - p)) == (n in (49, 69))
+    vr = VariationalReconstruction(m, dict(VR_HQM_PY, maxOrder=p, intOrder=order)).construct()
+    ev = EulerEvaluator(vr, dict(nVars=5, riemannSolverType=rs, muGas=0.0, ignoreVis=True))
+    u = vr.BuildUDof(5)
+    ev.InitializeUDOF(u, 2)
+    g = torch.Generator("cuda").manual_seed(2)
+    rand = lambda shape: torch.randn(shape, generator=g, dtype=torch.float64, device="cuda")  # noqa: E731
+    rec = 0.01 * rand((m.n_cell, vr.R, 5)) * u.abs().mean(0)
+    rec[:, :, 3] = 0
+    ev.EvaluateDt(torch.zeros(m.n_cell, dtype=torch.float64, device="cuda"), u, 1.0)
+    w, du, dr = rand(u.shape), rand(u.shape), rand(rec.shape)
+    a, b = ev.EvaluateRHSVJP(w, u, rec)
+    lhs = (w * ev.EvaluateRHSJVP(du, dr, u, rec)).flatten()
+    rhs = torch.cat([(a * du).flatten(), (b * dr).flatten()])
+    assert abs(float(lhs.sum() - rhs.sum())) < 1e-12 * float(lhs.abs().sum() + rhs.abs().sum())
